@@ -502,8 +502,12 @@ def lite_topk(q_idx8: torch.Tensor, k_idx8: torch.Tensor, weights: torch.Tensor,
               logits_workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Indexer + selection in one call: ``topk_idx`` [T, k] int32 (-1 padded) for the T query
     tokens at positions ``q_pos0 ...`` -- the input of ``union_qm`` / ``sparse_prefill``."""
-    logits = index_logits_fp8(q_idx8, k_idx8, weights, k_scale, q_pos0, out=logits_workspace)
     S = k_idx8.shape[0]
+    if logits_workspace is None:
+        # rows start on 16-byte boundaries whatever S is: the streaming selection kernels need that
+        logits_workspace = torch.empty((q_idx8.shape[0], (S + 3) // 4 * 4), dtype=torch.float32,
+                                       device=q_idx8.device)
+    logits = index_logits_fp8(q_idx8, k_idx8, weights, k_scale, q_pos0, out=logits_workspace)
     # a workspace wider than S: select over the first S columns of every row
     view = logits if logits.shape[1] == S else logits.as_strided((logits.shape[0], S), (logits.stride(0), 1))
     return topk_select(view, k, q_pos0=q_pos0)

@@ -61,6 +61,7 @@ struct LogitParams {
   const float* k_scale;     // [S] or null (1.0)
   float* logits;            // [T, ld]
   int T, Hi, S, q_pos0;
+  int tiles_per_split;      // key tiles of one CTA: blockIdx.y owns tiles [y * this, (y + 1) * this)
   long long ld;
   int epoch;
   unsigned long long wait_limit_ns;
@@ -95,9 +96,12 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   constexpr int tpa = kCols / HI;               // tokens per accumulator
   const int tok0 = blockIdx.x * 2 * tpa;        // first token of this CTA
   const int tok_end = min(p.T, tok0 + 2 * tpa);
-  // key tiles up to the causal bound of the CTA's last token
+  // key tiles up to the causal bound of the CTA's last token, and this CTA's share [j0, j0 + n)
   const int pos_max = p.q_pos0 + tok_end - 1;
-  const int n_tiles = min((p.S + kKeyTile - 1) / kKeyTile, pos_max / kKeyTile + 1);
+  const int all_tiles = (p.S + kKeyTile - 1) / kKeyTile;
+  const int causal_tiles = min(all_tiles, pos_max / kKeyTile + 1);
+  const int j0 = blockIdx.y * p.tiles_per_split, j_end = min(j0 + p.tiles_per_split, all_tiles);
+  const int n_tiles = max(min(j_end, causal_tiles) - j0, 0);
 
   if (threadIdx.x == 0) {
     mbar_init(&bar.q_full, 1);
@@ -125,7 +129,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    if (lane == 0 && n_tiles > 0) {
       const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
       mbar_arrive_expect_tx(&bar.q_full, 2 * kQTile);
       tma_load_2d_hint(sbase + kOffQ, &map_q, 0, tok0 * HI, &bar.q_full, pol_stream);
@@ -134,14 +138,14 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int s = j % kStages;
         if (j >= kStages && !mbar_wait(&bar.k_free[s], ((j / kStages) & 1) ^ 1, wt, kSiteKFree, j)) break;
         mbar_arrive_expect_tx(&bar.k_full[s], kKTile);
-        tma_load_2d_hint(sbase + kOffK + s * kKTile, &map_k, 0, j * kKeyTile, &bar.k_full[s], pol_keep);
+        tma_load_2d_hint(sbase + kOffK + s * kKTile, &map_k, 0, (j0 + j) * kKeyTile, &bar.k_full[s], pol_keep);
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue (one thread)
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc(0, 0, false, false, kKeyTile, kCols);
-      bool ok = mbar_wait(&bar.q_full, 0, wt, kSiteQFull, 0);
+      bool ok = n_tiles > 0 && mbar_wait(&bar.q_full, 0, wt, kSiteQFull, 0);
       for (int j = 0; j < n_tiles && ok; ++j) {
         const int s = j % kStages;
         ok = mbar_wait(&bar.k_full[s], (j / kStages) & 1, wt, kSiteKFull, j);
@@ -178,7 +182,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // Key tiles beyond the causal bound of the CTA's last token are not computed: their entries
     // are -inf for every token of the CTA (this warp's tokens and key rows).  Written first,
     // while the tensor core fills the first accumulators.
-    for (int j = n_tiles; j * kKeyTile < p.S; ++j) {
+    for (int j = j0 + n_tiles; j < j_end; ++j) {
       const int s_key = j * kKeyTile + krow;
       if (s_key < p.S) {
 #pragma unroll
@@ -190,7 +194,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     for (int j = 0; j < n_tiles; ++j) {
       // this key's scale is fetched before the wait, so its latency hides behind the MMAs
-      const int s_key = j * kKeyTile + krow;
+      const int s_key = (j0 + j) * kKeyTile + krow;
       const float ks = (p.k_scale && s_key < p.S) ? __ldg(p.k_scale + s_key) : 1.f;
       if (!mbar_wait(&bar.acc_full[a], j & 1, wt, kSiteAccFull, j)) break;
       __syncwarp();
@@ -241,7 +245,36 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncwarp();
     tmem_dealloc_cta(tmem, 512);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_status[3], 1);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(&g_status[3], 1);
+}
+
+// How many key ranges the grid splits every token group's keys into.  A CTA occupies an SM by
+// itself (all of TMEM) and works about one unit of time per key tile after a start-up worth about
+// four (TMEM and barrier set-up, the 64 KB of Q, the first K tile), so the launch takes
+// waves(ctas_x * splits) * (4 + tiles per split): few tokens need many splits to fill the SMs (36
+// tokens of 32 heads are 3 CTAs: 867 -> 22 us against 100K keys), many tokens a few so that the
+// last wave is full.
+static int sm_count() {
+  static thread_local int cached_dev = -1, cached = 148;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev != cached_dev) {
+    cudaDeviceGetAttribute(&cached, cudaDevAttrMultiProcessorCount, dev);
+    cached_dev = dev;
+  }
+  return cached;
+}
+static int pick_splits(int ctas_x, int tiles, int sms) {
+  int best = 1;
+  long long best_cost = -1;
+  const int most = tiles < 64 ? tiles : 64;
+  for (int n = 1; n <= most; ++n) {
+    const int per = (tiles + n - 1) / n;
+    const long long waves = ((long long)ctas_x * ((tiles + per - 1) / per) + sms - 1) / sms;
+    const long long cost = waves * (4 + per);
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = n; }
+  }
+  return best;
 }
 
 // ------------------------------------------------------------------ top-k selection
@@ -775,9 +808,69 @@ topk_select_stream_kernel(const SelParams p) {
 constexpr int kChunk = 16384;            // floats per chunk
 enum { kSiteSelChunk = 12 };
 
+// Block-wide: append the elements >= t_lo of one chunk (positions start .. start + kChunk - 1 of
+// the row, cut at n) to the survivor list, m_run entries long so far.  `release` runs on thread 0
+// once every thread has read the chunk out of its buffer.  fast turns false when the list is full
+// or a wait ran out.
+template <int NT, class Release>
+__device__ __forceinline__ void filter_chunk(SelShared& sh, const float* chunk, int start, int n, float t_lo,
+                                             bool landed, float* sval, uint32_t* spos, uint32_t& m_run,
+                                             bool& fast, Release release) {
+  constexpr int NQ = kChunk / 4 / NT;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const float4* buf = reinterpret_cast<const float4*>(chunk);
+  // this thread's NQ quads of the chunk: positions start + 4 * (q * NT + tid) .. + 3
+  float4 v[NQ];
+  uint32_t cnt = 0;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int pos = start + 4 * (q * NT + tid);
+    v[q] = pos < n ? buf[q * NT + tid] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    if (pos + 3 >= n) {      // the row's last quad may be cut: entries beyond n never survive
+      if (pos + 1 >= n) v[q].y = NAN;
+      if (pos + 2 >= n) v[q].z = NAN;
+      if (pos + 3 >= n) v[q].w = NAN;
+      if (pos >= n) v[q].x = NAN;
+    }
+    cnt += (v[q].x >= t_lo) + (v[q].y >= t_lo) + (v[q].z >= t_lo) + (v[q].w >= t_lo);
+  }
+  fence_proxy_async_smem();    // these reads are ordered before the next bulk write of the buffer
+  // block-wide exclusive scan of the counts (its barrier also frees the buffer)
+  uint32_t inc = cnt;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t a = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += a;
+  }
+  if (lane == 31) sh.wa[wid] = inc;
+  const bool all_landed = __syncthreads_and(landed);
+  if (tid == 0) release();
+  uint32_t wtot = lane < NT / 32 ? sh.wa[lane] : 0u, ws = wtot;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t a = __shfl_up_sync(0xffffffffu, ws, off);
+    if (lane >= off) ws += a;
+  }
+  uint32_t slot = m_run + __shfl_sync(0xffffffffu, ws - wtot, wid) + inc - cnt;
+  const uint32_t total = __shfl_sync(0xffffffffu, ws, NT / 32 - 1);
+  if (!all_landed || m_run + total > (uint32_t)kSurvCap) fast = false;   // block-uniform
+  if (fast) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const uint32_t pos = (uint32_t)(start + 4 * (q * NT + tid));
+      if (v[q].x >= t_lo) { sval[slot] = v[q].x; spos[slot] = pos; ++slot; }
+      if (v[q].y >= t_lo) { sval[slot] = v[q].y; spos[slot] = pos + 1; ++slot; }
+      if (v[q].z >= t_lo) { sval[slot] = v[q].z; spos[slot] = pos + 2; ++slot; }
+      if (v[q].w >= t_lo) { sval[slot] = v[q].w; spos[slot] = pos + 3; ++slot; }
+    }
+  }
+  m_run += total;
+  __syncthreads();             // sh.wa is reused by the next chunk's scan
+}
+
 __global__ void __launch_bounds__(kStreamThreads, 1)
 topk_select_chunked_kernel(const SelParams p) {
-  constexpr int NT = kStreamThreads, NQ = kChunk / 4 / NT;
+  constexpr int NT = kStreamThreads;
   extern __shared__ __align__(16) float cbuf[];       // 2 chunks | survivor values | survivor positions
   float* sval = cbuf + 2 * kChunk;
   uint32_t* spos = reinterpret_cast<uint32_t*>(sval + kSurvCap);
@@ -786,7 +879,7 @@ topk_select_chunked_kernel(const SelParams p) {
   __shared__ float red_a[NT / 32], red_b[NT / 32];
   __shared__ uint32_t eq_total;
   const Waiter wt{g_status, p.epoch, p.wait_limit_ns};
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x;
   auto len_of = [&](int t) -> int {
     return p.lengths ? min(max(p.lengths[t], 0), p.S) : min(p.S, max(p.q_pos0 + t + 1, 0));
   };
@@ -839,60 +932,96 @@ topk_select_chunked_kernel(const SelParams p) {
     const int nch = chunks_of(n);
     for (int c = 0; c < nch; ++c, ++gc) {
       const bool landed = mbar_wait(&bar[gc & 1], (gc >> 1) & 1, wt, kSiteSelChunk, c);
-      const float4* buf = reinterpret_cast<const float4*>(cbuf + (gc & 1) * kChunk);
-      const int start = c * kChunk;
-      // this thread's 8 quads of the chunk: positions start + 4 * (q * NT + tid) .. + 3
-      float4 v[NQ];
-      uint32_t cnt = 0;
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        const int pos = start + 4 * (q * NT + tid);
-        v[q] = pos < n ? buf[q * NT + tid] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-        if (pos + 3 >= n) {      // the row's last quad may be cut: entries beyond n never survive
-          if (pos + 1 >= n) v[q].y = NAN;
-          if (pos + 2 >= n) v[q].z = NAN;
-          if (pos + 3 >= n) v[q].w = NAN;
-          if (pos >= n) v[q].x = NAN;
-        }
-        cnt += (v[q].x >= t_lo) + (v[q].y >= t_lo) + (v[q].z >= t_lo) + (v[q].w >= t_lo);
-      }
-      fence_proxy_async_smem();    // these reads are ordered before the next bulk write of the buffer
-      // block-wide exclusive scan of the counts (its barrier also frees the buffer)
-      uint32_t inc = cnt;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t a = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += a;
-      }
-      if (lane == 31) sh.wa[wid] = inc;
-      const bool all_landed = __syncthreads_and(landed);
-      if (tid == 0) fetch_next();
-      uint32_t wtot = lane < NT / 32 ? sh.wa[lane] : 0u, ws = wtot;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t a = __shfl_up_sync(0xffffffffu, ws, off);
-        if (lane >= off) ws += a;
-      }
-      uint32_t slot = m_run + __shfl_sync(0xffffffffu, ws - wtot, wid) + inc - cnt;
-      const uint32_t total = __shfl_sync(0xffffffffu, ws, NT / 32 - 1);
-      if (!all_landed || m_run + total > (uint32_t)kSurvCap) fast = false;   // block-uniform
-      if (fast) {
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          const uint32_t pos = (uint32_t)(start + 4 * (q * NT + tid));
-          if (v[q].x >= t_lo) { sval[slot] = v[q].x; spos[slot] = pos; ++slot; }
-          if (v[q].y >= t_lo) { sval[slot] = v[q].y; spos[slot] = pos + 1; ++slot; }
-          if (v[q].z >= t_lo) { sval[slot] = v[q].z; spos[slot] = pos + 2; ++slot; }
-          if (v[q].w >= t_lo) { sval[slot] = v[q].w; spos[slot] = pos + 3; ++slot; }
-        }
-      }
-      m_run += total;
-      __syncthreads();             // sh.wa is reused by the next chunk's scan
+      filter_chunk<NT>(sh, cbuf + (gc & 1) * kChunk, c * kChunk, n, t_lo, landed, sval, spos, m_run, fast,
+                       [&]() { fetch_next(); });
     }
     if (m_run < (uint32_t)p.k) fast = false;       // the threshold was too high
     finish_row<NT>(sh, red_a, red_b, &eq_total, sval, spos, m_run, fast, row, n, p.k, out);
     __syncthreads();               // sh.* is reused by the next row
   }
+}
+
+// Few long rows: one CLUSTER per row, so that the SMs a row-per-CTA launch would leave idle share
+// the row.  CTA r filters the r-th of the row's equal segments (every CTA draws the same 2048
+// samples of the whole row, hence the same threshold); the survivors are then appended to the
+// leader's list through distributed shared memory in segment order and the leader finishes the
+// row like the kernels above.  Latency-bound: one CTA needs 27 us for a 100K-entry row.
+__global__ void __launch_bounds__(kStreamThreads, 1)
+topk_select_cluster_kernel(const SelParams p, int nc) {
+  constexpr int NT = kStreamThreads;
+  extern __shared__ __align__(16) float cbuf[];       // 2 chunks | survivor values | survivor positions
+  float* sval = cbuf + 2 * kChunk;
+  uint32_t* spos = reinterpret_cast<uint32_t*>(sval + kSurvCap);
+  __shared__ SelShared sh;
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ float red_a[NT / 32], red_b[NT / 32];
+  __shared__ uint32_t eq_total, seg_cnt[8];           // seg_cnt: leader CTA, survivors per segment
+  const Waiter wt{g_status, p.epoch, p.wait_limit_ns};
+  const int tid = threadIdx.x, rank = (int)cluster_ctarank(), t = blockIdx.x / nc;
+  const int n = p.lengths ? min(max(p.lengths[t], 0), p.S) : min(p.S, max(p.q_pos0 + t + 1, 0));
+  int32_t* out = p.out + (long long)t * p.k;
+  const float* row = p.logits + (long long)t * p.ld;
+  if (n <= p.k) {              // everything valid is selected (uniform over the cluster)
+    if (rank == 0)
+      for (int i = tid; i < p.k; i += NT) out[i] = i < n ? i : -1;
+    return;
+  }
+  const int seg = (((n + nc - 1) / nc) + 3) & ~3;
+  const int s0 = min(rank * seg, n), s1 = min(s0 + seg, n);
+  const int nch = (s1 - s0 + kChunk - 1) / kChunk;
+  auto fetch = [&](int c) {    // thread 0 only; whole 16-byte quads
+    const int start = s0 + c * kChunk;
+    const uint32_t bytes = (uint32_t)(min(kChunk, ((s1 + 3) & ~3) - start) * 4);
+    mbar_arrive_expect_tx(&bar[c & 1], bytes);
+    bulk_load_1d(smem_u32(cbuf + (c & 1) * kChunk), row + start, bytes, &bar[c & 1]);
+  };
+  if (tid == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    fence_mbar_init();
+    if (nch > 0) fetch(0);
+    if (nch > 1) fetch(1);
+    sh.n_cand = 0;
+  }
+  float smp[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) smp[i] = __ldg(row + (int)(((long long)(4 * tid + i) * n) >> 11));
+  __syncwarp();
+  cluster_sync_all();          // barriers initialised; every CTA of the cluster runs (remote stores below)
+  float t_lo = -INFINITY;
+  if (n > kSurvCap / 2) t_lo = sampled_threshold<NT>(sh, red_a, red_b, smp, n, p.k);
+
+  bool fast = true;
+  uint32_t m_run = 0;
+  for (int c = 0; c < nch; ++c) {
+    const bool landed = mbar_wait(&bar[c & 1], (c >> 1) & 1, wt, kSiteSelChunk, c);
+    filter_chunk<NT>(sh, cbuf + (c & 1) * kChunk, s0 + c * kChunk, s1, t_lo, landed, sval, spos, m_run, fast,
+                     [&]() { if (c + 2 < nch) fetch(c + 2); });
+  }
+  // a segment that did not fit says so with a count no list can hold
+  if (tid == 0)
+    st_cluster_u32(mapa(smem_u32(&seg_cnt[rank]), 0), fast ? m_run : (uint32_t)kSurvCap + 1u);
+  __syncwarp();
+  cluster_sync_all();
+  uint32_t before = 0, m_s = 0;
+  for (int i = 0; i < nc; ++i) {
+    const uint32_t c = ld_cluster_u32(mapa(smem_u32(&seg_cnt[i]), 0));
+    if (i < rank) before += c;
+    m_s += c;
+  }
+  if (m_s > (uint32_t)kSurvCap) fast = false;            // uniform over the cluster from here on
+  else if (rank > 0) {
+    const uint32_t dv = mapa(smem_u32(sval), 0), dp = mapa(smem_u32(spos), 0);
+    for (uint32_t i = tid; i < m_run; i += NT) {
+      st_cluster_u32(dv + 4 * (before + i), __float_as_uint(sval[i]));
+      st_cluster_u32(dp + 4 * (before + i), spos[i]);
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (rank > 0) return;
+  if (m_s < (uint32_t)p.k) fast = false;                 // the threshold was too high
+  finish_row<NT>(sh, red_a, red_b, &eq_total, sval, spos, m_s, fast, row, n, p.k, out);
 }
 
 }  // namespace idx
@@ -930,8 +1059,14 @@ extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, 
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
     return LITEDSA_ERR_CUDA;
   const int tok_per_cta = 2 * (kCols / Hi);
-  const int grid = (T + tok_per_cta - 1) / tok_per_cta;
-  kern<<<grid, kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream)>>>(map_q, map_k, p);
+  const int ctas_x = (T + tok_per_cta - 1) / tok_per_cta;
+  // the tiles that do work: up to the last token's causal bound
+  const int all_tiles = (S + kKeyTile - 1) / kKeyTile;
+  const int live_tiles = (int)min((long long)all_tiles, ((long long)q_pos0 + T - 1) / kKeyTile + 1);
+  const int splits = pick_splits(ctas_x, live_tiles, sm_count());
+  p.tiles_per_split = (live_tiles + splits - 1) / splits;
+  const int grid_y = (all_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+  kern<<<dim3(ctas_x, grid_y), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream)>>>(map_q, map_k, p);
   return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
 }
 
@@ -963,10 +1098,27 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
     return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
   };
   const bool aligned = (logits_row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  const int sms = sm_count();
+  const size_t chunk_dyn = (size_t)2 * kChunk * 4 + (size_t)kSurvCap * 8;
+  // Few rows: as many CTAs per row as the chip has for each, if every one of them gets at least
+  // 4096 entries (below that the extra cluster synchronisations cost what the shorter filter saves)
+  int nc = 8;
+  while (nc > 1 && ((long long)T * nc > sms || S < 4096 * nc)) nc >>= 1;
+  if (aligned && nc > 1) {
+    if (cudaFuncSetAttribute(topk_select_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)chunk_dyn) != cudaSuccess)
+      return LITEDSA_ERR_CUDA;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(T * nc)); cfg.blockDim = dim3(kStreamThreads);
+    cfg.dynamicSmemBytes = chunk_dyn; cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)nc; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel, (const SelParams)p, nc) == cudaSuccess
+               ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  }
   if (aligned && S <= kStreamThreads * 64) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = T < sms ? T : sms;
     auto kern = S <= kStreamThreads * 32 ? topk_select_stream_kernel<32> : topk_select_stream_kernel<64>;
     const size_t dyn = smem + (size_t)kSurvCap * 6;      // + survivor values (fp32) and positions (u16)
@@ -976,14 +1128,10 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
     return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
   }
   if (aligned) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t dyn = (size_t)2 * kChunk * 4 + (size_t)kSurvCap * 8;
     if (cudaFuncSetAttribute(topk_select_chunked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)dyn) != cudaSuccess)
+                             (int)chunk_dyn) != cudaSuccess)
       return LITEDSA_ERR_CUDA;
-    topk_select_chunked_kernel<<<T < sms ? T : sms, kStreamThreads, dyn, st>>>(p);
+    topk_select_chunked_kernel<<<T < sms ? T : sms, kStreamThreads, chunk_dyn, st>>>(p);
     return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
   }
   if (S <= kMaxSmemRow) return launch(topk_select_kernel<true>, kGenericThreads, smem);

@@ -247,3 +247,37 @@ def test_full_width_rows_sampled():
         ref_row = io.index_logits(q8[r:r + 1], k8, w[r:r + 1], ks, pos0 + r)[0]
         d = (gl[i, :n] - ref_row[:n]).abs().max().item()
         assert d <= 2e-5 * ref_row[:n].abs().max().item()
+
+
+@pytest.mark.parametrize("T,S,Hi,pos0", [
+    (1, 20001, 32, 20000),      # one token: as many key ranges as the grid takes, ragged last tile
+    (36, 9000, 32, 8964),       # three token groups, the last one short
+    (5, 4097, 64, 300),         # most key tiles beyond every token's position: written by the later ranges
+    (3, 130, 128, 127),         # two key tiles
+])
+def test_index_logits_with_the_keys_split_over_ctas(T, S, Hi, pos0):
+    q8, k8, w, ks = _ops(T, S, Hi, seed=S)
+    out = torch.full((T, S), 7.0, dtype=torch.float32, device=DEV)
+    api.index_logits_fp8(q8.to(DEV), k8.to(DEV), w.to(DEV), ks.to(DEV), pos0, out=out)
+    torch.cuda.synchronize()
+    assert api.index_status(reset=True)[0] == 0
+    ref = io.index_logits(q8, k8, w, ks, pos0)
+    got = out.cpu().double()
+    assert torch.equal(torch.isinf(got), torch.isinf(ref))
+    fin = torch.isfinite(ref)
+    # fp32 sums of Hi products: the bound of the other comparisons with the oracle in this file
+    assert float((got[fin] - ref[fin]).abs().max()) <= 2e-5 * float(ref[fin].abs().max())
+
+
+@pytest.mark.parametrize("T,S,k", [(1, 32768, 2048), (7, 40004, 1000), (18, 262148, 512), (2, 8192, 4096)])
+def test_topk_select_few_rows_shared_by_clusters(T, S, k):
+    # eight, four or two CTAs per row; lengths around the segment and chunk boundaries
+    x = _random_logits(T, S, seed=S + k)
+    x[0] = torch.round(x[0] * 8) / 8                      # ties at the k-th value: the exact path
+    edges = [S, S - 1, k, k + 1, 8 * 16384 + 5, S // 8 * 7 + 1, 16384, S // 2 + 2, 0]
+    lens = torch.tensor([min(S, edges[t % len(edges)]) for t in range(T)], dtype=torch.int32)
+    ref = io.topk_exact(x, k, lengths=lens)
+    got = api.topk_select(x.to(DEV), k, lengths=lens.to(DEV))
+    torch.cuda.synchronize()
+    assert api.index_status(reset=True)[0] == 0
+    assert np.array_equal(_canon(got), ref)
