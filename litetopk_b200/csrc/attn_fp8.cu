@@ -11,26 +11,34 @@
 // Those numerics are reproduced exactly so the two implementations agree to rounding.
 //
 // How it is organised here (written from scratch, raw PTX, no CuTe):
-//   * persistent: one cluster of 2 CTAs per SM pair walks tiles cid, cid + #clusters, ...;
-//     each CTA owns 64 query rows.  Both GEMMs are single tcgen05 cta_group::2 instructions
-//     spanning the pair: QK^T splits the 128 keys of a block across the CTAs (N split), PV
-//     splits the 512 value dims (N split).
-//   * 24 warps per CTA:
-//       warps 0-7   softmax, two groups of four warps on alternate key blocks (one TMEM lane
-//                   per thread, 64 S columns each);
-//       warps 8-15  KV row gather with 16-byte cp.async copies written straight into the
-//                   128-byte-swizzled tile layout (K: own 64 keys x 576 bytes; V: all 128 keys
-//                   x this CTA's 256 value bytes) and the Q tile (TMA);
-//       warp 16     MMA issue (leader CTA; whole warp polls, one elected lane issues);
-//       warps 17-18 relay "K / V landed" from the peer CTA to the leader's barriers;
-//       warp 19     index-validity bits;
-//       warps 20-23 tile epilogue: O out of TMEM, x out_scale / l, bf16, staged per warp and
-//                   written with TMA tile stores while the softmax warps already work on the
-//                   next tile.
+//   * persistent: one cluster of 2 CTAs per SM pair walks work items cid, cid + #clusters, ...
+//     (an item is a tile, or one of nsplit slices of a tile's key blocks); each CTA owns 64 query
+//     rows.  Both GEMMs are single tcgen05 cta_group::2 instructions spanning the pair: QK^T
+//     splits the 128 keys of a block across the CTAs (N split), PV splits the 512 value dims.
+//   * a block's K tile BECOMES its V tile.  CTA c gathers the 576-byte rows of its own 64 keys
+//     (column chunks 0-3 of 128 dims, rope chunk).  PV wants, per CTA, 256 value dims of all 128
+//     keys: for its own keys they are already there (chunks 2c, 2c + 1), and once QK^T has read
+//     the tile the other two chunks are dead -- the peer keys' rows of this CTA's 256 dims are
+//     gathered into them.  Both CTAs then hold keys 0-63 in chunks 0-1 and keys 64-127 in chunks
+//     2-3, which is what one pair-wide descriptor needs.  Against separate V tiles: 52 instead of
+//     68 KB fetched per block and CTA, and 36 instead of 68 KB of shared memory per block, i.e.
+//     four blocks in flight instead of two.
+//   * 32 warps per CTA:
+//       warps 0-15  softmax, two groups of eight warps on alternate key blocks (one TMEM lane and
+//                   32 S columns per thread: short chains, and eight warps per scheduler to hide
+//                   them);
+//       warps 16-23 KV row gather with 16-byte cp.async copies written straight into the
+//                   128-byte-swizzled tile layout;
+//       warp 24     MMA issue (leader CTA; whole warp polls, one elected lane issues);
+//       warps 25-26 relay "K / V landed" from the peer CTA to the leader's barriers;
+//       warp 27     index-validity bits;
+//       warps 28-31 Q tiles in (TMA, or bf16 rows quantised on the way) and tile epilogue: O out
+//                   of TMEM, x out_scale / l, bf16, staged per warp and written with TMA tile
+//                   stores while the softmax warps already work on the next item.
 //   * Q and K tiles are four 128-byte-swizzled column chunks per 64 rows plus a compact
-//     64-byte-swizzled chunk for the 64 rope bytes; V tiles two MN-major chunks per 128 keys.
+//     64-byte-swizzled chunk for the 64 rope bytes.
 //   * the 512 latent dims of every Q tile are moved from shared memory into TENSOR MEMORY once
-//     per tile (by the epilogue warps) and the QK^T MMAs read them from there (A operand in
+//     per item (by the epilogue warps) and the QK^T MMAs read them from there (A operand in
 //     TMEM); only the rope chunk of Q stays in shared memory.
 //   * completion is tracked with mbarriers only; every wait is bounded (common.cuh) and
 //     reports through a status word instead of trapping.
@@ -44,36 +52,35 @@ constexpr unsigned kIdleCheckEvery = 64;   // idle polls between two time-limit 
 constexpr unsigned kIdleSleepNs = 8;       // back-off of an idle poll
 
 
-constexpr int kSoftmaxWarps = 8, kProducerWarps = 8;
-constexpr int kWarpMma = 16, kWarpCopy = 17, kWarpRelay = 18, kWarpValid = 19, kWarpEpi0 = 20;
+constexpr int kSoftmaxWarps = 16, kProducerWarps = 8;
+constexpr int kWarpGather0 = 16, kWarpMma = 24, kWarpRelayK = 25, kWarpRelayV = 26, kWarpValid = 27, kWarpEpi0 = 28;
 constexpr int kEpiWarps = 4;
-constexpr int kAttnThreads = 768;
+constexpr int kAttnThreads = 1024;
 constexpr int kBlockKeys = 128;                      // keys per softmax block (whole pair)
 constexpr int kDQK = 576, kDV = 512;
 constexpr int kChunkBytes = 64 * 128;                // 64 rows x 128 B (dims 128j .. 128j+127)
 constexpr int kRopeChunkBytes = 64 * 64;             // 64 rows x 64 B (dims 512 .. 575), 64-byte swizzle
-constexpr uint32_t kQBytes = 4 * kChunkBytes + kRopeChunkBytes;  // 36864 (per CTA)
-constexpr uint32_t kKStage = kQBytes;                // 64 keys x 576 B
-constexpr uint32_t kVChunk = 128 * 128;              // 128 keys x 128 B
-constexpr uint32_t kVStage = 2 * kVChunk;            // 128 keys x 256 dims
+constexpr uint32_t kQLatent = 4 * kChunkBytes;       // 32768 (per CTA)
+constexpr uint32_t kStageKV = kQLatent + kRopeChunkBytes;        // 64 keys x 576 B
 constexpr uint32_t kPBytes = 64 * 128;               // 64 rows x 128 keys e4m3
-constexpr uint32_t kMiscBytes = 7168;
+constexpr uint32_t kMiscBytes = 10240;
 constexpr uint32_t kStageBytes = 4 * 4096;           // staged epilogue: one 4 KB slice per epilogue warp
+constexpr int kSlots = 5;                            // ring of 36 KB slots
 
-// Shared-memory plan: two K stages, two V stages, two P buffers, own output staging.  (A third
-// K stage fits only with a single P buffer and staging aliased onto the Q tile; measured
-// slower: the single P buffer then waits for PVs whose V tile landed late.)
-constexpr int kKStages = 2;
+// Shared-memory plan.  A ring of five slots carries, in order, each item's Q tile and its K tiles:
+// Q only passes through on its way to tensor memory (latent dims) and to a fixed 4 KB buffer (rope
+// chunk), so a landing area of its own would idle 19 blocks out of 20.  The entry number of running
+// block kb of item ordinal it is kb + it + 1, that of the item's Q (its first block's kb) + it.
+// What bounds the kernel is latency: a slot is held for a gather, a QK^T, a softmax chain and a PV,
+// about 9000 cycles, so blocks in flight are the throughput.
 struct Plan {
-  static constexpr int kPBufs = 2;
-  static constexpr uint32_t kOffQ = 0;
-  static constexpr uint32_t kOffK = kOffQ + kQBytes;
-  static constexpr uint32_t kOffV = kOffK + kKStages * kKStage;
-  static constexpr uint32_t kOffP = kOffV + 2 * kVStage;
-  static constexpr uint32_t kOffMisc = kOffP + kPBufs * kPBytes;
-  static constexpr uint32_t kOffStage = kOffMisc + kMiscBytes;
-  static constexpr uint32_t kSmem = kOffStage + kStageBytes + 1024;   // + alignment slack
-  static_assert(kOffV % 1024 == 0 && kOffP % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+  static constexpr uint32_t kOffKV = 0;
+  static constexpr uint32_t kOffRope = kOffKV + kSlots * kStageKV;
+  static constexpr uint32_t kOffP = kOffRope + kRopeChunkBytes;
+  static constexpr uint32_t kOffStage = kOffP + 2 * kPBytes;
+  static constexpr uint32_t kOffMisc = kOffStage + kStageBytes;
+  static constexpr uint32_t kSmem = kOffMisc + kMiscBytes + 1024;   // + alignment slack
+  static_assert(kStageKV % 1024 == 0 && kOffP % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static_assert(kSmem <= 232448, "shared-memory plan exceeds the 227 KB per-CTA limit");
 };
 
@@ -90,26 +97,29 @@ constexpr float kMInit = -1e30f;
 constexpr float kRescaleThreshold = 6.0f;
 
 struct Misc {
-  // in the leader CTA only: k_peer / v_peer (peer's K / V landed), s_free / p_ready (softmax
+  // in the leader CTA only: k_peer / v_peer (peer's K / V rows landed), s_free / p_ready (softmax
   // warps of both CTAs)
-  uint64_t k_peer[3], v_peer[2], s_free[2], p_ready[2];
-  // in every CTA.  qk_done is indexed by the running block number modulo 6: one barrier tells
-  // the softmax group of block kb (S buffer kb % 2) and the gather warps (K stage kb % 2 or
-  // kb % 3) that QK^T(kb) is complete, and none is reused before both have looked at it.
-  uint64_t k_land[3], v_land[2], qk_done[6], pv_done[2], valid_ready[2], valid_free[2];
+  uint64_t k_peer[8], v_peer[8], s_free[2], p_ready[2];
+  // in every CTA, indexed by the running block number modulo 8 (pv_done: modulo 4): with five
+  // slots everybody has looked at block kb's barriers before block kb + 8 can touch them
+  uint64_t k_land[8], v_land[8], qk_done[8], pv_done[4];
+  uint64_t slot_free[kSlots];       // the slot's entry is dead: block through its PV, or Q moved on
+  uint64_t valid_ready[2], valid_free[2];
   uint64_t m_pub[2];                // running max of block k published by softmax group k%2
-  uint64_t q_land;                  // every CTA: this CTA's Q tile has landed in shared memory
+  uint64_t q_land;                  // every CTA: this CTA's Q tile has landed in its slot (e4m3 q);
+                                    // its slot is free for the epilogue warps to fill (bf16 q)
   uint64_t qt_ready;                // leader CTA: Q's latent part is in tensor memory in both CTAs
-  uint64_t q_free;                  // all QK^T of the current tile are complete (Q tile reusable)
-  uint64_t o_free;                  // leader CTA: the tile's O has been read out of TMEM
-  uint64_t epi_ready;               // the tile's row scales are published (softmax warps)
+  uint64_t q_free;                  // all QK^T of the current item are complete (Q reusable)
+  uint64_t o_free;                  // leader CTA: the item's O has been read out of TMEM
+  uint64_t epi_ready;               // the item's row scales are published (softmax warps)
   uint32_t valid[2][4];             // 128 validity bits per stage
   uint32_t tmem_base;
   uint32_t pad;
-  float xbuf[2][2][128];            // [group][parity][lane]: row-max exchange between key halves
+  float xbuf[2][2][2][128];         // [group][parity][column half][lane]: row-max exchange
   float mshare[2][128];             // [group][lane]: running max after the group's latest block
-  float fin[3][256];                // end of tile: row sums, true maxima, last running max
-  float oscale[2][64];              // [tile parity][row]: out_scale / l, 0 for rows without a key
+  float fin_l[512];                 // end of item: row sums per thread ...
+  float fin_rm[128], fin_m[128];    // ... true maxima, last running max per (group, row)
+  float oscale[2][64];              // [item parity][row]: out_scale / l, 0 for rows without a key
 };
 static_assert(sizeof(Misc) <= kMiscBytes, "Misc too large");
 
@@ -136,7 +146,28 @@ struct AttnParams {
   float scale_log2, out_scale;
   int epoch;                          // this launch's epoch for the bounded waits
   unsigned long long wait_limit_ns;
+  // bf16 queries (dense packed layout), quantised to e4m3 on their way in: code = e4m3(q * q_inv);
+  // null: q arrives as e4m3 through map_q / map_q_rope
+  const uint4* q_bf16;
+  float q_inv;
+  // KV split inside the launch: nsplit > 1 slices per tile, each leaving its unnormalised O (fp32
+  // [ng * nsplit, 128, 512]) and (running max, row sum) for merge_parts_kernel
+  int nsplit;
+  float* part_o;
+  float2* part_ml;
 };
+
+// four e4m3 codes of two packed bf16 pairs, x inv (saturating): the arithmetic of quantize_e4m3
+__device__ __forceinline__ uint32_t e4m3x4_of_bf16(uint32_t lo, uint32_t hi, float inv) {
+  float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&lo));
+  float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hi));
+  a.x *= inv; a.y *= inv; b.x *= inv; b.y *= inv;
+  return (uint32_t)__nv_cvt_float2_to_fp8x2(a, __NV_SATFINITE, __NV_E4M3) |
+         ((uint32_t)__nv_cvt_float2_to_fp8x2(b, __NV_SATFINITE, __NV_E4M3) << 16);
+}
+
+// one work item: key blocks [k0, k0 + nb) of a tile; ranks >= lim are masked
+struct Item { int tile, k0, nb, lim; };
 
 // wait sites reported in the status word
 enum { kSiteQ = 1, kSiteKLand, kSiteKPeer, kSiteVLand, kSiteVPeer, kSiteQkDone, kSitePvDone,
@@ -146,23 +177,12 @@ enum { kSiteQ = 1, kSiteKLand, kSiteKPeer, kSiteVLand, kSiteVPeer, kSiteQkDone, 
 // status block of the FP8 attention kernels (layout: see Waiter in common.cuh)
 __device__ int g_attn_status[8];
 
-// a running block number's K stage / phase and its qk_done barrier / phase
-struct BlockIdx {
-  int ks, kph, b6, b6ph;
-  __device__ __forceinline__ explicit BlockIdx(int kb) {
-    ks = kb % kKStages; kph = (kb / kKStages) & 1;
-    b6 = kb % 6; b6ph = (kb / 6) & 1;
-  }
-};
-
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kAttnThreads, 1)
 masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_q_rope,
                       const __grid_constant__ OutMaps omaps, const AttnParams p) {
   using PL = Plan;
-  constexpr uint32_t kOffQ = PL::kOffQ, kOffK = PL::kOffK, kOffV = PL::kOffV, kOffP = PL::kOffP,
-                     kOffMisc = PL::kOffMisc, kOffStage = PL::kOffStage;
-  constexpr int kPBufs = PL::kPBufs;
+  constexpr uint32_t kOffRope = PL::kOffRope, kOffKV = PL::kOffKV, kOffP = PL::kOffP, kOffMisc = PL::kOffMisc, kOffStage = PL::kOffStage;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;       // 128B-swizzle tiles need 1024-byte alignment
@@ -170,22 +190,34 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   Misc& ms = *reinterpret_cast<Misc*>(sm + kOffMisc);
   const Waiter wt{g_attn_status, p.epoch, p.wait_limit_ns};
 
-  // Persistent: each cluster walks tiles cid, cid + #clusters, ...  Every role runs the same
-  // tile loop; stages, buffers and barrier phases are indexed by the cluster-wide running
-  // block number kb, so the next tile's Q / K / V loads and first QK^T overlap the previous
-  // tile's last softmax blocks and its epilogue.
+  // Persistent: each cluster walks items cid, cid + #clusters, ...  Every role runs the same
+  // item loop; stages, buffers and barrier phases are indexed by the cluster-wide running
+  // block number kb, so the next item's Q / K / V loads and first QK^T overlap the previous
+  // item's last softmax blocks and its epilogue.
   const uint32_t cta = cluster_ctarank();
   const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
+  const int n_items = p.ng * p.nsplit;
   // broadcast so the compiler knows the role index is warp-uniform
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  // live union entries of a tile; with per-token prefix bounds the block loop runs to the LAST
-  // token's bound (litedsa_attention_sm100.cuh:1846-1851)
-  auto tile_count = [&](int tile) -> int {
-    const int c = p.len_per_q ? p.len_per_q[(size_t)tile * p.G + (p.G - 1)]
-                              : (p.counts ? p.counts[tile] : p.cap);
-    return min(max(c, 0), p.cap);
+  auto item_of = [&](int w) -> Item {
+    Item t;
+    t.tile = p.nsplit == 1 ? w : w / p.nsplit;
+    // live union entries of the tile; with per-token prefix bounds the block loop runs to the LAST
+    // token's bound (litedsa_attention_sm100.cuh:1846-1851)
+    const int c = p.len_per_q ? p.len_per_q[(size_t)t.tile * p.G + (p.G - 1)]
+                              : (p.counts ? p.counts[t.tile] : p.cap);
+    t.lim = min(max(c, 0), p.cap);
+    t.k0 = 0;
+    t.nb = max((t.lim + kBlockKeys - 1) / kBlockKeys, 1);
+    if (p.nsplit > 1) {       // slice `part`; an empty slice runs one fully masked block
+      const int part = w - t.tile * p.nsplit, nbt = t.nb;
+      const int k1 = (part + 1) * nbt / p.nsplit;
+      t.k0 = part * nbt / p.nsplit;
+      t.nb = max(k1 - t.k0, 1);
+      t.lim = min(t.lim, k1 * kBlockKeys);
+    }
+    return t;
   };
-  auto blocks_of = [&](int count) -> int { return max((count + kBlockKeys - 1) / kBlockKeys, 1); };
 
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_land, 1);
@@ -193,25 +225,29 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
     mbar_init(&ms.epi_ready, kSoftmaxWarps);
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < 8; ++i) {
       mbar_init(&ms.k_peer[i], 1);
-      mbar_init(&ms.k_land[i], kProducerWarps * 32);        // one async arrival per gather thread
-    }
-    for (int i = 0; i < 6; ++i) mbar_init(&ms.qk_done[i], 1);
-    for (int i = 0; i < 2; ++i) {
       mbar_init(&ms.v_peer[i], 1);
-      mbar_init(&ms.s_free[i], 8);        // 4 warps of one softmax group x 2 CTAs
-      mbar_init(&ms.p_ready[i], 8);
-      mbar_init(&ms.v_land[i], kProducerWarps * 32);        // one async arrival per gather thread
-      mbar_init(&ms.pv_done[i], 1);
+      mbar_init(&ms.k_land[i], kProducerWarps * 32);        // one async arrival per gather thread
+      mbar_init(&ms.v_land[i], kProducerWarps * 32);
+      mbar_init(&ms.qk_done[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) mbar_init(&ms.pv_done[i], 1);
+    for (int i = 0; i < kSlots; ++i) mbar_init(&ms.slot_free[i], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&ms.s_free[i], 16);        // 8 warps of one softmax group x 2 CTAs
+      mbar_init(&ms.p_ready[i], 16);
       mbar_init(&ms.valid_ready[i], 1);
-      mbar_init(&ms.valid_free[i], 4);
-      mbar_init(&ms.m_pub[i], 4);
+      mbar_init(&ms.valid_free[i], 8);
+      mbar_init(&ms.m_pub[i], 8);
     }
     fence_mbar_init();
-    tma_prefetch_desc(&map_q);
-    tma_prefetch_desc(&map_q_rope);
-    for (int d = 0; d < p.n_out; ++d) tma_prefetch_desc(&omaps.m[d]);
+    if (p.q_bf16 == nullptr) {
+      tma_prefetch_desc(&map_q);
+      tma_prefetch_desc(&map_q_rope);
+    }
+    if (p.nsplit == 1)
+      for (int d = 0; d < p.n_out; ++d) tma_prefetch_desc(&omaps.m[d]);
   }
   __syncthreads();
   cluster_sync_all();
@@ -224,16 +260,23 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   tc_fence_after();
   const uint32_t tmem = ms.tmem_base;
 
+  // Registers: the block is launched with 64 per thread (8 warpgroups, 512 in sum); the softmax
+  // warps need more for their 32 scores, the epilogue for its 32 + 16 outputs, the others less:
+  // 80 x 4 + 40 x 2 + 40 + 72 = 512.  (With 64 everywhere a handful of values spilled, and with
+  // nearly all of L1 used as shared memory a spill is a round trip to L2.)
   if (warp < kSoftmaxWarps) {
-    // ------------------------------------------------------------ softmax + epilogue
-    // Two groups of four warps work on alternate key blocks (group g: blocks with kb % 2 == g),
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
+    // ------------------------------------------------------------ softmax
+    // Two groups of eight warps work on alternate key blocks (group g: blocks with kb % 2 == g),
     // so two blocks are in flight and the latencies of one chain (TMEM load, exchanges,
-    // fences) hide behind the other.  Within a group, thread = TMEM lane tl: tile row
-    // r = tl % 64, key half h = tl / 64 (64 S columns each).  The only state that crosses
-    // groups is the running max m, handed over through shared memory right after each
-    // block's row maxima are known; the row sum l is kept per group relative to the m of the
-    // group's latest block and merged at the end of the tile.
-    const int g = warp >> 2;                      // softmax group = block parity it serves
+    // fences) hide behind the other.  Within a group, thread = (TMEM lane tl, column half cs):
+    // tile row r = tl % 64, keys [64 h + 32 cs, +32) of the block with h = tl / 64.  (64 columns
+    // per thread in four warps made one block's chain 2.4 us, i.e. the kernel's pace.)  The only
+    // state that crosses groups is the running max m, handed over through shared memory right
+    // after each block's row maxima are known; the row sum l is kept per thread relative to the m
+    // of the group's latest block and merged at the end of the item.
+    const int g = warp >> 3;                      // softmax group = block parity it serves
+    const int cs = (warp >> 2) & 1;
     const int tl = ((warp & 3) << 5) | lane;
     const int r = tl & 63, h = tl >> 6;
     const int row = (int)cta * 64 + r;            // row of the 128-row tile
@@ -242,68 +285,65 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     const float c = p.scale_log2;
     const uint32_t a_s_free = mapa(smem_u32(&ms.s_free[g]), 0);
     const uint32_t a_p_ready = mapa(smem_u32(&ms.p_ready[g]), 0);
-    const uint32_t scol = tmem + lane_base + (g ? kTmemS1 : kTmemS0);
+    const uint32_t scol = tmem + lane_base + (g ? kTmemS1 : kTmemS0) + 32 * cs;
+    const int key0 = 64 * h + 32 * cs;            // first of this thread's keys within a block
     int kb0 = 0, it = 0;
 
-    for (int tile = cid; tile < p.ng; tile += ncl) {
-      const int nb = blocks_of(tile_count(tile));
-      const size_t trow = (size_t)tile * p.G + row / p.h_per_q;     // (tile, token) of this row
-      const uint32_t* mrow = p.memb ? p.memb + trow * capw + 2 * h : nullptr;
+    for (int w = cid; w < n_items; w += ncl) {
+      const Item item = item_of(w);
+      const int nb = item.nb;
+      const size_t trow = (size_t)item.tile * p.G + row / p.h_per_q;     // (tile, token) of this row
+      const uint32_t* mrow = p.memb ? p.memb + trow * capw + (size_t)item.k0 * 4 + (key0 >> 5) : nullptr;
       // per-token causal prefix: this row may attend union ranks < row_bound
       const int row_bound = p.len_per_q ? __ldg(p.len_per_q + trow) : 0x7fffffff;
       float m_mine = kMInit;      // the running max my row sum is relative to
       float li = 0.f, real_m = -INFINITY;
       const int k_first = (g - kb0) & 1;          // first local block with (kb0 + k) % 2 == g
-      uint2 mk = make_uint2(~0u, ~0u);
-      if (mrow && k_first < nb) mk = __ldcs(reinterpret_cast<const uint2*>(mrow + (size_t)k_first * 4));
+      uint32_t mk = ~0u;
+      if (mrow && k_first < nb) mk = __ldcs(mrow + (size_t)k_first * 4);
 
       for (int k = k_first; k < nb; k += 2) {
         const int kb = kb0 + k;
         const uint32_t ph = (kb >> 1) & 1;
-        uint2 mk_next = mk;
-        if (mrow && k + 2 < nb) mk_next = __ldcs(reinterpret_cast<const uint2*>(mrow + (size_t)(k + 2) * 4));
+        uint32_t mk_next = mk;
+        if (mrow && k + 2 < nb) mk_next = __ldcs(mrow + (size_t)(k + 2) * 4);
 
-        {
-          const BlockIdx bi(kb);
-          mbar_wait(&ms.qk_done[bi.b6], bi.b6ph, wt, kSiteQkDone, k);
-        }
+        mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteQkDone, k);
         __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
         tc_fence_after();
-        float sv[64];
+        float sv[32];
         tmem_ld32(scol, sv);
-        tmem_ld32(scol + 32, sv + 32);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(a_s_free);
 
         mbar_wait(&ms.valid_ready[g], ph, wt, kSiteValidReady, k);
-        uint32_t v0 = ms.valid[g][2 * h] & mk.x, v1 = ms.valid[g][2 * h + 1] & mk.y;
-        if (p.len_per_q) {     // ranks of my 64 columns: [128k + 64h, +64)
-          const int n = min(max(row_bound - (k * kBlockKeys + 64 * h), 0), 64);
-          const unsigned long long pm = n >= 64 ? ~0ull : ((1ull << n) - 1ull);
-          v0 &= (uint32_t)pm;
-          v1 &= (uint32_t)(pm >> 32);
+        uint32_t vm = ms.valid[g][key0 >> 5] & mk;
+        if (p.len_per_q) {     // ranks of my 32 columns
+          const int n = min(max(row_bound - ((item.k0 + k) * kBlockKeys + key0), 0), 32);
+          vm &= n >= 32 ? ~0u : ((1u << n) - 1u);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ms.valid_free[g]);
         mk = mk_next;
 
-        float cur = -INFINITY;
+        float c0 = -INFINITY, c1 = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          sv[j] = ((v0 >> j) & 1u) ? sv[j] : -INFINITY;
-          sv[32 + j] = ((v1 >> j) & 1u) ? sv[32 + j] : -INFINITY;
-          cur = fmaxf(cur, fmaxf(sv[j], sv[32 + j]));
+        for (int j = 0; j < 32; j += 2) {
+          sv[j] = ((vm >> j) & 1u) ? sv[j] : -INFINITY;
+          sv[j + 1] = ((vm >> (j + 1)) & 1u) ? sv[j + 1] : -INFINITY;
+          c0 = fmaxf(c0, sv[j]);
+          c1 = fmaxf(c1, sv[j + 1]);
         }
-        cur *= c;
-        float* xb = ms.xbuf[g][ph];
-        xb[tl] = cur;
-        if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-        else asm volatile("bar.sync 2, 128;" ::: "memory");
-        cur = fmaxf(cur, xb[tl ^ 64]);
+        float cur = fmaxf(c0, c1) * c;
+        float (*xb)[128] = ms.xbuf[g][ph];
+        xb[cs][tl] = cur;
+        if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+        else asm volatile("bar.sync 2, 256;" ::: "memory");
+        cur = fmaxf(fmaxf(xb[0][r], xb[1][r]), fmaxf(xb[0][r + 64], xb[1][r + 64]));
         real_m = fmaxf(real_m, cur);
-        // running max after block k-1 of this tile comes from the other group
+        // running max after block k-1 of this item comes from the other group
         float m_prev = kMInit;
         if (k > 0) {
           mbar_wait(&ms.m_pub[g ^ 1], ((kb - 1) >> 1) & 1, wt, kSiteMPub, k);
@@ -311,49 +351,46 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         const bool rescale = __any_sync(0xffffffffu, cur - m_prev > kRescaleThreshold);
         const float new_m = rescale ? fmaxf(cur, m_prev) : m_prev;
-        ms.mshare[g][tl] = new_m;
+        if (cs == 0) ms.mshare[g][tl] = new_m;
         __syncwarp();
         if (lane == 0) mbar_arrive(&ms.m_pub[g]);
         li *= fast_exp2(m_mine - new_m);
         m_mine = new_m;
 
         const float nm = -new_m + kPScaleLog2;
-        uint32_t pk[16];
+        uint32_t pk[8];
+        float l1 = 0.f;
 #pragma unroll
-        for (int j = 0; j < 64; j += 4) {
+        for (int j = 0; j < 32; j += 4) {
           float2 d0, d1;
           d0.x = fast_exp2(fmaf(sv[j], c, nm));
           d0.y = fast_exp2(fmaf(sv[j + 1], c, nm));
           d1.x = fast_exp2(fmaf(sv[j + 2], c, nm));
           d1.y = fast_exp2(fmaf(sv[j + 3], c, nm));
           li += d0.x + d0.y;
-          li += d1.x + d1.y;
+          l1 += d1.x + d1.y;
           const uint32_t lo = __nv_cvt_float2_to_fp8x2(d0, __NV_SATFINITE, __NV_E4M3);
           const uint32_t hi = __nv_cvt_float2_to_fp8x2(d1, __NV_SATFINITE, __NV_E4M3);
           pk[j >> 2] = lo | (hi << 16);
         }
-        // the P buffer was last read by the PV of block kb-2 (two buffers) or kb-1 (one)
-        if (kPBufs == 2) {
-          if (kb >= 2) mbar_wait(&ms.pv_done[g], ph ^ 1, wt, kSitePFree, k);
-        } else {
-          if (kb >= 1) mbar_wait(&ms.pv_done[g ^ 1], ((kb - 1) >> 1) & 1, wt, kSitePFree, k);
-        }
-        uint8_t* pdst = sm + kOffP + (kPBufs == 2 ? g : 0) * kPBytes + (4 * h) * 1024 + r * 16;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(pdst + i * 1024) =
-              make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+        li += l1;
+        // the P buffer was last read by the PV of block kb-2
+        if (kb >= 2) mbar_wait(&ms.pv_done[(kb - 2) & 3], ((kb - 2) >> 2) & 1, wt, kSitePFree, k);
+        uint8_t* pdst = sm + kOffP + g * kPBytes + (4 * h + 2 * cs) * 1024 + r * 16;
+        *reinterpret_cast<uint4*>(pdst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        *reinterpret_cast<uint4*>(pdst + 1024) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
 
         if (rescale && k > 0) {
           // O holds blocks [0, k) relative to m_prev: bring it to new_m once PV(k-1) is complete
-          mbar_wait(&ms.pv_done[g ^ 1], ((kb - 1) >> 1) & 1, wt, kSitePvDone, k);
+          // (each thread of the pair serving a TMEM lane takes half of the lane's columns)
+          mbar_wait(&ms.pv_done[(kb - 1) & 3], ((kb - 1) >> 2) & 1, wt, kSitePvDone, k);
           __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
           tc_fence_after();
           const float f = fast_exp2(m_prev - new_m);
           float o[32];
 #pragma unroll 1
-          for (int cc = 0; cc < 8; ++cc) {
-            const uint32_t ocol = tmem + lane_base + kTmemO + cc * 32;
+          for (int cc = 0; cc < 4; ++cc) {
+            const uint32_t ocol = tmem + lane_base + kTmemO + cs * 128 + cc * 32;
             tmem_ld32(ocol, o);
             tmem_wait_ld();
 #pragma unroll
@@ -368,175 +405,189 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) mbar_arrive_cluster(a_p_ready);
       }
 
-      // end of tile: merge the two groups' row sums (each relative to its own latest running max)
-      const int t = threadIdx.x;                    // 0..255 = g*128 + tl
-      ms.fin[0][t] = li;
-      ms.fin[1][t] = real_m;
-      ms.fin[2][t] = m_mine;
-      asm volatile("bar.sync 3, 256;" ::: "memory");
-      const int kbl = kb0 + nb - 1;                 // last block of the tile
-      const int last_g = kbl & 1;
-      float m = ms.fin[2][last_g * 128 + tl];       // running max after the last block
-      float lsum = 0.f;
-      real_m = -INFINITY;
-      // fixed summation order (even local blocks first, whichever group served them), so a
-      // tile's result does not depend on the blocks its cluster processed before
-      const int g_even = kb0 & 1;
+      // end of item: merge the row sums (each relative to its own group's latest running max)
+      // (the previous item's sums must have been read: every warp has arrived on its epi_ready)
+      if (it > 0) mbar_wait(&ms.epi_ready, (it - 1) & 1, wt, kSiteEpi, it);
+      ms.fin_l[(g * 2 + cs) * 128 + tl] = li;
+      if (cs == 0 && h == 0) {
+        ms.fin_rm[g * 64 + r] = real_m;
+        ms.fin_m[g * 64 + r] = m_mine;
+      }
+      asm volatile("bar.sync 3, 512;" ::: "memory");
+      if (g == 0 && cs == 0 && h == 0) {
+        const int last_g = (kb0 + nb - 1) & 1;      // group of the item's last block
+        float m = ms.fin_m[last_g * 64 + r];       // running max after the last block
+        float lsum = 0.f;
+        real_m = -INFINITY;
+        // fixed summation order (even local blocks first, whichever group served them), so an
+        // item's result does not depend on the blocks its cluster processed before
+        const int g_even = kb0 & 1;
 #pragma unroll
-      for (int gi = 0; gi < 2; ++gi) {
-        const int gg = gi ^ g_even;
+        for (int gi = 0; gi < 2; ++gi) {
+          const int gg = gi ^ g_even;
+          const float f = fast_exp2(ms.fin_m[gg * 64 + r] - m);
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int o = gg * 128 + hh * 64 + r;
-          lsum += ms.fin[0][o] * fast_exp2(ms.fin[2][o] - m);
-          real_m = fmaxf(real_m, ms.fin[1][o]);
+          for (int hc = 0; hc < 4; ++hc)
+            lsum += ms.fin_l[(gg * 2 + (hc & 1)) * 128 + (hc >> 1) * 64 + r] * f;
+          real_m = fmaxf(real_m, ms.fin_rm[gg * 64 + r]);
         }
-      }
-      li = lsum;
-      if (real_m == -INFINITY) { li = 0.f; m = -INFINITY; }
-      const size_t grow = (size_t)tile * 128 + row;
-      if (g == 0 && h == 0) {
-        float l = __logf(li) - kPScaleLn + m * kLn2;
-        if (!(li > 0.f)) l = INFINITY;
-        p.lse[grow] = l;
-        if (p.max_logits) p.max_logits[grow] = real_m * kLn2;
-      }
-      // Hand the tile over to the gather warps, which read O out of TMEM, scale it and store
-      // it while these warps already work on the next tile: all they need is 1 / l per row.
-      if (g == 0 && h == 0) {
-        // the sink joins the OUTPUT normaliser only (in l's units: x 7, relative to m)
-        float denom = li;
-        if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldg(p.sink + row) * kLog2e - m + kPScaleLog2);
-        ms.oscale[it & 1][r] = (li > 0.f) ? __fdividef(p.out_scale, denom) : 0.f;
+        li = lsum;
+        if (real_m == -INFINITY) { li = 0.f; m = -INFINITY; }
+        if (p.nsplit > 1) {
+          p.part_ml[(size_t)w * 128 + row] = make_float2(m, li);
+        } else {
+          const size_t grow = (size_t)item.tile * 128 + row;
+          float l = __logf(li) - kPScaleLn + m * kLn2;
+          if (!(li > 0.f)) l = INFINITY;
+          p.lse[grow] = l;
+          if (p.max_logits) p.max_logits[grow] = real_m * kLn2;
+          // the epilogue warps need 1 / l per row; the sink joins the OUTPUT normaliser only (in l's
+          // units: x 7, relative to m)
+          float denom = li;
+          if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldg(p.sink + row) * kLog2e - m + kPScaleLog2);
+          ms.oscale[it & 1][r] = (li > 0.f) ? __fdividef(p.out_scale, denom) : 0.f;
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&ms.epi_ready);
       kb0 += nb;
       ++it;
     }
-  } else if (warp < kSoftmaxWarps + kProducerWarps) {
-    // ------------------------------------------------------------ KV row gather (cp.async) and the Q tile (TMA)
+  } else if (warp < kWarpGather0 + kProducerWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    // ------------------------------------------------------------ KV row gather (cp.async)
     // The union rows are fetched with 16-byte cp.async copies issued by all 256 threads of
     // these eight warps: fire-and-forget, any number of blocks in flight, destination written
     // directly in the 128-byte-swizzled tile layout, completion reported to an mbarrier by an
     // asynchronous arrival.  (TMA gather4 was measured at one instruction per ~8.5 ns per SM,
-    // i.e. ~1 us per block for this tile shape: it, not the tensor pipe, set the pace.)
-    // Warp pw owns rows [8pw, 8pw+8) of this CTA's 64 keys (K tile: all 576 bytes, nine copies
-    // per lane) and rows [16pw, 16pw+16) of the block's 128 keys (V tile: this CTA's 256 value
-    // bytes, eight copies per lane).  K and V streams have different stage-free conditions
-    // (QK^T done vs PV done), so each warp advances two independent cursors and issues
-    // whichever is ready; neither tile is derived from the other, so no stage waits on a copy.
-    const int pw = warp - kSoftmaxWarps;
-    struct Cursor { int tile, it, k, nb, kb0; };
-    auto cur_init = [&](Cursor& c) {
-      c.tile = cid; c.it = 0; c.k = 0; c.kb0 = 0;
-      c.nb = c.tile < p.ng ? blocks_of(tile_count(c.tile)) : 0;
-    };
-    auto cur_next = [&](Cursor& c) {
-      if (++c.k == c.nb) {
-        c.kb0 += c.nb; c.k = 0; c.tile += ncl; ++c.it;
-        c.nb = c.tile < p.ng ? blocks_of(tile_count(c.tile)) : 0;
+    // i.e. the same ~60 GB/s per SM that the L2 -> SM path gives these copies.)
+    // Two cursors: K rows of block ck (this CTA's 64 keys, all 576 bytes: warp pw rows
+    // [8pw, 8pw + 8), nine copies per lane) as soon as the stage's previous block has been through
+    // its PV; V rows of block cv (the PEER's 64 keys, this CTA's 256 value bytes, four copies per
+    // lane) into the dead half of the same stage as soon as the block's QK^T is complete.
+    const int pw = warp - kWarpGather0;
+    struct Cursor { int w, k, nb, kb, slot, ring; const int32_t* idx; };   // slot, ring: entry = 5 ring + slot
+    // The Q entry in front of an item's K entries belongs to warp 0: once the slot is free it
+    // requests the tile (TMA) or, for bf16 q, hands the slot to the epilogue warps.  (Only here: a
+    // slot's barrier may be waited on once every older entry has been through it, which this
+    // warp's own K copies prove.)
+    int q_w = cid, q_slot = 0, q_ring = 0;
+    bool q_pending = pw == 0 && cid < n_items;
+    const uint64_t pol_stream = l2_policy_evict_first();
+    auto cur_load = [&](Cursor& c) {
+      c.nb = 0;
+      if (c.w < n_items) {
+        const Item t = item_of(c.w);
+        c.nb = t.nb; c.k = 0;
+        c.idx = p.indices + (size_t)t.tile * p.idx_stride + (size_t)t.k0 * kBlockKeys;
       }
     };
-    Cursor ck, cv;   // K gather, V gather
-    cur_init(ck);
-    cur_init(cv);
-    // q and out stream through once (evict-first TMA traffic), and so do the index lists and
-    // membership words (streaming loads): they must not push the re-read KV rows out of L2
-    const uint64_t pol_stream = l2_policy_evict_first();
-    // lane l < 16 holds the index of own key 8pw + l%8 (K tile rows), lane l >= 16 of key
-    // 16pw + l - 16 of the block's 128 keys (V tile rows)
-    const int my_key = lane < 16 ? 64 * (int)cta + 8 * pw + (lane & 7) : 16 * pw + (lane - 16);
-    auto load_idx = [&](const Cursor& c) -> int {
-      const int v = __ldcs(p.indices + (size_t)c.tile * p.idx_stride + (size_t)c.k * kBlockKeys + my_key);
-      return ((unsigned)v < (unsigned)p.s_kv) ? v : 0;     // out-of-range rows are masked later
+    auto advance = [&](Cursor& c) { if (++c.slot == kSlots) { c.slot = 0; ++c.ring; } };
+    auto cur_next = [&](Cursor& c) {
+      ++c.kb;
+      advance(c);
+      if (++c.k == c.nb) { c.w += ncl; cur_load(c); return true; }     // the next item's Q entry is next
+      return false;
     };
+    Cursor ck, cv;
+    ck.w = cv.w = cid;
+    ck.kb = cv.kb = 0;
+    ck.slot = cv.slot = 1;                         // entry 0 is the first item's Q
+    ck.ring = cv.ring = 0;
+    cur_load(ck);
+    cur_load(cv);
+    // lane l holds the index of key 8 pw + l % 8 of the CTA's own (K) / the peer's (V) 64 keys
+    const int own_key = 64 * (int)cta + 8 * pw + (lane & 7);
+    auto load_idx = [&](const Cursor& c, int key) -> int {
+      return __ldcs(c.idx + (size_t)c.k * kBlockKeys + key);
+    };
+    auto in_range = [&](int v) -> int { return ((unsigned)v < (unsigned)p.s_kv) ? v : 0; };   // masked later
     // The indices of a block are loaded right after the previous block's gather has been issued
-    // (one block ahead), so a cold index line from HBM is in flight while that gather lands.
+    // (one block ahead) and first looked at when the next gather goes out, so that nothing waits
+    // for a cold index line from HBM.
     int kidx = 0, vidx = 0;
-    if (ck.tile < p.ng) { kidx = load_idx(ck); vidx = load_idx(cv); }
+    if (ck.w < n_items) { kidx = load_idx(ck, own_key); vidx = load_idx(cv, own_key ^ 64); }
     const uint8_t* kvb = p.kv;
     const long long pitch = p.kv_pitch;
     const int cj = lane >> 3, cc = lane & 7;       // latent piece `lane`: chunk cj, 16-byte slot cc
-    int q_tile = cid, q_it = 0;                    // next Q tile to request (warp 0 only)
     unsigned long long idle_since = 0;
     unsigned idle_iters = 0;
     bool aborted = false;
-    while ((ck.tile < p.ng || cv.tile < p.ng || (pw == 0 && q_tile < p.ng)) && !aborted) {
+    while (cv.w < n_items && !aborted) {           // the V cursor never runs ahead of the K cursor
       bool did = false;
-      if (pw == 0 && q_tile < p.ng) {
-        // the previous tile's Q must have been consumed by its last QK^T
-        const bool okq = q_it == 0 || mbar_test(&ms.q_free, (q_it - 1) & 1);
-        if (__all_sync(0xffffffffu, okq)) {
-          if (lane == 0) {
-            mbar_arrive_expect_tx(&ms.q_land, kQBytes);
-            // this CTA's 64 rows of the tile = (token, head) pairs starting at row 64 cta
-            const int qh = (64 * (int)cta) % p.h_per_q;
-            const int qt = (q_tile / p.q_group_div) * p.G + (64 * (int)cta) / p.h_per_q;
-            for (int j = 0; j < 4; ++j)
-              tma_load_3d_hint(sbase + kOffQ + j * kChunkBytes, &map_q, 128 * j, qh, qt, &ms.q_land, pol_stream);
-            tma_load_3d_hint(sbase + kOffQ + 4 * kChunkBytes, &map_q_rope, 512, qh, qt, &ms.q_land, pol_stream);
+      // V first: its block is further along, and P waits for it next
+      {
+        // the block's K tile must have been read by its QK^T
+        const bool ok = cv.kb < ck.kb && mbar_test(&ms.qk_done[cv.kb & 7], (cv.kb >> 3) & 1);
+        if (__all_sync(0xffffffffu, ok)) {
+          const int vcur = in_range(vidx);
+          // the dead half of the K tile: chunks 2-3 in CTA 0, chunks 0-1 in CTA 1
+          const uint32_t vst = sbase + kOffKV + cv.slot * kStageKV + (cta == 0 ? 2 * kChunkBytes : 0);
+          // lane: row 8 pw + 2i + lane / 16 of the peer's keys, 16-byte piece lane % 16 of this
+          // CTA's 256 value bytes
+          const int pc = lane & 15, nbk = pc >> 3, c8 = pc & 7;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int rloc = 2 * i + (lane >> 4);
+            const int ri = __shfl_sync(0xffffffffu, vcur, rloc);
+            const int row = 8 * pw + rloc;
+            cp_async16(vst + nbk * kChunkBytes + row * 128 + ((c8 ^ (row & 7)) << 4),
+                       kvb + (size_t)ri * pitch + 256 * cta + 16 * pc);
           }
-          __syncwarp();
-          q_tile += ncl;
-          ++q_it;
+          cp_async_mbar_arrive_noinc(&ms.v_land[cv.kb & 7]);
+          if (cur_next(cv)) advance(cv);
+          if (cv.w < n_items) vidx = load_idx(cv, own_key ^ 64);
           did = true;
         }
       }
-      if (ck.tile < p.ng) {
-        const int kb = ck.kb0 + ck.k;
-        const BlockIdx bi(kb);
-        const int s = bi.ks;
-        // stage s held block kb - kKStages: its QK^T must have read it
-        bool ok = true;
-        if (kb >= kKStages) {
-          const BlockIdx prev(kb - kKStages);
-          ok = mbar_test(&ms.qk_done[prev.b6], prev.b6ph);
-        }
+      if (q_pending) {                             // warp-uniform; warp 0 only
+        const bool ok = q_ring == 0 || mbar_test(&ms.slot_free[q_slot], (q_ring - 1) & 1);
         if (__all_sync(0xffffffffu, ok)) {
-          const uint32_t kst = sbase + kOffK + s * kKStage;
+          if (lane == 0) {
+            if (p.q_bf16 != nullptr) {
+              mbar_arrive(&ms.q_land);
+            } else {
+              mbar_arrive_expect_tx(&ms.q_land, kStageKV);
+              // this CTA's 64 rows of the tile = (token, head) pairs starting at row 64 cta
+              const int qh = (64 * (int)cta) % p.h_per_q;
+              const int qt = item_of(q_w).tile / p.q_group_div * p.G + (64 * (int)cta) / p.h_per_q;
+              const uint32_t dst = sbase + kOffKV + q_slot * kStageKV;
+              for (int c = 0; c < 4; ++c)
+                tma_load_3d_hint(dst + c * kChunkBytes, &map_q, 128 * c, qh, qt, &ms.q_land, pol_stream);
+              tma_load_3d_hint(dst + kQLatent, &map_q_rope, 512, qh, qt, &ms.q_land, pol_stream);
+            }
+          }
+          __syncwarp();
+          q_pending = false;
+          did = true;
+        }
+      }
+      if (ck.w < n_items && !q_pending) {
+        // the slot's previous entry must be dead
+        const bool ok = ck.ring == 0 || mbar_test(&ms.slot_free[ck.slot], (ck.ring - 1) & 1);
+        if (__all_sync(0xffffffffu, ok)) {
+          const int kcur = in_range(kidx);
+          const uint32_t kst = sbase + kOffKV + ck.slot * kStageKV;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const int ri = __shfl_sync(0xffffffffu, kidx, i);
+            const int ri = __shfl_sync(0xffffffffu, kcur, i);
             const int row = 8 * pw + i;
             cp_async16(kst + cj * kChunkBytes + row * 128 + ((cc ^ (row & 7)) << 4),
                        kvb + (size_t)ri * pitch + 16 * lane);
           }
           {
-            const int ri = __shfl_sync(0xffffffffu, kidx, lane >> 2);
+            const int ri = __shfl_sync(0xffffffffu, kcur, lane >> 2);
             const int row = 8 * pw + (lane >> 2);
             // rope bytes: compact 64-byte rows, 64-byte swizzle (16-byte unit ^ ((row / 2) % 4))
-            cp_async16(kst + 4 * kChunkBytes + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4),
+            cp_async16(kst + kQLatent + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4),
                        kvb + (size_t)ri * pitch + 512 + 16 * (lane & 3));
           }
-          cp_async_mbar_arrive_noinc(&ms.k_land[s]);
-          cur_next(ck);
-          if (ck.tile < p.ng) kidx = load_idx(ck);
-          did = true;
-        }
-      }
-      if (cv.tile < p.ng) {
-        const int kb = cv.kb0 + cv.k;
-        const int s = kb & 1;
-        const uint32_t ph = (kb >> 1) & 1;
-        // V stage s was last read by the PV of block kb-2
-        const bool ok = kb < 2 || mbar_test(&ms.pv_done[s], ph ^ 1);
-        if (__all_sync(0xffffffffu, ok)) {
-          const uint32_t vst = sbase + kOffV + s * kVStage;
-          // lane: row 16pw + 2i + lane/16 of the block's 128 keys, 16-byte piece lane%16 of this
-          // CTA's 256 value bytes
-          const int pc = lane & 15, nbk = pc >> 3, c8 = pc & 7;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rloc = 2 * i + (lane >> 4);
-            const int ri = __shfl_sync(0xffffffffu, vidx, 16 + rloc);
-            const int row = 16 * pw + rloc;
-            cp_async16(vst + nbk * kVChunk + row * 128 + ((c8 ^ (row & 7)) << 4),
-                       kvb + (size_t)ri * pitch + 256 * cta + 16 * pc);
+          cp_async_mbar_arrive_noinc(&ms.k_land[ck.kb & 7]);
+          if (cur_next(ck)) {
+            if (pw == 0 && ck.w < n_items) { q_w = ck.w; q_slot = ck.slot; q_ring = ck.ring; q_pending = true; }
+            advance(ck);
           }
-          cp_async_mbar_arrive_noinc(&ms.v_land[s]);
-          cur_next(cv);
-          if (cv.tile < p.ng) vidx = load_idx(cv);
+          if (ck.w < n_items) kidx = load_idx(ck, own_key);
           did = true;
         }
       }
@@ -557,108 +608,161 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         aborted = __any_sync(0xffffffffu, stop);
       }
     }
-  } else {
+  } else if (warp < kWarpEpi0) {
+   asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
    if (warp == kWarpMma) {
     // ------------------------------------------------------------ MMA issue (leader CTA only)
     if (cta == 0) {   // the whole warp runs this loop; one elected lane issues
       constexpr uint32_t idesc_qk = umma_idesc(0, 0, false, false, 128, 128);
       constexpr uint32_t idesc_pv = umma_idesc(0, 0, false, true, 128, 256);
       const uint32_t a_qk_done0 = smem_u32(&ms.qk_done[0]), a_qk_done0_peer = mapa(a_qk_done0, 1);
-      const uint32_t a_pv_done_peer[2] = {mapa(smem_u32(&ms.pv_done[0]), 1), mapa(smem_u32(&ms.pv_done[1]), 1)};
+      const uint32_t a_pv_done0 = smem_u32(&ms.pv_done[0]), a_pv_done0_peer = mapa(a_pv_done0, 1);
+      const uint32_t a_slot_free0 = smem_u32(&ms.slot_free[0]), a_slot_free0_peer = mapa(a_slot_free0, 1);
       const uint32_t a_q_free_peer = mapa(smem_u32(&ms.q_free), 1);
       // S = Q K^T of block kb into S buffer kb%2
-      // The K / V tiles were written by cp.async (generic proxy) and are read by the tensor core
-      // through the async proxy: a cross-proxy fence sits between "landed" and the MMA.
+      // (the K / V rows were written by cp.async (generic proxy) and are read by the tensor core
+      // through the async proxy: a cross-proxy fence sits between "landed" and the MMA)
       // descriptor high words: 128-byte swizzle (8-row groups 1024 B apart) for the four latent
       // chunks, 64-byte swizzle (8-row groups 512 B apart) for the compact rope chunk
       const uint32_t hi128 = (uint32_t)(umma_desc(0, 16, 1024, kSwz128) >> 32);
       const uint32_t hi64 = (uint32_t)(umma_desc(0, 16, 512, kSwz64) >> 32);
-      auto issue_qk = [&](int k, int kb, const BlockIdx& bi) {
+      const uint32_t a_rope_lo = (uint32_t)umma_desc(sbase + kOffRope, 16, 512, kSwz64);
+      auto issue_qk = [&](int kb, int slot) {
         fence_proxy_async_smem();
         tc_fence_after();
         const uint32_t d = tmem + ((kb & 1) ? kTmemS1 : kTmemS0);
-        const uint32_t a_rope_lo = (uint32_t)umma_desc(sbase + kOffQ + 4 * kChunkBytes, 16, 512, kSwz64);
-        const uint32_t b_lo = (uint32_t)umma_desc(sbase + kOffK + bi.ks * kKStage, 16, 1024, kSwz128);
+        const uint32_t b_lo = (uint32_t)umma_desc(sbase + kOffKV + slot * kStageKV, 16, 1024, kSwz128);
         mma_f8_pair_qk18(d, idesc_qk, tmem + kTmemQ, b_lo, hi128, hi64, a_rope_lo);
-        mma_commit_pair_elect(a_qk_done0 + 8u * (uint32_t)bi.b6);
-        mma_commit_pair_elect(a_qk_done0_peer + 8u * (uint32_t)bi.b6);
+        mma_commit_pair_elect(a_qk_done0 + 8u * (uint32_t)(kb & 7));
+        mma_commit_pair_elect(a_qk_done0_peer + 8u * (uint32_t)(kb & 7));
       };
-      auto issue_pv = [&](int k, int kb) {
-        const int s = kb & 1;
+      auto issue_pv = [&](int k, int kb, int slot) {
         fence_proxy_async_smem();
         tc_fence_after();
-        const uint64_t ad = umma_desc(sbase + kOffP + (kPBufs == 2 ? s : 0) * kPBytes, 1024, 128, kSwzNone);
-        const uint64_t bd = umma_desc(sbase + kOffV + s * kVStage, kVChunk, 1024, kSwz128);
+        const uint64_t ad = umma_desc(sbase + kOffP + (kb & 1) * kPBytes, 1024, 128, kSwzNone);
+        const uint64_t bd = umma_desc(sbase + kOffKV + slot * kStageKV, kChunkBytes, 1024, kSwz128);
         mma_f8_pair_pv8(tmem + kTmemO, idesc_pv, (uint32_t)ad, (uint32_t)bd, (uint32_t)(ad >> 32),
                         (uint32_t)(bd >> 32), k ? 1u : 0u);
-        mma_commit_pair_elect(smem_u32(&ms.pv_done[s]));
-        mma_commit_pair_elect(a_pv_done_peer[s]);
+        mma_commit_pair_elect(a_slot_free0 + 8u * (uint32_t)slot);
+        mma_commit_pair_elect(a_slot_free0_peer + 8u * (uint32_t)slot);
+        mma_commit_pair_elect(a_pv_done0 + 8u * (uint32_t)(kb & 3));
+        mma_commit_pair_elect(a_pv_done0_peer + 8u * (uint32_t)(kb & 3));
       };
-      int kb0 = 0, it = 0;
+      // Ready-driven issue over two cursors: whichever of "next QK^T" (its K rows landed on both
+      // CTAs, its S buffer drained and, for an item's first block, its Q in place) and "next PV" (its
+      // P written, its V rows landed on both CTAs and, for an item's first PV, the previous item's O
+      // read out) is ready goes first.  QK^T runs into the next item while this item's last PVs are
+      // still waiting for their P, but not further: Q(it + 2) is brought in only after epilogue it.
+      struct Cursor { int w, k, nb, it, kb, slot; };
+      auto next = [&](Cursor& c) {
+        ++c.kb;
+        if (++c.slot == kSlots) c.slot = 0;
+        if (++c.k == c.nb) {
+          c.w += ncl; c.k = 0; ++c.it;
+          if (++c.slot == kSlots) c.slot = 0;
+          c.nb = c.w < n_items ? item_of(c.w).nb : 0;
+        }
+      };
+      Cursor q{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, 1}, v = q;
       bool aborted = false;
-      for (int tile = cid; tile < p.ng && !aborted; tile += ncl, ++it) {
-        const int nb = blocks_of(tile_count(tile));
-        mbar_wait(&ms.qt_ready, it & 1, wt, kSiteQ, it);
-        __syncwarp();
-        // Ready-driven issue: whichever of "next QK" (its K stage landed on both CTAs and its S
-        // buffer drained) and "next PV" (its P written, its V stage landed on both CTAs, and for
-        // the tile's first PV the previous tile's O read out) is ready goes first.
-        int qk_i = 0, pv_i = 0;
-        unsigned long long idle_since = 0;
-        unsigned idle_iters = 0;
-        while (pv_i < nb && !aborted) {
-          bool did = false;
-          {
-            const int kb = kb0 + pv_i;
-            const int s = kb & 1;
-            const uint32_t ph = (kb >> 1) & 1;
-            // lanes poll independently: act only on what every lane has seen (keeps the warp converged)
-            const bool ok = pv_i < qk_i && mbar_test(&ms.p_ready[s], ph) && mbar_test(&ms.v_land[s], ph) &&
-                            mbar_test(&ms.v_peer[s], ph) &&
-                            (pv_i > 0 || it == 0 || mbar_test(&ms.o_free, (it - 1) & 1));
-            if (__all_sync(0xffffffffu, ok)) {
-              issue_pv(pv_i, kb);
-              ++pv_i;
-              did = true;
-            }
-          }
-          if (qk_i < nb) {
-            const int kb = kb0 + qk_i;
-            const BlockIdx bi(kb);
-            const int s = kb & 1;
-            const uint32_t ph = (kb >> 1) & 1;
-            const bool ok = mbar_test(&ms.k_land[bi.ks], bi.kph) && mbar_test(&ms.k_peer[bi.ks], bi.kph) &&
-                            (kb < 2 || mbar_test(&ms.s_free[s], ph ^ 1));
-            if (__all_sync(0xffffffffu, ok)) {
-              issue_qk(qk_i, kb, bi);
-              ++qk_i;
-              if (qk_i == nb) {      // the Q tile is no longer needed once these MMAs complete
-                mma_commit_pair_elect(smem_u32(&ms.q_free));
-                mma_commit_pair_elect(a_q_free_peer);
-              }
-              did = true;
-            }
-          }
-          if (did) {
-            idle_since = 0;
-            idle_iters = 0;
-          } else if ((++idle_iters & (kIdleCheckEvery - 1)) != 0) {
-            __nanosleep(kIdleSleepNs);
-          } else {
-            const unsigned long long now = globaltimer_ns();
-            if (idle_since == 0) idle_since = now;
-            bool stop = wt.aborting();
-            if (now - idle_since > wt.limit_ns) {
-              if (lane == 0) wt.fail(kSiteMmaIdle, pv_i);
-              stop = true;
-            }
-            aborted = __any_sync(0xffffffffu, stop);
+      unsigned long long idle_since = 0;
+      unsigned idle_iters = 0;
+      while (v.w < n_items && !aborted) {
+        bool did = false;
+        {
+          const uint32_t ph = (v.kb >> 3) & 1;
+          // lanes poll independently: act only on what every lane has seen (keeps the warp converged)
+          const bool ok = v.kb < q.kb && mbar_test(&ms.p_ready[v.kb & 1], (v.kb >> 1) & 1) &&
+                          mbar_test(&ms.v_land[v.kb & 7], ph) && mbar_test(&ms.v_peer[v.kb & 7], ph) &&
+                          (v.k > 0 || v.it == 0 || mbar_test(&ms.o_free, (v.it - 1) & 1));
+          if (__all_sync(0xffffffffu, ok)) {
+            issue_pv(v.k, v.kb, v.slot);
+            next(v);
+            did = true;
           }
         }
-        kb0 += nb;
+        if (q.w < n_items && q.it - v.it <= 1) {
+          const uint32_t ph = (q.kb >> 3) & 1;
+          const bool ok = mbar_test(&ms.k_land[q.kb & 7], ph) && mbar_test(&ms.k_peer[q.kb & 7], ph) &&
+                          (q.kb < 2 || mbar_test(&ms.s_free[q.kb & 1], ((q.kb >> 1) & 1) ^ 1)) &&
+                          (q.k > 0 || mbar_test(&ms.qt_ready, q.it & 1));
+          if (__all_sync(0xffffffffu, ok)) {
+            issue_qk(q.kb, q.slot);
+            if (q.k == q.nb - 1) {      // Q is no longer needed once these MMAs complete
+              mma_commit_pair_elect(smem_u32(&ms.q_free));
+              mma_commit_pair_elect(a_q_free_peer);
+            }
+            next(q);
+            did = true;
+          }
+        }
+        if (did) {
+          idle_since = 0;
+          idle_iters = 0;
+        } else if ((++idle_iters & (kIdleCheckEvery - 1)) != 0) {
+          __nanosleep(kIdleSleepNs);
+        } else {
+          const unsigned long long now = globaltimer_ns();
+          if (idle_since == 0) idle_since = now;
+          bool stop = wt.aborting();
+          if (now - idle_since > wt.limit_ns) {
+            if (lane == 0) wt.fail(kSiteMmaIdle, v.kb);
+            stop = true;
+          }
+          aborted = __any_sync(0xffffffffu, stop);
+        }
       }
     }
-  } else if (warp >= kWarpEpi0) {
+  } else if (warp == kWarpRelayK || warp == kWarpRelayV) {
+    // ------------------------------------------------------------ "landed" relays to the leader CTA
+    // The MMA thread lives in the leader CTA and can only wait on its own barriers: in the
+    // peer CTA these warps forward "K rows landed" and "V rows landed".
+    if (cta == 1) {
+      const bool is_k = warp == kWarpRelayK;
+      const uint32_t a_peer0 = mapa(smem_u32(is_k ? &ms.k_peer[0] : &ms.v_peer[0]), 0);
+      int kb = 0;
+      for (int w = cid; w < n_items; w += ncl) {
+        const int nb = item_of(w).nb;
+        for (int k = 0; k < nb; ++k, ++kb) {
+          const int s = kb & 7;
+          mbar_wait(is_k ? &ms.k_land[s] : &ms.v_land[s], (kb >> 3) & 1, wt, is_k ? kSiteRelayK : kSiteRelayV, k);
+          fence_proxy_async_smem();     // this CTA's cp.async writes -> the leader's MMA reads
+          if (lane == 0) mbar_arrive_cluster_release(a_peer0 + 8u * (uint32_t)s);
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ index-validity bits (warp kWarpValid)
+    static_assert(kWarpValid == kWarpRelayV + 1 && kWarpValid + 1 == kWarpEpi0, "role layout");
+    int kb = 0;
+    for (int w = cid; w < n_items; w += ncl) {
+      const Item item = item_of(w);
+      const int32_t* idx_row = p.indices + (size_t)item.tile * p.idx_stride + (size_t)item.k0 * kBlockKeys;
+      int4 cur = __ldcs(reinterpret_cast<const int4*>(idx_row) + lane);
+      for (int k = 0; k < item.nb; ++k, ++kb) {
+        const int s = kb & 1;
+        const uint32_t ph = (kb >> 1) & 1;
+        int4 nxt = cur;
+        if (k + 1 < item.nb) nxt = __ldcs(reinterpret_cast<const int4*>(idx_row + (size_t)(k + 1) * kBlockKeys) + lane);
+        const int rank0 = (item.k0 + k) * kBlockKeys + lane * 4;
+        auto ok = [&](int idx, int rk) -> uint32_t {
+          return (idx >= 0 && idx < p.s_kv && rk < item.lim) ? 1u : 0u;
+        };
+        const uint32_t nib = ok(cur.x, rank0) | (ok(cur.y, rank0 + 1) << 1) |
+                             (ok(cur.z, rank0 + 2) << 2) | (ok(cur.w, rank0 + 3) << 3);
+        if (kb >= 2) mbar_wait(&ms.valid_free[s], ph ^ 1, wt, kSiteValidFree, k);
+        __syncwarp();
+        const uint32_t nib_hi = __shfl_down_sync(0xffffffffu, nib, 1);
+        if ((lane & 1) == 0)
+          reinterpret_cast<uint8_t*>(&ms.valid[s][0])[lane >> 1] = (uint8_t)(nib | (nib_hi << 4));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ms.valid_ready[s]);
+        cur = nxt;
+      }
+    }
+   }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 72;");
     // ------------------------------------------------------------ epilogue warps
     // O out of TMEM, x out_scale / l, bf16, TMA tile stores -- while the softmax warps already
     // work on the next tile.  A warp reads the TMEM lanes of its quarter (warp % 4): rows r of
@@ -666,72 +770,139 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     // box of 32 rows x 128 bytes in the warp's 4 KB slice (128-byte swizzle: the 16-byte stores
     // of eight consecutive rows hit distinct banks) and one lane hands the box to TMA:
     // full-line asynchronous writes, no barrier wider than the warp.
-    const int ew = warp - kWarpEpi0;
+    const int ew = warp - kWarpEpi0, e_tid = (int)threadIdx.x - 32 * kWarpEpi0;
     const int e_tl = ((warp & 3) << 5) | lane, e_r = e_tl & 63, e_h = e_tl >> 6;
     const uint32_t e_ocol = tmem + ((uint32_t)((warp & 3) * 32) << 16) + kTmemO;
     const uint32_t a_o_free = mapa(smem_u32(&ms.o_free), 0);
     const uint32_t a_qt_ready = mapa(smem_u32(&ms.qt_ready), 0);
     const uint64_t pol_stream = l2_policy_evict_first();
-    // These warps also move the latent part of every Q tile from shared memory (where TMA put
-    // it) into tensor memory, where the QK^T MMAs read it: lane = row (e_r, duplicated in lanes
-    // 64-127 as the 64-rows-per-CTA form of the instruction wants), chunk j -> 32 columns.  The
-    // tile's Q lands when the previous tile's last QK^T has completed, i.e. shortly before that
-    // tile's epilogue starts: transfer Q(t + 1), then write out O(t).
-    auto transfer_q = [&](int q_it) {
-      mbar_wait(&ms.q_land, q_it & 1, wt, kSiteQ, q_it);
-      __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
-      const uint8_t* qrow = sm + kOffQ + e_r * 128;
+    // These warps also bring the Q tiles in: from the ring slot where TMA has put the item's 64 rows
+    // -- or, bf16 q, where fill_q puts them: loaded, quantised and stored in the same swizzled layout
+    // by these 128 threads (one pass over q instead of the quantise kernel's read and write and this
+    // kernel's read) -- transfer_q moves the latent part into tensor memory, where the QK^T MMAs read
+    // it: lane = row (e_r, duplicated in lanes 64-127 as the 64-rows-per-CTA form of the
+    // instruction wants), chunk j -> 32 columns, and the rope chunk into its fixed buffer.  Order:
+    // move Q(t + 1) once item t's last QK^T is complete, then write out O(t).
+    auto fill_q = [&](int w, int j, int n) {
+      mbar_wait(&ms.q_land, j & 1, wt, kSiteQ, j);         // the slot is ours
+      __syncwarp();
+      const int qtile = item_of(w).tile / p.q_group_div;
+      const uint32_t qoff = kOffKV + (uint32_t)(n % kSlots) * kStageKV, rope = qoff + kQLatent;
+      {
+        const uint4* src = p.q_bf16 + ((size_t)qtile * 128 + 64 * cta) * (kDQK / 8);
 #pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
+        for (int i = 0; i < 18; i += 3) {      // 64 rows x 36 units of 16 codes = 18 units per thread
+          uint4 a[3], b[3];
+#pragma unroll
+          for (int u = 0; u < 3; ++u) {
+            const int unit = (i + u) * 128 + e_tid;
+            a[u] = __ldcs(src + 2 * unit);
+            b[u] = __ldcs(src + 2 * unit + 1);
+          }
+#pragma unroll
+          for (int u = 0; u < 3; ++u) {
+            const int unit = (i + u) * 128 + e_tid, row = unit / 36, c = unit - 36 * row;
+            const uint4 v = make_uint4(e4m3x4_of_bf16(a[u].x, a[u].y, p.q_inv), e4m3x4_of_bf16(a[u].z, a[u].w, p.q_inv),
+                                       e4m3x4_of_bf16(b[u].x, b[u].y, p.q_inv), e4m3x4_of_bf16(b[u].z, b[u].w, p.q_inv));
+            const uint32_t off = c < 32 ? qoff + (c >> 3) * kChunkBytes + row * 128 + (((c & 7) ^ (row & 7)) << 4)
+                                        : rope + row * 64 + (((c - 32) ^ ((row >> 1) & 3)) << 4);
+            *reinterpret_cast<uint4*>(sm + off) = v;
+          }
+        }
+        asm volatile("bar.sync 4, 128;" ::: "memory");
+      }
+    };
+    auto transfer_q = [&](int j, int n) {
+      if (j > 0) mbar_wait(&ms.q_free, (j - 1) & 1, wt, kSiteQFree, j);
+      if (p.q_bf16 == nullptr) mbar_wait(&ms.q_land, j & 1, wt, kSiteQ, j);
+      __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
+      tc_fence_after();
+      const int slot = n % kSlots;
+      const uint8_t* qtile = sm + kOffKV + slot * kStageKV;
+      const uint8_t* qrow = qtile + e_r * 128;
+      {                              // rope chunk: 4 KB, 32 bytes per thread
+        const uint4* src = reinterpret_cast<const uint4*>(qtile + kQLatent) + 2 * e_tid;
+        uint4* dst = reinterpret_cast<uint4*>(sm + kOffRope) + 2 * e_tid;
+        dst[0] = src[0];
+        dst[1] = src[1];
+      }
+#pragma unroll 1
+      for (int j4 = 0; j4 < 4; ++j4) {
         uint32_t v[32];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const uint4 t = *reinterpret_cast<const uint4*>(qrow + j * kChunkBytes + ((u ^ (e_r & 7)) << 4));
+          const uint4 t = *reinterpret_cast<const uint4*>(qrow + j4 * kChunkBytes + ((u ^ (e_r & 7)) << 4));
           v[4 * u] = t.x; v[4 * u + 1] = t.y; v[4 * u + 2] = t.z; v[4 * u + 3] = t.w;
         }
-        tmem_st32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + kTmemQ + 32 * j, reinterpret_cast<const float*>(v));
+        tmem_st32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + kTmemQ + 32 * j4, reinterpret_cast<const float*>(v));
       }
       tmem_wait_st();
       tc_fence_before();
-      fence_proxy_async_smem();      // these reads are ordered before the next TMA write of the tile
+      fence_proxy_async_smem();      // rope -> the MMAs' reads; these reads -> the slot's next TMA write
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(a_qt_ready);
+      asm volatile("bar.sync 4, 128;" ::: "memory");      // all four warps have read the slot
+      if (e_tid == 0) mbar_arrive(&ms.slot_free[slot]);
     };
     int kb0 = 0, it = 0;
-    if (cid < p.ng) transfer_q(0);
-    for (int tile = cid; tile < p.ng; tile += ncl, ++it) {
-      const int nb = blocks_of(tile_count(tile));
-      const int kbl = kb0 + nb - 1;                // last block of the tile
-      if (tile + ncl < p.ng) transfer_q(it + 1);
-      // the row scales are published and the tile's last PV has completed
+    if (cid < n_items) {
+      if (p.q_bf16 != nullptr) fill_q(cid, 0, 0);
+      transfer_q(0, 0);
+    }
+    for (int w = cid; w < n_items; w += ncl, ++it) {
+      const Item item = item_of(w);
+      const int tile = item.tile;
+      const int kbl = kb0 + item.nb - 1;           // last block of the item
+      if (w + ncl < n_items) {
+        const int n = kb0 + item.nb + it + 1;      // entry number of the next item's Q
+        if (p.q_bf16 != nullptr) fill_q(w + ncl, it + 1, n);
+        transfer_q(it + 1, n);
+      }
+      // the row scales are published and the item's last PV has completed
       mbar_wait(&ms.epi_ready, it & 1, wt, kSiteEpi, it);
-      mbar_wait(&ms.pv_done[kbl & 1], (kbl >> 1) & 1, wt, kSiteEpi, nb);
+      mbar_wait(&ms.pv_done[kbl & 3], (kbl >> 2) & 1, wt, kSiteEpi, item.nb);
       __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
       tc_fence_after();
+      if (p.nsplit > 1) {
+        // a slice: unnormalised fp32 O straight to its slot (few slices exist, all of them in L2)
+        float4* dst = reinterpret_cast<float4*>(p.part_o + ((size_t)w * 128 + 64 * cta + e_r) * kDV + 256 * e_h);
+        float o[32];
+#pragma unroll 1
+        for (int cc = 0; cc < 8; ++cc) {
+          tmem_ld32(e_ocol + cc * 32, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) dst[cc * 8 + j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(a_o_free);
+        kb0 += item.nb;
+        continue;
+      }
       const float oscale = ms.oscale[it & 1][e_r];
       const uint32_t emask = oscale != 0.f ? 0xffffffffu : 0u;
       // this warp's 32 rows of the tile = (token, head) pairs starting at row r0
       const int r0 = (int)cta * 64 + 32 * (warp & 1);
       const int out_head = r0 % p.h_per_q, out_tok = tile * p.G + r0 / p.h_per_q;
-      float ob[2][32];
-      tmem_ld32(e_ocol, ob[0]);
-#pragma unroll
+      float o[32];
+      tmem_ld32(e_ocol, o);
+#pragma unroll 1
       for (int cc = 0; cc < 8; ++cc) {
-        float* o = ob[cc & 1];
         tmem_wait_ld();
-        if (cc < 7) {
-          tmem_ld32(e_ocol + (cc + 1) * 32, ob[(cc + 1) & 1]);
-        } else {
-          // O has been read: the next tile's first PV may overwrite it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(a_o_free);
-        }
-        uint32_t w[16];
+        uint32_t wv[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           __nv_bfloat162 v2 = __floats2bfloat162_rn(o[2 * j] * oscale, o[2 * j + 1] * oscale);
-          w[j] = *reinterpret_cast<uint32_t*>(&v2) & emask;    // rows without a valid key: zeros
+          wv[j] = *reinterpret_cast<uint32_t*>(&v2) & emask;    // rows without a valid key: zeros
+        }
+        if (cc < 7) {
+          tmem_ld32(e_ocol + (cc + 1) * 32, o);
+        } else {
+          // O has been read: the next item's first PV may overwrite it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(a_o_free);
         }
         {
           // two rounds make one box of 32 rows x 128 bytes (128-byte swizzle) in the warp's 4 KB
@@ -745,7 +916,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             *reinterpret_cast<uint4*>(st_row + (((4 * (cc & 1) + j) ^ (e_r & 7)) << 4)) =
-                make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                make_uint4(wv[4 * j], wv[4 * j + 1], wv[4 * j + 2], wv[4 * j + 3]);
           if (cc & 1) {
             fence_proxy_async_smem();
             __syncwarp();
@@ -757,64 +928,10 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
           }
         }
       }
-      kb0 += nb;
+      kb0 += item.nb;
     }
     if (lane == 0) bulk_wait_all();   // output boxes written before the CTA retires
     tc_fence_before();
-  } else if (warp == kWarpCopy || warp == kWarpRelay) {
-    // ------------------------------------------------------------ "landed" relays to the leader CTA
-    // The MMA thread lives in the leader CTA and can only wait on its own barriers: in the
-    // peer CTA warp 17 forwards "K tile landed" and warp 18 "V tile landed".
-    if (cta == 1) {
-      const bool is_k = warp == kWarpCopy;
-      const uint32_t a_peer0 = mapa(smem_u32(is_k ? &ms.k_peer[0] : &ms.v_peer[0]), 0);
-      int kb0 = 0;
-      for (int tile = cid; tile < p.ng; tile += ncl) {
-        const int nb = blocks_of(tile_count(tile));
-        for (int k = 0; k < nb; ++k) {
-          const int kb = kb0 + k;
-          const BlockIdx bi(kb);
-          const int s = is_k ? bi.ks : (kb & 1);
-          const uint32_t ph = is_k ? (uint32_t)bi.kph : (uint32_t)((kb >> 1) & 1);
-          mbar_wait(is_k ? &ms.k_land[s] : &ms.v_land[s], ph, wt, is_k ? kSiteRelayK : kSiteRelayV, k);
-          fence_proxy_async_smem();     // this CTA's cp.async writes -> the leader's MMA reads
-          if (lane == 0) mbar_arrive_cluster_release(a_peer0 + 8u * (uint32_t)s);
-        }
-        kb0 += nb;
-      }
-    }
-  } else {
-    // ------------------------------------------------------------ index-validity bits (warp kWarpValid)
-    static_assert(kWarpValid == kWarpRelay + 1 && kWarpValid + 1 == kWarpEpi0, "role layout");
-    int kb0 = 0;
-    for (int tile = cid; tile < p.ng; tile += ncl) {
-      const int count = tile_count(tile);
-      const int nb = blocks_of(count);
-      const int32_t* idx_row = p.indices + (size_t)tile * p.idx_stride;
-      int4 cur = __ldcs(reinterpret_cast<const int4*>(idx_row) + lane);
-      for (int k = 0; k < nb; ++k) {
-        const int kb = kb0 + k;
-        const int s = kb & 1;
-        const uint32_t ph = (kb >> 1) & 1;
-        int4 nxt = cur;
-        if (k + 1 < nb) nxt = __ldcs(reinterpret_cast<const int4*>(idx_row + (size_t)(k + 1) * kBlockKeys) + lane);
-        const int rank0 = k * kBlockKeys + lane * 4;
-        auto ok = [&](int idx, int rk) -> uint32_t {
-          return (idx >= 0 && idx < p.s_kv && rk < count) ? 1u : 0u;
-        };
-        const uint32_t nib = ok(cur.x, rank0) | (ok(cur.y, rank0 + 1) << 1) |
-                             (ok(cur.z, rank0 + 2) << 2) | (ok(cur.w, rank0 + 3) << 3);
-        if (kb >= 2) mbar_wait(&ms.valid_free[s], ph ^ 1, wt, kSiteValidFree, k);
-        const uint32_t nib_hi = __shfl_down_sync(0xffffffffu, nib, 1);
-        if ((lane & 1) == 0)
-          reinterpret_cast<uint8_t*>(&ms.valid[s][0])[lane >> 1] = (uint8_t)(nib | (nib_hi << 4));
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ms.valid_ready[s]);
-        cur = nxt;
-      }
-      kb0 += nb;
-    }
-  }
   }
 
   // tear-down: nobody may still be reading TMEM of either CTA when it is released
@@ -854,7 +971,7 @@ static int launch_fp8_t(const CUtensorMap& map_q, const CUtensorMap& map_q_rope,
   auto kern = masked_mla_fp8_kernel;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::kSmem) != cudaSuccess)
     return LITEDSA_ERR_CUDA;
-  kern<<<2 * min(p.ng, max_clusters()), kAttnThreads, PL::kSmem, stream>>>(
+  kern<<<2 * min(p.ng * p.nsplit, max_clusters()), kAttnThreads, PL::kSmem, stream>>>(
       map_q, map_q_rope, omaps, p);
   return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
 }
@@ -881,7 +998,9 @@ static int launch_fp8(const Fp8Args& a, void* const* outs, int n_out, cudaStream
   // Q per CTA: four boxes of 128 bytes x 64 rows (128-byte swizzle) and the rope box of 64 bytes
   // x 64 rows (64-byte swizzle)
   const uint32_t qb_h = (uint32_t)min(h, 64);
-  if (!make_map_3d(&map_q, a.q8, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, (uint64_t)h,
+  if (a.q_is_bf16) {
+    map_q = map_q_rope = omaps.m[0];       // not used by the kernel
+  } else if (!make_map_3d(&map_q, a.q8, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, (uint64_t)h,
                    (uint64_t)(a.ng / qdiv) * G, q_hs, q_ts, 128, qb_h, 64 / qb_h) ||
       !make_map_3d(&map_q_rope, a.q8, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, (uint64_t)h,
                    (uint64_t)(a.ng / qdiv) * G, q_hs, q_ts, 64, qb_h, 64 / qb_h, CU_TENSOR_MAP_SWIZZLE_64B))
@@ -896,6 +1015,8 @@ static int launch_fp8(const Fp8Args& a, void* const* outs, int n_out, cudaStream
   p.idx_stride = a.indices_row_stride;
   p.scale_log2 = a.sm_scale * kLog2e; p.out_scale = a.out_scale;
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
+  p.q_bf16 = a.q_is_bf16 ? reinterpret_cast<const uint4*>(a.q8) : nullptr; p.q_inv = a.q_inv;
+  p.nsplit = a.nsplit; p.part_o = a.part_o; p.part_ml = reinterpret_cast<float2*>(a.part_ml);
   return launch_fp8_t(map_q, map_q_rope, omaps, p, stream);
 }
 

@@ -42,6 +42,14 @@ struct Fp8Args {
   // in-place ("zero-copy") addressing of q and out inside [T, H_padded, d] tensors that hold
   // h_per_q real heads per token: strides in ELEMENTS, 0 = the dense packed layout
   int64_t q_token_stride, q_head_stride, out_token_stride, out_head_stride;
+  // sparse_prefill only: q is bf16 (dense packed) and quantised by the kernel as e4m3(q * q_inv);
+  // nsplit > 1: every tile's blocks are cut into nsplit slices whose fp32 results go to part_o
+  // [ng * nsplit, 128, 512] / part_ml [ng * nsplit, 128] and are merged by a second launch
+  bool q_is_bf16 = false;
+  float q_inv = 0.f;
+  int nsplit = 1;
+  float* part_o = nullptr;
+  void* part_ml = nullptr;
 };
 int check_fp8_args(const Fp8Args& a);                                   // no CUDA call
 // attn_dsv4.cu: classify the tiles' index lists and enqueue the range kernel in rank mode, gated on
@@ -162,24 +170,29 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, const Waiter w,
-                                                   int site, int iter) {
-  const unsigned long long t0 = globaltimer_ns();
-  for (;;) {
-    for (int i = 0; i < 256; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
+// (One inlined loop and no call: a kernel that redistributes its registers with setmaxnreg cannot
+// contain calls.)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const Waiter& w, int site,
+                                          int iter = 0) {
+  unsigned long long t0 = 0;
+  for (uint32_t n = 1; !mbar_try_wait(bar, parity); ++n) {
+    if ((n & 255u) != 0) continue;
     if (w.aborting()) return false;
-    if (globaltimer_ns() - t0 > w.limit_ns) {
+    const unsigned long long now = globaltimer_ns();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > w.limit_ns) {
       w.fail(site, iter);
       return false;
     }
   }
+  return true;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const Waiter& w, int site,
-                                          int iter = 0) {
-  for (int i = 0; i < 64; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, w, site, iter);
+
+// the same for a whole converged warp whose further way depends on the result: all lanes get the
+// same answer
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const Waiter& w, int site,
+                                               int iter = 0) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, w, site, iter));
 }
 
 // release at cluster scope: orders this thread's earlier (distributed) shared-memory stores
@@ -403,8 +416,9 @@ __device__ __forceinline__ void mma_f8_pair_qk18(uint32_t d_tmem, uint32_t idesc
       ::"r"(d_tmem), "r"(idesc), "r"(q_tmem), "r"(b_lo), "r"(hi128), "r"(hi64), "r"(a_rope_lo)
       : "memory");
 }
-//   P V of one 128-key block: two N = 256 halves (D column offset 128, V chunk +1024) x four
-//   32-key steps (P +128, V +256 per step); `first` = 0 zeroes the accumulator in step 0
+//   P V of one 128-key block: two N = 256 halves (D column offset 128, V chunk +512) x four
+//   32-key steps (P +128; V: keys 0-63 in chunks 0-1, keys 64-127 in chunks 2-3 of 64 keys x 128
+//   bytes each, +256 per step inside a chunk); accumulate_first = 0 zeroes the accumulator in step 0
 #define LT_PV_STEP(DOFF, AINC, BINC, PRED)                              \
   "add.u32 dd, %0, " #DOFF ";\n\tadd.u32 alo, %2, " #AINC ";\n\tadd.u32 blo, %3, " #BINC ";\n\t" \
   "mov.b64 ad, {alo, %4};\n\tmov.b64 bd, {blo, %5};\n\t"                  \
@@ -415,9 +429,9 @@ __device__ __forceinline__ void mma_f8_pair_pv8(uint32_t d_tmem, uint32_t idesc,
   asm volatile(
       "{\n\t.reg .pred pf, po, pe;\n\t.reg .b32 alo, blo, dd;\n\t.reg .b64 ad, bd;\n\t"
       "setp.ne.b32 pf, %6, 0;\n\tsetp.eq.b32 po, 0, 0;\n\telect.sync _|pe, 0xffffffff;\n\t"
-      LT_PV_STEP(0, 0, 0, pf) LT_PV_STEP(0, 128, 256, po) LT_PV_STEP(0, 256, 512, po)
-      LT_PV_STEP(0, 384, 768, po)
-      LT_PV_STEP(128, 0, 1024, pf) LT_PV_STEP(128, 128, 1280, po) LT_PV_STEP(128, 256, 1536, po)
+      LT_PV_STEP(0, 0, 0, pf) LT_PV_STEP(0, 128, 256, po) LT_PV_STEP(0, 256, 1024, po)
+      LT_PV_STEP(0, 384, 1280, po)
+      LT_PV_STEP(128, 0, 512, pf) LT_PV_STEP(128, 128, 768, po) LT_PV_STEP(128, 256, 1536, po)
       LT_PV_STEP(128, 384, 1792, po)
       "}"
       ::"r"(d_tmem), "r"(idesc), "r"(a_lo), "r"(b_lo), "r"(a_hi), "r"(b_hi), "r"(accumulate_first)
