@@ -52,7 +52,9 @@ const char* litedsa_error_string(int code);
  * G*cap/32 <= 16384, 0 < seq_space <= 2^20 and a multiple of 1024.  Additionally
  * k % 4 == 0.
  * fill_tail == 0: words beyond the live prefixes are left untouched (the reference's
- * overwrite contract, litedsa_union.cuh:22-25); != 0: u_phys tail := -1, mask tail := 0.
+ * overwrite contract, litedsa_union.cuh:22-25); 2: u_phys := -1 from the live prefix to the next
+ * multiple of 128 entries (what the attention reads); any other value: u_phys tail := -1, mask
+ * tail := 0.
  */
 int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts,
                      uint32_t* memb_qm, const int32_t* req_pg, const int32_t* block_table,
@@ -114,6 +116,38 @@ int litedsa_masked_mla_fp8_ex(const void* q8, const void* kv8, const int32_t* in
                               const float* attn_sink, const int32_t* topk_length_per_q,
                               int q_group_div, int64_t q_token_stride, int64_t q_head_stride,
                               int64_t out_token_stride, int64_t out_head_stride, void* stream);
+
+/*
+ * litedsa_masked_mla_fp8 on bf16 queries [ng, 128, 576] (dense packed), quantised on their way into
+ * the kernel as e4m3(q / q_scale) -- the codes litedsa_quantize_e4m3 would give, without its pass
+ * over memory.  sm_scale includes q_scale and the cache's scale, as with e4m3 queries.
+ */
+int litedsa_masked_mla_fp8_bf16q(const void* q_bf16, float q_scale, const void* kv8,
+                                 const int32_t* indices, float sm_scale, float out_scale,
+                                 const int32_t* topk_length, const uint32_t* memb_qm, int h_per_q,
+                                 void* out, float* max_logits, float* lse, int ng, int s_kv, int topk,
+                                 int64_t kv_row_stride, int64_t indices_row_stride, void* stream);
+
+/*
+ * The whole path of one chunk of query tokens in one call: union_qm of the tiles' top-k lists and
+ * the masked attention over it (no counterpart in the reference, whose callers chain its operators).
+ *   q        [T, h, 576] dense: e4m3 codes (q_is_bf16 == 0) or bf16 (quantised with q_scale when kv is
+ *            FP8);  kv [s_kv, kv_row_stride] e4m3 codes with the scalar scale kv_scale
+ *            (kv_is_bf16 == 0) or bf16 rows (needs bf16 q; scales ignored); kv_row_stride in ELEMENTS
+ *   topk_idx [T, k] int32 (-1 padded), k % 4 == 0, (128 / h) * k % 128 == 0
+ *   sm_scale softmax scale on the unquantised values;  out [T, h, 512] bf16, lse [T, h] fp32
+ *   seq_space bound on the positions (multiple of 1024, <= 2^20)
+ *   policy_tokens >= T: tokens of the whole job.  Small jobs cut their tiles' lists into slices that
+ *            run in parallel and are merged in fp32; how many depends on this number only, so that
+ *            a job done in several calls gives the bits of the job done in one
+ *   workspace  256-byte aligned, litedsa_sparse_prefill_workspace(...) bytes
+ */
+int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
+                           const int32_t* topk_idx, float sm_scale, float q_scale, float kv_scale,
+                           void* out, float* lse, int T, int h, int k, int s_kv, int64_t kv_row_stride,
+                           int64_t seq_space, int policy_tokens, void* workspace,
+                           int64_t workspace_bytes, void* stream);
+int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens);
 
 /*
  * litedsa_masked_mla_fp8 with the all-gather of a query-sharded multi-GPU run folded into
@@ -212,6 +246,21 @@ int litedsa_dsv4_c128a_bf16(const void* q, const void* kv_comp, const void* kv_r
                             int64_t q_row_stride, int64_t kc_row_stride, int64_t kr_row_stride,
                             int64_t q_token_stride, int64_t q_head_stride, int64_t out_token_stride,
                             int64_t out_head_stride, void* stream);
+
+/*
+ * litedsa_dsv4_c128a_bf16 with the sink given per head (sink_len == h_per_q) or per packed row
+ * (sink_len == 128) and with an optional workspace (256-byte aligned).  A call of few tiles whose
+ * workspace has litedsa_dsv4_workspace(...) bytes cuts its tiles' key blocks into slices that run in
+ * parallel and merges them in fp32; without one the result is litedsa_dsv4_c128a_bf16's.
+ */
+int litedsa_dsv4_c128a_bf16_ws(const void* q, const void* kv_comp, const void* kv_raw, int ng, int h_per_q,
+                               int n_comp, int s_raw, int pos0, int window, int ratio, float sm_scale,
+                               const float* attn_sink, int sink_len, void* out, float* lse,
+                               int64_t q_row_stride, int64_t kc_row_stride, int64_t kr_row_stride,
+                               int64_t q_token_stride, int64_t q_head_stride, int64_t out_token_stride,
+                               int64_t out_head_stride, void* workspace, int64_t workspace_bytes,
+                               void* stream);
+int64_t litedsa_dsv4_workspace(int ng, int h_per_q, int n_comp, int pos0, int window, int ratio);
 
 /* Status block of the DSv4 kernel; same meaning and use as litedsa_attn_status. */
 int litedsa_dsv4_status(int* out4_host, int reset);

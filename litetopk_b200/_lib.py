@@ -33,6 +33,13 @@ SIGNATURES = {
                                              c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                              c_void_p, c_int, c_int, c_int, c_int64, c_int64,
                                              c_int64, c_void_p]),
+    "litedsa_masked_mla_fp8_bf16q": (c_int, [c_void_p, c_float, c_void_p, c_void_p, c_float, c_float,
+                                             c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                             c_int, c_int, c_int, c_int64, c_int64, c_void_p]),
+    "litedsa_sparse_prefill": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
+                                       c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64,
+                                       c_int64, c_int, c_void_p, c_int64, c_void_p]),
+    "litedsa_sparse_prefill_workspace": (c_int64, [c_int, c_int, c_int, c_int, c_int]),
     "litedsa_attn_status": (c_int, [c_void_p, c_int]),
     "litedsa_set_wait_limit_ns": (c_int, [c_uint64, c_void_p]),
     "litedsa_selftest_wait_timeout": (c_int, [c_uint64, c_void_p]),
@@ -46,6 +53,11 @@ SIGNATURES = {
     "litedsa_dsv4_c128a_bf16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                         c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int64,
                                         c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p]),
+    "litedsa_dsv4_c128a_bf16_ws": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                           c_int, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p, c_int64,
+                                           c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p,
+                                           c_int64, c_void_p]),
+    "litedsa_dsv4_workspace": (c_int64, [c_int, c_int, c_int, c_int, c_int, c_int]),
     "litedsa_dsv4_status": (c_int, [c_void_p, c_int]),
     "litedsa_dsv4_masked_mla_bf16": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                              c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p,

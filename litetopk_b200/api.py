@@ -29,6 +29,21 @@ def _stream(t: torch.Tensor) -> int:
     return torch.cuda.current_stream(t.device).cuda_stream
 
 
+# the current stream's handle without the Stream object around it (1.3 us of host time per call)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or \
+    (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
+def _on_device(dev: torch.device, fn, *args) -> int:
+    """``fn(*args, stream)`` on the current stream of ``dev``, which is made current if it is not."""
+    cur = torch.cuda.current_device()
+    index = cur if dev.index is None else dev.index
+    if index == cur:
+        return fn(*args, _raw_stream(index))
+    with torch.cuda.device(index):
+        return fn(*args, _raw_stream(index))
+
+
 def _need(t: torch.Tensor, name: str, dtype, ndim: Optional[int] = None) -> None:
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
@@ -646,6 +661,35 @@ def prepare_kv(kv_cache_fp8: torch.Tensor, kv_scale: Optional[float] = None,
     return kv
 
 
+def _derived_q_scale(q: torch.Tensor) -> float:
+    """Power-of-two e4m3 scale from max|q| (one device->host read)."""
+    amax = float(q.abs().amax().item())
+    return 2.0 ** max(-24, int(torch.tensor(max(amax, 1e-30) / 448.0).log2().ceil().item()))
+
+
+def _masked_mla_fp8_bf16q(q, q_scale, kv, indices, sm_scale, out_scale, counts, mask, h, out, ml, lse) -> None:
+    """The FP8 operator on contiguous bf16 q [T, h, 576], quantised inside the attention kernel; the
+    other tensors as masked_mla_fp8 has made or checked them."""
+    ng, topk = indices.shape[0], indices.shape[-1]
+    _need(kv, "kv", (torch.float8_e4m3fn, torch.uint8))
+    _need(indices, "indices", torch.int32)
+    _need(mask, "mask", (torch.int32, torch.uint32))
+    _need(counts, "counts", torch.int32, 1)
+    if kv.dim() == 3 and kv.shape[1] == 1:
+        kv = kv[:, 0]
+    if indices.dim() == 3 and indices.shape[1] == 1:
+        indices = indices[:, 0]
+    if kv.dim() != 2 or kv.shape[1] != 576 or kv.stride(1) != 1 or indices.stride(1) != 1 \
+            or ng * 128 != q.shape[0] * h:
+        raise ValueError("kv must be [s_kv,(1,)576] and indices [T*h/128,(1,)topk] with unit inner stride")
+    if mask.numel() != ng * (128 // h) * (topk // 32) or not mask.is_contiguous() \
+            or counts.shape[0] != ng or not counts.is_contiguous():
+        raise ValueError("mask must be a contiguous [ng, G, topk/32] and counts a contiguous [ng]")
+    check(_on_device(q.device, _lib.lib().litedsa_masked_mla_fp8_bf16q, _ptr(q), q_scale, _ptr(kv), _ptr(indices),
+                     sm_scale, out_scale, _ptr(counts), _ptr(mask), h, _ptr(out), _ptr(ml), _ptr(lse), ng,
+                     kv.shape[0], topk, kv.stride(0), indices.stride(0)), "masked_mla_fp8")
+
+
 def masked_mla_fp8(q: torch.Tensor, kv_cache_fp8: torch.Tensor, union_idx: torch.Tensor,
                    mask: torch.Tensor, sm_scale: float, *, counts: Optional[torch.Tensor] = None,
                    kv_scale: Optional[float] = None, q_scale: Optional[float] = None,
@@ -701,15 +745,14 @@ def masked_mla_fp8(q: torch.Tensor, kv_cache_fp8: torch.Tensor, union_idx: torch
     else:
         ks = 1.0 if kv_scale is None else float(kv_scale)
         if q.dtype == torch.bfloat16:
-            if q_scale is None:      # convenience: one device->host read
-                amax = float(q.abs().amax().item())
-                q_scale = 2.0 ** max(-24, int(torch.tensor(max(amax, 1e-30) / 448.0).log2().ceil().item()))
-            q8 = quantize_e4m3(q.contiguous(), q_scale)
+            if q_scale is None:
+                q_scale = _derived_q_scale(q)
+            _masked_mla_fp8_bf16q(q.contiguous(), float(q_scale), kv, union_idx, float(sm_scale) * q_scale * ks, ks,
+                                  counts, mask, h, out, ml, lse)
         else:
-            q8 = q.contiguous()
             q_scale = 1.0 if q_scale is None else q_scale
-        masked_mla_fp8_out(q8.view(ng, 128, 576), kv, union_idx, float(sm_scale) * q_scale * ks,
-                           ks, counts, mask, h, out, ml, lse)
+            masked_mla_fp8_out(q.contiguous().view(ng, 128, 576), kv, union_idx, float(sm_scale) * q_scale * ks,
+                               ks, counts, mask, h, out, ml, lse)
     res = (out.view(T, h, 512), lse.view(T, h))
     return res + (ml.view(T, h),) if return_max_logits else res
 
@@ -725,12 +768,57 @@ def sparse_prefill(q: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_idx: torch.
     several calls).  Returns ``(out [T,h,512] bf16, lse [T,h] f32)``, written into ``out`` /
     ``lse`` when given.
     """
-    h = q.shape[1]
-    u, m, c = union_qm(topk_idx, 128 // h,
-                       seq_space=seq_space if seq_space is not None else kv_cache_fp8.shape[0],
-                       return_counts=True)
-    return masked_mla_fp8(q, kv_cache_fp8, u, m, sm_scale, counts=c, kv_scale=kv_scale,
-                          q_scale=q_scale, out=out, lse=lse)
+    return _sparse_prefill(q, kv_cache_fp8, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse, q.shape[0])
+
+
+def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse, job_tokens):
+    """:func:`sparse_prefill` of a chunk of a job of ``job_tokens`` tokens (the library picks how a
+    small job is cut into slices from that number, so a chunk's bits do not depend on the chunking)."""
+    _need(q, "q", (torch.bfloat16, torch.uint8, torch.float8_e4m3fn), 3)
+    _need(topk_idx, "topk_idx", torch.int32, 2)
+    T, h, d = q.shape
+    if d != 576 or 128 % h or 128 // h > 16:
+        raise ValueError("q must be [T, h, 576] with h dividing 128 and 128/h <= 16")
+    k = topk_idx.shape[1]
+    if T % (128 // h) or topk_idx.shape[0] != T:
+        raise ValueError("token count must be a multiple of 128 // heads and match topk_idx")
+    kv = prepare_kv(kv_cache, kv_scale)
+    if kv.dim() == 3 and kv.shape[1] == 1:
+        kv = kv[:, 0]
+    _need(kv, "kv_cache", (torch.bfloat16, torch.uint8, torch.float8_e4m3fn), 2)
+    if kv.shape[1] != 576 or kv.stride(1) != 1:
+        raise ValueError("kv_cache must be [s_kv, 576] with unit inner stride (or packed 656-byte rows)")
+    kv_bf16, q_bf16 = kv.dtype == torch.bfloat16, q.dtype == torch.bfloat16
+    if kv_bf16 and not q_bf16:
+        raise TypeError("the bf16 route (cache with per-128 scales / bf16 workspace) needs bf16 q")
+    q, topk_idx, dev = q.contiguous(), topk_idx.contiguous(), q.device
+    if kv_scale is None:
+        kv_scale = 1.0
+    if q_scale is None:
+        q_scale = _derived_q_scale(q) if q_bf16 and not kv_bf16 else 1.0
+    if out is None:
+        out = torch.empty((T, h, 512), dtype=torch.bfloat16, device=dev)
+    else:
+        _need(out, "out", torch.bfloat16)
+        if out.numel() != T * h * 512 or not out.is_contiguous():
+            raise ValueError("out must be a contiguous [T,h,512] bf16 tensor")
+        out = out.view(T, h, 512)
+    if lse is None:
+        lse = torch.empty((T, h), dtype=torch.float32, device=dev)
+    else:
+        _need(lse, "lse", torch.float32)
+        if lse.numel() != T * h or not lse.is_contiguous():
+            raise ValueError("lse must be a contiguous [T,h] f32 tensor")
+        lse = lse.view(T, h)
+    lib = _lib.lib()
+    space = kv_cache.shape[0] if seq_space is None else int(seq_space)
+    ws = torch.empty((max(lib.litedsa_sparse_prefill_workspace(T, h, k, kv_bf16, job_tokens), 1),),
+                     dtype=torch.uint8, device=dev)
+    check(_on_device(dev, lib.litedsa_sparse_prefill, q.data_ptr(), q_bf16, kv.data_ptr(), kv_bf16,
+                     topk_idx.data_ptr(), sm_scale, q_scale, kv_scale, out.data_ptr(), lse.data_ptr(), T, h, k,
+                     kv.shape[0], kv.stride(0), (space + 1023) // 1024 * 1024, job_tokens, ws.data_ptr(),
+                     ws.numel()), "sparse_prefill")
+    return out, lse
 
 
 _SIDE_STREAMS = {}
@@ -842,8 +930,8 @@ def sparse_prefill_host(q_host: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_h
                 ev_in = torch.cuda.Event()
                 ev_in.record(s_in)
             cur.wait_event(ev_in)
-            sparse_prefill(qd[t0:t1], kv, idd[t0:t1], sm_scale, kv_scale=kv_scale, q_scale=q_scale,
-                           seq_space=space, out=od[t0:t1], lse=ld[t0:t1])
+            _sparse_prefill(qd[t0:t1], kv, idd[t0:t1], sm_scale, kv_scale, q_scale, space, od[t0:t1],
+                            ld[t0:t1], T)
             ev_c = torch.cuda.Event()
             ev_c.record(cur)
             s_out.wait_event(ev_c)
@@ -899,7 +987,7 @@ def dsv4_c128a_bf16(q: torch.Tensor, kv_compressed: Optional[torch.Tensor], kv_r
         _need(attn_sink, "attn_sink", torch.float32, 1)
         if attn_sink.shape[0] != h:
             raise ValueError("attn_sink must be [heads]")
-        sink = attn_sink.repeat(G).contiguous()            # per packed row
+        sink = attn_sink.contiguous()
     ng = T // G
     in_place_out = out is not None
     if in_place_out:
@@ -909,13 +997,15 @@ def dsv4_c128a_bf16(q: torch.Tensor, kv_compressed: Optional[torch.Tensor], kv_r
     else:
         out = torch.empty((T, h, 512), dtype=torch.bfloat16, device=q.device)
     lse = torch.empty((ng, 128), dtype=torch.float32, device=q.device)
-    with torch.cuda.device(q.device):
-        rc = _lib.lib().litedsa_dsv4_c128a_bf16(
-            _ptr(q), _ptr(kv_compressed) if n_comp else None, _ptr(kv_raw), ng, h, n_comp,
-            kv_raw.shape[0], int(q_pos0), int(window), int(ratio), float(sm_scale), _ptr(sink),
-            _ptr(out), _ptr(lse), q.stride(1), kv_compressed.stride(0) if n_comp else 576, kv_raw.stride(0),
-            q.stride(0), q.stride(1), out.stride(0), out.stride(1), _stream(q))
-    check(rc, "dsv4_c128a_bf16")
+    lib = _lib.lib()
+    ws_bytes = lib.litedsa_dsv4_workspace(ng, h, n_comp, int(q_pos0), int(window), int(ratio))
+    ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=q.device) if ws_bytes > 0 else None
+    check(_on_device(q.device, lib.litedsa_dsv4_c128a_bf16_ws, q.data_ptr(),
+                     kv_compressed.data_ptr() if n_comp else None, kv_raw.data_ptr(), ng, h, n_comp,
+                     kv_raw.shape[0], int(q_pos0), int(window), int(ratio), sm_scale, _ptr(sink), h,
+                     out.data_ptr(), lse.data_ptr(), q.stride(1), kv_compressed.stride(0) if n_comp else 576,
+                     kv_raw.stride(0), q.stride(0), q.stride(1), out.stride(0), out.stride(1), _ptr(ws), ws_bytes),
+          "dsv4_c128a_bf16")
     return out, lse.view(T, h)
 
 

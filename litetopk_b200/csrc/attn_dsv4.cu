@@ -69,7 +69,13 @@ static_assert(sizeof(Misc) <= kMiscBytes, "Misc too large");
 struct Params {
   __nv_bfloat16* out;        // [ng, 128, 512]
   float* lse;                // [ng, 128]
-  const float* sink;         // [128] per packed row, or null
+  const float* sink;         // natural-log units, indexed by packed row modulo sink_mod, or null
+  int sink_mod;              // 128: one value per packed row; h_per_q: one per head
+  // slices: every tile's blocks are cut into nsplit > 1 work items, each leaving its unnormalised
+  // O (fp32 [ng * nsplit, 128, 512]) and (running max, row sum) for merge_slices
+  int nsplit;
+  float* part_o;
+  float2* part_ml;
   int ng, n_comp, s_raw, G, h_per_q, pos0, window, ratio;
   float scale_log2;
   int epoch;                          // this launch's epoch for the bounded waits
@@ -95,13 +101,16 @@ enum { kSiteQ = 101, kSiteKFull, kSiteVFull, kSiteQkDone, kSitePvDone, kSiteSFre
 // status block of the DSv4 kernel (layout: see Waiter in common.cuh)
 __device__ int g_status[8];
 
-// key segments of a tile: compressed blocks first, then window blocks
+// key segments of a work item's tile: compressed blocks first, then window blocks; the item runs
+// the tile's blocks [b0, b0 + nb)
 struct TilePlan {
-  int p0, pref_max, wlo, count_w, nbc, nb, row_c;   // row_c: first row of the first segment
+  int tile, p0, pref_max, wlo, count_w, nbc, b0, nb, row_c;   // row_c: first row of the first segment
 };
-template <bool kRank>
-__device__ __forceinline__ TilePlan plan_tile(const Params& p, int tile) {
+template <bool kRank, bool kSliced>
+__device__ __forceinline__ TilePlan plan_item(const Params& p, int w) {
   TilePlan t;
+  const int tile = kSliced ? w / p.nsplit : w;
+  t.tile = tile;
   if (kRank) {
     const int4 r = __ldg(p.runs + tile);
     t.p0 = 0;
@@ -118,6 +127,14 @@ __device__ __forceinline__ TilePlan plan_tile(const Params& p, int tile) {
   t.nbc = (t.pref_max + kBlockKeys - 1) / kBlockKeys;
   t.nb = t.nbc + (t.count_w + kBlockKeys - 1) / kBlockKeys;
   if (t.nb == 0) t.nb = 1;      // an empty list: one fully masked block keeps the pipeline uniform
+  t.b0 = 0;
+  if (kSliced) {
+    // an empty slice repeats the tile's last block with every key masked (b0 beyond the list)
+    const int part = w - tile * p.nsplit, all = t.nb;
+    t.b0 = part * all / p.nsplit;
+    t.nb = (part + 1) * all / p.nsplit - t.b0;
+    if (t.nb == 0) { t.nb = 1; t.b0 = all; }
+  }
   return t;
 }
 // bits [0, x) of a 32-bit word (x may be negative or beyond 32)
@@ -134,7 +151,7 @@ __device__ __forceinline__ void mma_f16_elect(uint32_t d_tmem, uint64_t adesc, u
       : "memory");
 }
 
-template <bool kRank>
+template <bool kRank, bool kSliced>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kc32,
             const __grid_constant__ CUtensorMap map_kr32, const __grid_constant__ CUtensorMap map_kc64,
@@ -146,6 +163,8 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
   uint8_t* sm = smem_raw + (sbase - raw);
   Misc& ms = *reinterpret_cast<Misc*>(sm + kOffMisc);
   const Waiter wt{g_status, p.epoch, p.wait_limit_ns};
+  pdl_trigger();
+  pdl_wait();
   // device-side choice between this kernel and the gather kernel (uniform across the grid)
   if (p.gate != nullptr && *reinterpret_cast<const volatile int*>(p.gate) != p.gate_value) return;
   // the plan leaves less than 1024 bytes for aligning the base: refuse to run (uniformly, in
@@ -155,7 +174,8 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     return;
   }
 
-  // Persistent: each cluster walks tiles cid, cid + #clusters, ...  Stages, buffers and
+  const int n_items = kSliced ? p.ng * p.nsplit : p.ng;
+  // Persistent: each cluster walks items cid, cid + #clusters, ...  Stages, buffers and
   // barrier phases are indexed by the cluster-wide running block number kb, so the next
   // tile's Q / K / V loads and first QK^T overlap the previous tile's epilogue.
   const uint32_t cta = cluster_ctarank();
@@ -205,9 +225,9 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     const uint32_t a_s_free[2] = {mapa(smem_u32(&ms.s_free[0]), 0), mapa(smem_u32(&ms.s_free[1]), 0)};
     const uint32_t a_p_ready = mapa(smem_u32(&ms.p_ready), 0);
     int kb0 = 0, it = 0;
-   for (int tile = cid; tile < p.ng; tile += ncl) {
-    const TilePlan tp = plan_tile<kRank>(p, tile);
-    const int nb = tp.nb;
+   for (int w = cid; w < n_items; w += ncl) {
+    const TilePlan tp = plan_item<kRank, kSliced>(p, w);
+    const int nb = tp.nb, tile = tp.tile;
     int pref_q, lo_q, hi_q;
     if (kRank) {
       // list ranks this token may attend: rank < pref_q, or lo_q <= rank < hi_q (all < cnt)
@@ -243,8 +263,9 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
         // columns this thread holds: 32 consecutive list ranks starting at `off`, of which the
         // first `lim` exist in this segment; valid = existing and in one of the token's two
         // rank ranges -- one 32-bit mask per block
-        const bool seg0 = k < tp.nbc;
-        const int base = (seg0 ? k : k - tp.nbc) * kBlockKeys + 32 * h;
+        const int bk = tp.b0 + k;
+        const bool seg0 = bk < tp.nbc;
+        const int base = (seg0 ? bk : bk - tp.nbc) * kBlockKeys + 32 * h;
         const int lim = (seg0 ? tp.pref_max : tp.count_w) - base;
         const int off = (seg0 ? 0 : tp.pref_max) + base;
         const uint32_t vm = low_bits(lim) & (low_bits(pref_q - off) | (low_bits(hi_q - off) & ~low_bits(lo_q - off)));
@@ -256,11 +277,12 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
       } else {
         // columns this thread holds: keys [32h, 32h+32) of the block, as a contiguous valid range
         int v_lo, v_hi;
-        if (k < tp.nbc) {                       // compressed block: rank = 64k + j < pref_q
+        const int bk = tp.b0 + k;
+        if (bk < tp.nbc) {                      // compressed block: rank = 64 bk + j < pref_q
           v_lo = 0;
-          v_hi = pref_q - (k * kBlockKeys + 32 * h);
-        } else {                                // window block: lo_q <= 64(k-nbc) + j < hi_q
-          const int base = (k - tp.nbc) * kBlockKeys + 32 * h;
+          v_hi = pref_q - (bk * kBlockKeys + 32 * h);
+        } else {                                // window block: lo_q <= 64(bk-nbc) + j < hi_q
+          const int base = (bk - tp.nbc) * kBlockKeys + 32 * h;
           v_lo = lo_q - base;
           v_hi = hi_q - base;
         }
@@ -329,16 +351,20 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     asm volatile("bar.sync 1, 128;" ::: "memory");
     li += ms.xbuf[2][tl ^ 64];
     if (real_m == -INFINITY) { li = 0.f; m = -INFINITY; }
-    const size_t grow = (size_t)tile * 128 + row;
-    if (h == 0) {
-      float l = __logf(li) + m * kLn2;
-      if (!(li > 0.f)) l = INFINITY;
-      p.lse[grow] = l;
+    if (kSliced) {
+      if (h == 0) p.part_ml[(size_t)w * 128 + row] = make_float2(m, li);
+    } else {
+      const size_t grow = (size_t)tile * 128 + row;
+      if (h == 0) {
+        float l = __logf(li) + m * kLn2;
+        if (!(li > 0.f)) l = INFINITY;
+        p.lse[grow] = l;
+      }
+      // hand the tile over to the epilogue warps: all they need is 1 / normaliser per row
+      float denom = li;
+      if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldg(p.sink + row % p.sink_mod) * kLog2e - m);
+      if (h == 0) ms.oscale[it & 1][r] = (li > 0.f) ? __fdividef(1.0f, denom) : 0.f;
     }
-    // hand the tile over to the epilogue warps: all they need is 1 / normaliser per row
-    float denom = li;
-    if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldg(p.sink + row) * kLog2e - m);
-    if (h == 0) ms.oscale[it & 1][r] = (li > 0.f) ? __fdividef(1.0f, denom) : 0.f;
     __syncwarp();
     if (lane == 0) mbar_arrive(&ms.epi_ready);
     kb0 += nb;
@@ -352,9 +378,9 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
       const uint32_t a_v_full[2] = {mapa(smem_u32(&ms.v_full[0]), 0), mapa(smem_u32(&ms.v_full[1]), 0)};
       const uint64_t pol_stream = l2_policy_evict_first();     // q streams through once
       int kb0 = 0, it = 0;
-      for (int tile = cid; tile < p.ng; tile += ncl, ++it) {
-        const TilePlan tp = plan_tile<kRank>(p, tile);
-        const int nb = tp.nb;
+      for (int w = cid; w < n_items; w += ncl, ++it) {
+        const TilePlan tp = plan_item<kRank, kSliced>(p, w);
+        const int nb = tp.nb, tile = tp.tile;
         // the previous tile's Q must have been consumed by its last QK^T
         if (it > 0) mbar_wait(&ms.q_free, (it - 1) & 1, wt, kSiteQFree, it);
         if (cta == 0) mbar_arrive_expect_tx(&ms.q_full, 2 * kQBytes);
@@ -367,8 +393,9 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
           const int kb = kb0 + k;
           const int s = kb & 1;
           const uint32_t ph = (kb >> 1) & 1;
-          const bool comp = k < tp.nbc;
-          const int row0 = comp ? tp.row_c + k * kBlockKeys : tp.wlo + (k - tp.nbc) * kBlockKeys;
+          const int bk = tp.b0 + k;
+          const bool comp = bk < tp.nbc;
+          const int row0 = comp ? tp.row_c + bk * kBlockKeys : tp.wlo + (bk - tp.nbc) * kBlockKeys;
           const CUtensorMap* m32 = comp ? &map_kc32 : &map_kr32;
           const CUtensorMap* m64 = comp ? &map_kc64 : &map_kr64;
           if (kb >= 2) mbar_wait(&ms.qk_done[s], ph ^ 1, wt, kSiteKFree, k);   // K stage free
@@ -401,12 +428,30 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     const int sw = (r >> 1) & 3;
     const uint32_t a_o_free = mapa(smem_u32(&ms.o_free), 0);
     int kb0 = 0, it = 0;
-    for (int tile = cid; tile < p.ng; tile += ncl, ++it) {
-      const int nb = plan_tile<kRank>(p, tile).nb;
-      const int kbl = kb0 + nb - 1;                 // last block of the tile
+    for (int w = cid; w < n_items; w += ncl, ++it) {
+      const TilePlan tp = plan_item<kRank, kSliced>(p, w);
+      const int nb = tp.nb, tile = tp.tile;
+      const int kbl = kb0 + nb - 1;                 // last block of the item
       mbar_wait(&ms.epi_ready, it & 1, wt, kSiteEpi, it);
       mbar_wait(&ms.pv_done[kbl & 1], (kbl >> 1) & 1, wt, kSiteEpi, nb);
       tc_fence_after();
+      if (kSliced) {
+        // a slice: unnormalised fp32 O straight to its slot (few slices exist, all of them in L2)
+        float4* dst = reinterpret_cast<float4*>(p.part_o + ((size_t)w * 128 + 64 * cta + r) * kDV + 256 * h);
+        float o[32];
+#pragma unroll 1
+        for (int cc = 0; cc < 8; ++cc) {
+          tmem_ld32(ocol + cc * 32, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) dst[cc * 8 + j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(a_o_free);
+        kb0 += nb;
+        continue;
+      }
       const float oscale = ms.oscale[it & 1][r];
       const uint32_t emask = oscale != 0.f ? 0xffffffffu : 0u;
       // this warp's 32 rows of the tile = (token, head) pairs starting at row r0
@@ -426,11 +471,11 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(a_o_free);
         }
-        uint32_t w[16];
+        uint32_t wv[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           __nv_bfloat162 v2 = __floats2bfloat162_rn(o[2 * j] * oscale, o[2 * j + 1] * oscale);
-          w[j] = *reinterpret_cast<uint32_t*>(&v2) & emask;      // rows without a key: zeros
+          wv[j] = *reinterpret_cast<uint32_t*>(&v2) & emask;      // rows without a key: zeros
         }
         // the previous round's box must have been read out of the slice
         if (lane == 0) bulk_wait_read_all();
@@ -438,7 +483,7 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           *reinterpret_cast<uint4*>(st_row + ((j ^ sw) << 4)) =
-              make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+              make_uint4(wv[4 * j], wv[4 * j + 1], wv[4 * j + 2], wv[4 * j + 3]);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -458,8 +503,8 @@ dsv4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ C
     const uint32_t a_pv_done_peer[2] = {mapa(smem_u32(&ms.pv_done[0]), 1), mapa(smem_u32(&ms.pv_done[1]), 1)};
     const uint32_t a_q_free_peer = mapa(smem_u32(&ms.q_free), 1);
     int kb0 = 0, it = 0;
-    for (int tile = cid; tile < p.ng; tile += ncl, ++it) {
-      const int nb = plan_tile<kRank>(p, tile).nb;
+    for (int w = cid; w < n_items; w += ncl, ++it) {
+      const int nb = plan_item<kRank, kSliced>(p, w).nb;
       mbar_wait(&ms.q_full, it & 1, wt, kSiteQ, it);
       __syncwarp();
       for (int k = 0; k <= nb; ++k) {
@@ -553,11 +598,9 @@ static bool smem_alignment_ok() {
   return ok;
 }
 
-// how many 2-CTA clusters of this kernel the current device can hold at once
-static int max_clusters() {
+// how many 2-CTA clusters of this kernel device `dev` (the current one) can hold at once
+static int max_clusters(int dev) {
   static thread_local int cached_dev = -1, cached = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
   if (dev == cached_dev) return cached;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -569,12 +612,25 @@ static int max_clusters() {
   at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
   int q = 0;
-  if (cudaFuncSetAttribute(dsv4_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) == cudaSuccess &&
-      cudaOccupancyMaxActiveClusters(&q, dsv4_kernel<false>, &cfg) == cudaSuccess && q > 0)
+  if (ensure_smem<dsv4_kernel<false, false>>(dev, kSmem) &&
+      cudaOccupancyMaxActiveClusters(&q, dsv4_kernel<false, false>, &cfg) == cudaSuccess && q > 0)
     n = q;
   cudaGetLastError();
   cached_dev = dev; cached = n;
   return n;
+}
+
+// Launch of the range kernel over p.ng tiles of p.nsplit slices; a merge follows when they are sliced.
+template <bool kRank>
+static int launch(const CUtensorMap& mq, const CUtensorMap& mkc32, const CUtensorMap& mkr32, const CUtensorMap& mkc64,
+                  const CUtensorMap& mkr64, const CUtensorMap& mout, const Params& p, cudaStream_t stream) {
+  const int dev = current_device();
+  const bool sliced = p.nsplit > 1;
+  if (!(sliced ? ensure_smem<dsv4_kernel<kRank, true>>(dev, kSmem) : ensure_smem<dsv4_kernel<kRank, false>>(dev, kSmem)))
+    return LITEDSA_ERR_CUDA;
+  return launch_pdl(sliced ? dsv4_kernel<kRank, true> : dsv4_kernel<kRank, false>,
+                    dim3(2 * min(p.ng * p.nsplit, max_clusters(dev))), kThreads, kSmem, stream, mq, mkc32, mkr32,
+                    mkc64, mkr64, mout, p);
 }
 
 // One warp per tile: is the tile's gathered index list (its first counts[tile] entries) two
@@ -650,22 +706,47 @@ int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, con
                    CU_TENSOR_MAP_SWIZZLE_64B))
     return LITEDSA_ERR_CUDA;
   Params p;
-  p.out = reinterpret_cast<__nv_bfloat16*>(out); p.lse = lse; p.sink = attn_sink;
+  p.out = reinterpret_cast<__nv_bfloat16*>(out); p.lse = lse; p.sink = attn_sink; p.sink_mod = 128;
+  p.nsplit = 1; p.part_o = nullptr; p.part_ml = nullptr;
   p.ng = ng; p.n_comp = 0; p.s_raw = s_kv; p.G = G; p.h_per_q = h_per_q; p.pos0 = 0;
   p.window = 1; p.ratio = 1; p.scale_log2 = sm_scale * kLog2e;
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
   p.runs = runs; p.pref = pref; p.win_lo = win_lo; p.win_hi = win_hi; p.counts = counts;
   p.gate = gate; p.gate_value = 0;
-  if (cudaFuncSetAttribute(dsv4_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) !=
-      cudaSuccess)
-    return LITEDSA_ERR_CUDA;
-  dsv4_kernel<true><<<2 * min(ng, max_clusters()), kThreads, kSmem, stream>>>(mq, mk32, mk32, mk64, mk64, mout, p);
-  return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  return launch<true>(mq, mk32, mk32, mk64, mk64, mout, p, stream);
 }
 
 namespace dsv4 {
+
+// Slices of a tile when a call has `tiles` tiles of up to `blocks` 64-key blocks: as many as there
+// are idle clusters for, at least three blocks each (a slice costs an epilogue and its share of the
+// merge, as much as three blocks), none when more than half of the clusters have a tile anyway.
+static int pick_slices(int tiles, int blocks) {
+  constexpr int kClusters = 74;
+  int n = kClusters / tiles;
+  if (n > blocks / 3) n = blocks / 3;
+  if (n > kMaxSlices) n = kMaxSlices;
+  return n < 2 ? 1 : n;
+}
+// most 64-key blocks a tile of the call can have: its last tile has the longest prefix
+static int most_blocks(int ng, int G, int n_comp, int pos0, int window, int ratio) {
+  const int64_t last = (int64_t)pos0 + (int64_t)ng * G - 1;
+  const int64_t pref = min(last / ratio, (int64_t)n_comp);
+  return (int)((pref + kBlockKeys - 1) / kBlockKeys + (min(last + 1, (int64_t)window + G - 1) + kBlockKeys - 1) / kBlockKeys);
+}
+static int64_t slice_bytes(int ng, int nsplit) {
+  return nsplit < 2 ? 0 : (int64_t)ng * nsplit * 128 * (512 * 4 + 8);
+}
+
 }  // namespace dsv4
 }  // namespace lt
+
+// Bytes of workspace with which litedsa_dsv4_c128a_bf16_ws runs this shape in slices (0: it does not).
+extern "C" int64_t litedsa_dsv4_workspace(int ng, int h_per_q, int n_comp, int pos0, int window, int ratio) {
+  using namespace lt::dsv4;
+  if (ng <= 0 || h_per_q <= 0 || 128 % h_per_q || n_comp < 0 || pos0 < 0 || window <= 0 || ratio <= 0) return 0;
+  return slice_bytes(ng, pick_slices(ng, most_blocks(ng, 128 / h_per_q, n_comp, pos0, window, ratio)));
+}
 
 // DSv4 packed BF16 attention over (compressed prefix, sliding window).  Replaces the
 // reference operator dsv4_masked_mla_bf16 (kernels/b200/dsa/litedsa_dsv4.cu:50-55) for
@@ -679,6 +760,21 @@ extern "C" int litedsa_dsv4_c128a_bf16(const void* q, const void* kv_comp, const
                                        int64_t kr_row_stride, int64_t q_token_stride,
                                        int64_t q_head_stride, int64_t out_token_stride,
                                        int64_t out_head_stride, void* stream) {
+  return litedsa_dsv4_c128a_bf16_ws(q, kv_comp, kv_raw, ng, h_per_q, n_comp, s_raw, pos0, window, ratio, sm_scale,
+                                    attn_sink, 128, out, lse, q_row_stride, kc_row_stride, kr_row_stride,
+                                    q_token_stride, q_head_stride, out_token_stride, out_head_stride, nullptr, 0,
+                                    stream);
+}
+
+// The same with one sink per head (sink_len == h_per_q) or per packed row (128), and with a workspace
+// for calls of few tiles, whose key blocks are then cut into slices that run in parallel.
+extern "C" int litedsa_dsv4_c128a_bf16_ws(const void* q, const void* kv_comp, const void* kv_raw, int ng,
+                                          int h_per_q, int n_comp, int s_raw, int pos0, int window, int ratio,
+                                          float sm_scale, const float* attn_sink, int sink_len, void* out,
+                                          float* lse, int64_t q_row_stride, int64_t kc_row_stride,
+                                          int64_t kr_row_stride, int64_t q_token_stride, int64_t q_head_stride,
+                                          int64_t out_token_stride, int64_t out_head_stride, void* workspace,
+                                          int64_t workspace_bytes, void* stream) {
   using namespace lt;
   using namespace lt::dsv4;
   if (!q || !kv_raw || !out || !lse) return LITEDSA_ERR_ARG;
@@ -687,6 +783,7 @@ extern "C" int litedsa_dsv4_c128a_bf16(const void* q, const void* kv_comp, const
     return LITEDSA_ERR_SHAPE;
   if (h_per_q <= 0 || 128 % h_per_q != 0 || 128 / h_per_q > 16) return LITEDSA_ERR_SHAPE;
   const int G = 128 / h_per_q;
+  if (attn_sink && sink_len != 128 && sink_len != h_per_q) return LITEDSA_ERR_SHAPE;
   if ((int64_t)pos0 + (int64_t)ng * G > s_raw) return LITEDSA_ERR_SHAPE;   // queries sit inside the cache
   if (window + G - 1 > 8 * kBlockKeys * 64) return LITEDSA_ERR_UNSUPPORTED;
   // strides are in ELEMENTS (bf16); TMA needs 16-byte aligned bases and pitches
@@ -722,18 +819,27 @@ extern "C" int litedsa_dsv4_c128a_bf16(const void* q, const void* kv_comp, const
                    CU_TENSOR_MAP_SWIZZLE_64B))
     return LITEDSA_ERR_CUDA;
   Params p;
-  p.out = reinterpret_cast<__nv_bfloat16*>(out); p.lse = lse; p.sink = attn_sink;
+  p.out = reinterpret_cast<__nv_bfloat16*>(out); p.lse = lse; p.sink = attn_sink; p.sink_mod = sink_len;
+  p.nsplit = 1; p.part_o = nullptr; p.part_ml = nullptr;
+  if (workspace) {
+    if ((uintptr_t)workspace & 255) return LITEDSA_ERR_UNSUPPORTED;
+    const int ns = pick_slices(ng, most_blocks(ng, G, n_comp, pos0, window, ratio));
+    if (ns > 1 && workspace_bytes >= slice_bytes(ng, ns)) {
+      p.nsplit = ns;
+      p.part_o = reinterpret_cast<float*>(workspace);
+      p.part_ml = reinterpret_cast<float2*>(p.part_o + (size_t)ng * ns * 128 * kDV);
+    }
+  }
   p.ng = ng; p.n_comp = n_comp; p.s_raw = s_raw; p.G = G; p.h_per_q = h_per_q; p.pos0 = pos0;
   p.window = window; p.ratio = ratio; p.scale_log2 = sm_scale * kLog2e;
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
   if (!smem_alignment_ok()) return LITEDSA_ERR_UNSUPPORTED;   // first call per device: synchronous probe
   p.runs = nullptr; p.pref = p.win_lo = p.win_hi = p.counts = nullptr; p.gate = nullptr; p.gate_value = 0;
-  if (cudaFuncSetAttribute(dsv4_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) !=
-      cudaSuccess)
-    return LITEDSA_ERR_CUDA;
-  dsv4_kernel<false><<<2 * min(ng, max_clusters()), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream)>>>(
-      mq, mkc32, mkr32, mkc64, mkr64, mout, p);
-  return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int rc = launch<false>(mq, mkc32, mkr32, mkc64, mkr64, mout, p, st);
+  if (rc != LITEDSA_OK || p.nsplit == 1) return rc;
+  return merge_slices(p.part_o, p.part_ml, p.nsplit, ng, h_per_q, 1.f, 0.f, attn_sink, sink_len, out,
+                      (int64_t)(o_ts / 2), (int64_t)(o_hs / 2), lse, st);
 }
 
 // Status word of the DSv4 kernel (same meaning as litedsa_attn_status).

@@ -65,6 +65,7 @@ constexpr uint32_t kStageKV = kQLatent + kRopeChunkBytes;        // 64 keys x 57
 constexpr uint32_t kPBytes = 64 * 128;               // 64 rows x 128 keys e4m3
 constexpr uint32_t kMiscBytes = 10240;
 constexpr uint32_t kStageBytes = 4 * 4096;           // staged epilogue: one 4 KB slice per epilogue warp
+constexpr int kFillBatch = 6;                        // bf16 q: 32-byte loads in flight per thread while filling a Q tile
 constexpr int kSlots = 5;                            // ring of 36 KB slots
 
 // Shared-memory plan.  A ring of five slots carries, in order, each item's Q tile and its K tiles:
@@ -92,7 +93,7 @@ constexpr uint32_t kTmemQ = 384;                      // 128 columns: the 512 la
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kPScaleLog2 = 2.8073549220576042f;    // log2(7)
-constexpr float kPScaleLn = 1.9459101090932196f;      // ln(7)
+constexpr float kPScaleLn = kFp8LseOffset;            // ln(7)
 constexpr float kMInit = -1e30f;
 constexpr float kRescaleThreshold = 6.0f;
 
@@ -151,7 +152,7 @@ struct AttnParams {
   const uint4* q_bf16;
   float q_inv;
   // KV split inside the launch: nsplit > 1 slices per tile, each leaving its unnormalised O (fp32
-  // [ng * nsplit, 128, 512]) and (running max, row sum) for merge_parts_kernel
+  // [ng * nsplit, 128, 512]) and (running max, row sum) for merge_slices_kernel
   int nsplit;
   float* part_o;
   float2* part_ml;
@@ -166,8 +167,17 @@ __device__ __forceinline__ uint32_t e4m3x4_of_bf16(uint32_t lo, uint32_t hi, flo
          ((uint32_t)__nv_cvt_float2_to_fp8x2(b, __NV_SATFINITE, __NV_E4M3) << 16);
 }
 
-// one work item: key blocks [k0, k0 + nb) of a tile; ranks >= lim are masked
-struct Item { int tile, k0, nb, lim; };
+// One work item: nb blocks of a tile; ranks >= lim are masked.  A slice behind the first opens
+// with the tile's block 0 (lead = 1), of which only the row maxima count: its running max then
+// starts where the unsliced tile's does, so its P are rounded to e4m3 relative to the same value
+// (the max rarely moves after the first block) and slicing does not show in the result.
+template <bool kSliced>
+struct ItemT {
+  int tile, k0, nb, lim, lead;
+  // the tile's block that local block k is, and whether only its maxima count
+  __device__ __forceinline__ int block(int k) const { return !kSliced ? k : (k < lead ? 0 : k0 + k - lead); }
+  __device__ __forceinline__ bool leads(int k) const { return kSliced && k < lead; }
+};
 
 // wait sites reported in the status word
 enum { kSiteQ = 1, kSiteKLand, kSiteKPeer, kSiteVLand, kSiteVPeer, kSiteQkDone, kSitePvDone,
@@ -177,11 +187,14 @@ enum { kSiteQ = 1, kSiteKLand, kSiteKPeer, kSiteVLand, kSiteVPeer, kSiteQkDone, 
 // status block of the FP8 attention kernels (layout: see Waiter in common.cuh)
 __device__ int g_attn_status[8];
 
+// kSliced: p.nsplit > 1 (the unsliced kernel carries none of the slices' block arithmetic)
+template <bool kSliced>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kAttnThreads, 1)
 masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_q_rope,
                       const __grid_constant__ OutMaps omaps, const AttnParams p) {
   using PL = Plan;
+  using Item = ItemT<kSliced>;
   constexpr uint32_t kOffRope = PL::kOffRope, kOffKV = PL::kOffKV, kOffP = PL::kOffP, kOffMisc = PL::kOffMisc, kOffStage = PL::kOffStage;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -196,24 +209,25 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   // item's last softmax blocks and its epilogue.
   const uint32_t cta = cluster_ctarank();
   const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
-  const int n_items = p.ng * p.nsplit;
+  const int n_items = kSliced ? p.ng * p.nsplit : p.ng;
   // broadcast so the compiler knows the role index is warp-uniform
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   auto item_of = [&](int w) -> Item {
     Item t;
-    t.tile = p.nsplit == 1 ? w : w / p.nsplit;
+    t.tile = kSliced ? w / p.nsplit : w;
     // live union entries of the tile; with per-token prefix bounds the block loop runs to the LAST
     // token's bound (litedsa_attention_sm100.cuh:1846-1851)
     const int c = p.len_per_q ? p.len_per_q[(size_t)t.tile * p.G + (p.G - 1)]
                               : (p.counts ? p.counts[t.tile] : p.cap);
     t.lim = min(max(c, 0), p.cap);
-    t.k0 = 0;
+    t.k0 = t.lead = 0;
     t.nb = max((t.lim + kBlockKeys - 1) / kBlockKeys, 1);
-    if (p.nsplit > 1) {       // slice `part`; an empty slice runs one fully masked block
+    if (kSliced) {            // slice `part`; an empty slice runs one fully masked block
       const int part = w - t.tile * p.nsplit, nbt = t.nb;
       const int k1 = (part + 1) * nbt / p.nsplit;
       t.k0 = part * nbt / p.nsplit;
-      t.nb = max(k1 - t.k0, 1);
+      t.lead = part > 0 ? 1 : 0;
+      t.nb = max(k1 - t.k0, 1) + t.lead;
       t.lim = min(t.lim, k1 * kBlockKeys);
     }
     return t;
@@ -246,7 +260,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       tma_prefetch_desc(&map_q);
       tma_prefetch_desc(&map_q_rope);
     }
-    if (p.nsplit == 1)
+    if (!kSliced)
       for (int d = 0; d < p.n_out; ++d) tma_prefetch_desc(&omaps.m[d]);
   }
   __syncthreads();
@@ -259,6 +273,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ms.tmem_base;
+  pdl_trigger();
+  pdl_wait();
 
   // Registers: the block is launched with 64 per thread (8 warpgroups, 512 in sum); the softmax
   // warps need more for their 32 scores, the epilogue for its 32 + 16 outputs, the others less:
@@ -293,20 +309,20 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       const Item item = item_of(w);
       const int nb = item.nb;
       const size_t trow = (size_t)item.tile * p.G + row / p.h_per_q;     // (tile, token) of this row
-      const uint32_t* mrow = p.memb ? p.memb + trow * capw + (size_t)item.k0 * 4 + (key0 >> 5) : nullptr;
+      const uint32_t* mrow = p.memb ? p.memb + trow * capw + (key0 >> 5) : nullptr;
       // per-token causal prefix: this row may attend union ranks < row_bound
       const int row_bound = p.len_per_q ? __ldg(p.len_per_q + trow) : 0x7fffffff;
       float m_mine = kMInit;      // the running max my row sum is relative to
       float li = 0.f, real_m = -INFINITY;
       const int k_first = (g - kb0) & 1;          // first local block with (kb0 + k) % 2 == g
       uint32_t mk = ~0u;
-      if (mrow && k_first < nb) mk = __ldcs(mrow + (size_t)k_first * 4);
+      if (mrow && k_first < nb) mk = __ldcs(mrow + (size_t)item.block(k_first) * 4);
 
       for (int k = k_first; k < nb; k += 2) {
         const int kb = kb0 + k;
         const uint32_t ph = (kb >> 1) & 1;
         uint32_t mk_next = mk;
-        if (mrow && k + 2 < nb) mk_next = __ldcs(mrow + (size_t)(k + 2) * 4);
+        if (mrow && k + 2 < nb) mk_next = __ldcs(mrow + (size_t)item.block(k + 2) * 4);
 
         mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteQkDone, k);
         __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
@@ -321,7 +337,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         mbar_wait(&ms.valid_ready[g], ph, wt, kSiteValidReady, k);
         uint32_t vm = ms.valid[g][key0 >> 5] & mk;
         if (p.len_per_q) {     // ranks of my 32 columns
-          const int n = min(max(row_bound - ((item.k0 + k) * kBlockKeys + key0), 0), 32);
+          const int n = min(max(row_bound - (item.block(k) * kBlockKeys + key0), 0), 32);
           vm &= n >= 32 ? ~0u : ((1u << n) - 1u);
         }
         __syncwarp();
@@ -342,7 +358,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
         else asm volatile("bar.sync 2, 256;" ::: "memory");
         cur = fmaxf(fmaxf(xb[0][r], xb[1][r]), fmaxf(xb[0][r + 64], xb[1][r + 64]));
-        real_m = fmaxf(real_m, cur);
+        if (!item.leads(k)) real_m = fmaxf(real_m, cur);
         // running max after block k-1 of this item comes from the other group
         float m_prev = kMInit;
         if (k > 0) {
@@ -357,6 +373,10 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         li *= fast_exp2(m_mine - new_m);
         m_mine = new_m;
 
+        if (item.leads(k)) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sv[j] = -INFINITY;      // only the maxima of this block count
+        }
         const float nm = -new_m + kPScaleLog2;
         uint32_t pk[8];
         float l1 = 0.f;
@@ -433,7 +453,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         }
         li = lsum;
         if (real_m == -INFINITY) { li = 0.f; m = -INFINITY; }
-        if (p.nsplit > 1) {
+        if (kSliced) {
           p.part_ml[(size_t)w * 128 + row] = make_float2(m, li);
         } else {
           const size_t grow = (size_t)item.tile * 128 + row;
@@ -466,7 +486,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     // its PV; V rows of block cv (the PEER's 64 keys, this CTA's 256 value bytes, four copies per
     // lane) into the dead half of the same stage as soon as the block's QK^T is complete.
     const int pw = warp - kWarpGather0;
-    struct Cursor { int w, k, nb, kb, slot, ring; const int32_t* idx; };   // slot, ring: entry = 5 ring + slot
+    struct Cursor { int w, k, nb, kb, slot, ring, k0, lead; const int32_t* idx; };   // slot, ring: entry = 5 ring + slot
     // The Q entry in front of an item's K entries belongs to warp 0: once the slot is free it
     // requests the tile (TMA) or, for bf16 q, hands the slot to the epilogue warps.  (Only here: a
     // slot's barrier may be waited on once every older entry has been through it, which this
@@ -478,8 +498,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       c.nb = 0;
       if (c.w < n_items) {
         const Item t = item_of(c.w);
-        c.nb = t.nb; c.k = 0;
-        c.idx = p.indices + (size_t)t.tile * p.idx_stride + (size_t)t.k0 * kBlockKeys;
+        c.nb = t.nb; c.k = 0; c.k0 = t.k0; c.lead = t.lead;
+        c.idx = p.indices + (size_t)t.tile * p.idx_stride;
       }
     };
     auto advance = [&](Cursor& c) { if (++c.slot == kSlots) { c.slot = 0; ++c.ring; } };
@@ -499,7 +519,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     // lane l holds the index of key 8 pw + l % 8 of the CTA's own (K) / the peer's (V) 64 keys
     const int own_key = 64 * (int)cta + 8 * pw + (lane & 7);
     auto load_idx = [&](const Cursor& c, int key) -> int {
-      return __ldcs(c.idx + (size_t)c.k * kBlockKeys + key);
+      return __ldcs(c.idx + (size_t)(!kSliced ? c.k : (c.k < c.lead ? 0 : c.k0 + c.k - c.lead)) * kBlockKeys + key);
     };
     auto in_range = [&](int v) -> int { return ((unsigned)v < (unsigned)p.s_kv) ? v : 0; };   // masked later
     // The indices of a block are loaded right after the previous block's gather has been issued
@@ -737,14 +757,14 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     int kb = 0;
     for (int w = cid; w < n_items; w += ncl) {
       const Item item = item_of(w);
-      const int32_t* idx_row = p.indices + (size_t)item.tile * p.idx_stride + (size_t)item.k0 * kBlockKeys;
-      int4 cur = __ldcs(reinterpret_cast<const int4*>(idx_row) + lane);
+      const int32_t* idx_row = p.indices + (size_t)item.tile * p.idx_stride;
+      int4 cur = __ldcs(reinterpret_cast<const int4*>(idx_row + (size_t)item.block(0) * kBlockKeys) + lane);
       for (int k = 0; k < item.nb; ++k, ++kb) {
         const int s = kb & 1;
         const uint32_t ph = (kb >> 1) & 1;
         int4 nxt = cur;
-        if (k + 1 < item.nb) nxt = __ldcs(reinterpret_cast<const int4*>(idx_row + (size_t)(k + 1) * kBlockKeys) + lane);
-        const int rank0 = (item.k0 + k) * kBlockKeys + lane * 4;
+        if (k + 1 < item.nb) nxt = __ldcs(reinterpret_cast<const int4*>(idx_row + (size_t)item.block(k + 1) * kBlockKeys) + lane);
+        const int rank0 = item.block(k) * kBlockKeys + lane * 4;
         auto ok = [&](int idx, int rk) -> uint32_t {
           return (idx >= 0 && idx < p.s_kv && rk < item.lim) ? 1u : 0u;
         };
@@ -791,16 +811,16 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       {
         const uint4* src = p.q_bf16 + ((size_t)qtile * 128 + 64 * cta) * (kDQK / 8);
 #pragma unroll 1
-        for (int i = 0; i < 18; i += 3) {      // 64 rows x 36 units of 16 codes = 18 units per thread
-          uint4 a[3], b[3];
+        for (int i = 0; i < 18; i += kFillBatch) {      // 64 rows x 36 units of 16 codes = 18 units per thread
+          uint4 a[kFillBatch], b[kFillBatch];
 #pragma unroll
-          for (int u = 0; u < 3; ++u) {
+          for (int u = 0; u < kFillBatch; ++u) {
             const int unit = (i + u) * 128 + e_tid;
             a[u] = __ldcs(src + 2 * unit);
             b[u] = __ldcs(src + 2 * unit + 1);
           }
 #pragma unroll
-          for (int u = 0; u < 3; ++u) {
+          for (int u = 0; u < kFillBatch; ++u) {
             const int unit = (i + u) * 128 + e_tid, row = unit / 36, c = unit - 36 * row;
             const uint4 v = make_uint4(e4m3x4_of_bf16(a[u].x, a[u].y, p.q_inv), e4m3x4_of_bf16(a[u].z, a[u].w, p.q_inv),
                                        e4m3x4_of_bf16(b[u].x, b[u].y, p.q_inv), e4m3x4_of_bf16(b[u].z, b[u].w, p.q_inv));
@@ -863,7 +883,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       mbar_wait(&ms.pv_done[kbl & 3], (kbl >> 2) & 1, wt, kSiteEpi, item.nb);
       __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
       tc_fence_after();
-      if (p.nsplit > 1) {
+      if (kSliced) {
         // a slice: unnormalised fp32 O straight to its slot (few slices exist, all of them in L2)
         float4* dst = reinterpret_cast<float4*>(p.part_o + ((size_t)w * 128 + 64 * cta + e_r) * kDV + 256 * e_h);
         float o[32];
@@ -942,11 +962,9 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_attn_status[3], 1);
 }
 
-// how many 2-CTA clusters of this kernel the current device can hold at once
-static int max_clusters() {
+// how many 2-CTA clusters of this kernel device `dev` (the current one) can hold at once
+static int max_clusters(int dev) {
   static thread_local int cached_dev = -1, cached = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
   if (dev == cached_dev) return cached;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -956,9 +974,8 @@ static int max_clusters() {
   cudaLaunchAttribute at; at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
   int q = 0;
-  if (cudaFuncSetAttribute(masked_mla_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)Plan::kSmem) == cudaSuccess &&
-      cudaOccupancyMaxActiveClusters(&q, masked_mla_fp8_kernel, &cfg) == cudaSuccess && q > 0)
+  if (ensure_smem<masked_mla_fp8_kernel<false>>(dev, Plan::kSmem) &&
+      cudaOccupancyMaxActiveClusters(&q, masked_mla_fp8_kernel<false>, &cfg) == cudaSuccess && q > 0)
     n = q;
   cudaGetLastError();
   cached_dev = dev; cached = n;
@@ -967,13 +984,13 @@ static int max_clusters() {
 
 static int launch_fp8_t(const CUtensorMap& map_q, const CUtensorMap& map_q_rope, const OutMaps& omaps,
                         const AttnParams& p, cudaStream_t stream) {
-  using PL = Plan;
-  auto kern = masked_mla_fp8_kernel;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL::kSmem) != cudaSuccess)
+  const int dev = current_device();
+  const bool sliced = p.nsplit > 1;
+  if (!(sliced ? ensure_smem<masked_mla_fp8_kernel<true>>(dev, Plan::kSmem)
+               : ensure_smem<masked_mla_fp8_kernel<false>>(dev, Plan::kSmem)))
     return LITEDSA_ERR_CUDA;
-  kern<<<2 * min(p.ng * p.nsplit, max_clusters()), kAttnThreads, PL::kSmem, stream>>>(
-      map_q, map_q_rope, omaps, p);
-  return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  return launch_pdl(sliced ? masked_mla_fp8_kernel<true> : masked_mla_fp8_kernel<false>, dim3(2 * min(p.ng * p.nsplit, max_clusters(dev))), kAttnThreads,
+                    Plan::kSmem, stream, map_q, map_q_rope, omaps, p);
 }
 
 static int launch_fp8(const Fp8Args& a, void* const* outs, int n_out, cudaStream_t stream) {

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
+#include <atomic>
 #include <stdint.h>
 
 #include "../../include/litedsa_b200.h"
@@ -51,6 +52,7 @@ struct Fp8Args {
   float* part_o = nullptr;
   void* part_ml = nullptr;
 };
+constexpr float kFp8LseOffset = 1.9459101090932196f;   // ln 7: the FP8 kernel's P carry a factor 7
 int check_fp8_args(const Fp8Args& a);                                   // no CUDA call
 // attn_dsv4.cu: classify the tiles' index lists and enqueue the range kernel in rank mode, gated on
 // "every list is two contiguous runs" (workspace: 16 + 16 * ng bytes; word 0 is the gate)
@@ -62,6 +64,53 @@ int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, con
                       int64_t out_token_stride, int64_t out_head_stride, void* workspace,
                       cudaStream_t stream);
 int run_fp8(const Fp8Args& a, void* const* outs, int n_outs, void* stream);
+// prefill.cu: merge of the slices of ng tiles (see there); out strides in ELEMENTS
+constexpr int kMaxSlices = 16;
+int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
+                 const float* sink, int sink_mod, void* out, int64_t out_token_stride, int64_t out_head_stride,
+                 float* lse, cudaStream_t stream);
+
+// ---------------------------------------------------------------- launches
+// Raises a kernel's dynamic shared-memory limit on the current device, once per size (the call
+// costs as much host time as a launch).
+constexpr int kMaxDevices = 64;
+template <auto kKernel>
+inline bool ensure_smem(int dev, size_t bytes) {
+  static std::atomic<int> have[kMaxDevices];
+  if (dev < 0 || dev >= kMaxDevices) return false;
+  if (have[dev].load(std::memory_order_relaxed) >= (int)bytes) return true;
+  if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  int old = have[dev].load(std::memory_order_relaxed);
+  while (old < (int)bytes && !have[dev].compare_exchange_weak(old, (int)bytes)) {}
+  return true;
+}
+inline int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+// Launch that may start while its predecessor on the stream is still running (programmatic
+// dependent launch): launch latency, block scheduling and everything a kernel does before
+// pdl_wait() (barriers, tensor memory, shared-memory clears) overlap the predecessor's tail.  Every
+// kernel launched this way calls pdl_wait() before its first access to global memory; it
+// returns when the predecessor has completed, and since that one has waited too, everything
+// before it as well.  pdl_trigger(): this kernel's blocks are all running or done, successors may
+// be scheduled into whatever room is left.
+template <class K, class... A>
+inline int launch_pdl(K kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- addresses / cluster
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -111,6 +111,8 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
   }
+  pdl_trigger();
+  pdl_wait();
   // head weights of the CTA's tokens: column c of accumulator a is row tok0 * Hi + 256 a + c.
   // Halved: the drain computes relu(x) as (x + |x|) / 2 with the division folded in here.
   for (int i = threadIdx.x; i < 2 * kCols; i += kThreads) {
@@ -458,6 +460,8 @@ topk_select_kernel(const SelParams p) {
   constexpr int NT = kGenericThreads;
   extern __shared__ __align__(16) uint32_t rowkeys[];
   __shared__ SelShared sh;
+  pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x, tid = threadIdx.x;
   const int n = p.lengths ? min(max(p.lengths[t], 0), p.S) : min(p.S, max(p.q_pos0 + t + 1, 0));
   int32_t* out = p.out + (long long)t * p.k;
@@ -693,6 +697,8 @@ topk_select_stream_kernel(const SelParams p) {
     fence_mbar_init();
   }
   __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   if (tid == 0 && (int)blockIdx.x < p.T) fetch(blockIdx.x);
   uint32_t phase = 0;
 
@@ -899,6 +905,8 @@ topk_select_chunked_kernel(const SelParams p) {
     ++gf;
     if (++cf == chunks_of(n)) { cf = 0; tf += gridDim.x; skip_short(); }
   };
+  pdl_trigger();
+  pdl_wait();
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -957,6 +965,8 @@ topk_select_cluster_kernel(const SelParams p, int nc) {
   __shared__ float red_a[NT / 32], red_b[NT / 32];
   __shared__ uint32_t eq_total, seg_cnt[8];           // seg_cnt: leader CTA, survivors per segment
   const Waiter wt{g_status, p.epoch, p.wait_limit_ns};
+  pdl_trigger();
+  pdl_wait();
   const int tid = threadIdx.x, rank = (int)cluster_ctarank(), t = blockIdx.x / nc;
   const int n = p.lengths ? min(max(p.lengths[t], 0), p.S) : min(p.S, max(p.q_pos0 + t + 1, 0));
   int32_t* out = p.out + (long long)t * p.k;
@@ -1055,8 +1065,9 @@ extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, 
   p.weights = weights; p.k_scale = k_scale; p.logits = logits;
   p.T = T; p.Hi = Hi; p.S = S; p.q_pos0 = q_pos0; p.ld = logits_row_stride;
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
-  auto kern = Hi == 32 ? index_logits_kernel<32> : (Hi == 64 ? index_logits_kernel<64> : index_logits_kernel<128>);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
+  const int dev = current_device();
+  if (!(Hi == 32 ? ensure_smem<index_logits_kernel<32>>(dev, kSmem)
+                 : (Hi == 64 ? ensure_smem<index_logits_kernel<64>>(dev, kSmem) : ensure_smem<index_logits_kernel<128>>(dev, kSmem))))
     return LITEDSA_ERR_CUDA;
   const int tok_per_cta = 2 * (kCols / Hi);
   const int ctas_x = (T + tok_per_cta - 1) / tok_per_cta;
@@ -1066,8 +1077,8 @@ extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, 
   const int splits = pick_splits(ctas_x, live_tiles, sm_count());
   p.tiles_per_split = (live_tiles + splits - 1) / splits;
   const int grid_y = (all_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
-  kern<<<dim3(ctas_x, grid_y), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream)>>>(map_q, map_k, p);
-  return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  return launch_pdl(Hi == 32 ? index_logits_kernel<32> : (Hi == 64 ? index_logits_kernel<64> : index_logits_kernel<128>),
+                    dim3(ctas_x, grid_y), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_k, p);
 }
 
 // Exact top-k per row of `logits`: topk_idx[t, :] = the k positions i < len(t) with the largest
@@ -1087,55 +1098,48 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
   p.T = T; p.S = S; p.k = k; p.q_pos0 = q_pos0; p.ld = logits_row_stride;
   p.epoch = lt::next_launch_epoch(); p.wait_limit_ns = lt::wait_limit_ns();
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // rows up to 32768 entries live in registers (512 threads x 64 or 32 consecutive positions,
-  // transposed through shared memory); longer rows stay in shared memory up to 49152 entries
-  // and are re-read from memory by every pass beyond that
+  // aligned rows up to 32768 entries live in registers, longer ones stream through shared memory;
+  // unaligned ones are kept in shared memory up to 49152 entries and re-read from memory beyond
   const size_t smem = (((size_t)S + 3) & ~(size_t)3) * 4;      // whole 16-byte quads
-  auto launch = [&](auto kern, int threads, size_t dyn) -> int {
-    if (dyn && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
-      return LITEDSA_ERR_CUDA;
-    kern<<<T, threads, dyn, st>>>(p);
-    return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
-  };
+  const int dev = lt::current_device();
   const bool aligned = (logits_row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
-  const int sms = sm_count();
+  const int sms = sm_count(), grid = T < sms ? T : sms;
   const size_t chunk_dyn = (size_t)2 * kChunk * 4 + (size_t)kSurvCap * 8;
   // Few rows: as many CTAs per row as the chip has for each, if every one of them gets at least
   // 4096 entries (below that the extra cluster synchronisations cost what the shorter filter saves)
   int nc = 8;
   while (nc > 1 && ((long long)T * nc > sms || S < 4096 * nc)) nc >>= 1;
   if (aligned && nc > 1) {
-    if (cudaFuncSetAttribute(topk_select_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)chunk_dyn) != cudaSuccess)
-      return LITEDSA_ERR_CUDA;
+    if (!lt::ensure_smem<topk_select_cluster_kernel>(dev, chunk_dyn)) return LITEDSA_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(T * nc)); cfg.blockDim = dim3(kStreamThreads);
     cfg.dynamicSmemBytes = chunk_dyn; cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)nc; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.attrs = &at; cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)nc; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel, (const SelParams)p, nc) == cudaSuccess
                ? LITEDSA_OK : LITEDSA_ERR_CUDA;
   }
   if (aligned && S <= kStreamThreads * 64) {
-    const int grid = T < sms ? T : sms;
-    auto kern = S <= kStreamThreads * 32 ? topk_select_stream_kernel<32> : topk_select_stream_kernel<64>;
+    const bool small = S <= kStreamThreads * 32;
     const size_t dyn = smem + (size_t)kSurvCap * 6;      // + survivor values (fp32) and positions (u16)
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
+    if (!(small ? lt::ensure_smem<topk_select_stream_kernel<32>>(dev, dyn) : lt::ensure_smem<topk_select_stream_kernel<64>>(dev, dyn)))
       return LITEDSA_ERR_CUDA;
-    kern<<<grid, kStreamThreads, dyn, st>>>(p);
-    return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+    return lt::launch_pdl(small ? topk_select_stream_kernel<32> : topk_select_stream_kernel<64>, dim3(grid),
+                          kStreamThreads, dyn, st, p);
   }
   if (aligned) {
-    if (cudaFuncSetAttribute(topk_select_chunked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)chunk_dyn) != cudaSuccess)
-      return LITEDSA_ERR_CUDA;
-    topk_select_chunked_kernel<<<T < sms ? T : sms, kStreamThreads, chunk_dyn, st>>>(p);
-    return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+    if (!lt::ensure_smem<topk_select_chunked_kernel>(dev, chunk_dyn)) return LITEDSA_ERR_CUDA;
+    return lt::launch_pdl(topk_select_chunked_kernel, dim3(grid), kStreamThreads, chunk_dyn, st, p);
   }
-  if (S <= kMaxSmemRow) return launch(topk_select_kernel<true>, kGenericThreads, smem);
-  return launch(topk_select_kernel<false>, kGenericThreads, 0);
+  if (S <= kMaxSmemRow) {
+    if (!lt::ensure_smem<topk_select_kernel<true>>(dev, smem)) return LITEDSA_ERR_CUDA;
+    return lt::launch_pdl(topk_select_kernel<true>, dim3(T), kGenericThreads, smem, st, p);
+  }
+  return lt::launch_pdl(topk_select_kernel<false>, dim3(T), kGenericThreads, 0, st, p);
 }
 
 // Status block of the index-logits kernel (same layout as litedsa_attn_status).

@@ -1,0 +1,186 @@
+// The whole path of one chunk of query tokens behind one call: union of the tiles' top-k lists,
+// masked attention over it, and -- for chunks of few tokens -- the merge of the tiles' slices.
+//
+// What one call costs beyond its kernels matters for small chunks: as separate operators (each
+// with its own checks, output allocations and ctypes call) two tokens took 70 us of host time
+// around 38 us of kernels.  Here the intermediate tensors live in one caller-owned workspace.
+//
+// Few tiles leave most of the chip idle while each of them walks its union list serially (one
+// cluster of two SMs per tile, about 1.3 us per 128-key block).  Such tiles are cut into slices
+// (pick_slices) that run as separate work items of the attention kernel; every slice leaves its
+// unnormalised fp32 O with its running max and row sum, and merge_slices_kernel brings them to a
+// common max, normalises and rounds once -- the same fp32 accumulation as the unsliced tile, in
+// another order.  The reference leaves KV splits to its callers
+// (kernels/b200/dsa/litedsa_attention_sm100.cuh:1383-1385).
+#include "common.cuh"
+
+namespace lt {
+namespace prefill {
+
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLn2 = 0.6931471805599453f;
+
+// out = out_scale * sum_j O_j 2^(m_j - M) / (sum_j l_j 2^(m_j - M) + sink), lse = ln(sum) + M ln 2 - lse_off
+// (the sink joins the output's normaliser only; row r of a tile = token r / h, head r % h).
+// One warp per row: lane i holds dims 128 c + 4 i .. + 3 of the four 128-dim pieces.  HBM / L2
+// bound in principle (2 KB per slice and row), latency-bound at the sizes it runs at: all slices'
+// loads of a piece are independent.
+__global__ void __launch_bounds__(128)
+merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml, int nsplit, int n_rows, int h,
+                    float out_scale, float lse_off, const float* __restrict__ sink, int sink_mod,
+                    __nv_bfloat16* __restrict__ out, long long out_ts, long long out_hs, float* __restrict__ lse) {
+  const int row = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  if (row >= n_rows) return;
+  pdl_wait();
+  const int tile = row >> 7, r = row & 127;
+  const size_t p0 = (size_t)tile * nsplit * 128 + r;            // slice j of the row: p0 + 128 j
+  float2 ml = make_float2(-INFINITY, 0.f);
+  if (lane < nsplit) ml = __ldg(part_ml + p0 + (size_t)lane * 128);
+  float m = ml.y > 0.f ? ml.x : -INFINITY;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  const float f = ml.y > 0.f ? fast_exp2(ml.x - m) : 0.f;       // slices without a key weigh nothing
+  float l = ml.y * f;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+  float4 acc[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j = 0; j < nsplit; ++j) {
+    const float fj = __shfl_sync(0xffffffffu, f, j);
+    if (fj == 0.f) continue;                                    // warp-uniform
+    const float4* src = reinterpret_cast<const float4*>(part_o + (p0 + (size_t)j * 128) * 512) + lane;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float4 v = __ldg(src + 32 * c);
+      acc[c].x = fmaf(v.x, fj, acc[c].x);
+      acc[c].y = fmaf(v.y, fj, acc[c].y);
+      acc[c].z = fmaf(v.z, fj, acc[c].z);
+      acc[c].w = fmaf(v.w, fj, acc[c].w);
+    }
+  }
+  float denom = l;
+  if (sink != nullptr && l > 0.f) denom += fast_exp2(__ldg(sink + r % sink_mod) * kLog2e - m);
+  const float os = l > 0.f ? __fdividef(out_scale, denom) : 0.f;
+  uint2* dst = reinterpret_cast<uint2*>(out + (row / h) * out_ts + (row % h) * out_hs) + lane;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(acc[c].x * os, acc[c].y * os);
+    const __nv_bfloat162 b = __floats2bfloat162_rn(acc[c].z * os, acc[c].w * os);
+    dst[32 * c] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  }
+  if (lane == 0) lse[row] = l > 0.f ? __logf(l) + m * kLn2 - lse_off : INFINITY;
+}
+
+// How many slices a tile is cut into when a launch has `tiles` tiles of lists up to `cap` long: as
+// many as there are idle clusters for, at least 512 list entries each (a slice costs a block of its own
+// for the running max, an epilogue and its share of the merge), none when more
+// than half of the clusters have a tile of their own anyway.
+static int pick_slices(int tiles, int cap) {
+  constexpr int kClusters = 74;
+  int n = kClusters / tiles;
+  if (n > cap / 512) n = cap / 512;
+  if (n > kMaxSlices) n = kMaxSlices;
+  return n < 2 ? 1 : n;
+}
+
+// workspace layout: all offsets are multiples of 256 bytes
+struct Layout { int64_t counts, u, memb, part_o, part_ml, total; };
+static Layout layout_of(int ng, int G, int cap, int nsplit) {
+  auto up = [](int64_t b) { return (b + 255) & ~(int64_t)255; };
+  Layout l;
+  l.counts = 0;
+  l.u = up(4 * (int64_t)ng);
+  l.memb = l.u + up(4 * (int64_t)ng * cap);
+  l.part_o = l.memb + up(4 * (int64_t)ng * G * (cap / 32));
+  l.part_ml = l.part_o + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 512 * 4) : 0);
+  l.total = l.part_ml + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 8) : 0);
+  return l;
+}
+
+static int check_shape(int T, int h, int k, int policy_tokens) {
+  if (h <= 0 || 128 % h != 0 || 128 / h > 16 || T <= 0 || T % (128 / h) != 0 || k <= 0) return LITEDSA_ERR_SHAPE;
+  if (policy_tokens < T) return LITEDSA_ERR_SHAPE;
+  if ((int64_t)(128 / h) * k > 65536) return LITEDSA_ERR_UNSUPPORTED;      // 16-bit ranks (union_qm)
+  return LITEDSA_OK;
+}
+
+}  // namespace prefill
+
+int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
+                 const float* sink, int sink_mod, void* out, int64_t out_token_stride, int64_t out_head_stride,
+                 float* lse, cudaStream_t stream) {
+  return launch_pdl(prefill::merge_slices_kernel, dim3((ng * 128 + 3) / 4), 128, 0, stream, part_o, part_ml, nsplit,
+                    ng * 128, h, out_scale, lse_off, sink, sink_mod, reinterpret_cast<__nv_bfloat16*>(out),
+                    (long long)out_token_stride, (long long)out_head_stride, lse);
+}
+}  // namespace lt
+
+// Bytes of workspace litedsa_sparse_prefill needs (0: the shape is not supported).
+extern "C" int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens) {
+  using namespace lt::prefill;
+  if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
+  const int G = 128 / h, cap = G * k;
+  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, cap);
+  return layout_of(T / G, G, cap, ns).total;
+}
+
+// union_qm + masked attention of T query tokens in one call; see include/litedsa_b200.h.
+extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
+                                      const int32_t* topk_idx, float sm_scale, float q_scale, float kv_scale,
+                                      void* out, float* lse, int T, int h, int k, int s_kv,
+                                      int64_t kv_row_stride, int64_t seq_space, int policy_tokens,
+                                      void* workspace, int64_t workspace_bytes, void* stream) {
+  using namespace lt;
+  using namespace lt::prefill;
+  if (!q || !kv || !topk_idx || !out || !lse || !workspace) return LITEDSA_ERR_ARG;
+  int rc = check_shape(T, h, k, policy_tokens);
+  if (rc != LITEDSA_OK) return rc;
+  if (kv_is_bf16 && !q_is_bf16) return LITEDSA_ERR_UNSUPPORTED;
+  if (!kv_is_bf16 && q_is_bf16 && !(q_scale > 0.f)) return LITEDSA_ERR_SHAPE;
+  if (((uintptr_t)workspace & 255) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)topk_idx & 15))
+    return LITEDSA_ERR_UNSUPPORTED;
+  const int G = 128 / h, ng = T / G, cap = G * k;
+  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, cap);
+  const Layout l = layout_of(ng, G, cap, ns);
+  if (workspace_bytes < l.total) return LITEDSA_ERR_SHAPE;
+  char* ws = reinterpret_cast<char*>(workspace);
+  int32_t* counts = reinterpret_cast<int32_t*>(ws + l.counts);
+  int32_t* u = reinterpret_cast<int32_t*>(ws + l.u);
+  uint32_t* memb = reinterpret_cast<uint32_t*>(ws + l.memb);
+  // fill mode 2: lists padded to whole 128-key blocks, nothing written beyond
+  rc = litedsa_union_qm(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
+  if (rc != LITEDSA_OK) return rc;
+  if (kv_is_bf16)
+    return litedsa_masked_mla_bf16(q, kv, u, sm_scale, counts, memb, h, out, nullptr, lse, ng, s_kv, cap, 576, 576,
+                                   kv_row_stride, cap, nullptr, stream);
+  Fp8Args a{q, kv, u, sm_scale * q_scale * kv_scale, kv_scale, counts, memb, h, nullptr, lse,
+            ng, s_kv, cap, 576, kv_row_stride, cap, nullptr, nullptr, 1};
+  a.q_is_bf16 = q_is_bf16 != 0;
+  a.q_inv = 1.0f / q_scale;
+  a.nsplit = ns;
+  a.part_o = reinterpret_cast<float*>(ws + l.part_o);
+  a.part_ml = ws + l.part_ml;
+  void* outs[1] = {out};
+  rc = run_fp8(a, outs, 1, stream);
+  if (rc != LITEDSA_OK || ns == 1) return rc;
+  return merge_slices(a.part_o, reinterpret_cast<const float2*>(a.part_ml), ns, ng, h, kv_scale, kFp8LseOffset,
+                      nullptr, 1, out, (int64_t)h * 512, 512, lse, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// litedsa_masked_mla_fp8 on bf16 queries, quantised inside the attention kernel.
+extern "C" int litedsa_masked_mla_fp8_bf16q(const void* q_bf16, float q_scale, const void* kv8, const int32_t* indices,
+                                            float sm_scale, float out_scale, const int32_t* topk_length,
+                                            const uint32_t* memb_qm, int h_per_q, void* out, float* max_logits,
+                                            float* lse, int ng, int s_kv, int topk, int64_t kv_row_stride,
+                                            int64_t indices_row_stride, void* stream) {
+  using namespace lt;
+  if (!memb_qm || !out) return LITEDSA_ERR_ARG;
+  if (!(q_scale > 0.f)) return LITEDSA_ERR_SHAPE;
+  Fp8Args a{q_bf16, kv8, indices, sm_scale, out_scale, topk_length, memb_qm, h_per_q, max_logits, lse,
+            ng, s_kv, topk, 576, kv_row_stride, indices_row_stride, nullptr, nullptr, 1};
+  a.q_is_bf16 = true;
+  a.q_inv = 1.0f / q_scale;
+  void* outs[1] = {out};
+  return run_fp8(a, outs, 1, stream);
+}

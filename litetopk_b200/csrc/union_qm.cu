@@ -35,7 +35,7 @@ struct UnionParams {
   int k, G, cap, s_words;   // s_words = seq_space / 32
   int rank_shift;           // rank table holds one entry per (1 << rank_shift) bitmap words
   int stage_list;           // 1: sorted list staged in smem
-  int fill_tail;            // 1: also write -1 / 0 beyond the live prefixes
+  int fill_tail;            // 1: also write -1 / 0 beyond the live prefixes; 2: -1 up to the next multiple of 128
 };
 
 // Shared-memory carve-up (bytes): bitmap | rank table (u16) | qm accumulator | list stage
@@ -85,6 +85,8 @@ union_qm_kernel(const UnionParams p) {
     uint4* b4 = reinterpret_cast<uint4*>(bm);
     for (int i = tid; i < (s_words >> 2); i += kUnionThreads) b4[i] = make_uint4(0, 0, 0, 0);
   }
+  pdl_trigger();
+  pdl_wait();
   // issue the tile's loads while the clear drains
   const int4* src = reinterpret_cast<const int4*>(p.idx + (size_t)g * total);
   const int nquad = total >> 2;
@@ -197,7 +199,7 @@ union_qm_kernel(const UnionParams p) {
   // sorted list -> global, 16-byte stores (the last quad is padded with -1)
   if (p.stage_list) {
     const int q_live = (live + 3) >> 2;
-    const int q_end = p.fill_tail ? (cap >> 2) : q_live;
+    const int q_end = p.fill_tail == 1 ? (cap >> 2) : (p.fill_tail == 2 ? ((live + 127) >> 7) << 5 : q_live);
     int4* dst = reinterpret_cast<int4*>(out_row);
     for (int i = tid; i < q_end; i += kUnionThreads) {
       int4 o;
@@ -209,13 +211,14 @@ union_qm_kernel(const UnionParams p) {
       dst[i] = o;
     }
   } else if (p.fill_tail) {
-    for (int i = live + tid; i < cap; i += kUnionThreads) out_row[i] = -1;
+    const int end = p.fill_tail == 1 ? cap : ((live + 127) >> 7) << 7;
+    for (int i = live + tid; i < end; i += kUnionThreads) out_row[i] = -1;
   }
 
   // phase 5: dump the live mask words (whole rows when fill_tail)
   {
     const int a4 = active >> 2, c4 = capw >> 2;
-    const int per_row = p.fill_tail ? c4 : a4;
+    const int per_row = p.fill_tail == 1 ? c4 : a4;
     uint4* dst = reinterpret_cast<uint4*>(p.memb + (size_t)g * p.G * capw);
     const uint4* s4 = reinterpret_cast<const uint4*>(qm_s);
     for (int i = tid; i < p.G * per_row; i += kUnionThreads) {
@@ -229,11 +232,11 @@ template <int NT, int VPT>
 static int launch_union(const UnionParams& p, int ng, size_t smem, cudaStream_t stream) {
   constexpr int kUnionThreads = NT;
   const bool plain = p.btab == nullptr && p.rank_shift == 0;
-  auto kern = plain ? union_qm_kernel<NT, VPT, true> : union_qm_kernel<NT, VPT, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return LITEDSA_ERR_CUDA;
-  kern<<<ng, kUnionThreads, smem, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  const int dev = current_device();
+  if (!(plain ? ensure_smem<union_qm_kernel<NT, VPT, true>>(dev, smem) : ensure_smem<union_qm_kernel<NT, VPT, false>>(dev, smem)))
+    return LITEDSA_ERR_CUDA;
+  return launch_pdl(plain ? union_qm_kernel<NT, VPT, true> : union_qm_kernel<NT, VPT, false>, dim3(ng), kUnionThreads,
+                    smem, stream, p);
 }
 
 }  // namespace lt
@@ -266,7 +269,7 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
   p.bt_stride = bt_blocks; p.bt_blocks = bt_blocks; p.bsz = block_table ? block_size : 1;
   p.bsz_mul = fast_div_mul(int64_t(s_words) * 32, p.bsz);
   p.kq = k / 4; p.kq_mul = fast_div_mul(int64_t(G) * (k / 4), k / 4);
-  p.k = k; p.G = G; p.cap = cap; p.s_words = s_words; p.fill_tail = fill_tail ? 1 : 0;
+  p.k = k; p.G = G; p.cap = cap; p.s_words = s_words; p.fill_tail = fill_tail == 2 ? 2 : (fill_tail ? 1 : 0);
   // pick the richest shared-memory plan that fits (227 KB per CTA on sm_100)
   const size_t limit = 220 * 1024;
   p.rank_shift = 0; p.stage_list = 1;

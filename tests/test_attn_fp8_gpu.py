@@ -444,3 +444,40 @@ def test_path_agrees_with_the_stock_per_token_sparse_mla_kernel():
     assert cos >= 0.9995, (mad, cos)                     # e4m3 P against a bf16 kernel
     assert float((lse - lse_ref).abs().max()) <= TOL_LSE
     assert api.attn_status()[0] == 0
+
+
+@pytest.mark.parametrize("tokens,heads,topk,s_kv", [
+    (2, 64, 2048, 32768),       # one tile, four slices of five blocks
+    (2, 64, 512, 4096),         # too short to slice
+    (34, 64, 1024, 8192),       # 17 tiles, two slices
+    (8, 16, 2048, 20000),       # one tile of eight tokens, sixteen slices
+    (300, 32, 256, 5000),       # 75 tiles: one more than clusters
+])
+@pytest.mark.parametrize("qdtype", ["bf16", "e4m3"])
+def test_sparse_prefill_in_one_call_equals_its_operators(tokens, heads, topk, s_kv, qdtype):
+    def mutate(idx):
+        idx = idx.clone()
+        idx[0, topk // 2:] = -1             # a short list
+        idx[1, :] = -1                      # a token without a key
+        return idx
+    w, idx, kv, q = _case(tokens, heads, topk, s_kv, (0.6, 0.8), seed=11, mutate=mutate)
+    q8, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    qd = q.to(DEV) if qdtype == "bf16" else q8.view(tokens, heads, 576).to(DEV)
+    kvd, idd = kv8.to(DEV), idx.to(DEV)
+    u, m, c = api.union_qm(idd, w.group, seq_space=s_kv, return_counts=True)
+    api.attn_status(reset=True)
+    want_o, want_l = api.masked_mla_fp8(q8.view(tokens, heads, 576).to(DEV), kvd, u, m, synth.SM_SCALE, counts=c,
+                                        kv_scale=ks, q_scale=qs)
+    # a chunk of a large job: no slices, the same kernels on the same operands
+    o1, l1 = api._sparse_prefill(qd, kvd, idd, synth.SM_SCALE, ks, qs, None, None, None, 100000)
+    assert torch.equal(o1, want_o) and torch.equal(l1, want_l)
+    # on its own: slices.  Their running maxima differ from the unsliced tile's, hence the e4m3
+    # rounding of P (relative 2^-4 at most per weight): the bounds of the KV-split test above
+    o2, l2 = api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    torch.cuda.synchronize()
+    assert api.attn_status()[0] == 0
+    mad, cos = ao.compare(o2.cpu(), want_o.cpu())
+    assert mad <= 0.1 and cos >= 0.9995, (mad, cos)
+    fin = torch.isfinite(want_l)
+    assert torch.equal(torch.isfinite(l2), fin) and bool((o2[~fin] == 0).all())
+    assert float((l2[fin] - want_l[fin]).abs().max()) <= TOL_LSE

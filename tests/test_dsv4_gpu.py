@@ -93,3 +93,24 @@ def test_dsv4_in_place_padded_heads(h, hpad):
     assert got_o.data_ptr() == out_pad.data_ptr()
     assert torch.equal(out_pad[:, :h], want_o) and torch.equal(got_l, want_l)
     assert bool((out_pad[:, h:] == 7.0).all())
+
+
+@pytest.mark.parametrize("T,h,S,Nc,pos0,sink", [
+    (24, 16, 77777, 607, 77777 - 24, True),     # three tiles, four slices each, sink per head
+    (8, 16, 131072, 1024, 131072 - 8, False),   # one tile of 19 blocks, six slices
+    (16, 8, 40000, 312, 20001, True),           # one tile of sixteen tokens in the middle of the cache
+    (2, 64, 9000, 70, 300, False),              # five blocks: one slice
+])
+def test_dsv4_few_tiles_run_in_slices(T, h, S, Nc, pos0, sink):
+    _run(T, h, S, Nc, pos0, sink=sink, seed=T + h)
+    # slices in the model's own padded output tensor
+    g = torch.Generator(device=DEV).manual_seed(3)
+    q = torch.randn((T, h, 576), generator=g, device=DEV).to(torch.bfloat16)
+    kc = torch.randn((Nc, 576), generator=g, device=DEV).to(torch.bfloat16)
+    kr = torch.randn((S, 576), generator=g, device=DEV).to(torch.bfloat16)
+    want_o, want_l = api.dsv4_c128a_bf16(q, kc, kr, pos0, synth.SM_SCALE)
+    out = torch.full((T, h + 8, 512), 7.0, dtype=torch.bfloat16, device=DEV)
+    got_o, got_l = api.dsv4_c128a_bf16(q, kc, kr, pos0, synth.SM_SCALE, heads=h, out=out)
+    torch.cuda.synchronize()
+    assert torch.equal(out[:, :h], want_o) and torch.equal(got_l, want_l) and bool((out[:, h:] == 7.0).all())
+    assert api.dsv4_status()[0] == 0
