@@ -109,6 +109,7 @@ struct Misc {
   uint64_t m_pub[2];                // running max of block k published by softmax group k%2
   uint64_t q_land;                  // every CTA: this CTA's Q tile has landed in its slot (e4m3 q);
                                     // its slot is free for the epilogue warps to fill (bf16 q)
+  uint64_t q_taken;                 // every CTA: the item's Q has been moved out of its slot
   uint64_t qt_ready;                // leader CTA: Q's latent part is in tensor memory in both CTAs
   uint64_t q_free;                  // all QK^T of the current item are complete (Q reusable)
   uint64_t o_free;                  // leader CTA: the item's O has been read out of TMEM
@@ -235,6 +236,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_land, 1);
+    mbar_init(&ms.q_taken, 1);
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
@@ -491,7 +493,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     // requests the tile (TMA) or, for bf16 q, hands the slot to the epilogue warps.  (Only here: a
     // slot's barrier may be waited on once every older entry has been through it, which this
     // warp's own K copies prove.)
-    int q_w = cid, q_slot = 0, q_ring = 0;
+    // The previous item's Q must have been moved on: with short items its bytes could still be in flight.
+    int q_w = cid, q_slot = 0, q_ring = 0, q_n = 0;      // q_n: items whose Q has been requested
     bool q_pending = pw == 0 && cid < n_items;
     const uint64_t pol_stream = l2_policy_evict_first();
     auto cur_load = [&](Cursor& c) {
@@ -561,7 +564,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         }
       }
       if (q_pending) {                             // warp-uniform; warp 0 only
-        const bool ok = q_ring == 0 || mbar_test(&ms.slot_free[q_slot], (q_ring - 1) & 1);
+        const bool ok = (q_ring == 0 || mbar_test(&ms.slot_free[q_slot], (q_ring - 1) & 1)) &&
+                        (q_n == 0 || mbar_test(&ms.q_taken, (q_n - 1) & 1));
         if (__all_sync(0xffffffffu, ok)) {
           if (lane == 0) {
             if (p.q_bf16 != nullptr) {
@@ -579,6 +583,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
           }
           __syncwarp();
           q_pending = false;
+          ++q_n;
           did = true;
         }
       }
@@ -630,14 +635,34 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp < kWarpEpi0) {
    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+   // running position of an MMA-issuing warp: work item, block of the item, blocks of the item, item
+   // ordinal, running block number, ring slot
+   struct MmaCursor { int w, k, nb, it, kb, slot; };
+   auto mma_next = [&](MmaCursor& c) {
+     ++c.kb;
+     if (++c.slot == kSlots) c.slot = 0;
+     if (++c.k == c.nb) {
+       c.w += ncl; c.k = 0; ++c.it;
+       if (++c.slot == kSlots) c.slot = 0;       // the next item's Q entry
+       c.nb = c.w < n_items ? item_of(c.w).nb : 0;
+     }
+   };
+   // the time-limit and abort check of a wait that has not been satisfied yet (warp-uniform answer)
+   auto mma_idle = [&](unsigned long long& since, int site, int kb) -> bool {
+     const unsigned long long now = globaltimer_ns();
+     if (since == 0) since = now;
+     bool stop = wt.aborting();
+     if (now - since > wt.limit_ns) {
+       if (lane == 0) wt.fail(site, kb);
+       stop = true;
+     }
+     return __any_sync(0xffffffffu, stop);
+   };
    if (warp == kWarpMma) {
     // ------------------------------------------------------------ MMA issue (leader CTA only)
     if (cta == 0) {   // the whole warp runs this loop; one elected lane issues
       constexpr uint32_t idesc_qk = umma_idesc(0, 0, false, false, 128, 128);
-      constexpr uint32_t idesc_pv = umma_idesc(0, 0, false, true, 128, 256);
       const uint32_t a_qk_done0 = smem_u32(&ms.qk_done[0]), a_qk_done0_peer = mapa(a_qk_done0, 1);
-      const uint32_t a_pv_done0 = smem_u32(&ms.pv_done[0]), a_pv_done0_peer = mapa(a_pv_done0, 1);
-      const uint32_t a_slot_free0 = smem_u32(&ms.slot_free[0]), a_slot_free0_peer = mapa(a_slot_free0, 1);
       const uint32_t a_q_free_peer = mapa(smem_u32(&ms.q_free), 1);
       // S = Q K^T of block kb into S buffer kb%2
       // (the K / V rows were written by cp.async (generic proxy) and are read by the tensor core
@@ -656,6 +681,37 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         mma_commit_pair_elect(a_qk_done0 + 8u * (uint32_t)(kb & 7));
         mma_commit_pair_elect(a_qk_done0_peer + 8u * (uint32_t)(kb & 7));
       };
+      // Two warps issue the MMAs, this one QK^T and the next one PV: each waits for its own operands and
+      // the tensor pipe takes what comes first.  One flat loop over a cursor whose every decision is a
+      // vote: the compiler then keeps the MMA operands in uniform registers (nested loops with
+      // breaks: 53 cycles to issue an MMA instead of 23).
+      MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, 1};
+      bool aborted = false;
+      unsigned long long since = 0;
+      while (c.w < n_items && !aborted) {
+        // K rows landed on both CTAs, S buffer drained and, for an item's first block, Q in place
+        const uint32_t ph = (c.kb >> 3) & 1;
+        const bool ok = (c.k > 0 || mbar_try_wait(&ms.qt_ready, c.it & 1)) && mbar_try_wait(&ms.k_land[c.kb & 7], ph) &&
+                        mbar_try_wait(&ms.k_peer[c.kb & 7], ph) &&
+                        (c.kb < 2 || mbar_try_wait(&ms.s_free[c.kb & 1], ((c.kb >> 1) & 1) ^ 1));
+        if (__all_sync(0xffffffffu, ok)) {
+          issue_qk(c.kb, c.slot);
+          if (c.k == c.nb - 1) {      // Q is no longer needed once these MMAs complete
+            mma_commit_pair_elect(smem_u32(&ms.q_free));
+            mma_commit_pair_elect(a_q_free_peer);
+          }
+          mma_next(c);
+          since = 0;
+        } else {
+          aborted = mma_idle(since, kSiteKLand, c.kb);
+        }
+      }
+    }
+   } else if (warp == kWarpRelayK && cta == 0) {
+      // ---------------------------------------------------------- PV issue (leader CTA)
+      constexpr uint32_t idesc_pv = umma_idesc(0, 0, false, true, 128, 256);
+      const uint32_t a_pv_done0 = smem_u32(&ms.pv_done[0]), a_pv_done0_peer = mapa(a_pv_done0, 1);
+      const uint32_t a_slot_free0 = smem_u32(&ms.slot_free[0]), a_slot_free0_peer = mapa(a_slot_free0, 1);
       auto issue_pv = [&](int k, int kb, int slot) {
         fence_proxy_async_smem();
         tc_fence_after();
@@ -668,71 +724,24 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         mma_commit_pair_elect(a_pv_done0 + 8u * (uint32_t)(kb & 3));
         mma_commit_pair_elect(a_pv_done0_peer + 8u * (uint32_t)(kb & 3));
       };
-      // Ready-driven issue over two cursors: whichever of "next QK^T" (its K rows landed on both
-      // CTAs, its S buffer drained and, for an item's first block, its Q in place) and "next PV" (its
-      // P written, its V rows landed on both CTAs and, for an item's first PV, the previous item's O
-      // read out) is ready goes first.  QK^T runs into the next item while this item's last PVs are
-      // still waiting for their P, but not further: Q(it + 2) is brought in only after epilogue it.
-      struct Cursor { int w, k, nb, it, kb, slot; };
-      auto next = [&](Cursor& c) {
-        ++c.kb;
-        if (++c.slot == kSlots) c.slot = 0;
-        if (++c.k == c.nb) {
-          c.w += ncl; c.k = 0; ++c.it;
-          if (++c.slot == kSlots) c.slot = 0;
-          c.nb = c.w < n_items ? item_of(c.w).nb : 0;
-        }
-      };
-      Cursor q{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, 1}, v = q;
+      MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, 1};
       bool aborted = false;
-      unsigned long long idle_since = 0;
-      unsigned idle_iters = 0;
-      while (v.w < n_items && !aborted) {
-        bool did = false;
-        {
-          const uint32_t ph = (v.kb >> 3) & 1;
-          // lanes poll independently: act only on what every lane has seen (keeps the warp converged)
-          const bool ok = v.kb < q.kb && mbar_test(&ms.p_ready[v.kb & 1], (v.kb >> 1) & 1) &&
-                          mbar_test(&ms.v_land[v.kb & 7], ph) && mbar_test(&ms.v_peer[v.kb & 7], ph) &&
-                          (v.k > 0 || v.it == 0 || mbar_test(&ms.o_free, (v.it - 1) & 1));
-          if (__all_sync(0xffffffffu, ok)) {
-            issue_pv(v.k, v.kb, v.slot);
-            next(v);
-            did = true;
-          }
-        }
-        if (q.w < n_items && q.it - v.it <= 1) {
-          const uint32_t ph = (q.kb >> 3) & 1;
-          const bool ok = mbar_test(&ms.k_land[q.kb & 7], ph) && mbar_test(&ms.k_peer[q.kb & 7], ph) &&
-                          (q.kb < 2 || mbar_test(&ms.s_free[q.kb & 1], ((q.kb >> 1) & 1) ^ 1)) &&
-                          (q.k > 0 || mbar_test(&ms.qt_ready, q.it & 1));
-          if (__all_sync(0xffffffffu, ok)) {
-            issue_qk(q.kb, q.slot);
-            if (q.k == q.nb - 1) {      // Q is no longer needed once these MMAs complete
-              mma_commit_pair_elect(smem_u32(&ms.q_free));
-              mma_commit_pair_elect(a_q_free_peer);
-            }
-            next(q);
-            did = true;
-          }
-        }
-        if (did) {
-          idle_since = 0;
-          idle_iters = 0;
-        } else if ((++idle_iters & (kIdleCheckEvery - 1)) != 0) {
-          __nanosleep(kIdleSleepNs);
+      unsigned long long since = 0;
+      while (c.w < n_items && !aborted) {
+        // V rows landed on both CTAs, P written; an item's first PV overwrites O: the previous item
+        // must have read it out
+        const uint32_t ph = (c.kb >> 3) & 1;
+        const bool ok = mbar_try_wait(&ms.v_land[c.kb & 7], ph) && mbar_try_wait(&ms.v_peer[c.kb & 7], ph) &&
+                        (c.k > 0 || c.it == 0 || mbar_try_wait(&ms.o_free, (c.it - 1) & 1)) &&
+                        mbar_try_wait(&ms.p_ready[c.kb & 1], (c.kb >> 1) & 1);
+        if (__all_sync(0xffffffffu, ok)) {
+          issue_pv(c.k, c.kb, c.slot);
+          mma_next(c);
+          since = 0;
         } else {
-          const unsigned long long now = globaltimer_ns();
-          if (idle_since == 0) idle_since = now;
-          bool stop = wt.aborting();
-          if (now - idle_since > wt.limit_ns) {
-            if (lane == 0) wt.fail(kSiteMmaIdle, v.kb);
-            stop = true;
-          }
-          aborted = __any_sync(0xffffffffu, stop);
+          aborted = mma_idle(since, kSitePReady, c.kb);
         }
       }
-    }
   } else if (warp == kWarpRelayK || warp == kWarpRelayV) {
     // ------------------------------------------------------------ "landed" relays to the leader CTA
     // The MMA thread lives in the leader CTA and can only wait on its own barriers: in the
@@ -862,7 +871,10 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(a_qt_ready);
       asm volatile("bar.sync 4, 128;" ::: "memory");      // all four warps have read the slot
-      if (e_tid == 0) mbar_arrive(&ms.slot_free[slot]);
+      if (e_tid == 0) {
+        mbar_arrive(&ms.slot_free[slot]);
+        mbar_arrive(&ms.q_taken);
+      }
     };
     int kb0 = 0, it = 0;
     if (cid < n_items) {

@@ -162,14 +162,15 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                "r"(bytes)
                : "memory");
 }
+constexpr uint32_t kSuspendHintNs = 20000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendHintNs)
       : "memory");
   return ok != 0;
 }
@@ -225,7 +226,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
                                           int iter = 0) {
   unsigned long long t0 = 0;
   for (uint32_t n = 1; !mbar_try_wait(bar, parity); ++n) {
-    if ((n & 255u) != 0) continue;
+    if ((n & 15u) != 0) continue;
     if (w.aborting()) return false;
     const unsigned long long now = globaltimer_ns();
     if (t0 == 0) t0 = now;
@@ -235,13 +236,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     }
   }
   return true;
-}
-
-// the same for a whole converged warp whose further way depends on the result: all lanes get the
-// same answer
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const Waiter& w, int site,
-                                               int iter = 0) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, w, site, iter));
 }
 
 // release at cluster scope: orders this thread's earlier (distributed) shared-memory stores
@@ -303,6 +297,11 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst_smem, const CUtens
       ".L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
       ::"r"(dst_smem), "l"(map), "r"(x), "r"(y), "r"(smem_u32(mbar)), "l"(pol)
       : "memory");
+}
+// the same tile brought into L2 only
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+               ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
 }
 // untiled bulk copy global -> this CTA's shared memory (both addresses 16-byte aligned, size a
 // multiple of 16), completion bytes on this CTA's own barrier

@@ -403,3 +403,14 @@ def test_dsv4_reference_signature_in_a_cuda_graph_switches_kernels_with_the_data
         torch.cuda.synchronize()
         assert torch.equal(out, want[0]) and torch.equal(lse, want[1])
     assert api.dsv4_status()[0] == 0 and api.bf16_status()[0] == 0
+
+
+@pytest.mark.parametrize("tokens,heads,topk", [(800, 64, 64), (320, 64, 96 * 2), (1200, 16, 32)])
+def test_native_many_short_tiles(tokens, heads, topk):
+    # several tiles per cluster with one to a few key blocks each (lists of 64 to 256 entries)
+    w, idx, kv, q = _native_case(tokens, heads, topk, 4096, (0.5, 0.9), seed=14)
+    api.bf16_status(reset=True)
+    out, lse = api.sparse_prefill(q.to(DEV), kv.to(DEV), idx.to(DEV), synth.SM_SCALE)
+    torch.cuda.synchronize()
+    assert api.bf16_status()[0] == 0
+    _check_exact(out, lse, q, kv, idx, tag="short tiles")

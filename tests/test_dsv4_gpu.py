@@ -114,3 +114,8 @@ def test_dsv4_few_tiles_run_in_slices(T, h, S, Nc, pos0, sink):
     torch.cuda.synchronize()
     assert torch.equal(out[:, :h], want_o) and torch.equal(got_l, want_l) and bool((out[:, h:] == 7.0).all())
     assert api.dsv4_status()[0] == 0
+
+
+def test_dsv4_many_short_tiles():
+    # 192 tiles of two to four blocks at the start of the sequence: short prefixes, clipped windows
+    _run(384, 64, 512, 4, 0, seed=9)
