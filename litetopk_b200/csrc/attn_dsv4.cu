@@ -66,7 +66,8 @@ static int pick_slices(int tiles, int blocks) {
 static int most_blocks(int ng, int G, int n_comp, int pos0, int window, int ratio) {
   const int64_t last = (int64_t)pos0 + (int64_t)ng * G - 1;
   const int64_t pref = min(last / ratio, (int64_t)n_comp);
-  return (int)((pref + kBlockKeys - 1) / kBlockKeys + (min(last + 1, (int64_t)window + G - 1) + kBlockKeys - 1) / kBlockKeys);
+  const int64_t halves = (pref + kOwnKeys - 1) / kOwnKeys + (min(last + 1, (int64_t)window + G - 1) + kOwnKeys - 1) / kOwnKeys;
+  return (int)((halves + 1) / 2);
 }
 static int64_t slice_bytes(int ng, int nsplit) {
   return nsplit < 2 ? 0 : (int64_t)ng * nsplit * 128 * (512 * 4 + 8);

@@ -151,10 +151,13 @@ enum { kSiteQ = 101, kSiteKFull, kSiteVFull, kSiteQkDone, kSitePvDone, kSiteVali
 // status block of the kernels of this translation unit (layout: see Waiter in common.cuh)
 static __device__ int g_status[8];
 
-// One work item: blocks [k0, k0 + nb) of a tile.  kRange / kRank: the first nbc blocks of the tile
-// walk len0 rows from row0, the others len1 rows from row1.  kGather: len0 list entries.
+// One work item: blocks [k0, k0 + nb) of a tile.  Half block 2 b + c (32 keys, the ones CTA c loads) is the
+// unit in which a tile's keys are laid out.  kRange / kRank: the first nh0 half blocks walk len0 rows
+// from row0, the others len1 rows from row1 -- a block may hold the end of one segment and the
+// start of the other (128-key windows of two tokens are 129 keys: five half blocks, not three
+// blocks).  kGather: len0 list entries.
 struct Item {
-  int tile, k0, nb, nbc, row0, len0, row1, len1;
+  int tile, k0, nb, nh0, row0, len0, row1, len1;
 };
 
 // bits [0, x) of a 32-bit word (x may be negative or beyond 32)
@@ -264,7 +267,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const int n_items = kSliced ? p.ng * p.nsplit : p.ng;
   // broadcast so the compiler knows the role index is warp-uniform
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  auto blocks_of = [](int n) -> int { return (n + kBlockKeys - 1) / kBlockKeys; };
+  auto halves_of = [](int n) -> int { return (n + kOwnKeys - 1) / kOwnKeys; };
   auto item_of = [&](int w) -> Item {
     Item t;
     t.tile = kSliced ? w / p.nsplit : w;
@@ -281,9 +284,9 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     } else {
       t.len0 = min(max(p.counts ? __ldg(p.counts + t.tile) : p.cap, 0), p.cap);
     }
-    t.nbc = blocks_of(t.len0);
+    t.nh0 = halves_of(t.len0);
     t.k0 = 0;
-    t.nb = max(t.nbc + blocks_of(t.len1), 1);     // an empty list: one fully masked block
+    t.nb = max((t.nh0 + halves_of(t.len1) + 1) / 2, 1);     // an empty list: one fully masked block
     if (kSliced) {            // slice `part`; an empty one runs a block beyond the list: fully masked
       const int part = w - t.tile * p.nsplit, all = t.nb;
       t.k0 = part * all / p.nsplit;
@@ -412,9 +415,9 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
         uint32_t vm;
         {
-          const int bk = item.k0 + k;
-          const bool seg0 = kSrc == kGather || bk < item.nbc;
-          const int base = (seg0 ? bk : bk - item.nbc) * kBlockKeys + 32 * h;   // within the segment
+          const int hb = 2 * (item.k0 + k) + h;
+          const bool seg0 = kSrc == kGather || hb < item.nh0;
+          const int base = (seg0 ? hb : hb - item.nh0) * kOwnKeys;            // within the segment
           const int off = (seg0 ? 0 : item.len0) + base;                      // list rank of column 0
           if (kSrc == kGather && mrow)
             vm = mk;
@@ -686,9 +689,9 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         if (!ok) break;
         for (int k = 0; k < item.nb; ++k, ++kb) {
-          const int bk = item.k0 + k;
-          const bool seg0 = bk < item.nbc;
-          const int row0 = seg0 ? item.row0 + bk * kBlockKeys : item.row1 + (bk - item.nbc) * kBlockKeys;
+          const int hb = 2 * (item.k0 + k) + (is_v ? (int)cta ^ 1 : (int)cta);
+          const bool seg0 = hb < item.nh0;
+          const int row0 = seg0 ? item.row0 + hb * kOwnKeys : item.row1 + (hb - item.nh0) * kOwnKeys;
           const CUtensorMap* m = seg0 ? &map_kv0 : &map_kv1;
           const uint32_t dst = sbase + PL::kOffKV + slot * PL::kSlot;
           if (!is_v) {
@@ -697,7 +700,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             if (!ok) break;
             if (cta == 0) mbar_arrive_expect_tx(&ms.k_full[kb & 7], 2 * PL::kSlot);
             for (int j = 0; j < kChunks; ++j)
-              tma_load_2d_pair(dst + j * kChunkBytes, m, 64 * j, row0 + kOwnKeys * (int)cta, a_k_full + 8u * (uint32_t)(kb & 7));
+              tma_load_2d_pair(dst + j * kChunkBytes, m, 64 * j, row0, a_k_full + 8u * (uint32_t)(kb & 7));
           } else {
             // the peer's 32 keys, this CTA's 256 value dims, once QK^T has read the tile
             ok = mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, kb);
@@ -705,7 +708,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             if (cta == 0) mbar_arrive_expect_tx(&ms.v_full[kb & 7], 2 * 4 * kChunkBytes);
             for (int j = 0; j < 4; ++j)
               tma_load_2d_pair(dst + ((cta == 0 ? 4 : 0) + j) * kChunkBytes, m, 256 * (int)cta + 64 * j,
-                               row0 + kOwnKeys * (int)(cta ^ 1), a_v_full + 8u * (uint32_t)(kb & 7));
+                               row0, a_v_full + 8u * (uint32_t)(kb & 7));
           }
           advance();
         }
