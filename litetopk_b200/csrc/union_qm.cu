@@ -8,14 +8,16 @@
 //   memb_qm[g,q,w]   bit b set  <=>  rank 32*w+b is in token q's own list
 // Only the algorithmic idea "a position bitmap makes sort + dedup a scan" is shared
 // with the reference; this kernel is laid out for B200 differently:
-//   * 256-thread CTAs (several resident per SM, so one tile's barrier phases overlap
-//     another tile's loads) instead of one 1024-thread CTA per SM slot;
+//   * small CTAs, several resident per SM, so one tile's barrier phases overlap another
+//     tile's loads, instead of one 1024-thread CTA per SM slot;
 //   * the tile's indices are read from HBM ONCE with 16-byte loads and stay in
 //     registers for the second (rank) pass;
 //   * a per-word exclusive rank table makes the rank lookup one popcount;
-//   * the sorted list is staged in shared memory and leaves the SM as 16-byte
-//     coalesced stores.
-// Integer-only, HBM-bound work: no tensor cores, no TMA.
+//   * the sorted list is staged in shared memory and leaves the SM as 16-byte coalesced stores.
+// Integer-only work: no tensor cores, no TMA.  It moves the index lists and the union once (65536
+// tokens of 16 heads, top-2048 of 131072: 0.8 GB, 120 us), and is bound by the instructions and
+// shared-memory cycles per candidate: insert (one atomic), rank (two loads), membership (one atomic),
+// list entry (one store; expanding the list from the bitmap instead was 5 % slower).
 #include "common.cuh"
 
 namespace lt {
@@ -33,19 +35,14 @@ struct UnionParams {
   int kq;                   // k / 4: 16-byte loads per token row
   uint32_t kq_mul;          // ceil(2^32 / kq), or 0: divide
   int k, G, cap, s_words;   // s_words = seq_space / 32
-  int rank_shift;           // rank table holds one entry per (1 << rank_shift) bitmap words
-  int stage_list;           // 1: sorted list staged in smem
+  int quads_per_thread;     // 16-byte bitmap quads a thread counts: 1 or odd (conflict-free reads)
+  int window;               // list entries staged in shared memory; later ones are written directly
   int fill_tail;            // 1: also write -1 / 0 beyond the live prefixes; 2: -1 up to the next multiple of 128
 };
 
-// Shared-memory carve-up (bytes): bitmap | rank table (u16) | qm accumulator | list stage
-__host__ __device__ inline size_t union_smem_bytes(int s_words, int rank_shift, int G, int cap,
-                                                   int stage_list) {
-  size_t b = (size_t)s_words * 4;
-  b += (((size_t)(s_words >> rank_shift) * 2) + 15) & ~(size_t)15;
-  b += (size_t)G * (cap / 32) * 4;
-  if (stage_list) b += (size_t)cap * 4;
-  return b;
+// Shared-memory carve-up (bytes): bitmap | rank table (u16) | qm accumulator | list window
+__host__ __device__ inline size_t union_smem_bytes(int s_words, int rank_shift, int G, int cap, int window) {
+  return (size_t)s_words * 4 + (size_t)(s_words >> rank_shift) * 2 + (size_t)G * (cap / 32) * 4 + (size_t)window * 4;
 }
 
 // n / d through a multiply-high when the host proved it exact (n * d < 2^32, d > 1)
@@ -57,33 +54,29 @@ inline uint32_t fast_div_mul(int64_t n_max, int d) {
   return (uint32_t)(((int64_t(1) << 32) + d - 1) / d);
 }
 
-// NT threads per tile; VPT int4 loads cached per thread (0: nothing cached, the second
-// pass re-reads the tile).  PLAIN: no block table and one rank-table entry per bitmap word
-// (the common case), so the candidate pass carries neither the translation nor the
-// partial-rank loop.  (Forcing 32 registers per thread so that every warp slot of the SM is
-// filled was measured 3-8 % slower: the kernel is bound by shared-memory transactions, not
-// by occupancy.)
-template <int NT, int VPT, bool PLAIN>
+// NT threads per tile; VPT int4 loads cached per thread (0: nothing cached, the second pass re-reads
+// the tile).  RS: the rank table holds one entry per (1 << RS) bitmap words.  BT: block table.
+template <int NT, int VPT, int RS, bool BT>
 __global__ void __launch_bounds__(NT)
 union_qm_kernel(const UnionParams p) {
-  constexpr int kUnionThreads = NT;
+  constexpr int NW = NT / 32;
   extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ int warp_tot[kUnionThreads / 32];
+  __shared__ int warp_tot[NW];
 
   const int g = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int s_words = p.s_words, cap = p.cap, capw = cap >> 5, total = p.G * p.k;
-  const int S = s_words << 5;
-  uint32_t* bm = smem;
+  const uint32_t S = (uint32_t)s_words << 5;
+  uint32_t* bm = smem;                                          // s_words % 32 == 0: all parts are 16-byte aligned
   uint16_t* rtab = reinterpret_cast<uint16_t*>(bm + s_words);
-  const int rt_entries = s_words >> p.rank_shift;
-  uint32_t* qm_s = reinterpret_cast<uint32_t*>(
-      reinterpret_cast<char*>(rtab) + ((((size_t)rt_entries * 2) + 15) & ~(size_t)15));
+  uint32_t* qm_s = reinterpret_cast<uint32_t*>(rtab + (s_words >> RS));
   int32_t* list_s = reinterpret_cast<int32_t*>(qm_s + (size_t)p.G * capw);
 
-  // phase 0: clear bitmap
+  // ---- clear the bitmap and the membership words (own memory: before the wait for the previous kernel)
   {
     uint4* b4 = reinterpret_cast<uint4*>(bm);
-    for (int i = tid; i < (s_words >> 2); i += kUnionThreads) b4[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < (s_words >> 2); i += NT) b4[i] = make_uint4(0, 0, 0, 0);
+    uint4* q4 = reinterpret_cast<uint4*>(qm_s);
+    for (int i = tid; i < (p.G * capw >> 2); i += NT) q4[i] = make_uint4(0, 0, 0, 0);
   }
   pdl_trigger();
   pdl_wait();
@@ -94,33 +87,36 @@ union_qm_kernel(const UnionParams p) {
   if (VPT > 0) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int qd = i * kUnionThreads + tid;
+      const int qd = i * NT + tid;
       v[i] = qd < nquad ? __ldg(src + qd) : make_int4(-1, -1, -1, -1);
     }
   }
   __syncthreads();
 
-  // phase 1: insert
+  // ---- insert
   auto insert = [&](int pos) {
-    if ((unsigned)pos < (unsigned)S) atomicOr(&bm[pos >> 5], 1u << (pos & 31));
+    if ((uint32_t)pos < S) atomicOr(&bm[pos >> 5], 1u << (pos & 31));
   };
   if (VPT > 0) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) { insert(v[i].x); insert(v[i].y); insert(v[i].z); insert(v[i].w); }
   } else {
-    for (int qd = tid; qd < nquad; qd += kUnionThreads) {
+    for (int qd = tid; qd < nquad; qd += NT) {
       const int4 t = __ldg(src + qd);
       insert(t.x); insert(t.y); insert(t.z); insert(t.w);
     }
   }
   __syncthreads();
 
-  // phase 2: per-thread popcount of a contiguous run of words; warp scan, then every
-  // thread adds the totals of the warps before its own
-  const int wpt = (s_words + kUnionThreads - 1) / kUnionThreads;   // words per thread
-  const int w0 = min(tid * wpt, s_words), w1 = min(w0 + wpt, s_words);
+  // ---- rank of every word: each thread counts a run of quads; warp scan, then a scan of the warp totals
+  const int nq_bm = s_words >> 2;
+  const int q0 = min(tid * p.quads_per_thread, nq_bm), q1 = min(q0 + p.quads_per_thread, nq_bm);
+  const uint4* b4 = reinterpret_cast<const uint4*>(bm);
   int mine = 0;
-  for (int w = w0; w < w1; ++w) mine += __popc(bm[w]);
+  for (int i = q0; i < q1; ++i) {
+    const uint4 b = b4[i];
+    mine += __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
+  }
   int incl = mine;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
@@ -129,114 +125,115 @@ union_qm_kernel(const UnionParams p) {
   }
   if (lane == 31) warp_tot[wid] = incl;
   __syncthreads();
-  int before = 0, count = 0;
+  const int wt = lane < NW ? warp_tot[lane] : 0;
+  int wincl = wt;
 #pragma unroll
-  for (int i = 0; i < kUnionThreads / 32; ++i) {
-    const int t = warp_tot[i];
-    before += i < wid ? t : 0;
-    count += t;
+  for (int off = 1; off < NW; off <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, wincl, off);
+    if (lane >= off) wincl += t;
   }
-  const int live = min(count, cap);
-  if (tid == 0) p.counts[g] = count;
-
-  // phase 3: exclusive rank of every bitmap word (or every 2^rank_shift-th word)
-  {
-    int r = before + incl - mine;
-    const int rank_shift = PLAIN ? 0 : p.rank_shift;
-    const int rmask = (1 << rank_shift) - 1;
-    for (int w = w0; w < w1; ++w) {
-      if ((w & rmask) == 0) rtab[w >> rank_shift] = (uint16_t)r;
-      r += __popc(bm[w]);
+  const int live = __shfl_sync(0xffffffffu, wincl, NW - 1);     // <= G * k = cap
+  int r0 = __shfl_sync(0xffffffffu, wincl - wt, wid) + incl - mine;
+  if (tid == 0) p.counts[g] = live;
+  for (int i = q0; i < q1; ++i) {
+    const uint4 b = b4[i];
+    if (RS == 0) {
+      const int r1 = r0 + __popc(b.x), r2 = r1 + __popc(b.y), r3 = r2 + __popc(b.z);
+      reinterpret_cast<uint2*>(rtab)[i] = make_uint2((uint32_t)r0 | (uint32_t)r1 << 16, (uint32_t)r2 | (uint32_t)r3 << 16);
+      r0 = r3 + __popc(b.w);
+    } else {
+      static_assert(RS == 0 || RS == 2, "one rank per word or per quad");
+      rtab[i] = (uint16_t)r0;
+      r0 += __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
     }
   }
-  // live mask words per query row: max(4, roundup4(ceil(live / 32)))
-  const int active = max(4, (((live + 31) >> 5) + 3) & ~3);
-  for (int i = tid; i < p.G * active; i += kUnionThreads) qm_s[i] = 0u;
   __syncthreads();
 
-  // phase 4: every candidate looks up its rank, sets its token's membership bit and
-  // writes its own slot of the sorted list (duplicates write the same value)
-  const int32_t* bt_row = (!PLAIN && p.btab) ? p.btab + (size_t)p.req_pg[g] * p.bt_stride : nullptr;
+  // ---- every candidate looks up its rank, sets its token's membership bit and writes its own entry of
+  // the sorted list (duplicates write the same value)
+  const int32_t* bt_row = BT ? p.btab + (size_t)p.req_pg[g] * p.bt_stride : nullptr;
   int32_t* out_row = p.u_phys + (size_t)g * cap;
-  int32_t* list_dst = p.stage_list ? list_s : out_row;
-  auto mark = [&](int pos, int qrow) {
-    if ((unsigned)pos >= (unsigned)S) return;
-    const int w = pos >> 5;
-    int r;
-    if (PLAIN) {
-      r = rtab[w];
-    } else {
-      r = rtab[w >> p.rank_shift];
-      if (p.rank_shift)
-        for (int x = (w >> p.rank_shift) << p.rank_shift; x < w; ++x) r += __popc(bm[x]);
+  auto mark = [&](int pos, uint32_t* row) {
+    if ((uint32_t)pos < S) {
+      const int w = pos >> 5;
+      int r = rtab[w >> RS];
+      if (RS)
+        for (int x = (w >> RS) << RS; x < w; ++x) r += __popc(bm[x]);
+      r += __popc(bm[w] & ((1u << (pos & 31)) - 1u));
+      atomicOr(row + (r >> 5), 1u << (r & 31));
+      int phys = pos;
+      if (BT) {
+        const int blk = fast_div(pos, p.bsz, p.bsz_mul);
+        phys = blk < p.bt_blocks ? bt_row[blk] * p.bsz + (pos - blk * p.bsz) : -1;
+      }
+      if (r < p.window) list_s[r] = phys;
+      else out_row[r] = phys;
     }
-    r += __popc(bm[w] & ((1u << (pos & 31)) - 1u));
-    if (r >= cap) return;
-    atomicOr(&qm_s[qrow + (r >> 5)], 1u << (r & 31));
-    int phys = pos;
-    if (!PLAIN && bt_row) {
-      const int blk = fast_div(pos, p.bsz, p.bsz_mul);
-      phys = blk < p.bt_blocks ? bt_row[blk] * p.bsz + (pos - blk * p.bsz) : -1;
-    }
-    list_dst[r] = phys;
   };
   if (VPT > 0) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      // k % 4 == 0: the four candidates of one 16-byte load belong to one token
-      const int qrow = fast_div(i * kUnionThreads + tid, p.kq, p.kq_mul) * active;
-      mark(v[i].x, qrow); mark(v[i].y, qrow); mark(v[i].z, qrow); mark(v[i].w, qrow);
+      // k % 4 == 0: the four candidates of one 16-byte load belong to one token (loads past the tile
+      // are all -1)
+      uint32_t* row = qm_s + fast_div(i * NT + tid, p.kq, p.kq_mul) * capw;
+      mark(v[i].x, row); mark(v[i].y, row); mark(v[i].z, row); mark(v[i].w, row);
     }
   } else {
-    for (int qd = tid; qd < nquad; qd += kUnionThreads) {
+    for (int qd = tid; qd < nquad; qd += NT) {
       const int4 t = __ldg(src + qd);
-      const int qrow = fast_div(qd, p.kq, p.kq_mul) * active;
-      mark(t.x, qrow); mark(t.y, qrow); mark(t.z, qrow); mark(t.w, qrow);
+      uint32_t* row = qm_s + fast_div(qd, p.kq, p.kq_mul) * capw;
+      mark(t.x, row); mark(t.y, row); mark(t.z, row); mark(t.w, row);
     }
   }
   __syncthreads();
 
-  // sorted list -> global, 16-byte stores (the last quad is padded with -1)
-  if (p.stage_list) {
-    const int q_live = (live + 3) >> 2;
-    const int q_end = p.fill_tail == 1 ? (cap >> 2) : (p.fill_tail == 2 ? ((live + 127) >> 7) << 5 : q_live);
-    int4* dst = reinterpret_cast<int4*>(out_row);
-    for (int i = tid; i < q_end; i += kUnionThreads) {
-      int4 o;
+  // ---- staged list -> global, 16-byte stores; the last quad is padded with -1
+  {
+    const int end = p.fill_tail == 1 ? cap : (p.fill_tail == 2 ? ((live + 127) >> 7) << 7 : (live + 3) & ~3);
+    for (int i = tid; i < end >> 2; i += NT) {
       const int b = i << 2;
-      o.x = b + 0 < live ? list_s[b + 0] : -1;
-      o.y = b + 1 < live ? list_s[b + 1] : -1;
-      o.z = b + 2 < live ? list_s[b + 2] : -1;
-      o.w = b + 3 < live ? list_s[b + 3] : -1;
-      dst[i] = o;
+      if (b >= p.window && b + 3 < live) continue;              // written above (window % 4 == 0)
+      if (b >= p.window && b < live) {                          // the last quad, partly written above
+        for (int e = live; e < b + 4; ++e) out_row[e] = -1;
+        continue;
+      }
+      int4 o = make_int4(-1, -1, -1, -1);
+      if (b < live) {
+        o = reinterpret_cast<const int4*>(list_s)[i];
+        if (b + 1 >= live) o.y = -1;
+        if (b + 2 >= live) o.z = -1;
+        if (b + 3 >= live) o.w = -1;
+      }
+      reinterpret_cast<int4*>(out_row)[i] = o;
     }
-  } else if (p.fill_tail) {
-    const int end = p.fill_tail == 1 ? cap : ((live + 127) >> 7) << 7;
-    for (int i = live + tid; i < end; i += kUnionThreads) out_row[i] = -1;
   }
 
-  // phase 5: dump the live mask words (whole rows when fill_tail)
+  // ---- live mask words, max(4, roundup4(ceil(live / 32))) per token (whole rows when fill_tail is 1;
+  // the words beyond are still zero)
   {
-    const int a4 = active >> 2, c4 = capw >> 2;
-    const int per_row = p.fill_tail == 1 ? c4 : a4;
+    const int c4 = capw >> 2;
+    const int per_row = p.fill_tail == 1 ? c4 : max(1, (live + 127) >> 7);
+    const int runs = (per_row + 31) >> 5;                       // warp-wide pieces of a row
     uint4* dst = reinterpret_cast<uint4*>(p.memb + (size_t)g * p.G * capw);
     const uint4* s4 = reinterpret_cast<const uint4*>(qm_s);
-    for (int i = tid; i < p.G * per_row; i += kUnionThreads) {
-      const int q = i / per_row, j = i - q * per_row;
-      dst[q * c4 + j] = j < a4 ? s4[q * a4 + j] : make_uint4(0, 0, 0, 0);
+    for (int c = wid; c < p.G * runs; c += NW) {
+      const int q = c / runs, j = 32 * (c - q * runs) + lane;
+      if (j < per_row) dst[q * c4 + j] = s4[q * c4 + j];
     }
   }
 }
 
-template <int NT, int VPT>
-static int launch_union(const UnionParams& p, int ng, size_t smem, cudaStream_t stream) {
-  constexpr int kUnionThreads = NT;
-  const bool plain = p.btab == nullptr && p.rank_shift == 0;
+template <int NT, int VPT, int RS>
+static int launch_union_rs(const UnionParams& p, int ng, size_t smem, cudaStream_t stream) {
   const int dev = current_device();
-  if (!(plain ? ensure_smem<union_qm_kernel<NT, VPT, true>>(dev, smem) : ensure_smem<union_qm_kernel<NT, VPT, false>>(dev, smem)))
+  if (!(p.btab ? ensure_smem<union_qm_kernel<NT, VPT, RS, true>>(dev, smem) : ensure_smem<union_qm_kernel<NT, VPT, RS, false>>(dev, smem)))
     return LITEDSA_ERR_CUDA;
-  return launch_pdl(plain ? union_qm_kernel<NT, VPT, true> : union_qm_kernel<NT, VPT, false>, dim3(ng), kUnionThreads,
-                    smem, stream, p);
+  return launch_pdl(p.btab ? union_qm_kernel<NT, VPT, RS, true> : union_qm_kernel<NT, VPT, RS, false>, dim3(ng), NT, smem,
+                    stream, p);
+}
+template <int NT, int VPT>
+static int launch_union(const UnionParams& p, int rank_shift, int ng, size_t smem, cudaStream_t stream) {
+  return rank_shift ? launch_union_rs<NT, VPT, 2>(p, ng, smem, stream) : launch_union_rs<NT, VPT, 0>(p, ng, smem, stream);
 }
 
 }  // namespace lt
@@ -270,28 +267,39 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
   p.bsz_mul = fast_div_mul(int64_t(s_words) * 32, p.bsz);
   p.kq = k / 4; p.kq_mul = fast_div_mul(int64_t(G) * (k / 4), k / 4);
   p.k = k; p.G = G; p.cap = cap; p.s_words = s_words; p.fill_tail = fill_tail == 2 ? 2 : (fill_tail ? 1 : 0);
-  // pick the richest shared-memory plan that fits (227 KB per CTA on sm_100)
+  // Shared memory (227 KB per CTA on sm_100): the whole list is staged if two CTAs fit on an SM then,
+  // else its first 8192 entries (a union is usually well below G * k); one rank per bitmap word if
+  // that fits, else one per quad.
   const size_t limit = 220 * 1024;
-  p.rank_shift = 0; p.stage_list = 1;
-  if (union_smem_bytes(s_words, 0, G, cap, 1) > limit) p.stage_list = 0;
-  if (union_smem_bytes(s_words, 0, G, cap, p.stage_list) > limit) p.rank_shift = 2;
-  const size_t smem = union_smem_bytes(s_words, p.rank_shift, G, cap, p.stage_list);
+  int rank_shift = 0;
+  p.window = cap;
+  if (union_smem_bytes(s_words, 0, G, cap, cap) > 110 * 1024) p.window = cap < 8192 ? cap : 8192;
+  if (union_smem_bytes(s_words, 0, G, cap, p.window) > limit) p.window = cap < 1024 ? cap : 1024;
+  if (union_smem_bytes(s_words, 0, G, cap, p.window) > limit) rank_shift = 2;
+  const size_t smem = union_smem_bytes(s_words, rank_shift, G, cap, p.window);
   if (smem > limit) return LITEDSA_ERR_UNSUPPORTED;
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int quads = G * k / 4;
-  // small tiles: 256-thread CTAs, several per SM; tiles whose shared memory leaves room for
-  // only a few CTAs per SM get 1024 threads each to keep the SM's warp slots filled
-  if (smem <= 48 * 1024) {
-    const int qpt = (quads + 255) / 256;
-    if (qpt <= 1) return launch_union<256, 1>(p, ng, smem, st);
-    if (qpt <= 4) return launch_union<256, 4>(p, ng, smem, st);
-    if (qpt <= 16) return launch_union<256, 16>(p, ng, smem, st);
-    return launch_union<256, 0>(p, ng, smem, st);
+  // At most one tile per SM and more than 256 loads or bitmap quads in it: 1024 threads shorten the
+  // tile's own chain of phases.  Otherwise 256 threads (512 for tiles that need more registers),
+  // several tiles per SM.  (65536 tokens of 16 heads, top-2048 of 131072: 610 us with one CTA of 1024
+  // threads per SM, 440 with two of 512; 16384 x 32 heads, top-1024 of 65536: 72 -> 55.)
+  const bool small = quads <= 256 && s_words <= 1024;
+  const int nt = ng <= 148 && !small ? 1024 : (quads <= 2048 ? 256 : 512);
+  const int qpt = (s_words / 4 + nt - 1) / nt;
+  p.quads_per_thread = qpt == 1 ? 1 : (qpt | 1);
+  const int vpt = (quads + nt - 1) / nt;
+  if (nt == 1024) {
+    if (vpt <= 1) return launch_union<1024, 1>(p, rank_shift, ng, smem, st);
+    if (vpt <= 4) return launch_union<1024, 4>(p, rank_shift, ng, smem, st);
+    return launch_union<1024, 0>(p, rank_shift, ng, smem, st);
   }
-  const int qpt = (quads + 1023) / 1024;
-  if (qpt <= 2) return launch_union<1024, 2>(p, ng, smem, st);
-  if (qpt <= 4) return launch_union<1024, 4>(p, ng, smem, st);
-  if (qpt <= 8) return launch_union<1024, 8>(p, ng, smem, st);
-  return launch_union<1024, 0>(p, ng, smem, st);
+  if (nt == 256) {
+    if (vpt <= 1) return launch_union<256, 1>(p, rank_shift, ng, smem, st);
+    if (vpt <= 4) return launch_union<256, 4>(p, rank_shift, ng, smem, st);
+    return launch_union<256, 8>(p, rank_shift, ng, smem, st);
+  }
+  if (vpt <= 8) return launch_union<512, 8>(p, rank_shift, ng, smem, st);
+  return launch_union<512, 0>(p, rank_shift, ng, smem, st);
 }

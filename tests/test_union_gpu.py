@@ -116,3 +116,30 @@ def test_union_full_size_properties():
     u2, m2, c2 = api.union_qm(u[:, :w.cap // 2 * 2].reshape(-1, w.cap).contiguous(), 1,
                               seq_space=w.s_kv, return_counts=True)
     assert torch.equal(c2, c)
+
+
+@pytest.mark.parametrize("ng", [1, 148, 149])                # one tile per SM at most / more
+@pytest.mark.parametrize("G,k,space", [
+    (2, 512, 4096),           # one load per thread
+    (2, 1984, 1024 * 33),     # 256 threads, four loads; bitmap quads do not divide by the threads
+    (4, 2048, 1 << 16),       # eight loads
+    (8, 2048, 1 << 18),       # 512 threads; unions beyond the staged part of the list
+    (16, 2048, 1 << 15),      # nothing cached, two staged windows' worth of list
+    (16, 2048, 1 << 20),      # one rank per quad
+])
+def test_union_plans(ng, G, k, space):
+    gen = torch.Generator().manual_seed(ng + k)
+    idx = torch.randint(0, space, (G, k), generator=gen, dtype=torch.int32)
+    idx[0, ::97] = -1
+    # tiles share the lists, each with its own shift, so that a few tiles checked on the CPU stand for all
+    shift = torch.arange(ng, dtype=torch.int32) * 37
+    full = torch.where(idx[None] >= 0, (idx[None] + shift[:, None, None]) % space, idx[None]).reshape(ng * G, k).contiguous()
+    for fill in (False, True):
+        got = _run(full, G, space, fill=fill)
+        for t in sorted({0, ng // 2, ng - 1}):
+            want = uo.union_qm_oracle(full[t * G:(t + 1) * G].numpy(), G, space)
+            ok, msg = uo.live_equal([x[t:t + 1] for x in got], want, G * k)
+            assert ok, (t, msg)
+            live = int(want[1][0])
+            beyond = got[0][t, (live + 3) // 4 * 4:]         # the quad that is cut is padded in any case
+            assert (beyond == (-1 if fill else -7)).all() and (got[0][t, live:(live + 3) // 4 * 4] == -1).all()
