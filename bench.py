@@ -934,7 +934,7 @@ def main():
                     help="run only the indexer + top-k leg on the chosen config's shape (profiling aid)")
     ap.add_argument("--only-native", action="store_true",
                     help="run only the native-cache (bf16 route) record of the workload and print it "
-                         "(profiling aid for masked_mla_bf16_kernel)")
+                         "(profiling aid for the gathering mla_bf16_kernel)")
     ap.add_argument("--measure-fp8-peak", action="store_true",
                     help="print the tcgen05 dense rates measured by the library's probe and exit")
     ap.add_argument("--ref-module-worker", action="store_true", help=argparse.SUPPRESS)
@@ -980,7 +980,7 @@ def main():
                 "warmup": args.warmup, "ms_per_step": rec["ms_per_step"], "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "bf16", "data": "synthetic",
                 "config": config_dict(w, args), "effective_tflops": rec["effective_tflops"],
-                "roofline": {"kernel": "dsv4_kernel", "bound": "tensor", "achieved": rec["effective_tflops"],
+                "roofline": {"kernel": "mla_bf16_kernel", "bound": "tensor", "achieved": rec["effective_tflops"],
                              "peak": peaks["bf16_tflops"], "unit": "TFLOP/s", "frac": rec["frac"], "traffic": None,
                              "peak_source": f"bf16 dense (cuBLAS) of {peaks['source']}", "tcgen05_probe": probe},
                 "record": rec, "gpu_launches": args.steps, "cpu_baseline": None, "e2e": None}

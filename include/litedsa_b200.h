@@ -235,10 +235,6 @@ int litedsa_repack_kv656(const void* kv656, void* kv576, int s_kv, int64_t out_p
  * q_token_stride, q_head_stride, out_token_stride, out_head_stride (ELEMENTS; 0 = the dense
  * packed layout) address q and out in place inside [T, H_padded, d] tensors with h_per_q real
  * heads per token (see litedsa_masked_mla_fp8_ex; kernels/b200/dsa/DSV4_ZEROCOPY_PLAN.md:50-76).
- * The kernel uses all 227 KB of shared memory and needs its dynamic base within 768 bytes of
- * a 1024-byte boundary: the first call on each device launches a one-thread probe and reads
- * its answer back synchronously (make that call outside stream capture); when the base
- * does not fit the call returns LITEDSA_ERR_UNSUPPORTED.
  */
 int litedsa_dsv4_c128a_bf16(const void* q, const void* kv_comp, const void* kv_raw, int ng,
                             int h_per_q, int n_comp, int s_raw, int pos0, int window, int ratio,

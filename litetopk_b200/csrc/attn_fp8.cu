@@ -181,9 +181,9 @@ struct ItemT {
 };
 
 // wait sites reported in the status word
-enum { kSiteQ = 1, kSiteKLand, kSiteKPeer, kSiteVLand, kSiteVPeer, kSiteQkDone, kSitePvDone,
-       kSiteSFree, kSitePReady, kSiteValidReady, kSiteValidFree, kSiteKFree, kSiteKCopied,
-       kSiteVFree, kSitePFree, kSiteEpi, kSiteRelayK, kSiteRelayV, kSiteMPub, kSiteMmaIdle, kSiteQFree, kSiteOFree, kSiteSelfTest };
+enum { kSiteQ = 1, kSiteKLand, kSiteQkDone, kSitePvDone,
+       kSiteSFree, kSitePReady, kSiteValidReady, kSiteValidFree, kSiteKFree,
+       kSiteVFree, kSitePFree, kSiteEpi, kSiteRelayK, kSiteRelayV, kSiteMPub, kSiteQFree, kSiteOFree, kSiteSelfTest };
 
 // status block of the FP8 attention kernels (layout: see Waiter in common.cuh)
 __device__ int g_attn_status[8];

@@ -319,26 +319,13 @@ __device__ __forceinline__ void tma_store_3d_hint(const void* map, uint32_t src_
                " [%0, {%2, %3, %4}], [%1], %5;"
                :: "l"(map), "r"(src_smem), "r"(x), "r"(y), "r"(z), "l"(pol) : "memory");
 }
-__device__ __forceinline__ void tma_store_3d(const void* map, uint32_t src_smem, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               :: "l"(map), "r"(src_smem), "r"(x), "r"(y), "r"(z) : "memory");
-}
 
-// TMA tile store shared -> global (bulk async-group completion)
-__device__ __forceinline__ void tma_store_2d(const void* map, uint32_t src_smem, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               :: "l"(map), "r"(src_smem), "r"(x), "r"(y) : "memory");
-}
 __device__ __forceinline__ void bulk_commit_group() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // all committed bulk groups of this thread have finished READING their shared-memory source
 __device__ __forceinline__ void bulk_wait_read_all() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-// ... all but the most recent one
-__device__ __forceinline__ void bulk_wait_read_1() {
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
 // all committed bulk groups of this thread are complete (writes performed)
 __device__ __forceinline__ void bulk_wait_all() {
@@ -366,21 +353,6 @@ __device__ __forceinline__ uint64_t l2_policy_evict_last() {
 // memory); without the operand the same builds run, bit-identical and at the same speed.
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
-}
-__device__ __forceinline__ void tma_store_2d_hint(const void* map, uint32_t src_smem, int x, int y,
-                                                  uint64_t pol) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint"
-               " [%0, {%2, %3}], [%1], %4;"
-               :: "l"(map), "r"(src_smem), "r"(x), "r"(y), "l"(pol) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t dst_smem, const CUtensorMap* map,
-                                                      int x, int y, uint32_t mbar_cluster_addr,
-                                                      uint64_t pol) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes.cta_group::2"
-      ".L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
-      ::"r"(dst_smem), "l"(map), "r"(x), "r"(y), "r"(mbar_cluster_addr), "l"(pol)
-      : "memory");
 }
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -144,7 +144,7 @@ struct Params {
   const int32_t* counts;     // [ng] or null
 };
 
-enum { kSiteQ = 101, kSiteKFull, kSiteVFull, kSiteQkDone, kSitePvDone, kSiteValidReady, kSiteValidFree,
+enum { kSiteQ = 101, kSiteKFull, kSiteQkDone, kSitePvDone, kSiteValidReady, kSiteValidFree,
        kSiteKFree, kSiteVFree, kSitePFree, kSiteEpi, kSiteQFree, kSiteMPub, kSiteRelayK, kSiteRelayV,
        kSiteSFree, kSiteOFree, kSitePReady };
 
