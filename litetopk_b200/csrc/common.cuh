@@ -458,6 +458,18 @@ __device__ __forceinline__ void mma_f8_pair_pv8(uint32_t d_tmem, uint32_t idesc,
       : "memory");
 }
 
+// 16 lanes x 32 columns as 16 x 256-bit fragments: thread l gets, for i = 0 .. 3, columns
+// 8 i + 2 (l % 4) + {0, 1} of row l / 4 in v[4 i], v[4 i + 1] and of row l / 4 + 8 in v[4 i + 2], v[4 i + 3]
+__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, float (&v)[16]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32"
+      " {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 // 32 lanes x 32 consecutive fp32 columns: thread i of the warp gets lane (base_lane + i)
 // the same, issued by one elected lane of a fully converged warp (keeps the caller warp-uniform)
 __device__ __forceinline__ void mma_commit_pair_elect(uint32_t cluster_addr) {

@@ -15,14 +15,15 @@
 // counterpart in the reference to be checked against; the CPU oracle restates the formula.
 //
 // index_logits_kernel (tensor-bound): the product is computed TRANSPOSED, keys on the M axis,
-// so that the head sum of a (token, key) pair is a sum along one accumulator row, i.e. inside
-// one thread.  One CTA owns 2 x 256 / Hi tokens: their q rows are the B operand of two
-// N = 256 accumulators (512 TMEM columns); the K tiles (128 keys x 128 bytes, TMA, four
-// stages) are the A operand and are streamed once per CTA, up to the causal bound of its
-// last token.  While the tensor core fills one accumulator, eight warps drain the other
-// (lane quarter x column half): tcgen05.ld, relu, multiply by the head weight, add; then
-// x k_scale, causal mask, and 128 consecutive fp32 logits per token leave each warp as
-// coalesced stores.
+// so that the head sum of a (token, key) pair is a sum along one accumulator row.  One CTA owns
+// 512 / Hi tokens: their q rows are the B operand of four N = 128 accumulators (512 TMEM columns);
+// the K tiles (128 keys x 128 bytes, TMA, four stages) are the A operand and are streamed once per
+// CTA, up to the causal bound of its last token.  While the tensor core fills one accumulator,
+// sixteen warps (accumulator x lane quarter) drain the others: tcgen05.ld, relu, multiply by the head
+// weight, add; then x k_scale, causal mask, and 128 consecutive fp32 logits per token leave each warp
+// as coalesced stores.  The drain paces the kernel (2070 cycles per key tile, of which the MMAs need
+// 1024): 4096 tokens x 32768 keys x 64 heads 934 us; 966 with two N = 256 accumulators, weights from shared
+// memory and the warps of a scheduler in two phases instead of four.
 //
 // topk_select (memory-bound): exact selection per token row.  Rows up to 32768 entries go
 // through persistent CTAs that prefetch the next row with a bulk copy while the current one
@@ -37,21 +38,23 @@ namespace lt {
 namespace idx {
 
 // ------------------------------------------------------------------ index logits
-constexpr int kThreads = 640;             // TMA, MMA, TMEM warps + 16 drain warps
+constexpr int kThreads = 576;             // TMA and MMA warps + 16 drain warps
+constexpr int kDrainWarp0 = 2;
 constexpr int kKeyTile = 128;             // keys per MMA (M)
-constexpr int kCols = 256;                // (token, head) columns per accumulator (N)
+constexpr int kCols = 128;                // (token, head) columns per accumulator (N)
+constexpr int kAccs = 4;                  // accumulators: all 512 TMEM columns
 constexpr int kDim = 128;                 // index head dim = bytes per row
 constexpr int kStages = 4;
-constexpr uint32_t kQTile = kCols * kDim;       // 32 KB
+constexpr uint32_t kQTile = kCols * kDim;       // 16 KB
 constexpr uint32_t kKTile = kKeyTile * kDim;    // 16 KB
 constexpr uint32_t kOffQ = 0;
-constexpr uint32_t kOffK = kOffQ + 2 * kQTile;
+constexpr uint32_t kOffK = kOffQ + kAccs * kQTile;
 constexpr uint32_t kOffW = kOffK + kStages * kKTile;
-constexpr uint32_t kOffBar = kOffW + 2 * kCols * 4;
+constexpr uint32_t kOffBar = kOffW + kAccs * kCols * 4;
 constexpr uint32_t kSmem = kOffBar + 256 + 1024;   // + alignment slack
 
 struct Bars {
-  uint64_t q_full, k_full[kStages], k_free[kStages], acc_full[2], acc_free[2];
+  uint64_t q_full, k_full[kStages], k_free[kStages], acc_full[kAccs], acc_free[kAccs];
   uint32_t tmem_base;
 };
 static_assert(sizeof(Bars) <= 256, "barrier block too large");
@@ -80,6 +83,12 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 
 __device__ int g_status[8];
 
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
 template <int HI>
 __global__ void __launch_bounds__(kThreads, 1)
 index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -94,8 +103,8 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   constexpr int tpa = kCols / HI;               // tokens per accumulator
-  const int tok0 = blockIdx.x * 2 * tpa;        // first token of this CTA
-  const int tok_end = min(p.T, tok0 + 2 * tpa);
+  const int tok0 = blockIdx.x * kAccs * tpa;    // first token of this CTA
+  const int tok_end = min(p.T, tok0 + kAccs * tpa);
   // key tiles up to the causal bound of the CTA's last token, and this CTA's share [j0, j0 + n)
   const int pos_max = p.q_pos0 + tok_end - 1;
   const int all_tiles = (p.S + kKeyTile - 1) / kKeyTile;
@@ -106,21 +115,21 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   if (threadIdx.x == 0) {
     mbar_init(&bar.q_full, 1);
     for (int i = 0; i < kStages; ++i) { mbar_init(&bar.k_full[i], 1); mbar_init(&bar.k_free[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bar.acc_full[i], 1); mbar_init(&bar.acc_free[i], 8); }
+    for (int i = 0; i < kAccs; ++i) { mbar_init(&bar.acc_full[i], 1); mbar_init(&bar.acc_free[i], 4); }
     fence_mbar_init();
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
   }
   pdl_trigger();
   pdl_wait();
-  // head weights of the CTA's tokens: column c of accumulator a is row tok0 * Hi + 256 a + c.
+  // head weights of the CTA's tokens: column c of accumulator a is row tok0 * Hi + 128 a + c.
   // Halved: the drain computes relu(x) as (x + |x|) / 2 with the division folded in here.
-  for (int i = threadIdx.x; i < 2 * kCols; i += kThreads) {
+  for (int i = threadIdx.x; i < kAccs * kCols; i += kThreads) {
     const long long r = (long long)tok0 * HI + i;
     wsm[i] = r < (long long)p.T * HI ? 0.5f * __ldg(p.weights + r) : 0.f;
   }
   __syncthreads();
-  if (warp == 2) {
+  if (warp == 0) {
     tmem_alloc_cta(&bar.tmem_base, 512);
     tmem_relinquish_cta();
   }
@@ -133,9 +142,9 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0 && n_tiles > 0) {
       const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
-      mbar_arrive_expect_tx(&bar.q_full, 2 * kQTile);
-      tma_load_2d_hint(sbase + kOffQ, &map_q, 0, tok0 * HI, &bar.q_full, pol_stream);
-      tma_load_2d_hint(sbase + kOffQ + kQTile, &map_q, 0, tok0 * HI + kCols, &bar.q_full, pol_stream);
+      mbar_arrive_expect_tx(&bar.q_full, kAccs * kQTile);
+      for (int a = 0; a < kAccs; ++a)
+        tma_load_2d_hint(sbase + kOffQ + a * kQTile, &map_q, 0, tok0 * HI + a * kCols, &bar.q_full, pol_stream);
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % kStages;
         if (j >= kStages && !mbar_wait(&bar.k_free[s], ((j / kStages) & 1) ^ 1, wt, kSiteKFree, j)) break;
@@ -144,8 +153,8 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issue (one thread)
-    if (lane == 0) {
+    // ---------------------------------------------------------------- MMA issue (one elected thread)
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc(0, 0, false, false, kKeyTile, kCols);
       bool ok = n_tiles > 0 && mbar_wait(&bar.q_full, 0, wt, kSiteQFull, 0);
       for (int j = 0; j < n_tiles && ok; ++j) {
@@ -153,7 +162,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         ok = mbar_wait(&bar.k_full[s], (j / kStages) & 1, wt, kSiteKFull, j);
         if (!ok) break;
         const uint64_t ad = umma_desc(sbase + kOffK + s * kKTile, 16, 1024, kSwz128);
-        for (int a = 0; a < 2 && ok; ++a) {
+        for (int a = 0; a < kAccs && ok; ++a) {
           // accumulator a still holds tile j-1 until its four warps have read it
           if (j > 0) ok = mbar_wait(&bar.acc_free[a], (j - 1) & 1, wt, kSiteAccFree, j);
           if (!ok) break;
@@ -164,23 +173,30 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             mma_f8_cta(tmem + a * kCols, ad + 2 * kk, bd + 2 * kk, idesc, kk ? 1u : 0u);
           mma_commit_cta(&bar.acc_full[a]);
         }
-        mma_commit_cta(&bar.k_free[s]);     // both accumulators have read the K tile
+        mma_commit_cta(&bar.k_free[s]);     // all accumulators have read the K tile
       }
     }
-  } else if (warp >= 4) {
+    __syncwarp();
+  } else {
     // ---------------------------------------------------------------- accumulator drain
-    // Sixteen warps: accumulator a, column half hf (128 columns = tpa / 2 whole tokens), TMEM
-    // lane quarter q4.  relu(x) * w is computed as (x + |x|) * (w / 2): an add with an absolute-
-    // value operand and a packed fma, both on the fma pipe (a max would go to the half-rate
-    // integer pipe, which then paces the kernel).
-    const int dw = warp - 4;
-    const int a = dw >> 3, hf = (dw >> 2) & 1;
-    const int q4 = warp & 3;                            // TMEM lane quarter of this warp
-    const int krow = 32 * q4 + lane;                    // key row of the tile = TMEM lane
-    const uint32_t tcol = tmem + ((uint32_t)(32 * q4) << 16) + a * kCols + 128 * hf;
-    const float* w = wsm + a * kCols + 128 * hf;
-    constexpr int tph = tpa / 2;                        // tokens per column half
-    const int t_base = tok0 + a * tpa + hf * tph;
+    // Sixteen warps: accumulator a, TMEM lane quarter q4.  The four warps of one scheduler (one lane
+    // quarter) serve four accumulators, which are filled in turn, so that they are in different phases:
+    // with two accumulators of 256 columns the warps waited, multiplied and reduced in lockstep.
+    // relu(x) * w is computed as (x + |x|) * (w / 2): an add with an absolute-value operand and a
+    // packed fma, both on the fma pipe (a max would go to the half-rate integer pipe).
+    // The accumulator is read as 16 x 256-bit fragments: lane l gets columns 8 i + 2 (l % 4) + {0, 1}
+    // of rows l / 4 and l / 4 + 8, so it needs a quarter of the weights and keeps them in registers.
+    // (With one key row per lane every lane needs every weight; as 16-byte broadcasts from shared
+    // memory those take 1024 of its cycles per key tile, beside 1024 for the MMAs' operands.)
+    const int a = (warp - kDrainWarp0) >> 2, q4 = warp & 3;
+    // the key row whose sums this lane ends up with (below)
+    const int krow = 32 * q4 + 16 * ((lane >> 1) & 1) + 8 * (lane & 1) + (lane >> 2);
+    const uint32_t tcol = tmem + ((uint32_t)(32 * q4) << 16) + a * kCols;
+    const int t_base = tok0 + a * tpa;
+    float2 w[kCols / 8];                                // columns 8 i + 2 (lane % 4) + {0, 1}
+#pragma unroll
+    for (int i = 0; i < kCols / 8; ++i)
+      w[i] = *reinterpret_cast<const float2*>(wsm + a * kCols + 8 * i + 2 * (lane & 3));
     // Key tiles beyond the causal bound of the CTA's last token are not computed: their entries
     // are -inf for every token of the CTA (this warp's tokens and key rows).  Written first,
     // while the tensor core fills the first accumulators.
@@ -188,62 +204,80 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int s_key = j * kKeyTile + krow;
       if (s_key < p.S) {
 #pragma unroll
-        for (int tt = 0; tt < tph; ++tt) {
-          const int t = t_base + tt;
-          if (t < p.T) p.logits[(long long)t * p.ld + s_key] = -INFINITY;
-        }
+        for (int tt = 0; tt < tpa; ++tt)
+          if (t_base + tt < p.T) p.logits[(long long)(t_base + tt) * p.ld + s_key] = -INFINITY;
       }
     }
-    for (int j = 0; j < n_tiles; ++j) {
-      // this key's scale is fetched before the wait, so its latency hides behind the MMAs
+    // tiles below this one lie inside the cache and inside every token's causal bound
+    const int j_plain = min(p.S, p.q_pos0 + tok0 + 1) / kKeyTile - j0;
+    const bool all_toks = t_base + tpa <= p.T;
+    auto scale_of = [&](int j) -> float {
       const int s_key = (j0 + j) * kKeyTile + krow;
-      const float ks = (p.k_scale && s_key < p.S) ? __ldg(p.k_scale + s_key) : 1.f;
-      if (!mbar_wait(&bar.acc_full[a], j & 1, wt, kSiteAccFull, j)) break;
-      __syncwarp();
+      return (p.k_scale && s_key < p.S) ? __ldg(p.k_scale + s_key) : 1.f;
+    };
+    float* out = p.logits + (long long)t_base * p.ld + (long long)j0 * kKeyTile + krow;
+    float ks_next = n_tiles > 0 ? scale_of(0) : 1.f;    // fetched a tile ahead
+    for (int j = 0; j < n_tiles; ++j, out += kKeyTile) {
+      const float ks = ks_next;
+      if (j + 1 < n_tiles) ks_next = scale_of(j + 1);
+      const bool landed = mbar_wait(&bar.acc_full[a], j & 1, wt, kSiteAccFull, j);
+      if (!__all_sync(0xffffffffu, landed)) break;
       tc_fence_after();
-      float acc[tph];
-      float x[2][32];
-      tmem_ld32(tcol, x[0]);
-      // two packed fma chains (four independent partial sums), carried over the 32-column chunks
-      // of one token and folded when the token's last chunk is done (a chunk never straddles two
-      // tokens)
-      float2 s0 = make_float2(0.f, 0.f), s1 = make_float2(0.f, 0.f);
+      // step m: 32 columns (chunk m / 2) of 16 rows (half m % 2).  One packed chain per row, carried
+      // over the chunks of a token (a chunk never straddles two tokens).
+      float acc[tpa];
+      float x[2][16];
+      float2 sum[2][2];                                 // [row half][row l / 4, + 8]
+      tmem_ld_16x256b_x4(tcol, x[0]);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int m = 0; m < kCols / 16; ++m) {
+        const int c = m >> 1, rh = m & 1;
         tmem_wait_ld();
-        if (c < 3) tmem_ld32(tcol + 32 * (c + 1), x[(c + 1) & 1]);
-        const float* xc = x[c & 1];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 w4 = *reinterpret_cast<const float4*>(w + 32 * c + i);
-          s0 = fma2(make_float2(xc[i] + fabsf(xc[i]), xc[i + 1] + fabsf(xc[i + 1])), make_float2(w4.x, w4.y), s0);
-          s1 = fma2(make_float2(xc[i + 2] + fabsf(xc[i + 2]), xc[i + 3] + fabsf(xc[i + 3])),
-                    make_float2(w4.z, w4.w), s1);
+        if (m + 1 < kCols / 16) {
+          tmem_ld_16x256b_x4(tcol + 32 * ((m + 1) >> 1) + ((uint32_t)(16 * ((m + 1) & 1)) << 16), x[(m + 1) & 1]);
+        } else {
+          tc_fence_before();                            // everything has been read
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar.acc_free[a]);
         }
-        if ((32 * (c + 1)) % HI == 0 || c == 3) {
-          acc[(32 * c) / HI] = (s0.x + s0.y) + (s1.x + s1.y);
-          s0 = make_float2(0.f, 0.f);
-          s1 = make_float2(0.f, 0.f);
+        const float* xc = x[m & 1];
+        if ((32 * c) % HI == 0) sum[rh][0] = sum[rh][1] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          sum[rh][0] = fma2(make_float2(xc[4 * i] + fabsf(xc[4 * i]), xc[4 * i + 1] + fabsf(xc[4 * i + 1])),
+                            w[4 * c + i], sum[rh][0]);
+          sum[rh][1] = fma2(make_float2(xc[4 * i + 2] + fabsf(xc[4 * i + 2]), xc[4 * i + 3] + fabsf(xc[4 * i + 3])),
+                            w[4 * c + i], sum[rh][1]);
+        }
+        if (rh == 1 && (32 * (c + 1)) % HI == 0) {
+          // the four lanes of a row group hold a quarter of the columns each; two exchanges leave
+          // lane l with the whole sum of row 16 (l / 2 % 2) + 8 (l % 2) + l / 4
+          float v[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const float lo = sum[r][0].x + sum[r][0].y, hi = sum[r][1].x + sum[r][1].y;
+            v[r] = ((lane & 1) ? hi : lo) + __shfl_xor_sync(0xffffffffu, (lane & 1) ? lo : hi, 1);
+          }
+          acc[(32 * c) / HI] = ((lane & 2) ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, (lane & 2) ? v[0] : v[1], 2);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.acc_free[a]);
-      // scale, causal mask, store: lanes of a warp hold 32 consecutive keys
-      if (s_key < p.S) {
+      // scale, causal mask, store: the lanes of a warp hold 32 consecutive keys
+      if (j < j_plain && all_toks) {
 #pragma unroll
-        for (int tt = 0; tt < tph; ++tt) {
+        for (int tt = 0; tt < tpa; ++tt) out[tt * p.ld] = acc[tt] * ks;
+      } else {
+        const int s_key = (j0 + j) * kKeyTile + krow;
+#pragma unroll
+        for (int tt = 0; tt < tpa; ++tt) {
           const int t = t_base + tt;
-          if (t >= p.T) continue;
-          const float v = s_key <= p.q_pos0 + t ? acc[tt] * ks : -INFINITY;
-          p.logits[(long long)t * p.ld + s_key] = v;
+          if (t < p.T && s_key < p.S) out[tt * p.ld] = s_key <= p.q_pos0 + t ? acc[tt] * ks : -INFINITY;
         }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 2) {
+  if (warp == 0) {
     __syncwarp();
     tmem_dealloc_cta(tmem, 512);
   }
@@ -1069,7 +1103,7 @@ extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, 
   if (!(Hi == 32 ? ensure_smem<index_logits_kernel<32>>(dev, kSmem)
                  : (Hi == 64 ? ensure_smem<index_logits_kernel<64>>(dev, kSmem) : ensure_smem<index_logits_kernel<128>>(dev, kSmem))))
     return LITEDSA_ERR_CUDA;
-  const int tok_per_cta = 2 * (kCols / Hi);
+  const int tok_per_cta = kAccs * (kCols / Hi);
   const int ctas_x = (T + tok_per_cta - 1) / tok_per_cta;
   // the tiles that do work: up to the last token's causal bound
   const int all_tiles = (S + kKeyTile - 1) / kKeyTile;
