@@ -547,15 +547,16 @@ __device__ __forceinline__ void block_fmax_fmin(float* red_a, float* red_b, floa
 // threshold bin, its keys ranked by counting), then every survivor >= the k-th value is written
 // out (thread i owns a contiguous run of survivor slots; one block-wide exclusive scan).  When
 // the fast path does not apply -- or stops applying: NaN / infinite values, a single value,
-// more threshold-bin keys than threads, a tie at the k-th value that must be cut by position --
-// the row is finished exactly from memory: bitwise radix select (unless the k-th value is
-// already known) and ordered emission.
+// more threshold-bin keys or tied values than threads -- the row is finished exactly from memory:
+// bitwise radix select (unless the k-th value is already known) and ordered emission.  One such row
+// costs about 30 us, and of 4096 rows of 30K logits one has a tie to be cut: cut among the survivors
+// (260 -> 229 us on such data).
 template <int NT, class PosT>
 __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* red_b, uint32_t* eq_total,
                                            const float* sval, const PosT* spos, uint32_t m_s, bool fast,
                                            const float* row, int n, int k, int32_t* out) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  uint32_t kth = 0, ties = 0;
+  uint32_t kth = 0, ties = 0, tie_end = 0xffffffffu;      // tie_end: last position selected among the tied
   bool have_kth = false;
   if (fast) {
     float vmax = -INFINITY, vmin = INFINITY, chk = 0.f;
@@ -600,7 +601,31 @@ __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* r
         __syncthreads();
         kth = sh.kth; ties = sh.ties;
         have_kth = true;
-        if (ties != *eq_total) fast = false;      // the tie at the k-th value must be cut by position
+        if (ties != *eq_total) {                  // the tie at the k-th value must be cut by position
+          const float kv = okey_inv(kth);
+          __syncthreads();
+          if (tid == 0) sh.n_cand = 0;
+          __syncthreads();
+          for (uint32_t i = tid; i < m_s; i += NT)
+            if (sval[i] == kv) {
+              const uint32_t c = atomicAdd(&sh.n_cand, 1u);
+              if (c < (uint32_t)NT) sh.cand[c] = spos[i];
+            }
+          __syncthreads();
+          const uint32_t me = sh.n_cand;
+          if (me <= (uint32_t)NT) {
+            if (tid < (int)me) {
+              const uint32_t mine = sh.cand[tid];
+              uint32_t r = 0;
+              for (uint32_t j = 0; j < me; ++j) r += sh.cand[j] < mine;
+              if (r + 1 == ties) sh.kth = mine;
+            }
+            __syncthreads();
+            tie_end = sh.kth;
+          } else {
+            fast = false;
+          }
+        }
       } else {
         fast = false;
       }
@@ -611,30 +636,34 @@ __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* r
   }
   if (fast) {
     const float kv = okey_inv(kth);
-    const uint32_t per = (m_s + NT - 1) / NT;
-    const uint32_t i0 = min((uint32_t)tid * per, m_s), i1 = min(i0 + per, m_s);
-    uint32_t cnt = 0;
-    for (uint32_t i = i0; i < i1; ++i) cnt += sval[i] >= kv;
-    uint32_t inc = cnt;
+    auto emit = [&](auto selected) {
+      const uint32_t per = (m_s + NT - 1) / NT;
+      const uint32_t i0 = min((uint32_t)tid * per, m_s), i1 = min(i0 + per, m_s);
+      uint32_t cnt = 0;
+      for (uint32_t i = i0; i < i1; ++i) cnt += selected(i);
+      uint32_t inc = cnt;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xffffffffu, inc, off);
-      if (lane >= off) inc += a;
-    }
-    if (lane == 31) sh.wa[wid] = inc;
-    __syncthreads();
-    uint32_t wtot = lane < NT / 32 ? sh.wa[lane] : 0u, ws = wtot;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xffffffffu, ws, off);
-      if (lane >= off) ws += a;
-    }
-    uint32_t o = __shfl_sync(0xffffffffu, ws - wtot, wid) + inc - cnt;
-    for (uint32_t i = i0; i < i1; ++i)
-      if (sval[i] >= kv) {
-        if (o < (uint32_t)k) out[o] = (int32_t)spos[i];
-        ++o;
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += a;
       }
+      if (lane == 31) sh.wa[wid] = inc;
+      __syncthreads();
+      uint32_t wtot = lane < NT / 32 ? sh.wa[lane] : 0u, ws = wtot;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xffffffffu, ws, off);
+        if (lane >= off) ws += a;
+      }
+      uint32_t o = __shfl_sync(0xffffffffu, ws - wtot, wid) + inc - cnt;
+      for (uint32_t i = i0; i < i1; ++i)
+        if (selected(i)) {
+          if (o < (uint32_t)k) out[o] = (int32_t)spos[i];
+          ++o;
+        }
+    };
+    if (tie_end == 0xffffffffu) emit([&](uint32_t i) { return sval[i] >= kv; });
+    else emit([&](uint32_t i) { return sval[i] > kv || (sval[i] == kv && (uint32_t)spos[i] <= tie_end); });
   } else {
     auto key_mem = [&](int i) -> uint32_t { return okey(__ldg(row + i)); };
     if (!have_kth) {
@@ -696,7 +725,7 @@ __device__ __forceinline__ float sampled_threshold(SelShared& sh, float* red_a, 
 //   5. survivors >= the k-th value are written out (block-wide scan of per-thread counts).
 // The output order is fixed but not ascending.  Whatever the fast path does not cover -- too
 // few or too many survivors, NaN or infinite values, a single value, more threshold-bin keys
-// than threads, a tie at the k-th value that must be cut by position -- is finished by the
+// or values tied at the k-th than threads -- is finished by the
 // exact bitwise radix select and the ordered emission over the row re-read from memory.
 constexpr int kStreamThreads = 512;
 enum { kSiteSelRow = 11 };

@@ -182,6 +182,21 @@ def test_topk_select_when_the_sampled_threshold_misleads(kind, S):
     assert np.array_equal(_canon(got), ref)
 
 
+@pytest.mark.parametrize("T,S", [(300, 8192), (300, 32768), (5, 70000), (160, 70000)])   # registers, cluster, chunks
+@pytest.mark.parametrize("tied", [2, 3, 600])              # in the survivors / more than there are threads
+def test_topk_select_cuts_a_tie_at_the_kth_value_by_position(T, S, tied):
+    k = 2048
+    x = _random_logits(T, S, seed=S + tied)
+    order = torch.argsort(x, dim=1, descending=True, stable=True)
+    # ranks k - 1 - tied / 2 ... share one value: some of them belong to the top k, the others do not
+    ranks = order[:, k - 1 - tied // 2: k - 1 - tied // 2 + tied]
+    x.scatter_(1, ranks, x.gather(1, ranks[:, :1]).expand(-1, tied))
+    ref = io.topk_exact(x, k, q_pos0=S - 1)
+    got = api.topk_select(x.to(DEV), k, q_pos0=S - 1)
+    torch.cuda.synchronize()
+    assert np.array_equal(_canon(got), ref)
+
+
 def test_topk_select_with_lengths_and_row_pitch():
     T, S, k = 12, 2048, 256
     x = _random_logits(T, 2304, seed=4)
