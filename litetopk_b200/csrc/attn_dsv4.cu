@@ -53,12 +53,14 @@ classify_runs_kernel(const int32_t* __restrict__ indices, long long idx_stride, 
 
 
 // Slices of a tile when a call has `tiles` tiles of up to `blocks` key blocks: as many as there are
-// idle clusters for, at least three blocks each (a slice costs an epilogue and its share of the merge,
-// as much as three blocks), none when more than half of the clusters have a tile anyway.
+// idle clusters for, at least five blocks each, none below 20 blocks.  Slices cost about 5 us (a launch for the
+// merge, fp32 partial results), a block of an unsliced tile 0.75 us.  (With slices from six blocks on,
+// 24 tokens against 77777 positions took 25.5 us, unsliced 20.)
 static int pick_slices(int tiles, int blocks) {
   constexpr int kClusters = 74;
+  if (blocks < 20) return 1;
   int n = kClusters / tiles;
-  if (n > blocks / 3) n = blocks / 3;
+  if (n > blocks / 5) n = blocks / 5;
   if (n > kMaxSlices) n = kMaxSlices;
   return n < 2 ? 1 : n;
 }

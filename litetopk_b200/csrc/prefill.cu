@@ -72,14 +72,19 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
   if (lane == 0) lse[row] = l > 0.f ? __logf(l) + m * kLn2 - lse_off : INFINITY;
 }
 
-// How many slices a tile is cut into when a launch has `tiles` tiles of lists up to `cap` long: as
-// many as there are idle clusters for, at least 512 list entries each (a slice costs a block of its own
-// for the running max, an epilogue and its share of the merge), none when more
-// than half of the clusters have a tile of their own anyway.
-static int pick_slices(int tiles, int cap) {
+// How many slices a tile is cut into when a launch has `tiles` tiles of G lists of k entries.  A union
+// is not known on the host; neighbouring tokens share about three quarters of their lists, so it is
+// taken as k (3 + G) / 4 entries.  Slices cost about 6 us (a launch for the merge, fp32 partial
+// results) and a block each for the running max, a block of an unsliced tile 1.1 us: from 12 blocks on
+// there are slices, of at least four blocks, at most as many as there are idle clusters for.  (Slices of two
+// or three blocks from lists of 8 blocks on: 36 tokens x 32 heads, top-1024 33 us, now 27 (unsliced 29); 64 x 16,
+// top-1024 36, now 30 (39); 64 x 64, top-512 26, now 19; two tokens x 64, top-2048 26 both (34).)
+static int pick_slices(int tiles, int G, int k) {
   constexpr int kClusters = 74;
+  const int blocks = (int)((int64_t)k * (3 + G) / 4 / 128);
+  if (blocks < 12) return 1;
   int n = kClusters / tiles;
-  if (n > cap / 512) n = cap / 512;
+  if (n > blocks / 4) n = blocks / 4;
   if (n > kMaxSlices) n = kMaxSlices;
   return n < 2 ? 1 : n;
 }
@@ -121,7 +126,7 @@ extern "C" int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_
   using namespace lt::prefill;
   if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
   const int G = 128 / h, cap = G * k;
-  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, cap);
+  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, G, k);
   return layout_of(T / G, G, cap, ns).total;
 }
 
@@ -141,7 +146,7 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   if (((uintptr_t)workspace & 255) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)topk_idx & 15))
     return LITEDSA_ERR_UNSUPPORTED;
   const int G = 128 / h, ng = T / G, cap = G * k;
-  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, cap);
+  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, G, k);
   const Layout l = layout_of(ng, G, cap, ns);
   if (workspace_bytes < l.total) return LITEDSA_ERR_SHAPE;
   char* ws = reinterpret_cast<char*>(workspace);
