@@ -32,6 +32,10 @@ struct Args {
   // in-place addressing of q / out inside [T, H_padded, d] tensors (ELEMENTS, 0 = dense packed)
   int64_t q_token_stride, q_head_stride, out_token_stride, out_head_stride;
   const int* gate = nullptr;      // run only if *gate == 1 (see Params)
+  // nsplit > 1 (d = 576): every tile's blocks are cut into slices whose fp32 results go to part_o / part_ml
+  int nsplit = 1;
+  float* part_o = nullptr;
+  float2* part_ml = nullptr;
 };
 
 // argument rules shared by both entry points (no CUDA call)
@@ -73,6 +77,10 @@ static int run(const Args& a, void* stream) {
   p.memb = a.memb; p.s_kv = a.s_kv; p.cap = a.topk;
   p.pref = a.pref; p.win_lo = a.win_lo; p.win_hi = a.win_hi; p.counts = a.counts;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (a.nsplit > 1) {
+    p.nsplit = a.nsplit; p.part_o = a.part_o; p.part_ml = a.part_ml;
+    return launch<576, kGather, true>(mq, mq, mq, mout, p, st);
+  }
   return a.d == 576 ? launch<576, kGather, false>(mq, mq, mq, mout, p, st)
                     : launch<512, kGather, false>(mq, mq, mq, mout, p, st);
 }
@@ -118,6 +126,16 @@ __global__ void __launch_bounds__(256) dequant_kv656_kernel(const uint8_t* __res
 }
 
 }  // namespace b16
+
+// the union form on dense packed operands of 576 dims, in nsplit slices (prefill.cu)
+int run_bf16_slices(const void* q, const void* kv, const int32_t* indices, float sm_scale, const int32_t* counts,
+                    const uint32_t* memb, int h, void* out, float* lse, int ng, int s_kv, int cap, int64_t kv_row_stride,
+                    int nsplit, float* part_o, float2* part_ml, void* stream) {
+  b16::Args a{q, kv, indices, counts, memb, nullptr, nullptr, nullptr, nullptr, out, nullptr, lse,
+              ng, s_kv, cap, 576, h, 576, kv_row_stride, cap, sm_scale, 0, 0, 0, 0};
+  a.nsplit = nsplit; a.part_o = part_o; a.part_ml = part_ml;
+  return b16::run(a, stream);
+}
 }  // namespace lt
 
 // The reference's DSv4 operator with its own argument list

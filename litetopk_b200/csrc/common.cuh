@@ -64,6 +64,9 @@ int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, con
                       int64_t out_token_stride, int64_t out_head_stride, void* workspace,
                       cudaStream_t stream);
 int run_fp8(const Fp8Args& a, void* const* outs, int n_outs, void* stream);
+int run_bf16_slices(const void* q, const void* kv, const int32_t* indices, float sm_scale, const int32_t* counts,
+                    const uint32_t* memb, int h, void* out, float* lse, int ng, int s_kv, int cap, int64_t kv_row_stride,
+                    int nsplit, float* part_o, float2* part_ml, void* stream);      // attn_bf16.cu
 // prefill.cu: merge of the slices of ng tiles (see there); out strides in ELEMENTS
 constexpr int kMaxSlices = 16;
 int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,

@@ -395,13 +395,13 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       float li = 0.f, real_m = -INFINITY;
       const int k_first = (g - kb0) & 1;          // first local block with (kb0 + k) % 2 == g
       uint32_t mk = 0u;
-      if (mrow && k_first < nb) mk = __ldcs(mrow + 2 * k_first);
+      if (mrow && k_first < nb) mk = __ldcs(mrow + 2 * (item.k0 + k_first));
 
       for (int k = k_first; k < nb; k += 2) {
         const int kb = kb0 + k;
         const uint32_t ph = (kb >> 1) & 1;
         uint32_t mk_next = 0u;
-        if (kSrc == kGather && mrow && k + 2 < nb) mk_next = __ldcs(mrow + 2 * (k + 2));
+        if (kSrc == kGather && mrow && k + 2 < nb) mk_next = __ldcs(mrow + 2 * (item.k0 + k + 2));
 
         mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteQkDone, k);
         __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops

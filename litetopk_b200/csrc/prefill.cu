@@ -79,12 +79,14 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
 // there are slices, of at least four blocks, at most as many as there are idle clusters for.  (Slices of two
 // or three blocks from lists of 8 blocks on: 36 tokens x 32 heads, top-1024 33 us, now 27 (unsliced 29); 64 x 16,
 // top-1024 36, now 30 (39); 64 x 64, top-512 26, now 19; two tokens x 64, top-2048 26 both (34).)
-static int pick_slices(int tiles, int G, int k) {
+// The bf16 kernel's blocks are 64 keys and take 0.8 us: from 20 on, at least five per slice.  (Native cache,
+// two tokens x 64 heads, top-2048: 52 -> 26 us; 36 x 32, top-1024: 41 -> 27; 64 x 16, top-2048: 103 -> 45.)
+static int pick_slices(int tiles, int G, int k, bool bf16) {
   constexpr int kClusters = 74;
-  const int blocks = (int)((int64_t)k * (3 + G) / 4 / 128);
-  if (blocks < 12) return 1;
+  const int blocks = (int)((int64_t)k * (3 + G) / 4 / (bf16 ? 64 : 128));
+  if (blocks < (bf16 ? 20 : 12)) return 1;
   int n = kClusters / tiles;
-  if (n > blocks / 4) n = blocks / 4;
+  if (n > blocks / (bf16 ? 5 : 4)) n = blocks / (bf16 ? 5 : 4);
   if (n > kMaxSlices) n = kMaxSlices;
   return n < 2 ? 1 : n;
 }
@@ -126,7 +128,7 @@ extern "C" int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_
   using namespace lt::prefill;
   if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
   const int G = 128 / h, cap = G * k;
-  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, G, k);
+  const int ns = pick_slices(policy_tokens / G, G, k, kv_is_bf16 != 0);
   return layout_of(T / G, G, cap, ns).total;
 }
 
@@ -146,7 +148,7 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   if (((uintptr_t)workspace & 255) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)topk_idx & 15))
     return LITEDSA_ERR_UNSUPPORTED;
   const int G = 128 / h, ng = T / G, cap = G * k;
-  const int ns = kv_is_bf16 ? 1 : pick_slices(policy_tokens / G, G, k);
+  const int ns = pick_slices(policy_tokens / G, G, k, kv_is_bf16 != 0);
   const Layout l = layout_of(ng, G, cap, ns);
   if (workspace_bytes < l.total) return LITEDSA_ERR_SHAPE;
   char* ws = reinterpret_cast<char*>(workspace);
@@ -156,6 +158,14 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   // fill mode 2: lists padded to whole 128-key blocks, nothing written beyond
   rc = litedsa_union_qm(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
   if (rc != LITEDSA_OK) return rc;
+  if (kv_is_bf16 && ns > 1) {
+    float* part_o = reinterpret_cast<float*>(ws + l.part_o);
+    float2* part_ml = reinterpret_cast<float2*>(ws + l.part_ml);
+    rc = run_bf16_slices(q, kv, u, sm_scale, counts, memb, h, out, lse, ng, s_kv, cap, kv_row_stride, ns, part_o, part_ml, stream);
+    if (rc != LITEDSA_OK) return rc;
+    return merge_slices(part_o, part_ml, ns, ng, h, 1.f, 0.f, nullptr, 1, out, (int64_t)h * 512, 512, lse,
+                        reinterpret_cast<cudaStream_t>(stream));
+  }
   if (kv_is_bf16)
     return litedsa_masked_mla_bf16(q, kv, u, sm_scale, counts, memb, h, out, nullptr, lse, ng, s_kv, cap, 576, 576,
                                    kv_row_stride, cap, nullptr, stream);

@@ -414,3 +414,32 @@ def test_native_many_short_tiles(tokens, heads, topk):
     torch.cuda.synchronize()
     assert api.bf16_status()[0] == 0
     _check_exact(out, lse, q, kv, idx, tag="short tiles")
+
+
+@pytest.mark.parametrize("tokens,heads,topk", [
+    (2, 64, 2048),         # one tile, eight slices
+    (24, 32, 1536),        # six tiles, eight slices
+    (8, 16, 2048),         # one tile of eight tokens, sixteen slices
+    (30, 64, 1984),        # 15 tiles, four slices; a list that is not a multiple of the block
+])
+def test_native_few_tiles_run_in_slices(tokens, heads, topk):
+    w, idx, kv, q = _native_case(tokens, heads, topk, 20000, (0.6, 0.8), seed=15)
+    idx = idx.clone()
+    idx[0, topk // 2:] = -1                 # a short list
+    api.bf16_status(reset=True)
+    out, lse = api.sparse_prefill(q.to(DEV), kv.to(DEV), idx.to(DEV), synth.SM_SCALE)
+    torch.cuda.synchronize()
+    assert api.bf16_status()[0] == 0
+    _check_exact(out, lse, q, kv, idx, tag="slices")
+    # unions shorter than the slices: some are empty
+    idx[:, 16:] = -1
+    out, lse = api.sparse_prefill(q.to(DEV), kv.to(DEV), idx.to(DEV), synth.SM_SCALE)
+    torch.cuda.synchronize()
+    assert api.bf16_status()[0] == 0
+    _check_exact(out, lse, q, kv, idx, tag="empty slices")
+    # the last tile without any key (not part of the comparison above: the cosine of zeros is undefined)
+    idx[-(128 // heads):] = -1
+    out, lse = api.sparse_prefill(q.to(DEV), kv.to(DEV), idx.to(DEV), synth.SM_SCALE)
+    last = slice(tokens - 128 // heads, tokens)
+    assert bool((out[last] == 0).all()) and bool(torch.isposinf(lse[last]).all())
+    assert bool(torch.isfinite(out.float()).all())
