@@ -94,7 +94,7 @@ struct Misc {
   // in every CTA
   uint64_t qk_done[8], pv_done[4], slot_free[kSlots], valid_ready[2], valid_free[2], m_pub[2];
   uint64_t q_land;                  // this CTA's Q chunks for tensor memory have landed in their slot
-  uint64_t q_taken;                 // they have been moved out of it
+  uint64_t q_taken[2];              // they have been moved out of it, by parity of the item ordinal
   uint64_t qt_ready;                // leader CTA: they are in tensor memory in both CTAs
   uint64_t q_free;                  // all QK^T of the current item are complete
   uint64_t o_free;                  // leader CTA: the item's O has been read out of TMEM
@@ -299,7 +299,6 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_res, 1);
     mbar_init(&ms.q_land, kQEntries);
-    mbar_init(&ms.q_taken, 1);
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
@@ -319,6 +318,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(&ms.valid_ready[i], 1);
       mbar_init(&ms.valid_free[i], 4);
       mbar_init(&ms.m_pub[i], 4);
+      mbar_init(&ms.q_taken[i], 1);
     }
     fence_mbar_init();
     tma_prefetch_desc(&map_q);
@@ -679,7 +679,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       for (int w = cid; w < n_items && ok; w += ncl, ++it) {
         const Item item = item_of(w);
         // the previous item's Q must have been moved on: with short items its bytes could still be in flight
-        if (!is_v && it > 0) ok = mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQFree, kb);
+        if (!is_v && it > 0) ok = mbar_wait(&ms.q_taken[(it - 1) & 1], ((it - 1) >> 1) & 1, wt, kSiteQFree, kb);
         for (int e = 0; e < kQEntries && ok; ++e) {
           if (!is_v) {
             if (ring > 0) ok = mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteQFree, kb);
@@ -814,7 +814,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (lane == 0) mbar_arrive_cluster(a_qt_ready);
       asm volatile("bar.sync 4, 128;" ::: "memory");      // all four warps have read the slots
       if (e_tid < kQEntries) mbar_arrive(&ms.slot_free[(n + e_tid) % kSlots]);
-      if (e_tid == 0) mbar_arrive(&ms.q_taken);
+      if (e_tid == 0) mbar_arrive(&ms.q_taken[j & 1]);
     };
     int kb0 = 0, it = 0;
     if (cid < n_items) bring_q(cid, 0, 0);
@@ -894,11 +894,19 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // (this CTA's 32 keys, all dims) once its slot is free.
     const int pw = warp - kWarpGather0;
     struct Cursor { int w, k, nb, kb, slot, ring, k0, len; const int32_t* idx; };   // ring entry = kSlots ring + slot
-    // The Q entries in front of an item's K entries belong to warp 0.  (A slot's barrier may be waited
-    // on only once every older entry has been through it, which this warp's own K copies prove.)
-    // (And the previous item's Q must have been moved on.)
+    // The Q entries in front of an item's K entries are requested by warp 0, once the previous item's Q
+    // has been moved on.  A parity test of slot_free answers for the slot's latest entry only if the
+    // warp knows that the one before it is dead, which it does when it filled the latest entry itself.
+    // The other warps have not: for them a slot that last held Q is free once that item's q_taken says
+    // so.  (Stepping over the Q entries and testing slot_free behind them let items of one or two blocks
+    // copy K over a block whose PV was pending.)  Two q_taken barriers are enough: the item after the
+    // next cannot have its Q moved before this warp has copied the next one's K.
+    // q_held: four bits per slot -- 1: Q was its last entry, 2: that item's ordinal % 2, 4: its phase.
     int q_w = cid, q_slot = 0, q_ring = 0, q_left = pw == 0 && cid < n_items ? kQEntries : 0;
     int q_n = 0;                                   // items whose Q has been requested
+    uint32_t q_held = 0x11u;                       // the first item's Q entries: slots 0 and 1
+    int k_it = 0;                                  // item ordinal of the K cursor
+    static_assert(kQEntries == 2 && kSlots <= 8, "q_held layout");
     auto cur_load = [&](Cursor& c) {
       c.nb = 0;
       if (c.w < n_items) {
@@ -958,7 +966,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
       if (q_left > 0) {                            // warp-uniform; warp 0 only
         const bool ok = (q_ring == 0 || mbar_test(&ms.slot_free[q_slot], (q_ring - 1) & 1)) &&
-                        (q_n == 0 || mbar_test(&ms.q_taken, (q_n - 1) & 1));
+                        (q_n == 0 || mbar_test(&ms.q_taken[(q_n - 1) & 1], ((q_n - 1) >> 1) & 1));
         if (__all_sync(0xffffffffu, ok)) {
           if (lane == 0) request_q(q_w, kQEntries - q_left, q_slot);
           __syncwarp();
@@ -968,8 +976,11 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       }
       if (ck.w < n_items && q_left == 0) {
-        const bool ok = ck.ring == 0 || mbar_test(&ms.slot_free[ck.slot], (ck.ring - 1) & 1);
+        const uint32_t held = q_held >> (4 * ck.slot);
+        const bool ok = (held & 1u) ? mbar_test(&ms.q_taken[(held >> 1) & 1u], (held >> 2) & 1u)
+                                    : (ck.ring == 0 || mbar_test(&ms.slot_free[ck.slot], (ck.ring - 1) & 1));
         if (__all_sync(0xffffffffu, ok)) {
+          q_held &= ~(15u << (4 * ck.slot));
           const int kcur = in_range(kidx);
           const uint32_t kst = sbase + PL::kOffKV + ck.slot * PL::kSlot;
 #pragma unroll
@@ -988,8 +999,11 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           cp_async_mbar_arrive_noinc(&ms.k_full[ck.kb & 7]);
           if (cur_next(ck)) {
             if (pw == 0 && ck.w < n_items) { q_w = ck.w; q_slot = ck.slot; q_ring = ck.ring; q_left = kQEntries; }
-            advance(ck);
-            advance(ck);
+            ++k_it;
+            for (int e = 0; e < kQEntries; ++e) {
+              q_held = (q_held & ~(15u << (4 * ck.slot))) | ((1u | (uint32_t)(k_it & 3) << 1) << (4 * ck.slot));
+              advance(ck);
+            }
           }
           if (ck.w < n_items) kidx = load_idx(ck, (int)cta);
           did = true;

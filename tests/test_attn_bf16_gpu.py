@@ -443,3 +443,26 @@ def test_native_few_tiles_run_in_slices(tokens, heads, topk):
     last = slice(tokens - 128 // heads, tokens)
     assert bool((out[last] == 0).all()) and bool(torch.isposinf(lse[last]).all())
     assert bool(torch.isfinite(out.float()).all())
+
+
+@pytest.mark.parametrize("counts", [(1, 2, 1, 1, 2, 1), (1, 1, 2, 1, 1, 1), (2, 1, 1, 1, 2, 1)])
+def test_native_items_of_one_and_two_blocks_in_a_row(counts):
+    # every cluster of the launch gets items of these numbers of key blocks one after the other: the
+    # orders in which a K copy behind two Q entries could meet a slot whose PV was still pending
+    clusters = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    T, s_kv = 2 * clusters * len(counts), 4096
+    g = torch.Generator().manual_seed(16)
+    idx = torch.full((T, 64), -1, dtype=torch.int32)
+    for tile in range(T // 2):
+        pos = torch.randperm(s_kv, generator=g)[:128].to(torch.int32).sort().values
+        two = counts[tile // clusters] == 2
+        idx[2 * tile] = pos[0::2]
+        idx[2 * tile + 1] = pos[1::2] if two else pos[0::2]     # a union of 128 or of 64 keys
+    kv = synth.make_kv_cache(s_kv, seed=16, mode="native")
+    q = synth.make_q(T, 64, seed=16, mode="native")
+    api.bf16_status(reset=True)
+    for _ in range(3):
+        out, lse = api.sparse_prefill(q.to(DEV), kv.to(DEV), idx.to(DEV), synth.SM_SCALE)
+        torch.cuda.synchronize()
+        assert api.bf16_status()[0] == 0
+        _check_exact(out, lse, q, kv, idx, tag=f"blocks {counts}")
