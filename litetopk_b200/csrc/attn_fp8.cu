@@ -113,7 +113,9 @@ struct Misc {
   uint64_t qt_ready;                // leader CTA: Q's latent part is in tensor memory in both CTAs
   uint64_t q_free;                  // all QK^T of the current item are complete (Q reusable)
   uint64_t o_free;                  // leader CTA: the item's O has been read out of TMEM
-  uint64_t epi_ready;               // the item's row scales are published (softmax warps)
+  uint64_t epi_ready[2];            // the item's row scales are published (softmax warps), by parity of
+                                    // the item ordinal: with items of one or two blocks the next item's can
+                                    // be complete before the epilogue has looked at this one's
   uint32_t valid[2][4];             // 128 validity bits per stage
   uint32_t tmem_base;
   uint32_t pad;
@@ -240,7 +242,6 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
-    mbar_init(&ms.epi_ready, kSoftmaxWarps);
     for (int i = 0; i < 8; ++i) {
       mbar_init(&ms.k_peer[i], 1);
       mbar_init(&ms.v_peer[i], 1);
@@ -256,6 +257,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       mbar_init(&ms.valid_ready[i], 1);
       mbar_init(&ms.valid_free[i], 8);
       mbar_init(&ms.m_pub[i], 8);
+      mbar_init(&ms.epi_ready[i], kSoftmaxWarps);
     }
     fence_mbar_init();
     if (p.q_bf16 == nullptr) {
@@ -429,7 +431,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
 
       // end of item: merge the row sums (each relative to its own group's latest running max)
       // (the previous item's sums must have been read: every warp has arrived on its epi_ready)
-      if (it > 0) mbar_wait(&ms.epi_ready, (it - 1) & 1, wt, kSiteEpi, it);
+      if (it > 0) mbar_wait(&ms.epi_ready[(it - 1) & 1], ((it - 1) >> 1) & 1, wt, kSiteEpi, it);
       ms.fin_l[(g * 2 + cs) * 128 + tl] = li;
       if (cs == 0 && h == 0) {
         ms.fin_rm[g * 64 + r] = real_m;
@@ -471,7 +473,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ms.epi_ready);
+      if (lane == 0) mbar_arrive(&ms.epi_ready[it & 1]);
       kb0 += nb;
       ++it;
     }
@@ -891,7 +893,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         transfer_q(it + 1, n);
       }
       // the row scales are published and the item's last PV has completed
-      mbar_wait(&ms.epi_ready, it & 1, wt, kSiteEpi, it);
+      mbar_wait(&ms.epi_ready[it & 1], (it >> 1) & 1, wt, kSiteEpi, it);
       mbar_wait(&ms.pv_done[kbl & 3], (kbl >> 2) & 1, wt, kSiteEpi, item.nb);
       __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
       tc_fence_after();

@@ -98,7 +98,9 @@ struct Misc {
   uint64_t qt_ready;                // leader CTA: they are in tensor memory in both CTAs
   uint64_t q_free;                  // all QK^T of the current item are complete
   uint64_t o_free;                  // leader CTA: the item's O has been read out of TMEM
-  uint64_t epi_ready;               // the item's row scales are published
+  uint64_t epi_ready[2];            // the item's row scales are published, by parity of the item ordinal: with
+                                    // items of one or two blocks the next item's can be complete before the
+                                    // epilogue has looked at this one's
   uint32_t valid[2][2];             // 64 validity bits per stage (gather)
   uint32_t tmem_base, pad;
   float xbuf[2][2][128];            // [group][parity][lane]: row-max exchange between key halves
@@ -302,7 +304,6 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
-    mbar_init(&ms.epi_ready, kSoftmaxWarps);
     for (int i = 0; i < 8; ++i) {
       mbar_init(&ms.k_full[i], kTma ? 1 : kGatherWarps * 32);     // gather: one async arrival per thread
       mbar_init(&ms.v_full[i], kTma ? 1 : kGatherWarps * 32);
@@ -318,6 +319,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(&ms.valid_ready[i], 1);
       mbar_init(&ms.valid_free[i], 4);
       mbar_init(&ms.m_pub[i], 4);
+      mbar_init(&ms.epi_ready[i], kSoftmaxWarps);
       mbar_init(&ms.q_taken[i], 1);
     }
     fence_mbar_init();
@@ -515,7 +517,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
       // end of item: merge the row sums (each relative to its own group's latest running max; the
       // previous item's sums have been read once every warp has arrived on its epi_ready)
-      if (it > 0) mbar_wait(&ms.epi_ready, (it - 1) & 1, wt, kSiteEpi, it);
+      if (it > 0) mbar_wait(&ms.epi_ready[(it - 1) & 1], ((it - 1) >> 1) & 1, wt, kSiteEpi, it);
       ms.fin_l[g * 128 + tl] = li;
       if (h == 0) {
         ms.fin_rm[g * 64 + r] = real_m;
@@ -555,7 +557,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ms.epi_ready);
+      if (lane == 0) mbar_arrive(&ms.epi_ready[it & 1]);
       kb0 += nb;
       ++it;
     }
@@ -823,7 +825,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const int kbl = kb0 + item.nb - 1;           // last block of the item
       if (w + ncl < n_items) bring_q(w + ncl, it + 1, kb0 + item.nb + kQEntries * (it + 1));
       // the row scales are published and the item's last PV has completed
-      mbar_wait(&ms.epi_ready, it & 1, wt, kSiteEpi, it);
+      mbar_wait(&ms.epi_ready[it & 1], (it >> 1) & 1, wt, kSiteEpi, it);
       mbar_wait(&ms.pv_done[kbl & 3], (kbl >> 2) & 1, wt, kSiteEpi, item.nb);
       __syncwarp();
       tc_fence_after();

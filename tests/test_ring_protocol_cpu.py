@@ -162,3 +162,11 @@ def test_no_copy_overwrites_a_slot_in_use(source):
     ring = _constants(source)
     bad = [s for s in SEQUENCES if "overwrite" in _explore(s, **ring)]
     assert not bad, bad
+
+
+@pytest.mark.parametrize("source", ["mla_bf16.cuh", "attn_fp8.cu"])
+def test_every_order_of_steps_ends(source):
+    # a barrier that completes twice before a waiter looks leaves that waiter behind for good
+    ring = _constants(source)
+    bad = [s for s in SEQUENCES if _explore(s, **ring)]
+    assert not bad, bad
