@@ -315,7 +315,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       const size_t trow = (size_t)item.tile * p.G + row / p.h_per_q;     // (tile, token) of this row
       const uint32_t* mrow = p.memb ? p.memb + trow * capw + (key0 >> 5) : nullptr;
       // per-token causal prefix: this row may attend union ranks < row_bound
-      const int row_bound = p.len_per_q ? __ldg(p.len_per_q + trow) : 0x7fffffff;
+      const int row_bound = p.len_per_q ? __ldcg(p.len_per_q + trow) : 0x7fffffff;
       float m_mine = kMInit;      // the running max my row sum is relative to
       float li = 0.f, real_m = -INFINITY;
       const int k_first = (g - kb0) & 1;          // first local block with (kb0 + k) % 2 == g
@@ -468,7 +468,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
           // the epilogue warps need 1 / l per row; the sink joins the OUTPUT normaliser only (in l's
           // units: x 7, relative to m)
           float denom = li;
-          if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldg(p.sink + row) * kLog2e - m + kPScaleLog2);
+          if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldcg(p.sink + row) * kLog2e - m + kPScaleLog2);
           ms.oscale[it & 1][r] = (li > 0.f) ? __fdividef(p.out_scale, denom) : 0.f;
         }
       }

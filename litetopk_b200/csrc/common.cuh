@@ -101,7 +101,9 @@ inline int current_device() {
 // kernel launched this way calls pdl_wait() before its first access to global memory; it
 // returns when the predecessor has completed, and since that one has waited too, everything
 // before it as well.  pdl_trigger(): this kernel's blocks are all running or done, successors may
-// be scheduled into whatever room is left.
+// be scheduled into whatever room is left.  Such a kernel is alive while others still
+// write what it will read, so it reads global memory with __ldcg, __ldcs or plain loads, never through
+// the read-only path (__ldg), which takes the data to be constant for the whole life of the grid.
 template <class K, class... A>
 inline int launch_pdl(K kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
   cudaLaunchConfig_t cfg = {};

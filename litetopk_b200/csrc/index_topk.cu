@@ -126,7 +126,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // Halved: the drain computes relu(x) as (x + |x|) / 2 with the division folded in here.
   for (int i = threadIdx.x; i < kAccs * kCols; i += kThreads) {
     const long long r = (long long)tok0 * HI + i;
-    wsm[i] = r < (long long)p.T * HI ? 0.5f * __ldg(p.weights + r) : 0.f;
+    wsm[i] = r < (long long)p.T * HI ? 0.5f * __ldcg(p.weights + r) : 0.f;
   }
   __syncthreads();
   if (warp == 0) {
@@ -213,7 +213,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const bool all_toks = t_base + tpa <= p.T;
     auto scale_of = [&](int j) -> float {
       const int s_key = (j0 + j) * kKeyTile + krow;
-      return (p.k_scale && s_key < p.S) ? __ldg(p.k_scale + s_key) : 1.f;
+      return (p.k_scale && s_key < p.S) ? __ldcg(p.k_scale + s_key) : 1.f;
     };
     float* out = p.logits + (long long)t_base * p.ld + (long long)j0 * kKeyTile + krow;
     float ks_next = n_tiles > 0 ? scale_of(0) : 1.f;    // fetched a tile ahead
@@ -506,13 +506,13 @@ topk_select_kernel(const SelParams p) {
   }
   uint32_t kmax = 0u, kmin = 0xffffffffu;
   for (int i = tid; i < n; i += NT) {
-    const uint32_t u = okey(__ldg(row + i));
+    const uint32_t u = okey(__ldcg(row + i));
     if (kSmemRow) rowkeys[i] = u;
     kmax = max(kmax, u);
     kmin = min(kmin, u);
   }
   block_max_min<NT>(sh, kmax, kmin);         // barrier: the shared-memory row is complete
-  auto key_at = [&](int i) -> uint32_t { return kSmemRow ? rowkeys[i] : okey(__ldg(row + i)); };
+  auto key_at = [&](int i) -> uint32_t { return kSmemRow ? rowkeys[i] : okey(__ldcg(row + i)); };
   uint32_t ties = 0;
   const uint32_t kth = radix_kth<NT>(sh, key_at, n, kmax, kmin, (uint32_t)p.k, &ties);
   emit_ordered<NT>(sh, key_at, n, kth, ties, out, p.k);
@@ -665,7 +665,7 @@ __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* r
     if (tie_end == 0xffffffffu) emit([&](uint32_t i) { return sval[i] >= kv; });
     else emit([&](uint32_t i) { return sval[i] > kv || (sval[i] == kv && (uint32_t)spos[i] <= tie_end); });
   } else {
-    auto key_mem = [&](int i) -> uint32_t { return okey(__ldg(row + i)); };
+    auto key_mem = [&](int i) -> uint32_t { return okey(__ldcg(row + i)); };
     if (!have_kth) {
       uint32_t kmax = 0u, kmin = 0xffffffffu;
       for (int i = tid; i < n; i += NT) {
@@ -992,7 +992,7 @@ topk_select_chunked_kernel(const SelParams p) {
     // 2048 evenly spaced samples, read from memory while the first chunk lands
     float smp[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) smp[i] = __ldg(row + (int)(((long long)(4 * tid + i) * n) >> 11));
+    for (int i = 0; i < 4; ++i) smp[i] = __ldcg(row + (int)(((long long)(4 * tid + i) * n) >> 11));
     if (tid == 0) sh.n_cand = 0;
     float t_lo = -INFINITY;
     if (n > kSurvCap / 2) t_lo = sampled_threshold<NT>(sh, red_a, red_b, smp, n, p.k);
@@ -1058,7 +1058,7 @@ topk_select_cluster_kernel(const SelParams p, int nc) {
   }
   float smp[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) smp[i] = __ldg(row + (int)(((long long)(4 * tid + i) * n) >> 11));
+  for (int i = 0; i < 4; ++i) smp[i] = __ldcg(row + (int)(((long long)(4 * tid + i) * n) >> 11));
   __syncwarp();
   cluster_sync_all();          // barriers initialised; every CTA of the cluster runs (remote stores below)
   float t_lo = -INFINITY;

@@ -280,11 +280,11 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       t.row1 = max(0, p0 - p.window + 1);
       t.len1 = plast - t.row1 + 1;
     } else if (kSrc == kRank) {
-      const int4 r = __ldg(p.runs + t.tile);
+      const int4 r = __ldcg(p.runs + t.tile);
       t.row0 = r.x; t.len0 = max(r.y, 0);
       t.row1 = r.z; t.len1 = max(r.w, 0);
     } else {
-      t.len0 = min(max(p.counts ? __ldg(p.counts + t.tile) : p.cap, 0), p.cap);
+      t.len0 = min(max(p.counts ? __ldcg(p.counts + t.tile) : p.cap, 0), p.cap);
     }
     t.nh0 = halves_of(t.len0);
     t.k0 = 0;
@@ -388,10 +388,10 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         mrow = p.memb + trow * capw + h;
       } else {
         const int total = item.len0 + item.len1;
-        const int cnt = p.counts ? min(max(__ldg(p.counts + item.tile), 0), total) : total;
-        pref = min(__ldg(p.pref + trow), cnt);
-        lo = __ldg(p.win_lo + trow);
-        hi = min(__ldg(p.win_hi + trow), cnt);
+        const int cnt = p.counts ? min(max(__ldcg(p.counts + item.tile), 0), total) : total;
+        pref = min(__ldcg(p.pref + trow), cnt);
+        lo = __ldcg(p.win_lo + trow);
+        hi = min(__ldcg(p.win_hi + trow), cnt);
       }
       float m_mine = kMInit;      // the running max my row sum is relative to
       float li = 0.f, real_m = -INFINITY;
@@ -552,7 +552,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           if (p.max_logits) p.max_logits[grow] = real_m * kLn2;
           // the epilogue warps need 1 / normaliser per row; the sink joins it here only
           float denom = li;
-          if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldg(p.sink + row % p.sink_mod) * kLog2e - m);
+          if (p.sink != nullptr && li > 0.f) denom += fast_exp2(__ldcg(p.sink + row % p.sink_mod) * kLog2e - m);
           ms.oscale[it & 1][r] = (li > 0.f) ? __fdividef(1.0f, denom) : 0.f;
         }
       }

@@ -35,7 +35,7 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
   const int tile = row >> 7, r = row & 127;
   const size_t p0 = (size_t)tile * nsplit * 128 + r;            // slice j of the row: p0 + 128 j
   float2 ml = make_float2(-INFINITY, 0.f);
-  if (lane < nsplit) ml = __ldg(part_ml + p0 + (size_t)lane * 128);
+  if (lane < nsplit) ml = __ldcg(part_ml + p0 + (size_t)lane * 128);
   float m = ml.y > 0.f ? ml.x : -INFINITY;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -52,7 +52,7 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
     const float4* src = reinterpret_cast<const float4*>(part_o + (p0 + (size_t)j * 128) * 512) + lane;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const float4 v = __ldg(src + 32 * c);
+      const float4 v = __ldcg(src + 32 * c);
       acc[c].x = fmaf(v.x, fj, acc[c].x);
       acc[c].y = fmaf(v.y, fj, acc[c].y);
       acc[c].z = fmaf(v.z, fj, acc[c].z);
@@ -60,7 +60,7 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
     }
   }
   float denom = l;
-  if (sink != nullptr && l > 0.f) denom += fast_exp2(__ldg(sink + r % sink_mod) * kLog2e - m);
+  if (sink != nullptr && l > 0.f) denom += fast_exp2(__ldcg(sink + r % sink_mod) * kLog2e - m);
   const float os = l > 0.f ? __fdividef(out_scale, denom) : 0.f;
   uint2* dst = reinterpret_cast<uint2*>(out + (row / h) * out_ts + (row % h) * out_hs) + lane;
 #pragma unroll

@@ -88,7 +88,7 @@ union_qm_kernel(const UnionParams p) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int qd = i * NT + tid;
-      v[i] = qd < nquad ? __ldg(src + qd) : make_int4(-1, -1, -1, -1);
+      v[i] = qd < nquad ? __ldcg(src + qd) : make_int4(-1, -1, -1, -1);
     }
   }
   __syncthreads();
@@ -102,7 +102,7 @@ union_qm_kernel(const UnionParams p) {
     for (int i = 0; i < VPT; ++i) { insert(v[i].x); insert(v[i].y); insert(v[i].z); insert(v[i].w); }
   } else {
     for (int qd = tid; qd < nquad; qd += NT) {
-      const int4 t = __ldg(src + qd);
+      const int4 t = __ldcg(src + qd);
       insert(t.x); insert(t.y); insert(t.z); insert(t.w);
     }
   }
@@ -180,7 +180,7 @@ union_qm_kernel(const UnionParams p) {
     }
   } else {
     for (int qd = tid; qd < nquad; qd += NT) {
-      const int4 t = __ldg(src + qd);
+      const int4 t = __ldcg(src + qd);
       uint32_t* row = qm_s + fast_div(qd, p.kq, p.kq_mul) * capw;
       mark(t.x, row); mark(t.y, row); mark(t.z, row); mark(t.w, row);
     }

@@ -1,0 +1,18 @@
+"""Rules on the CUDA sources that no single run can show broken."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "litetopk_b200" / "csrc"
+
+
+def _code(path):
+    return re.sub(r"//[^\n]*", "", path.read_text())
+
+
+def test_dependent_launches_do_not_read_through_the_read_only_path():
+    # a kernel that waits with pdl_wait() is alive while its predecessors still write: ld.global.nc
+    # (__ldg) would take what they write to be constant
+    files = [f for f in sorted(CSRC.glob("*.cu*")) if f.name != "common.cuh" and "pdl_wait()" in _code(f)]
+    assert {f.name for f in files} >= {"attn_fp8.cu", "mla_bf16.cuh", "index_topk.cu", "prefill.cu", "union_qm.cu"}
+    for f in files:
+        assert "__ldg(" not in _code(f) and ".nc" not in _code(f), f.name
