@@ -64,7 +64,8 @@ struct LogitParams {
   const float* k_scale;     // [S] or null (1.0)
   float* logits;            // [T, ld]
   int T, Hi, S, q_pos0;
-  int tiles_per_split;      // key tiles of one CTA: blockIdx.y owns tiles [y * this, (y + 1) * this)
+  int live_tiles;           // key tiles up to the last token's causal bound
+  int tiles_per_split;      // of these, blockIdx.y owns tiles [y * this, (y + 1) * this)
   long long ld;
   int epoch;
   unsigned long long wait_limit_ns;
@@ -109,7 +110,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int pos_max = p.q_pos0 + tok_end - 1;
   const int all_tiles = (p.S + kKeyTile - 1) / kKeyTile;
   const int causal_tiles = min(all_tiles, pos_max / kKeyTile + 1);
-  const int j0 = blockIdx.y * p.tiles_per_split, j_end = min(j0 + p.tiles_per_split, all_tiles);
+  const int j0 = blockIdx.y * p.tiles_per_split, j_end = min(j0 + p.tiles_per_split, p.live_tiles);
   const int n_tiles = max(min(j_end, causal_tiles) - j0, 0);
 
   if (threadIdx.x == 0) {
@@ -199,15 +200,21 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       w[i] = *reinterpret_cast<const float2*>(wsm + a * kCols + 8 * i + 2 * (lane & 3));
     // Key tiles beyond the causal bound of the CTA's last token are not computed: their entries
     // are -inf for every token of the CTA (this warp's tokens and key rows).  Written first,
-    // while the tensor core fills the first accumulators.
-    for (int j = j0 + n_tiles; j < j_end; ++j) {
-      const int s_key = j * kKeyTile + krow;
-      if (s_key < p.S) {
+    // while the tensor core fills the first accumulators: those of the CTA's own range, and its share of
+    // the tiles beyond every token's bound.
+    auto fill = [&](int ja, int jb) {
+      for (int j = ja; j < jb; ++j) {
+        const int s_key = j * kKeyTile + krow;
+        if (s_key < p.S) {
 #pragma unroll
-        for (int tt = 0; tt < tpa; ++tt)
-          if (t_base + tt < p.T) p.logits[(long long)(t_base + tt) * p.ld + s_key] = -INFINITY;
+          for (int tt = 0; tt < tpa; ++tt)
+            if (t_base + tt < p.T) p.logits[(long long)(t_base + tt) * p.ld + s_key] = -INFINITY;
+        }
       }
-    }
+    };
+    fill(j0 + n_tiles, j_end);
+    const long long dead = all_tiles - p.live_tiles;
+    fill(p.live_tiles + (int)(dead * blockIdx.y / gridDim.y), p.live_tiles + (int)(dead * (blockIdx.y + 1) / gridDim.y));
     // tiles below this one lie inside the cache and inside every token's causal bound
     const int j_plain = min(p.S, p.q_pos0 + tok0 + 1) / kKeyTile - j0;
     const bool all_toks = t_base + tpa <= p.T;
@@ -289,7 +296,10 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 // four (TMEM and barrier set-up, the 64 KB of Q, the first K tile), so the launch takes
 // waves(ctas_x * splits) * (4 + tiles per split): few tokens need many splits to fill the SMs (36
 // tokens of 32 heads are 3 CTAs: 867 -> 22 us against 100K keys), many tokens a few so that the
-// last wave is full.
+// last wave is full.  The tiles beyond every token's position are only filled with -inf, at about a 90th of
+// a unit per tile and token of the CTA, and shared out among the same CTAs.  (A CTA per range of the
+// whole cache paid the start-up for each of them: 150 tokens of 128 heads at position 0 of 131072
+// 507 us; with ranges of the live tiles alone 20.)
 static int sm_count() {
   static thread_local int cached_dev = -1, cached = 148;
   int dev = 0;
@@ -300,14 +310,14 @@ static int sm_count() {
   }
   return cached;
 }
-static int pick_splits(int ctas_x, int tiles, int sms) {
+static int pick_splits(int ctas_x, int live, int dead, int tok_per_cta, int sms) {
   int best = 1;
   long long best_cost = -1;
-  const int most = tiles < 64 ? tiles : 64;
-  for (int n = 1; n <= most; ++n) {
-    const int per = (tiles + n - 1) / n;
-    const long long waves = ((long long)ctas_x * ((tiles + per - 1) / per) + sms - 1) / sms;
-    const long long cost = waves * (4 + per);
+  for (int n = 1; n <= 64 && n <= live + dead; ++n) {
+    const int per = (live + n - 1) / n;
+    const long long ranges = dead > 0 ? n : (live + per - 1) / per;      // CTAs with something to do
+    const long long waves = (ctas_x * ranges + sms - 1) / sms;
+    const long long cost = waves * (90LL * (4 + per) + (long long)((dead + n - 1) / n) * tok_per_cta);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = n; }
   }
   return best;
@@ -1104,8 +1114,8 @@ topk_select_cluster_kernel(const SelParams p, int nc) {
 //   q_idx8  [T, Hi, 128] e4m3 codes, dense; Hi in {32, 64, 128}
 //   k_idx8  [S, 128] e4m3 codes, rows k_row_stride bytes apart (multiple of 16)
 //   weights [T, Hi] fp32;  k_scale [S] fp32 or null (1.0)
-//   logits  [T, logits_row_stride] fp32: entries s <= q_pos0 + t are written, entries beyond a
-//           token's position inside the processed tiles are -inf, later ones are left untouched
+//   logits  [T, logits_row_stride] fp32: the first S entries of every row are written, those beyond
+//           the token's position (s > q_pos0 + t) as -inf
 // No counterpart in the reference (its indexer was removed); asynchronous on `stream`.
 extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, const float* weights,
                                         const float* k_scale, float* logits, int T, int Hi, int S,
@@ -1137,9 +1147,11 @@ extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, 
   // the tiles that do work: up to the last token's causal bound
   const int all_tiles = (S + kKeyTile - 1) / kKeyTile;
   const int live_tiles = (int)min((long long)all_tiles, ((long long)q_pos0 + T - 1) / kKeyTile + 1);
-  const int splits = pick_splits(ctas_x, live_tiles, sm_count());
+  const int dead_tiles = all_tiles - live_tiles;
+  const int splits = pick_splits(ctas_x, live_tiles, dead_tiles, tok_per_cta, sm_count());
+  p.live_tiles = live_tiles;
   p.tiles_per_split = (live_tiles + splits - 1) / splits;
-  const int grid_y = (all_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+  const int grid_y = dead_tiles > 0 ? splits : (live_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
   return launch_pdl(Hi == 32 ? index_logits_kernel<32> : (Hi == 64 ? index_logits_kernel<64> : index_logits_kernel<128>),
                     dim3(ctas_x, grid_y), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_k, p);
 }

@@ -296,3 +296,24 @@ def test_topk_select_few_rows_shared_by_clusters(T, S, k):
     torch.cuda.synchronize()
     assert api.index_status(reset=True)[0] == 0
     assert np.array_equal(_canon(got), ref)
+
+
+def test_index_logits_of_a_long_cache_before_its_tokens_arrive():
+    # tokens at the start of a cache of more than 65535 key tiles, all but the first beyond their positions
+    T, S, Hi, pos0 = 3, 65536 * 128 + 5, 64, 70
+    q8, k8, w, ks = _ops(T, 256, Hi, seed=5)
+    keys = torch.zeros((S, 128), dtype=torch.uint8, device=DEV)
+    keys[:256] = k8.to(DEV).view(torch.uint8)
+    scale = torch.ones((S,), device=DEV)
+    scale[:256] = ks.to(DEV)
+    got = torch.full((T, S), 7.0, device=DEV)
+    api.index_logits_fp8(q8.to(DEV), keys, w.to(DEV), scale, pos0, out=got)
+    torch.cuda.synchronize()
+    assert api.index_status(reset=True)[0] == 0
+    ref = io.index_logits(q8, k8, w, ks, pos0)
+    head = got[:, :256].cpu().double()
+    fin = torch.isfinite(ref)
+    assert torch.equal(torch.isinf(head), ~fin)
+    # fp32 sums of Hi products: the bound of the other comparisons with the oracle in this file
+    assert float((head[fin] - ref[fin]).abs().max()) <= 2e-5 * float(ref[fin].abs().max())
+    assert bool(torch.isneginf(got[:, 256:]).all())
