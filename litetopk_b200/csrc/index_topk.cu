@@ -1107,6 +1107,32 @@ topk_select_cluster_kernel(const SelParams p, int nc) {
   finish_row<NT>(sh, red_a, red_b, &eq_total, sval, spos, m_s, fast, row, n, p.k, out);
 }
 
+constexpr size_t kChunkDyn = (size_t)2 * kChunk * 4 + (size_t)kSurvCap * 8;
+
+// how many clusters of nc (2, 4 or 8) CTAs of topk_select_cluster_kernel device `dev` holds at once
+static int row_clusters(int dev, int nc, int sms) {
+  static thread_local int cached_dev = -1, cached[3];
+  if (dev != cached_dev) {
+    for (int i = 0; i < 3; ++i) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)((sms >> (i + 1)) << (i + 1))); cfg.blockDim = dim3(kStreamThreads);
+      cfg.dynamicSmemBytes = kChunkDyn;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = 2u << i; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+      cfg.attrs = &at; cfg.numAttrs = 1;
+      int n = 0;
+      if (!ensure_smem<topk_select_cluster_kernel>(dev, kChunkDyn) ||
+          cudaOccupancyMaxActiveClusters(&n, topk_select_cluster_kernel, &cfg) != cudaSuccess)
+        n = 0;
+      cudaGetLastError();
+      cached[i] = n;
+    }
+    cached_dev = dev;
+  }
+  return cached[nc == 8 ? 2 : nc >> 2];
+}
+
 }  // namespace idx
 }  // namespace lt
 
@@ -1179,16 +1205,19 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
   const int dev = lt::current_device();
   const bool aligned = (logits_row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
   const int sms = sm_count(), grid = T < sms ? T : sms;
-  const size_t chunk_dyn = (size_t)2 * kChunk * 4 + (size_t)kSurvCap * 8;
-  // Few rows: as many CTAs per row as the chip has for each, if every one of them gets at least
-  // 4096 entries (below that the extra cluster synchronisations cost what the shorter filter saves)
-  int nc = 8;
-  while (nc > 1 && ((long long)T * nc > sms || S < 4096 * nc)) nc >>= 1;
-  if (aligned && nc > 1) {
-    if (!lt::ensure_smem<topk_select_cluster_kernel>(dev, chunk_dyn)) return LITEDSA_ERR_CUDA;
+  // Few long rows: the largest clusters of which the chip holds one per row at once, if every CTA gets at
+  // least 8192 entries.  Below 24576 entries the cluster synchronisations cost more than the shorter
+  // filter saves (20000 entries, k = 2048: 11.9 us, one CTA per row 10.3; 32768: 12.2 and 12.3; 131072:
+  // 14.1 and 28.8).  What counts is how many clusters fit, not how many SMs there are: 18 clusters of eight are
+  // 144 CTAs but more than the chip's GPCs hold, and the second wave made 18 rows of 32768 entries take
+  // 20.3 us.
+  int nc = aligned ? 8 : 1;
+  while (nc > 1 && (S <= 24576 || S < 8192 * nc || T > row_clusters(dev, nc, sms))) nc >>= 1;
+  if (nc > 1) {
+    if (!lt::ensure_smem<topk_select_cluster_kernel>(dev, kChunkDyn)) return LITEDSA_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(T * nc)); cfg.blockDim = dim3(kStreamThreads);
-    cfg.dynamicSmemBytes = chunk_dyn; cfg.stream = st;
+    cfg.dynamicSmemBytes = kChunkDyn; cfg.stream = st;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)nc; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -1207,8 +1236,8 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
                           kStreamThreads, dyn, st, p);
   }
   if (aligned) {
-    if (!lt::ensure_smem<topk_select_chunked_kernel>(dev, chunk_dyn)) return LITEDSA_ERR_CUDA;
-    return lt::launch_pdl(topk_select_chunked_kernel, dim3(grid), kStreamThreads, chunk_dyn, st, p);
+    if (!lt::ensure_smem<topk_select_chunked_kernel>(dev, kChunkDyn)) return LITEDSA_ERR_CUDA;
+    return lt::launch_pdl(topk_select_chunked_kernel, dim3(grid), kStreamThreads, kChunkDyn, st, p);
   }
   if (S <= kMaxSmemRow) {
     if (!lt::ensure_smem<topk_select_kernel<true>>(dev, smem)) return LITEDSA_ERR_CUDA;

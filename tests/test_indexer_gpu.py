@@ -284,7 +284,8 @@ def test_index_logits_with_the_keys_split_over_ctas(T, S, Hi, pos0):
     assert float((got[fin] - ref[fin]).abs().max()) <= 2e-5 * float(ref[fin].abs().max())
 
 
-@pytest.mark.parametrize("T,S,k", [(1, 32768, 2048), (7, 40004, 1000), (18, 262148, 512), (2, 8192, 4096)])
+@pytest.mark.parametrize("T,S,k", [(1, 32768, 2048), (7, 40004, 1000), (18, 262148, 512), (2, 8192, 4096),
+                                   (40, 33332, 512), (15, 65540, 2048)])
 def test_topk_select_few_rows_shared_by_clusters(T, S, k):
     # eight, four or two CTAs per row; lengths around the segment and chunk boundaries
     x = _random_logits(T, S, seed=S + k)
