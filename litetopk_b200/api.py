@@ -667,6 +667,18 @@ def _derived_q_scale(q: torch.Tensor) -> float:
     return 2.0 ** max(-24, int(torch.tensor(max(amax, 1e-30) / 448.0).log2().ceil().item()))
 
 
+def _quantise_first(ng: int, G: int, cap: int) -> bool:
+    """Whether bf16 queries of an FP8 call get a quantisation pass of their own, or are quantised by the
+    attention kernel on their way in.  The kernel's epilogue warps do that between two outputs, about
+    10 us per tile, which only tiles of five key blocks or more hide; a pass costs 3 us per tile and
+    cluster.  With one token per tile that is a list of up to 512 entries (4096 tokens x 128 heads, in
+    the kernel / with the pass: top-256 579 / 445 us, top-512 614 / 543, top-1024 823 / 843).  The union
+    of several tokens is not known here: only tiles of a single block (4096 x 64 heads, top-64 278 / 221
+    and 288 / 268 us at half and nine tenths sharing; top-256 302 / 252 but 327 / 344).  Few tiles
+    have nothing to hide."""
+    return ng > 296 and cap <= (512 if G == 1 else 128)
+
+
 def _masked_mla_fp8_bf16q(q, q_scale, kv, indices, sm_scale, out_scale, counts, mask, h, out, ml, lse) -> None:
     """The FP8 operator on contiguous bf16 q [T, h, 576], quantised inside the attention kernel; the
     other tensors as masked_mla_fp8 has made or checked them."""
@@ -747,10 +759,15 @@ def masked_mla_fp8(q: torch.Tensor, kv_cache_fp8: torch.Tensor, union_idx: torch
         if q.dtype == torch.bfloat16:
             if q_scale is None:
                 q_scale = _derived_q_scale(q)
-            _masked_mla_fp8_bf16q(q.contiguous(), float(q_scale), kv, union_idx, float(sm_scale) * q_scale * ks, ks,
-                                  counts, mask, h, out, ml, lse)
+            q = q.contiguous()
+            if _quantise_first(ng, G, union_idx.shape[-1]):
+                q = quantize_e4m3(q, q_scale)
         else:
             q_scale = 1.0 if q_scale is None else q_scale
+        if q.dtype == torch.bfloat16:
+            _masked_mla_fp8_bf16q(q, float(q_scale), kv, union_idx, float(sm_scale) * q_scale * ks, ks,
+                                  counts, mask, h, out, ml, lse)
+        else:
             masked_mla_fp8_out(q.contiguous().view(ng, 128, 576), kv, union_idx, float(sm_scale) * q_scale * ks,
                                ks, counts, mask, h, out, ml, lse)
     res = (out.view(T, h, 512), lse.view(T, h))
@@ -796,6 +813,8 @@ def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_spac
         kv_scale = 1.0
     if q_scale is None:
         q_scale = _derived_q_scale(q) if q_bf16 and not kv_bf16 else 1.0
+    if q_bf16 and not kv_bf16 and _quantise_first(T * h // 128, 128 // h, 128 // h * k):
+        q, q_bf16 = quantize_e4m3(q, q_scale), False
     if out is None:
         out = torch.empty((T, h, 512), dtype=torch.bfloat16, device=dev)
     else:

@@ -500,3 +500,19 @@ def test_many_one_block_tiles(qdtype):
     assert mad <= TOL_ABS * max(1.0, float(ref[0].float().abs().max())) and cos >= TOL_COS, (mad, cos)
     assert float((lse.cpu().view(w.tiles, 128) - ref[1]).abs().max()) <= TOL_LSE
     assert api.attn_status()[0] == 0
+
+
+@pytest.mark.parametrize("tokens,heads,topk", [(600, 64, 64), (600, 64, 128), (300, 128, 512), (300, 128, 640)])
+def test_bf16_queries_give_the_same_bits_however_they_are_quantised(tokens, heads, topk):
+    # on both sides of the rule that gives many tiles of short lists a quantisation pass of their own
+    w, idx, kv, q = _case(tokens, heads, topk, 4096, (0.8, 0.8), seed=18)
+    q8, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    qd, kvd, idd = q.to(DEV), kv8.to(DEV), idx.to(DEV)
+    assert api._quantise_first(w.tiles, w.group, w.cap) == ((heads, topk) in ((64, 64), (128, 512)))
+    want_o, want_l = api.sparse_prefill(q8.view(tokens, heads, 576).to(DEV), kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    out, lse = api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    assert torch.equal(out, want_o) and torch.equal(lse, want_l)
+    u, m, c = api.union_qm(idd, w.group, seq_space=w.s_kv, return_counts=True)
+    out, lse = api.masked_mla_fp8(qd, kvd, u, m, synth.SM_SCALE, counts=c, kv_scale=ks, q_scale=qs)
+    assert torch.equal(out, want_o) and torch.equal(lse, want_l)
+    assert api.attn_status()[0] == 0
