@@ -53,16 +53,17 @@ classify_runs_kernel(const int32_t* __restrict__ indices, long long idx_stride, 
 
 
 // Slices of a tile when a call has `tiles` tiles of up to `blocks` key blocks: as many as there are
-// idle clusters for, at least five blocks each, none below 20 blocks.  Slices cost about 5 us (a launch for the
-// merge, fp32 partial results), a block of an unsliced tile 0.75 us.  (With slices from six blocks on,
-// 24 tokens against 77777 positions took 25.5 us, unsliced 20.)
+// idle clusters for, at least five blocks each, none below 20 blocks.  They cost a launch for the merge and
+// fp32 partial results, which grow with their number, so they have to shorten a tile by at least 4 +
+// 0.1 tiles n of its blocks of 0.75 us.  (24 tokens against 77777 positions in slices from six blocks on
+// 25.5 us, unsliced 20; 37 tiles of 20 blocks in two slices 26.6, unsliced 24.7, of 26 blocks 28.8 and 29.3;
+// one tile of 26 blocks in five 18.4 and 28.4.)
 static int pick_slices(int tiles, int blocks) {
-  constexpr int kClusters = 74;
   if (blocks < 20) return 1;
-  int n = kClusters / tiles;
+  int n = sm_count() / 2 / tiles;
   if (n > blocks / 5) n = blocks / 5;
   if (n > kMaxSlices) n = kMaxSlices;
-  return n < 2 ? 1 : n;
+  return n >= 2 && blocks - (double)blocks / n >= 4.0 + 0.1 * tiles * n ? n : 1;
 }
 // most blocks a tile of the call can have: its last tile has the longest prefix
 static int most_blocks(int ng, int G, int n_comp, int pos0, int window, int ratio) {

@@ -94,6 +94,16 @@ inline int current_device() {
   int dev = -1;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
 }
+// SMs of the current device
+inline int sm_count() {
+  static thread_local int cached_dev = -1, cached = 148;
+  const int dev = current_device();
+  if (dev >= 0 && dev != cached_dev &&
+      cudaDeviceGetAttribute(&cached, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+    cached_dev = dev;
+  cudaGetLastError();
+  return cached;
+}
 
 // Launch that may start while its predecessor on the stream is still running (programmatic
 // dependent launch): launch latency, block scheduling and everything a kernel does before

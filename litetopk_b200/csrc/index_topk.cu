@@ -300,16 +300,6 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 // a unit per tile and token of the CTA, and shared out among the same CTAs.  (A CTA per range of the
 // whole cache paid the start-up for each of them: 150 tokens of 128 heads at position 0 of 131072
 // 507 us; with ranges of the live tiles alone 20.)
-static int sm_count() {
-  static thread_local int cached_dev = -1, cached = 148;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev != cached_dev) {
-    cudaDeviceGetAttribute(&cached, cudaDevAttrMultiProcessorCount, dev);
-    cached_dev = dev;
-  }
-  return cached;
-}
 static int pick_splits(int ctas_x, int live, int dead, int tok_per_cta, int sms) {
   int best = 1;
   long long best_cost = -1;
@@ -1204,7 +1194,7 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
   const size_t smem = (((size_t)S + 3) & ~(size_t)3) * 4;      // whole 16-byte quads
   const int dev = lt::current_device();
   const bool aligned = (logits_row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
-  const int sms = sm_count(), grid = T < sms ? T : sms;
+  const int sms = lt::sm_count(), grid = T < sms ? T : sms;
   // Few long rows: the largest clusters of which the chip holds one per row at once, if every CTA gets at
   // least 8192 entries.  Below 24576 entries the cluster synchronisations cost more than the shorter
   // filter saves (20000 entries, k = 2048: 11.9 us, one CTA per row 10.3; 32768: 12.2 and 12.3; 131072:

@@ -72,23 +72,27 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
   if (lane == 0) lse[row] = l > 0.f ? __logf(l) + m * kLn2 - lse_off : INFINITY;
 }
 
-// How many slices a tile is cut into when a launch has `tiles` tiles of G lists of k entries.  A union
-// is not known on the host; neighbouring tokens share about three quarters of their lists, so it is
-// taken as k (3 + G) / 4 entries.  Slices cost about 6 us (a launch for the merge, fp32 partial
-// results) and a block each for the running max, a block of an unsliced tile 1.1 us: from 12 blocks on
-// there are slices, of at least four blocks, at most as many as there are idle clusters for.  (Slices of two
-// or three blocks from lists of 8 blocks on: 36 tokens x 32 heads, top-1024 33 us, now 27 (unsliced 29); 64 x 16,
-// top-1024 36, now 30 (39); 64 x 64, top-512 26, now 19; two tokens x 64, top-2048 26 both (34).)
-// The bf16 kernel's blocks are 64 keys and take 0.8 us: from 20 on, at least five per slice.  (Native cache,
-// two tokens x 64 heads, top-2048: 52 -> 26 us; 36 x 32, top-1024: 41 -> 27; 64 x 16, top-2048: 103 -> 45.)
+// How many slices a tile is cut into when a launch has `tiles` tiles of G lists of k entries: as many as
+// there are idle clusters for, of at least four 128-key blocks (bf16 kernel: five of 64), if a tile has
+// 12 (20).  A union is not known on the host; neighbouring tokens share about three quarters of their
+// lists, so it is taken as k (3 + G) / 4 entries.  Slices cost a launch for the merge, a block each for the
+// running max, and fp32 partial results, which grow with their number; a block of an unsliced tile takes
+// 1.1 us (0.8).  FP8 slices that shorten a tile by less than 4 + 0.08 tiles n blocks even when only half of
+// the lists is shared are not made (128 heads, 37 tiles of 12 blocks: 30.5 us in two slices, 25.6 whole).
+// Graph replays of 1440 calls (8 to 128 heads, 1 to 37 tiles, 256 to 3072 entries, 50 to 90 % sharing): FP8
+// 0.80 of the unsliced time in the mean, 59 of 660 calls more than 2 % slower, all of them with unions
+// much shorter than taken here (8 heads, 24 tiles, top-384: nine tenths shared 28.8 and 23.1 us, half
+// shared 36.0 and 41.8); bf16 0.61 and 6 of 780.  Two tokens x 64 heads, top-2048:
+// FP8 32.2 -> 24.1 us.
 static int pick_slices(int tiles, int G, int k, bool bf16) {
-  constexpr int kClusters = 74;
   const int blocks = (int)((int64_t)k * (3 + G) / 4 / (bf16 ? 64 : 128));
   if (blocks < (bf16 ? 20 : 12)) return 1;
-  int n = kClusters / tiles;
+  int n = sm_count() / 2 / tiles;
   if (n > blocks / (bf16 ? 5 : 4)) n = blocks / (bf16 ? 5 : 4);
   if (n > kMaxSlices) n = kMaxSlices;
-  return n < 2 ? 1 : n;
+  if (n < 2) return 1;
+  const double half = (double)k * (1 + G) / 2 / 128;
+  return bf16 || half - (half / n + 1.0) >= 4.0 + 0.08 * tiles * n ? n : 1;
 }
 
 // workspace layout: all offsets are multiples of 256 bytes

@@ -286,7 +286,7 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
   // several tiles per SM.  (65536 tokens of 16 heads, top-2048 of 131072: 610 us with one CTA of 1024
   // threads per SM, 440 with two of 512; 16384 x 32 heads, top-1024 of 65536: 72 -> 55.)
   const bool small = quads <= 256 && s_words <= 1024;
-  const int nt = ng <= 148 && !small ? 1024 : (quads <= 2048 ? 256 : 512);
+  const int nt = ng <= sm_count() && !small ? 1024 : (quads <= 2048 ? 256 : 512);
   const int qpt = (s_words / 4 + nt - 1) / nt;
   p.quads_per_thread = qpt == 1 ? 1 : (qpt | 1);
   const int vpt = (quads + nt - 1) / nt;

@@ -451,6 +451,7 @@ def test_path_agrees_with_the_stock_per_token_sparse_mla_kernel():
     (2, 64, 512, 4096),         # too short to slice
     (34, 64, 1024, 8192),       # 17 tiles, too short to slice
     (34, 64, 1536, 16384),      # 17 tiles, three slices
+    (34, 64, 2048, 16384),      # 17 tiles, four slices
     (8, 16, 2048, 20000),       # one tile of eight tokens, eleven slices
     (8, 16, 4096, 20000),       # ... sixteen slices
     (300, 32, 256, 5000),       # 75 tiles: one more than clusters
