@@ -74,21 +74,30 @@ int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng,
                  float* lse, cudaStream_t stream);
 
 // ---------------------------------------------------------------- launches
-// Raises a kernel's dynamic shared-memory limit on the current device, once per size (the call
-// costs as much host time as a launch).
+// Raises a kernel's dynamic shared-memory limit on the current device to all that its static part leaves,
+// once (the call costs as much host time as a launch); true if `bytes` fit.  The limit does not depend
+// on `bytes`: with the size of each call, a thread that set a smaller one last could leave the limit
+// below what another had recorded.
 constexpr int kMaxDevices = 64;
 template <auto kKernel>
 inline bool ensure_smem(int dev, size_t bytes) {
-  static std::atomic<int> have[kMaxDevices];
+  static std::atomic<int> limit[kMaxDevices];
   if (dev < 0 || dev >= kMaxDevices) return false;
-  if (have[dev].load(std::memory_order_relaxed) >= (int)bytes) return true;
-  if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
+  int have = limit[dev].load(std::memory_order_acquire);
+  if (have == 0) {
+    cudaFuncAttributes fa;
+    int most = 0;
+    if (cudaFuncGetAttributes(&fa, kKernel) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    have = most - (int)fa.sharedSizeBytes;
+    limit[dev].store(have, std::memory_order_release);
   }
-  int old = have[dev].load(std::memory_order_relaxed);
-  while (old < (int)bytes && !have[dev].compare_exchange_weak(old, (int)bytes)) {}
-  return true;
+  return bytes <= (size_t)have;
 }
 inline int current_device() {
   int dev = -1;

@@ -16,3 +16,13 @@ def test_dependent_launches_do_not_read_through_the_read_only_path():
     assert {f.name for f in files} >= {"attn_fp8.cu", "mla_bf16.cuh", "index_topk.cu", "prefill.cu", "union_qm.cu"}
     for f in files:
         assert "__ldg(" not in _code(f) and ".nc" not in _code(f), f.name
+
+
+def test_a_kernels_shared_memory_limit_does_not_depend_on_the_call():
+    # two threads that set a kernel's limit to their own sizes can leave it below what one of them has
+    # recorded; every caller sets the same one
+    calls = [c for f in sorted(CSRC.glob("*.cu*"))
+             for c in re.findall(r"cudaFuncSetAttribute\(([^;{]*)", _code(f)) if "MaxDynamicSharedMemorySize" in c]
+    assert calls
+    for c in calls:
+        assert not re.search(r"\b(bytes|dyn|smem)\b", c), c
