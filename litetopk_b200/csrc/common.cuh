@@ -114,6 +114,14 @@ inline int sm_count() {
   return cached;
 }
 
+// The status of a launch.  A refused one is reported here and nowhere else: the runtime would hand its
+// error to the next caller of cudaGetLastError(), in this library or outside it.
+inline int launch_result(cudaError_t e) {
+  if (e == cudaSuccess) return LITEDSA_OK;
+  cudaGetLastError();
+  return LITEDSA_ERR_CUDA;
+}
+
 // Launch that may start while its predecessor on the stream is still running (programmatic
 // dependent launch): launch latency, block scheduling and everything a kernel does before
 // pdl_wait() (barriers, tensor memory, shared-memory clears) overlap the predecessor's tail.  Every
@@ -131,7 +139,7 @@ inline int launch_pdl(K kern, dim3 grid, int threads, size_t smem, cudaStream_t 
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+  return launch_result(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

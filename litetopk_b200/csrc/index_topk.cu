@@ -1214,8 +1214,7 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel, (const SelParams)p, nc) == cudaSuccess
-               ? LITEDSA_OK : LITEDSA_ERR_CUDA;
+    return lt::launch_result(cudaLaunchKernelEx(&cfg, topk_select_cluster_kernel, (const SelParams)p, nc));
   }
   if (aligned && S <= kStreamThreads * 64) {
     const bool small = S <= kStreamThreads * 32;

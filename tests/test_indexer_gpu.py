@@ -318,3 +318,27 @@ def test_index_logits_of_a_long_cache_before_its_tokens_arrive():
     # fp32 sums of Hi products: the bound of the other comparisons with the oracle in this file
     assert float((head[fin] - ref[fin]).abs().max()) <= 2e-5 * float(ref[fin].abs().max())
     assert bool(torch.isneginf(got[:, 256:]).all())
+
+
+@pytest.mark.parametrize("T,S", [(4, 65536), (300, 1024)])           # the cluster launch, a plain one
+def test_a_refused_launch_is_reported_once(T, S):
+    # a stream whose capture has been invalidated (by synchronising it) refuses launches
+    import ctypes
+    from litetopk_b200 import _lib
+    rt = ctypes.CDLL("libcudart.so.12")
+    x = _random_logits(T, S, seed=2).to(DEV)
+    sel = torch.empty((T, 64), dtype=torch.int32, device=DEV)
+    api.topk_select(x, 64, q_pos0=S, out=sel)
+    torch.cuda.synchronize()
+    stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(ctypes.byref(stream), 1) == 0
+    assert rt.cudaStreamBeginCapture(stream, 2) == 0
+    assert rt.cudaStreamSynchronize(stream) != 0
+    rt.cudaGetLastError()
+    rc = _lib.lib().litedsa_topk_select(x.data_ptr(), None, sel.data_ptr(), T, S, 64, S, S, stream)
+    left = rt.cudaGetLastError()
+    rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+    rt.cudaGetLastError()
+    assert rt.cudaStreamDestroy(stream) == 0
+    assert rc == 4 and left == 0, (rc, left)
+    torch.cuda.synchronize()
