@@ -143,7 +143,7 @@ int litedsa_masked_mla_fp8_bf16q(const void* q_bf16, float q_scale, const void* 
  *   workspace  256-byte aligned, litedsa_sparse_prefill_workspace(...) bytes
  */
 int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
-                           const int32_t* topk_idx, float sm_scale, float q_scale, float kv_scale,
+                           const int32_t* topk_idx, double sm_scale, double q_scale, double kv_scale,
                            void* out, float* lse, int T, int h, int k, int s_kv, int64_t kv_row_stride,
                            int64_t seq_space, int policy_tokens, void* workspace,
                            int64_t workspace_bytes, void* stream);

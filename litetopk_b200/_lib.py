@@ -6,7 +6,7 @@ resolved, importing `lib()` raises.
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_int, c_int64, c_uint64, c_float, c_void_p, c_char_p
+from ctypes import c_int, c_int64, c_uint64, c_double, c_float, c_void_p, c_char_p
 from pathlib import Path
 
 _PKG = Path(__file__).resolve().parent
@@ -36,8 +36,8 @@ SIGNATURES = {
     "litedsa_masked_mla_fp8_bf16q": (c_int, [c_void_p, c_float, c_void_p, c_void_p, c_float, c_float,
                                              c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                              c_int, c_int, c_int, c_int64, c_int64, c_void_p]),
-    "litedsa_sparse_prefill": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_float, c_float,
-                                       c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64,
+    "litedsa_sparse_prefill": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_double, c_double,
+                                       c_double, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64,
                                        c_int64, c_int, c_void_p, c_int64, c_void_p]),
     "litedsa_sparse_prefill_workspace": (c_int64, [c_int, c_int, c_int, c_int, c_int]),
     "litedsa_attn_status": (c_int, [c_void_p, c_int]),

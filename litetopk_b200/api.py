@@ -834,7 +834,7 @@ def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_spac
     ws = torch.empty((max(lib.litedsa_sparse_prefill_workspace(T, h, k, kv_bf16, job_tokens), 1),),
                      dtype=torch.uint8, device=dev)
     check(_on_device(dev, lib.litedsa_sparse_prefill, q.data_ptr(), q_bf16, kv.data_ptr(), kv_bf16,
-                     topk_idx.data_ptr(), sm_scale, q_scale, kv_scale, out.data_ptr(), lse.data_ptr(), T, h, k,
+                     topk_idx.data_ptr(), float(sm_scale), float(q_scale), float(kv_scale), out.data_ptr(), lse.data_ptr(), T, h, k,
                      kv.shape[0], kv.stride(0), (space + 1023) // 1024 * 1024, job_tokens, ws.data_ptr(),
                      ws.numel()), "sparse_prefill")
     return out, lse

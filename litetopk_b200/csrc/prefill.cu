@@ -138,7 +138,7 @@ extern "C" int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_
 
 // union_qm + masked attention of T query tokens in one call; see include/litedsa_b200.h.
 extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
-                                      const int32_t* topk_idx, float sm_scale, float q_scale, float kv_scale,
+                                      const int32_t* topk_idx, double sm_scale, double q_scale, double kv_scale,
                                       void* out, float* lse, int T, int h, int k, int s_kv,
                                       int64_t kv_row_stride, int64_t seq_space, int policy_tokens,
                                       void* workspace, int64_t workspace_bytes, void* stream) {
@@ -148,7 +148,7 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   int rc = check_shape(T, h, k, policy_tokens);
   if (rc != LITEDSA_OK) return rc;
   if (kv_is_bf16 && !q_is_bf16) return LITEDSA_ERR_UNSUPPORTED;
-  if (!kv_is_bf16 && q_is_bf16 && !(q_scale > 0.f)) return LITEDSA_ERR_SHAPE;
+  if (!kv_is_bf16 && q_is_bf16 && !((float)q_scale > 0.f)) return LITEDSA_ERR_SHAPE;
   if (((uintptr_t)workspace & 255) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)topk_idx & 15))
     return LITEDSA_ERR_UNSUPPORTED;
   const int G = 128 / h, ng = T / G, cap = G * k;
@@ -165,25 +165,26 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   if (kv_is_bf16 && ns > 1) {
     float* part_o = reinterpret_cast<float*>(ws + l.part_o);
     float2* part_ml = reinterpret_cast<float2*>(ws + l.part_ml);
-    rc = run_bf16_slices(q, kv, u, sm_scale, counts, memb, h, out, lse, ng, s_kv, cap, kv_row_stride, ns, part_o, part_ml, stream);
+    rc = run_bf16_slices(q, kv, u, (float)sm_scale, counts, memb, h, out, lse, ng, s_kv, cap, kv_row_stride, ns, part_o, part_ml, stream);
     if (rc != LITEDSA_OK) return rc;
     return merge_slices(part_o, part_ml, ns, ng, h, 1.f, 0.f, nullptr, 1, out, (int64_t)h * 512, 512, lse,
                         reinterpret_cast<cudaStream_t>(stream));
   }
   if (kv_is_bf16)
-    return litedsa_masked_mla_bf16(q, kv, u, sm_scale, counts, memb, h, out, nullptr, lse, ng, s_kv, cap, 576, 576,
+    return litedsa_masked_mla_bf16(q, kv, u, (float)sm_scale, counts, memb, h, out, nullptr, lse, ng, s_kv, cap, 576, 576,
                                    kv_row_stride, cap, nullptr, stream);
-  Fp8Args a{q, kv, u, sm_scale * q_scale * kv_scale, kv_scale, counts, memb, h, nullptr, lse,
+  // one rounding to fp32 of the whole product, as a caller of the operators makes it
+  Fp8Args a{q, kv, u, (float)(sm_scale * q_scale * kv_scale), (float)kv_scale, counts, memb, h, nullptr, lse,
             ng, s_kv, cap, 576, kv_row_stride, cap, nullptr, nullptr, 1};
   a.q_is_bf16 = q_is_bf16 != 0;
-  a.q_inv = 1.0f / q_scale;
+  a.q_inv = 1.0f / (float)q_scale;
   a.nsplit = ns;
   a.part_o = reinterpret_cast<float*>(ws + l.part_o);
   a.part_ml = ws + l.part_ml;
   void* outs[1] = {out};
   rc = run_fp8(a, outs, 1, stream);
   if (rc != LITEDSA_OK || ns == 1) return rc;
-  return merge_slices(a.part_o, reinterpret_cast<const float2*>(a.part_ml), ns, ng, h, kv_scale, kFp8LseOffset,
+  return merge_slices(a.part_o, reinterpret_cast<const float2*>(a.part_ml), ns, ng, h, a.out_scale, kFp8LseOffset,
                       nullptr, 1, out, (int64_t)h * 512, 512, lse, reinterpret_cast<cudaStream_t>(stream));
 }
 

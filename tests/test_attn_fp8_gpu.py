@@ -517,3 +517,17 @@ def test_bf16_queries_give_the_same_bits_however_they_are_quantised(tokens, head
     out, lse = api.masked_mla_fp8(qd, kvd, u, m, synth.SM_SCALE, counts=c, kv_scale=ks, q_scale=qs)
     assert torch.equal(out, want_o) and torch.equal(lse, want_l)
     assert api.attn_status()[0] == 0
+
+
+def test_scales_that_are_no_powers_of_two_are_rounded_once():
+    # the product of the scales reaches the kernel as one fp32 number, in the one-call form as in the chain
+    tokens, heads = 64, 64
+    w, idx, kv, q = _case(tokens, heads, 512, 4096, (0.8, 0.8), seed=19)
+    q8, kv8, _, _ = synth.refcompat_operands(q, kv)
+    sm, qs, ks = 0.743, 0.0131, 0.0229          # logits of some tens, where one fp32 step shows
+    assert np.float32(np.float32(sm) * np.float32(qs)) * np.float32(ks) != np.float32(sm * qs * ks)
+    q8, kvd, idd = q8.view(tokens, heads, 576).to(DEV), kv8.to(DEV), idx.to(DEV)
+    u, m, c = api.union_qm(idd, w.group, seq_space=w.s_kv, return_counts=True)
+    want_o, want_l = api.masked_mla_fp8(q8, kvd, u, m, sm, counts=c, kv_scale=ks, q_scale=qs)
+    out, lse = api.sparse_prefill(q8, kvd, idd, sm, kv_scale=ks, q_scale=qs)
+    assert torch.equal(out, want_o) and torch.equal(lse, want_l)
