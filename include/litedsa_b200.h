@@ -52,9 +52,7 @@ const char* litedsa_error_string(int code);
  * G*cap/32 <= 16384, 0 < seq_space <= 2^20 and a multiple of 1024.  Additionally
  * k % 4 == 0.
  * fill_tail == 0: words beyond the live prefixes are left untouched (the reference's
- * overwrite contract, litedsa_union.cuh:22-25); 2: u_phys := -1 from the live prefix to the next
- * multiple of 128 entries (what the attention reads); any other value: u_phys tail := -1, mask
- * tail := 0.
+ * overwrite contract, litedsa_union.cuh:22-25); != 0: u_phys tail := -1, mask tail := 0.
  */
 int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts,
                      uint32_t* memb_qm, const int32_t* req_pg, const int32_t* block_table,

@@ -159,8 +159,8 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   int32_t* counts = reinterpret_cast<int32_t*>(ws + l.counts);
   int32_t* u = reinterpret_cast<int32_t*>(ws + l.u);
   uint32_t* memb = reinterpret_cast<uint32_t*>(ws + l.memb);
-  // fill mode 2: lists padded to whole 128-key blocks, nothing written beyond
-  rc = litedsa_union_qm(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
+  // fill 2: lists padded to whole 128-key blocks, nothing written beyond
+  rc = run_union(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
   if (rc != LITEDSA_OK) return rc;
   if (kv_is_bf16 && ns > 1) {
     float* part_o = reinterpret_cast<float*>(ws + l.part_o);

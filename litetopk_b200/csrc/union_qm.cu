@@ -236,17 +236,10 @@ static int launch_union(const UnionParams& p, int rank_shift, int ng, size_t sme
   return rank_shift ? launch_union_rs<NT, VPT, 2>(p, ng, smem, stream) : launch_union_rs<NT, VPT, 0>(p, ng, smem, stream);
 }
 
-}  // namespace lt
-
-// C-ABI entry point; argument order and meaning follow the reference operator
-// union_qm(topk_indices, u_phys, counts, memb_qm, req_pg, block_table, block_size, seq_space)
-// (kernels/b200/dsa/litedsa.cu:31-75), with tensor shapes passed as integers.
-extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts,
-                                uint32_t* memb_qm, const int32_t* req_pg,
-                                const int32_t* block_table, int T, int k, int ng, int cap, int G,
-                                int bt_rows, int bt_blocks, int block_size, int64_t seq_space,
-                                int fill_tail, void* stream) {
-  using namespace lt;
+// Checks and launch behind litedsa_union_qm and litedsa_sparse_prefill; fill as UnionParams::fill_tail.
+int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uint32_t* memb_qm, const int32_t* req_pg,
+              const int32_t* block_table, int T, int k, int ng, int cap, int G, int bt_rows, int bt_blocks,
+              int block_size, int64_t seq_space, int fill, void* stream) {
   // same argument checks as the reference launcher (litedsa.cu:43-59)
   if (!topk_indices || !u_phys || !counts || !memb_qm) return LITEDSA_ERR_ARG;
   if (ng <= 0 || G <= 0 || k <= 0 || T != ng * G) return LITEDSA_ERR_SHAPE;
@@ -266,7 +259,7 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
   p.bt_stride = bt_blocks; p.bt_blocks = bt_blocks; p.bsz = block_table ? block_size : 1;
   p.bsz_mul = fast_div_mul(int64_t(s_words) * 32, p.bsz);
   p.kq = k / 4; p.kq_mul = fast_div_mul(int64_t(G) * (k / 4), k / 4);
-  p.k = k; p.G = G; p.cap = cap; p.s_words = s_words; p.fill_tail = fill_tail == 2 ? 2 : (fill_tail ? 1 : 0);
+  p.k = k; p.G = G; p.cap = cap; p.s_words = s_words; p.fill_tail = fill;
   // Shared memory (227 KB per CTA on sm_100): the whole list is staged if two CTAs fit on an SM then,
   // else its first 8192 entries (a union is usually well below G * k); one rank per bitmap word if
   // that fits, else one per quad.
@@ -302,4 +295,18 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
   }
   if (vpt <= 8) return launch_union<512, 8>(p, rank_shift, ng, smem, st);
   return launch_union<512, 0>(p, rank_shift, ng, smem, st);
+}
+
+}  // namespace lt
+
+// C-ABI entry point; argument order and meaning follow the reference operator
+// union_qm(topk_indices, u_phys, counts, memb_qm, req_pg, block_table, block_size, seq_space)
+// (kernels/b200/dsa/litedsa.cu:31-75), with tensor shapes passed as integers.
+extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts,
+                                uint32_t* memb_qm, const int32_t* req_pg,
+                                const int32_t* block_table, int T, int k, int ng, int cap, int G,
+                                int bt_rows, int bt_blocks, int block_size, int64_t seq_space,
+                                int fill_tail, void* stream) {
+  return lt::run_union(topk_indices, u_phys, counts, memb_qm, req_pg, block_table, T, k, ng, cap, G, bt_rows, bt_blocks,
+                       block_size, seq_space, fill_tail != 0 ? 1 : 0, stream);
 }

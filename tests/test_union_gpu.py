@@ -143,3 +143,20 @@ def test_union_plans(ng, G, k, space):
             live = int(want[1][0])
             beyond = got[0][t, (live + 3) // 4 * 4:]         # the quad that is cut is padded in any case
             assert (beyond == (-1 if fill else -7)).all() and (got[0][t, live:(live + 3) // 4 * 4] == -1).all()
+
+
+@pytest.mark.parametrize("fill", [1, 2, -1])
+def test_union_any_nonzero_fill_tail_fills_whole_rows(fill):
+    # the C entry's flag is a truth value
+    from litetopk_b200 import _lib
+    ng, G, k = 2, 2, 512
+    cap = G * k
+    idx = (torch.arange(ng * G * k, dtype=torch.int32, device=DEV).reshape(ng * G, k) * 3 % 200).contiguous()
+    u = torch.full((ng, cap), -7, dtype=torch.int32, device=DEV)
+    m = torch.full((ng, G, cap // 32), -7, dtype=torch.int32, device=DEV)
+    c = torch.empty((ng,), dtype=torch.int32, device=DEV)
+    rc = _lib.lib().litedsa_union_qm(idx.data_ptr(), u.data_ptr(), c.data_ptr(), m.data_ptr(), None, None, ng * G, k, ng,
+                                     cap, G, 0, 0, 1, 1024, fill, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and c.tolist() == [200, 200]
+    assert bool((u[:, 200:] == -1).all()) and bool((m[:, :, 7:] == 0).all())
