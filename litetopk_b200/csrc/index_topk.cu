@@ -546,9 +546,9 @@ __device__ __forceinline__ void block_fmax_fmin(float* red_a, float* red_b, floa
 // most kSurvCap entries.  Steps: exact selection among the survivors (value-linear histogram,
 // threshold bin, its keys ranked by counting), then every survivor >= the k-th value is written
 // out (thread i owns a contiguous run of survivor slots; one block-wide exclusive scan).  When
-// the fast path does not apply -- or stops applying: NaN / infinite values, a single value,
-// more threshold-bin keys or tied values than threads -- the row is finished exactly from memory:
-// bitwise radix select (unless the k-th value is already known) and ordered emission.  One such row
+// the fast path does not apply -- or stops applying: infinite values, a single value, more
+// threshold-bin keys than threads (ties share a bin) -- the row is finished exactly from memory:
+// bitwise radix select and ordered emission.  One such row
 // costs about 30 us, and of 4096 rows of 30K logits one has a tie to be cut: cut among the survivors
 // (260 -> 229 us on such data).
 template <int NT, class PosT>
@@ -557,7 +557,6 @@ __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* r
                                            const float* row, int n, int k, int32_t* out) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   uint32_t kth = 0, ties = 0, tie_end = 0xffffffffu;      // tie_end: last position selected among the tied
-  bool have_kth = false;
   if (fast) {
     float vmax = -INFINITY, vmin = INFINITY, chk = 0.f;
     for (uint32_t i = tid; i < m_s; i += NT) {
@@ -600,31 +599,23 @@ __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* r
         }
         __syncthreads();
         kth = sh.kth; ties = sh.ties;
-        have_kth = true;
         if (ties != *eq_total) {                  // the tie at the k-th value must be cut by position
           const float kv = okey_inv(kth);
           __syncthreads();
           if (tid == 0) sh.n_cand = 0;
           __syncthreads();
           for (uint32_t i = tid; i < m_s; i += NT)
-            if (sval[i] == kv) {
-              const uint32_t c = atomicAdd(&sh.n_cand, 1u);
-              if (c < (uint32_t)NT) sh.cand[c] = spos[i];
-            }
+            if (sval[i] == kv) sh.cand[atomicAdd(&sh.n_cand, 1u)] = spos[i];
           __syncthreads();
-          const uint32_t me = sh.n_cand;
-          if (me <= (uint32_t)NT) {
-            if (tid < (int)me) {
-              const uint32_t mine = sh.cand[tid];
-              uint32_t r = 0;
-              for (uint32_t j = 0; j < me; ++j) r += sh.cand[j] < mine;
-              if (r + 1 == ties) sh.kth = mine;
-            }
-            __syncthreads();
-            tie_end = sh.kth;
-          } else {
-            fast = false;
+          const uint32_t me = sh.n_cand;          // equal values share the threshold bin: at most its m keys
+          if (tid < (int)me) {
+            const uint32_t mine = sh.cand[tid];
+            uint32_t r = 0;
+            for (uint32_t j = 0; j < me; ++j) r += sh.cand[j] < mine;
+            if (r + 1 == ties) sh.kth = mine;
           }
+          __syncthreads();
+          tie_end = sh.kth;
         }
       } else {
         fast = false;
@@ -666,16 +657,14 @@ __device__ __forceinline__ void finish_row(SelShared& sh, float* red_a, float* r
     else emit([&](uint32_t i) { return sval[i] > kv || (sval[i] == kv && (uint32_t)spos[i] <= tie_end); });
   } else {
     auto key_mem = [&](int i) -> uint32_t { return okey(__ldcg(row + i)); };
-    if (!have_kth) {
-      uint32_t kmax = 0u, kmin = 0xffffffffu;
-      for (int i = tid; i < n; i += NT) {
-        const uint32_t u = key_mem(i);
-        kmax = max(kmax, u);
-        kmin = min(kmin, u);
-      }
-      block_max_min<NT>(sh, kmax, kmin);
-      kth = radix_kth<NT>(sh, key_mem, n, kmax, kmin, (uint32_t)k, &ties);
+    uint32_t kmax = 0u, kmin = 0xffffffffu;
+    for (int i = tid; i < n; i += NT) {
+      const uint32_t u = key_mem(i);
+      kmax = max(kmax, u);
+      kmin = min(kmin, u);
     }
+    block_max_min<NT>(sh, kmax, kmin);
+    kth = radix_kth<NT>(sh, key_mem, n, kmax, kmin, (uint32_t)k, &ties);
     emit_ordered<NT>(sh, key_mem, n, kth, ties, out, k);
   }
 }
@@ -724,8 +713,8 @@ __device__ __forceinline__ float sampled_threshold(SelShared& sh, float* red_a, 
 //      exactly by counting;
 //   5. survivors >= the k-th value are written out (block-wide scan of per-thread counts).
 // The output order is fixed but not ascending.  Whatever the fast path does not cover -- too
-// few or too many survivors, NaN or infinite values, a single value, more threshold-bin keys
-// or values tied at the k-th than threads -- is finished by the
+// few or too many survivors, infinite values, a single value, more threshold-bin keys than
+// threads -- is finished by the
 // exact bitwise radix select and the ordered emission over the row re-read from memory.
 constexpr int kStreamThreads = 512;
 enum { kSiteSelRow = 11 };
