@@ -136,8 +136,10 @@ int litedsa_masked_mla_fp8_bf16q(const void* q_bf16, float q_scale, const void* 
  *   sm_scale softmax scale on the unquantised values;  out [T, h, 512] bf16, lse [T, h] fp32
  *   seq_space bound on the positions (multiple of 1024, <= 2^20)
  *   policy_tokens >= T: tokens of the whole job.  Small jobs cut their tiles' lists into slices that
- *            run in parallel and are merged in fp32; how many depends on this number only, so that
- *            a job done in several calls gives the bits of the job done in one
+ *            run in parallel and are merged in fp32 (a slice rounds its softmax weights relative to its
+ *            own running max, so a sliced tile can differ from the whole one by that rounding); how many
+ *            depends on this number only, so that a job done in several calls gives the bits of the
+ *            job done in one
  *   workspace  256-byte aligned, litedsa_sparse_prefill_workspace(...) bytes
  */
 int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,

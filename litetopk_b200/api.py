@@ -777,15 +777,26 @@ def masked_mla_fp8(q: torch.Tensor, kv_cache_fp8: torch.Tensor, union_idx: torch
 def sparse_prefill(q: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_idx: torch.Tensor,
                    sm_scale: float, *, kv_scale: Optional[float] = None,
                    q_scale: Optional[float] = None, seq_space: Optional[int] = None,
-                   out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None):
+                   out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None,
+                   job_tokens: Optional[int] = None):
     """The whole hot path for one chunk of query tokens: union_qm + masked attention.
 
     q [T,h,576], topk_idx [T,k] int32, kv_cache_fp8 as in :func:`masked_mla_fp8` (already
     resident on the device; pass the result of :func:`prepare_kv` when the same cache serves
     several calls).  Returns ``(out [T,h,512] bf16, lse [T,h] f32)``, written into ``out`` /
     ``lse`` when given.
+
+    A call of few tokens cuts its tiles' lists into slices that run in parallel and are merged in
+    fp32.  A slice rounds its softmax weights relative to its own running maximum, so the result of
+    a few tokens alone and inside a larger call can differ by that rounding (e4m3 or bf16; neither is
+    closer to the exact result).  How a tile is cut depends on ``job_tokens`` alone, by default the
+    call's own number of tokens: state the tokens of the whole job when this call is a part of it, and
+    its tokens get the bits that they have in one call of the job.
     """
-    return _sparse_prefill(q, kv_cache_fp8, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse, q.shape[0])
+    if job_tokens is not None and int(job_tokens) < q.shape[0]:
+        raise ValueError("job_tokens must be at least the call's number of tokens")
+    return _sparse_prefill(q, kv_cache_fp8, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse,
+                           q.shape[0] if job_tokens is None else int(job_tokens))
 
 
 def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse, job_tokens):
@@ -979,6 +990,10 @@ def dsv4_c128a_bf16(q: torch.Tensor, kv_compressed: Optional[torch.Tensor], kv_r
     the first ``heads`` head slots per token are real; it is read in place (any strides with unit
     inner stride), and the result is written in place into ``out`` ``[T, H_padded, 512]`` when
     given (else a dense ``[T, heads, 512]`` is returned).  lse is ``[T, heads]``.
+
+    A call of few tokens with long key ranges cuts them into slices that run in parallel and are merged in
+    fp32; a slice rounds its softmax weights to bf16 relative to its own running maximum, so the result of a
+    few tokens alone and inside a larger call can differ by that rounding.
     """
     _need(q, "q", torch.bfloat16, 3)
     _need(kv_raw, "kv_raw", torch.bfloat16, 2)

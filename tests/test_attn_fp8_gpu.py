@@ -531,3 +531,18 @@ def test_scales_that_are_no_powers_of_two_are_rounded_once():
     want_o, want_l = api.masked_mla_fp8(q8, kvd, u, m, sm, counts=c, kv_scale=ks, q_scale=qs)
     out, lse = api.sparse_prefill(q8, kvd, idd, sm, kv_scale=ks, q_scale=qs)
     assert torch.equal(out, want_o) and torch.equal(lse, want_l)
+
+
+def test_a_part_of_a_job_gives_the_bits_of_the_job():
+    # four tokens alone would run in slices; as a part of a job of 80 they do not
+    tokens, part = 80, 4
+    w, idx, kv, q = _case(tokens, 64, 2048, 16384, (0.6, 0.8), seed=20)
+    q8, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    qd, kvd, idd = q.to(DEV), kv8.to(DEV), idx.to(DEV)
+    want_o, want_l = api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    for t0 in (0, 40, tokens - part):
+        out, lse = api.sparse_prefill(qd[t0:t0 + part], kvd, idd[t0:t0 + part], synth.SM_SCALE, kv_scale=ks, q_scale=qs,
+                                      job_tokens=tokens)
+        assert torch.equal(out, want_o[t0:t0 + part]) and torch.equal(lse, want_l[t0:t0 + part])
+    with pytest.raises(ValueError, match="job_tokens"):
+        api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs, job_tokens=tokens - 2)
