@@ -506,8 +506,8 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, float (&v)[16
       : "r"(taddr)
       : "memory");
 }
-// 32 lanes x 32 consecutive fp32 columns: thread i of the warp gets lane (base_lane + i)
-// the same, issued by one elected lane of a fully converged warp (keeps the caller warp-uniform)
+// commit of the pair's earlier MMAs to one barrier, issued by one elected lane of a fully converged warp
+// (keeps the caller warp-uniform)
 __device__ __forceinline__ void mma_commit_pair_elect(uint32_t cluster_addr) {
   asm volatile(
       "{\n\t.reg .pred pe;\n\telect.sync _|pe, 0xffffffff;\n\t"
@@ -515,6 +515,7 @@ __device__ __forceinline__ void mma_commit_pair_elect(uint32_t cluster_addr) {
       ::"r"(cluster_addr)
       : "memory");
 }
+// 32 lanes x 32 consecutive fp32 columns: thread i of the warp gets lane (base_lane + i)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
   asm volatile(
@@ -553,7 +554,7 @@ __device__ __forceinline__ void tmem_wait_st() {
 // Shared-memory matrix descriptor (sm_100 format, version field = 1):
 //   [0,14) start address >> 4, [16,30) leading byte offset >> 4, [32,46) stride byte offset >> 4,
 //   [46,48) = 1, [61,64) swizzle: 0 none, 2 = 128 B, 4 = 64 B, 6 = 32 B.
-enum : uint32_t { kSwzNone = 0, kSwz128 = 2, kSwz64 = 4, kSwz32 = 6 };
+enum : uint32_t { kSwzNone = 0, kSwz128 = 2, kSwz64 = 4 };
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo_bytes,
                                               uint32_t sbo_bytes, uint32_t swizzle) {
   uint64_t d = 0;

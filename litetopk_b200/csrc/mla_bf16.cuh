@@ -13,7 +13,9 @@
 //   kGather  an index list per tile (rank ranges or membership bits), 16-byte cp.async row gather.
 //
 // Organisation: persistent clusters of 2 CTAs (64 query rows each), tcgen05 cta_group::2 kind::f16
-// MMAs, 64-key blocks (the reference's, so the running max takes the same course).  One block's
+// MMAs, 64-key blocks.  With kGather they are the reference's, so the running max takes the same course;
+// kRange and kRank lay each of the two segments out in half blocks of 32 keys, so a block holds other
+// keys and P can be rounded relative to another running max.  One block's
 // chain of loads, QK^T, softmax and PV takes about 5000 cycles, its 44 MMAs about 1250, so four blocks
 // or more have to be in flight.  To make room for them:
 //   * a block's K tile BECOMES its V tile (as in the FP8 kernel, attn_fp8.cu): CTA c loads the rows of
