@@ -150,6 +150,20 @@ int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_
 int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens);
 
 /*
+ * litedsa_sparse_prefill with the rows of a tile chosen by the size of the job: jobs of many tokens of up to
+ * 64 heads with an FP8 cache unite the lists of 64 query rows instead of 128 and run
+ * in blocks of 64 keys, which is faster (shorter unions).  Softmax weights are then rounded to e4m3 relative
+ * to other running maxima than litedsa_sparse_prefill's (no further from the exact result).  Other jobs give
+ * litedsa_sparse_prefill's bits, and as there a job done in several calls gives the bits of the job done in one.
+ */
+int litedsa_sparse_prefill_job(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
+                               const int32_t* topk_idx, double sm_scale, double q_scale, double kv_scale,
+                               void* out, float* lse, int T, int h, int k, int s_kv, int64_t kv_row_stride,
+                               int64_t seq_space, int job_tokens, void* workspace,
+                               int64_t workspace_bytes, void* stream);
+int64_t litedsa_sparse_prefill_job_workspace(int T, int h, int k, int kv_is_bf16, int job_tokens);
+
+/*
  * litedsa_masked_mla_fp8 with the all-gather of a query-sharded multi-GPU run folded into
  * the kernel's epilogue.  Every output box is written to n_outs (1..8) destinations with
  * TMA tile stores: outs[0] is this GPU's [ng, 128, 512] bf16 buffer, outs[1..] are

@@ -40,6 +40,10 @@ SIGNATURES = {
                                        c_double, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64,
                                        c_int64, c_int, c_void_p, c_int64, c_void_p]),
     "litedsa_sparse_prefill_workspace": (c_int64, [c_int, c_int, c_int, c_int, c_int]),
+    "litedsa_sparse_prefill_job": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_double, c_double,
+                                           c_double, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64,
+                                           c_int64, c_int, c_void_p, c_int64, c_void_p]),
+    "litedsa_sparse_prefill_job_workspace": (c_int64, [c_int, c_int, c_int, c_int, c_int]),
     "litedsa_attn_status": (c_int, [c_void_p, c_int]),
     "litedsa_set_wait_limit_ns": (c_int, [c_uint64, c_void_p]),
     "litedsa_selftest_wait_timeout": (c_int, [c_uint64, c_void_p]),

@@ -787,21 +787,23 @@ def sparse_prefill(q: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_idx: torch.
     ``lse`` when given.
 
     A call of few tokens cuts its tiles' lists into slices that run in parallel and are merged in
-    fp32.  A slice rounds its softmax weights relative to its own running maximum, so the result of
-    a few tokens alone and inside a larger call can differ by that rounding (e4m3 or bf16; neither is
-    closer to the exact result).  How a tile is cut depends on ``job_tokens`` alone, by default the
-    call's own number of tokens: state the tokens of the whole job when this call is a part of it, and
-    its tokens get the bits that they have in one call of the job.
+    fp32; one of many tokens with an FP8 cache and up to 64 heads unites the lists of 64 query rows
+    instead of 128.  Either way softmax weights are rounded relative to another running maximum, so the
+    result of some tokens alone and inside a larger call can differ by that rounding (e4m3 or bf16; none
+    is closer to the exact result).  What a tile is and how it is cut depends on ``job_tokens`` alone, by
+    default the call's own number of tokens: state the tokens of the whole job when this call is a part of
+    it, and its tokens get the bits that they have in one call of the job.
     """
     if job_tokens is not None and int(job_tokens) < q.shape[0]:
         raise ValueError("job_tokens must be at least the call's number of tokens")
     return _sparse_prefill(q, kv_cache_fp8, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse,
-                           q.shape[0] if job_tokens is None else int(job_tokens))
+                           q.shape[0] if job_tokens is None else int(job_tokens), True)
 
 
-def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse, job_tokens):
+def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse, job_tokens, by_job=False):
     """:func:`sparse_prefill` of a chunk of a job of ``job_tokens`` tokens (the library picks how a
-    small job is cut into slices from that number, so a chunk's bits do not depend on the chunking)."""
+    small job is cut into slices from that number and, ``by_job``, whether a tile has 64 rows instead of
+    128, so a chunk's bits do not depend on the chunking)."""
     _need(q, "q", (torch.bfloat16, torch.uint8, torch.float8_e4m3fn), 3)
     _need(topk_idx, "topk_idx", torch.int32, 2)
     T, h, d = q.shape
@@ -842,12 +844,12 @@ def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_spac
         lse = lse.view(T, h)
     lib = _lib.lib()
     space = kv_cache.shape[0] if seq_space is None else int(seq_space)
-    ws = torch.empty((max(lib.litedsa_sparse_prefill_workspace(T, h, k, kv_bf16, job_tokens), 1),),
-                     dtype=torch.uint8, device=dev)
-    check(_on_device(dev, lib.litedsa_sparse_prefill, q.data_ptr(), q_bf16, kv.data_ptr(), kv_bf16,
-                     topk_idx.data_ptr(), float(sm_scale), float(q_scale), float(kv_scale), out.data_ptr(), lse.data_ptr(), T, h, k,
-                     kv.shape[0], kv.stride(0), (space + 1023) // 1024 * 1024, job_tokens, ws.data_ptr(),
-                     ws.numel()), "sparse_prefill")
+    fn, size = (lib.litedsa_sparse_prefill_job, lib.litedsa_sparse_prefill_job_workspace) if by_job else \
+        (lib.litedsa_sparse_prefill, lib.litedsa_sparse_prefill_workspace)
+    ws = torch.empty((max(size(T, h, k, kv_bf16, job_tokens), 1),), dtype=torch.uint8, device=dev)
+    check(_on_device(dev, fn, q.data_ptr(), q_bf16, kv.data_ptr(), kv_bf16, topk_idx.data_ptr(), float(sm_scale),
+                     float(q_scale), float(kv_scale), out.data_ptr(), lse.data_ptr(), T, h, k, kv.shape[0], kv.stride(0),
+                     (space + 1023) // 1024 * 1024, job_tokens, ws.data_ptr(), ws.numel()), "sparse_prefill")
     return out, lse
 
 
@@ -961,7 +963,7 @@ def sparse_prefill_host(q_host: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_h
                 ev_in.record(s_in)
             cur.wait_event(ev_in)
             _sparse_prefill(qd[t0:t1], kv, idd[t0:t1], sm_scale, kv_scale, q_scale, space, od[t0:t1],
-                            ld[t0:t1], T)
+                            ld[t0:t1], T, True)
             ev_c = torch.cuda.Event()
             ev_c.record(cur)
             s_out.wait_event(ev_c)

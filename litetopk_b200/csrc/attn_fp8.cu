@@ -1089,6 +1089,8 @@ int run_fp8(const Fp8Args& a, void* const* outs, int n_outs, void* stream) {
 
 }  // namespace lt
 
+#include "attn_fp8_r64.cuh"
+
 // Masked FP8 MLA prefill; replaces the reference operator
 //   masked_mla_fp8(q, kv, indices, sm_scale, out_scale, topk_length, memb_qm, h_per_q,
 //                  out, max_logits, lse)            (kernels/b200/dsa/litedsa.cu:77-135)

@@ -116,6 +116,19 @@ static int check_shape(int T, int h, int k, int policy_tokens) {
   return LITEDSA_OK;
 }
 
+// Whether a job of `tokens` tokens runs on 64-row tiles (attn_fp8_r64.cuh) instead of 128-row ones: with an FP8
+// cache, up to 64 heads, lists of a tile of 256 entries and more, a tile for every other SM and at least ten key
+// blocks per SM.  (Fewer tiles run faster as slices of 128-row ones: 40 tiles of 16 heads, top-2048, 60 us
+// against 65; with less work both forms take the 23 us of a call's launches.)  128-row / 64-row tiles, e4m3 queries, half and nine tenths of the lists shared, us: 74 tiles x 64 heads, top-2048 39 / 30 and
+// 35 / 29; 16 heads, top-2048 71 / 59 and 45 / 39; 222 x 32 heads, top-2048 104 / 76
+// and 63 / 65; 1184 tiles x 64 heads, top-256 59 / 51 and 84 / 51, top-2048 276 / 199 and 233 / 202; 32 heads
+// 430 / 295 and 263 / 246; 16 heads 770 / 456 and 376 / 296; 8 heads 1403 / 806 and 572 / 429.
+static bool use_rows64(int tokens, int h, int k, bool kv_bf16) {
+  if (kv_bf16 || h > 64 || (int64_t)(128 / h) * k % 128 != 0) return false;
+  const int64_t tiles = (int64_t)tokens * h / 64, list = (int64_t)(64 / h) * k;
+  return list >= 256 && tiles >= sm_count() / 2 && tiles * list >= (int64_t)10 * 64 * sm_count();
+}
+
 }  // namespace prefill
 
 int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
@@ -127,23 +140,31 @@ int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng,
 }
 }  // namespace lt
 
-// Bytes of workspace litedsa_sparse_prefill needs (0: the shape is not supported).
-extern "C" int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens) {
-  using namespace lt::prefill;
-  if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
-  const int G = 128 / h, cap = G * k;
-  const int ns = pick_slices(policy_tokens / G, G, k, kv_is_bf16 != 0);
-  return layout_of(T / G, G, cap, ns).total;
+namespace lt {
+namespace prefill {
+
+// rows of a tile and length of its list; the slices of a tile
+struct Route { int ng, G, cap, ns; bool rows64; };
+static Route route_of(int T, int h, int k, bool kv_bf16, int policy_tokens, bool by_job) {
+  Route r;
+  r.rows64 = by_job && use_rows64(policy_tokens, h, k, kv_bf16);
+  r.G = (r.rows64 ? 64 : 128) / h;
+  r.ng = T / r.G;
+  r.cap = r.rows64 ? (r.G * k + 127) / 128 * 128 : r.G * k;
+  r.ns = r.rows64 ? 1 : pick_slices(policy_tokens / r.G, r.G, k, kv_bf16);
+  return r;
 }
 
-// union_qm + masked attention of T query tokens in one call; see include/litedsa_b200.h.
-extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
-                                      const int32_t* topk_idx, double sm_scale, double q_scale, double kv_scale,
-                                      void* out, float* lse, int T, int h, int k, int s_kv,
-                                      int64_t kv_row_stride, int64_t seq_space, int policy_tokens,
-                                      void* workspace, int64_t workspace_bytes, void* stream) {
-  using namespace lt;
-  using namespace lt::prefill;
+static int64_t workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens, bool by_job) {
+  if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
+  const Route r = route_of(T, h, k, kv_is_bf16 != 0, policy_tokens, by_job);
+  return layout_of(r.ng, r.G, r.cap, r.ns).total;
+}
+
+static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, const int32_t* topk_idx, double sm_scale,
+               double q_scale, double kv_scale, void* out, float* lse, int T, int h, int k, int s_kv,
+               int64_t kv_row_stride, int64_t seq_space, int policy_tokens, bool by_job, void* workspace,
+               int64_t workspace_bytes, void* stream) {
   if (!q || !kv || !topk_idx || !out || !lse || !workspace) return LITEDSA_ERR_ARG;
   int rc = check_shape(T, h, k, policy_tokens);
   if (rc != LITEDSA_OK) return rc;
@@ -151,8 +172,8 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   if (!kv_is_bf16 && q_is_bf16 && !((float)q_scale > 0.f)) return LITEDSA_ERR_SHAPE;
   if (((uintptr_t)workspace & 255) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) || ((uintptr_t)topk_idx & 15))
     return LITEDSA_ERR_UNSUPPORTED;
-  const int G = 128 / h, ng = T / G, cap = G * k;
-  const int ns = pick_slices(policy_tokens / G, G, k, kv_is_bf16 != 0);
+  const Route r = route_of(T, h, k, kv_is_bf16 != 0, policy_tokens, by_job);
+  const int G = r.G, ng = r.ng, cap = r.cap, ns = r.ns;
   const Layout l = layout_of(ng, G, cap, ns);
   if (workspace_bytes < l.total) return LITEDSA_ERR_SHAPE;
   char* ws = reinterpret_cast<char*>(workspace);
@@ -178,6 +199,7 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
             ng, s_kv, cap, 576, kv_row_stride, cap, nullptr, nullptr, 1};
   a.q_is_bf16 = q_is_bf16 != 0;
   a.q_inv = 1.0f / (float)q_scale;
+  if (r.rows64) return run_fp8_rows64(a, out, stream);
   a.nsplit = ns;
   a.part_o = reinterpret_cast<float*>(ws + l.part_o);
   a.part_ml = ws + l.part_ml;
@@ -186,6 +208,37 @@ extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* 
   if (rc != LITEDSA_OK || ns == 1) return rc;
   return merge_slices(a.part_o, reinterpret_cast<const float2*>(a.part_ml), ns, ng, h, a.out_scale, kFp8LseOffset,
                       nullptr, 1, out, (int64_t)h * 512, 512, lse, reinterpret_cast<cudaStream_t>(stream));
+}
+
+}  // namespace prefill
+}  // namespace lt
+
+// Bytes of workspace litedsa_sparse_prefill needs (0: the shape is not supported).
+extern "C" int64_t litedsa_sparse_prefill_workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens) {
+  return lt::prefill::workspace(T, h, k, kv_is_bf16, policy_tokens, false);
+}
+extern "C" int64_t litedsa_sparse_prefill_job_workspace(int T, int h, int k, int kv_is_bf16, int job_tokens) {
+  return lt::prefill::workspace(T, h, k, kv_is_bf16, job_tokens, true);
+}
+
+// union_qm + masked attention of T query tokens in one call; see include/litedsa_b200.h.
+extern "C" int litedsa_sparse_prefill(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
+                                      const int32_t* topk_idx, double sm_scale, double q_scale, double kv_scale,
+                                      void* out, float* lse, int T, int h, int k, int s_kv,
+                                      int64_t kv_row_stride, int64_t seq_space, int policy_tokens,
+                                      void* workspace, int64_t workspace_bytes, void* stream) {
+  return lt::prefill::run(q, q_is_bf16, kv, kv_is_bf16, topk_idx, sm_scale, q_scale, kv_scale, out, lse, T, h, k, s_kv,
+                          kv_row_stride, seq_space, policy_tokens, false, workspace, workspace_bytes, stream);
+}
+
+// The same, the rows of a tile chosen by the size of the job; see include/litedsa_b200.h.
+extern "C" int litedsa_sparse_prefill_job(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16,
+                                          const int32_t* topk_idx, double sm_scale, double q_scale, double kv_scale,
+                                          void* out, float* lse, int T, int h, int k, int s_kv, int64_t kv_row_stride,
+                                          int64_t seq_space, int job_tokens, void* workspace, int64_t workspace_bytes,
+                                          void* stream) {
+  return lt::prefill::run(q, q_is_bf16, kv, kv_is_bf16, topk_idx, sm_scale, q_scale, kv_scale, out, lse, T, h, k, s_kv,
+                          kv_row_stride, seq_space, job_tokens, true, workspace, workspace_bytes, stream);
 }
 
 // litedsa_masked_mla_fp8 on bf16 queries, quantised inside the attention kernel.

@@ -243,7 +243,7 @@ int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uin
   // same argument checks as the reference launcher (litedsa.cu:43-59)
   if (!topk_indices || !u_phys || !counts || !memb_qm) return LITEDSA_ERR_ARG;
   if (ng <= 0 || G <= 0 || k <= 0 || T != ng * G) return LITEDSA_ERR_SHAPE;
-  if (cap != G * k || cap % 128 != 0) return LITEDSA_ERR_SHAPE;
+  if (cap < G * k || cap % 128 != 0) return LITEDSA_ERR_SHAPE;
   if (G > 16 || (int64_t)G * (cap / 32) > 16 * 1024) return LITEDSA_ERR_SHAPE;
   if (seq_space <= 0 || seq_space > (1 << 20)) return LITEDSA_ERR_SHAPE;
   const int s_words = (int)((seq_space + 31) / 32);
@@ -307,6 +307,7 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
                                 const int32_t* block_table, int T, int k, int ng, int cap, int G,
                                 int bt_rows, int bt_blocks, int block_size, int64_t seq_space,
                                 int fill_tail, void* stream) {
+  if (topk_indices && u_phys && counts && memb_qm && cap != G * k) return LITEDSA_ERR_SHAPE;
   return lt::run_union(topk_indices, u_phys, counts, memb_qm, req_pg, block_table, T, k, ng, cap, G, bt_rows, bt_blocks,
                        block_size, seq_space, fill_tail != 0 ? 1 : 0, stream);
 }

@@ -546,3 +546,52 @@ def test_a_part_of_a_job_gives_the_bits_of_the_job():
         assert torch.equal(out, want_o[t0:t0 + part]) and torch.equal(lse, want_l[t0:t0 + part])
     with pytest.raises(ValueError, match="job_tokens"):
         api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs, job_tokens=tokens - 2)
+
+
+@pytest.mark.parametrize("tokens,heads,topk,s_kv", [
+    (380, 64, 256, 4096),        # one token per tile, four blocks
+    (602, 64, 960, 7777),        # a list that is no multiple of 128, ten more tiles in the last round
+    (1300, 32, 512, 5001),       # two tokens per tile
+    (2376, 16, 256, 3000),       # four
+    (4752, 8, 272, 2500),        # eight
+])
+def test_calls_of_many_tokens_on_64_row_tiles(tokens, heads, topk, s_kv):
+    g = torch.Generator().manual_seed(21)
+
+    def mutate(idx):
+        idx = idx.clone()
+        n = torch.randint(0, topk + 1, (tokens, 1), generator=g)
+        n[torch.rand((tokens, 1), generator=g) < 0.5] = topk
+        for i, m in enumerate((0, 1, 63, 64, 65, 127, 128, 129)):       # around the blocks' edges, whole tiles
+            n[16 * i:16 * i + 16] = m
+        idx[torch.arange(topk)[None] >= n] = -1
+        idx[150:160, 1::2] = idx[150:160, 0::2]                         # duplicates count once
+        return idx
+    w, idx, kv, q = _case(tokens, heads, topk, s_kv, (0.5, 0.9), seed=22, mutate=mutate)
+    q8, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    q8, kvd, idd = q8.view(tokens, heads, 576), kv8.to(DEV), idx.to(DEV)
+    api.attn_status(reset=True)
+    out, lse = api.sparse_prefill(q8.to(DEV), kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    out_b, lse_b = api.sparse_prefill(q.to(DEV), kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    torch.cuda.synchronize()
+    assert api.attn_status()[0] == 0
+    assert torch.equal(out, out_b) and torch.equal(lse, lse_b)          # bf16 queries are quantised to the same codes
+    # the 128-row form: the same keys for every row, other roundings of P (the bounds of the slices' test above)
+    want_o, want_l = api._sparse_prefill(q8.to(DEV), kvd, idd, synth.SM_SCALE, ks, qs, None, None, None, tokens)
+    fin = torch.isfinite(want_l)
+    assert torch.equal(torch.isfinite(lse), fin) and bool((out[~fin] == 0).all())
+    assert float((lse[fin] - want_l[fin]).abs().max()) <= TOL_LSE
+    mad, cos = ao.compare(out.cpu(), want_o.cpu())
+    assert cos >= 0.9995 and mad <= 0.1 * max(1.0, float(want_o.float().abs().max())), (mad, cos)
+    part = slice(tokens // 2, tokens // 2 + 128 // heads)               # a part of the job has the job's bits
+    out_p, lse_p = api.sparse_prefill(q8[part].to(DEV), kvd, idd[part], synth.SM_SCALE, kv_scale=ks, q_scale=qs, job_tokens=tokens)
+    assert torch.equal(out_p, out[part]) and torch.equal(lse_p, lse[part])
+    some = [t for t in [*range(16, min(170, tokens), 3), *range(170, tokens, tokens // 30)] if bool((idx[t] >= 0).any())]
+    kvf = kv8.view(torch.float8_e4m3fn).float() * ks
+    uniq = torch.full((len(some), topk), -1, dtype=torch.int32)
+    for i, t in enumerate(some):
+        u = idx[t][idx[t] >= 0].unique()
+        uniq[i, :len(u)] = u
+    out_e, lse_e = ao.mla_exact(q8[some].view(torch.float8_e4m3fn).float() * qs, kvf, uniq, synth.SM_SCALE)
+    mad, cos = ao.compare(out[some].cpu(), out_e)
+    assert cos >= 0.9995 and float((lse[some].cpu() - lse_e.float()).abs().max()) <= TOL_LSE, (mad, cos)
