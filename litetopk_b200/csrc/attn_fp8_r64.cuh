@@ -56,7 +56,8 @@ struct Misc {
   uint64_t s_free[kGroups], valid_ready[kGroups], valid_free[kGroups];
   uint64_t m_pub[kGroups];          // running max after the group's latest block published
   uint64_t pair_max;                // row maxima of an item's second block published
-  uint64_t q_land;                  // the item's Q tile has landed in its slot (e4m3 q); its slot is free to fill (bf16 q)
+  uint64_t q_codes;                 // bf16 q: the item's codes are in q_codes
+  uint64_t q_land;                  // the item's Q tile has landed in its slot
   uint64_t q_taken;                 // the item's Q has been moved out of its slot
   uint64_t qt_ready;                // Q's latent dims are in tensor memory
   uint64_t q_free;                  // all QK^T of the current item are complete
@@ -82,7 +83,10 @@ struct Params {
   float scale_log2, out_scale;
   int epoch;
   unsigned long long wait_limit_ns;
-  const uint4* q_bf16;       // bf16 queries, quantised on their way in; null: e4m3 through map_q / map_q_rope
+  // bf16 queries, quantised by the epilogue warps an item ahead into q_codes [2][CTAs][64, 576] (map_q and
+  // map_q_rope are of that then); null: e4m3
+  const uint4* q_bf16;
+  uint8_t* q_codes;
   float q_inv;
 };
 
@@ -154,6 +158,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return v;
 }
 
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_rope,
                           const __grid_constant__ CUtensorMap map_out, const Params p) {
@@ -185,6 +195,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       mbar_init(&ms.m_pub[i], kGroupWarps);
     }
     mbar_init(&ms.pair_max, kGroupWarps);
+    mbar_init(&ms.q_codes, 1);
     mbar_init(&ms.q_land, kGatherWarps);
     mbar_init(&ms.q_taken, 1);
     mbar_init(&ms.qt_ready, kEpiWarps);
@@ -193,10 +204,8 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     mbar_init(&ms.fin_ready, kGroups * kGroupWarps);
     mbar_init(&ms.fin_free, kEpiWarps);
     fence_mbar_init();
-    if (p.q_bf16 == nullptr) {
-      tma_prefetch_desc(&map_q);
-      tma_prefetch_desc(&map_q_rope);
-    }
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_q_rope);
     tma_prefetch_desc(&map_out);
   }
   if (warp == kWarpQk) {
@@ -396,18 +405,20 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       // and a Q counts as landed only when all of them have -- those of its set also through its slot's
       // barrier --, so that none is overtaken and tests a phase that is two ahead.
       if (it > 0) mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
+      if (p.q_bf16 != nullptr && tile < ng) mbar_wait(&ms.q_codes, it & 1, wt, kSiteQ, it);
       const bool q_mine = (e & 1) == set;
       if (q_mine && ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
       __syncwarp();
       if (lane == 0) {
-        if (!q_mine || pw != 0 || p.q_bf16 != nullptr || tile >= ng) {
+        if (!q_mine || pw != 0 || tile >= ng) {
           mbar_arrive(&ms.q_land);
         } else {
           mbar_arrive_expect_tx(&ms.q_land, kSlot);
           const uint32_t dst = sbase + kOffKV + slot * kSlot;
+          const int z = p.q_bf16 != nullptr ? (it & 1) * ncta + cid : tile * p.G;
           for (int x = 0; x < 4; ++x)
-            tma_load_3d_hint(dst + x * kChunkBytes, &map_q, 128 * x, 0, tile * p.G, &ms.q_land, pol_stream);
-          tma_load_3d_hint(dst + kQLatent, &map_q_rope, 512, 0, tile * p.G, &ms.q_land, pol_stream);
+            tma_load_3d_hint(dst + x * kChunkBytes, &map_q, 128 * x, 0, z, &ms.q_land, pol_stream);
+          tma_load_3d_hint(dst + kQLatent, &map_q_rope, 512, 0, z, &ms.q_land, pol_stream);
         }
       }
       __syncwarp();
@@ -589,11 +600,11 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     const int e_r = e_tid & 63, e_h = e_tid >> 6;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t e_ocol = tmem + lane_base + kTmemO;
-    auto fill_q = [&](int tile, int j, int n) {
-      mbar_wait(&ms.q_land, j & 1, wt, kSiteQ, j);         // the slot is ours
-      __syncwarp();
-      const uint32_t qoff = kOffKV + (uint32_t)(n % kSlots) * kSlot, rope = qoff + kQLatent;
+    // bf16 q: item j's codes into q_codes, an item ahead.  (Straight into the Q's ring slot, which is free only when
+    // the item before it ends, the loads' latency held up each item by some 6000 cycles.)
+    auto quantise_q = [&](int tile, int j) {
       const uint4* src = p.q_bf16 + (size_t)tile * kRows * (kDQK / 8);
+      uint4* dst = reinterpret_cast<uint4*>(p.q_codes + (size_t)((j & 1) * ncta + cid) * kSlot);
 #pragma unroll 1
       for (int i = 0; i < 18; i += kFillBatch) {      // 64 rows x 36 units of 16 codes = 18 units per thread
         uint4 a[kFillBatch], b[kFillBatch];
@@ -604,30 +615,26 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
           b[u] = __ldcs(src + 2 * unit + 1);
         }
 #pragma unroll
-        for (int u = 0; u < kFillBatch; ++u) {
-          const int unit = (i + u) * 128 + e_tid, row = unit / 36, c = unit - 36 * row;
-          const uint4 v = make_uint4(e4m3x4_of_bf16(a[u].x, a[u].y, p.q_inv), e4m3x4_of_bf16(a[u].z, a[u].w, p.q_inv),
-                                     e4m3x4_of_bf16(b[u].x, b[u].y, p.q_inv), e4m3x4_of_bf16(b[u].z, b[u].w, p.q_inv));
-          const uint32_t off = c < 32 ? qoff + (c >> 3) * kChunkBytes + row * 128 + (((c & 7) ^ (row & 7)) << 4)
-                                      : rope + row * 64 + (((c - 32) ^ ((row >> 1) & 3)) << 4);
-          *reinterpret_cast<uint4*>(sm + off) = v;
-        }
+        for (int u = 0; u < kFillBatch; ++u)
+          dst[(i + u) * 128 + e_tid] =
+              make_uint4(e4m3x4_of_bf16(a[u].x, a[u].y, p.q_inv), e4m3x4_of_bf16(a[u].z, a[u].w, p.q_inv),
+                         e4m3x4_of_bf16(b[u].x, b[u].y, p.q_inv), e4m3x4_of_bf16(b[u].z, b[u].w, p.q_inv));
       }
+      __threadfence();
+      asm volatile("fence.proxy.async;" ::: "memory");      // these stores -> the TMA loads of the codes
       asm volatile("bar.sync 5, 128;" ::: "memory");
+      if (e_tid == 0) mbar_arrive(&ms.q_codes);
     };
     auto transfer_q = [&](int j, int n) {
       if (j > 0) mbar_wait(&ms.q_free, (j - 1) & 1, wt, kSiteQFree, j);
-      if (p.q_bf16 == nullptr) mbar_wait(&ms.q_land, j & 1, wt, kSiteQ, j);
+      mbar_wait(&ms.q_land, j & 1, wt, kSiteQ, j);
       __syncwarp();
       tc_fence_after();
       const uint8_t* qtile = sm + kOffKV + (n % kSlots) * kSlot;
       const uint8_t* qrow = qtile + e_r * 128;
-      {                              // rope chunk: 4 KB, 32 bytes per thread
-        const uint4* src = reinterpret_cast<const uint4*>(qtile + kQLatent) + 2 * e_tid;
-        uint4* dst = reinterpret_cast<uint4*>(sm + kOffRope) + 2 * e_tid;
-        dst[0] = src[0];
-        dst[1] = src[1];
-      }
+      // rope chunk: 4 KB, 32 bytes per thread
+      reinterpret_cast<uint4*>(sm + kOffRope)[e_tid] = reinterpret_cast<const uint4*>(qtile + kQLatent)[e_tid];
+      reinterpret_cast<uint4*>(sm + kOffRope)[e_tid + 128] = reinterpret_cast<const uint4*>(qtile + kQLatent)[e_tid + 128];
 #pragma unroll 1
       for (int j4 = 0; j4 < 4; ++j4) {
         uint32_t v[32];
@@ -643,7 +650,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       fence_proxy_async_smem();      // rope -> the MMAs' reads; these reads -> the slot's next TMA write
       __syncwarp();
       if (lane == 0) mbar_arrive(&ms.qt_ready);
-      asm volatile("bar.sync 5, 128;" ::: "memory");      // all four warps have read the slot
+      asm volatile("bar.sync 5, 128;" ::: "memory");      // all warps have read the slot
       if (e_tid == 0) mbar_arrive(&ms.q_taken);
     };
     // the slot of entry n is dead (its TMA reads included)
@@ -654,7 +661,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       if (e_tid == 0) mbar_arrive(&ms.slot_free[n % kSlots]);
     };
     int kb0 = 0, it = 0, nb_next = blocks_of(cid);
-    if (p.q_bf16 != nullptr) fill_q(cid, 0, 0);
+    if (p.q_bf16 != nullptr) quantise_q(cid, 0);
     transfer_q(0, 0);
     release(0);
     for (int tile = cid; tile < ng; tile += ncta, ++it) {
@@ -662,7 +669,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       nb_next = blocks_of(tile + ncta);
       const int n = kb0 + nb + it + 1;             // entry number of the next item's Q
       if (tile + ncta < ng) {
-        if (p.q_bf16 != nullptr) fill_q(tile + ncta, it + 1, n);
+        if (p.q_bf16 != nullptr) quantise_q(tile + ncta, it + 1);
         transfer_q(it + 1, n);
       } else {
         mbar_wait(&ms.q_land, (it + 1) & 1, wt, kSiteQ, it + 1);      // an empty entry
@@ -682,7 +689,8 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       if (lane == 0) mbar_arrive(&ms.fin_free);
       if (e_h == 0) p.lse[(size_t)tile * kRows + e_r] = li > 0.f ? __logf(li) - kPScaleLn + m * kLn2 : INFINITY;
       const float oscale = li > 0.f ? __fdividef(p.out_scale, li) : 0.f;
-      const uint32_t emask = oscale != 0.f ? 0xffffffffu : 0u;
+      const bool no_key = oscale == 0.f, some_no_key = __any_sync(0xffffffffu, no_key);
+      const uint64_t os2 = pack2(oscale, oscale);
       mbar_wait(&ms.pv_done[kbl & 7], (kbl >> 3) & 1, wt, kSiteEpi, nb);
       __syncwarp();
       tc_fence_after();
@@ -690,47 +698,45 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       const int r0 = 32 * (warp & 1);
       const int out_head = r0 % p.h_per_q, out_tok = tile * p.G + r0 / p.h_per_q;
       const uint32_t stage = kOffKV + (uint32_t)(n % kSlots) * kSlot + (uint32_t)ew * 8192;
-      float o[32];
-      tmem_ld32(e_ocol, o);
+      // Four boxes of 32 rows x 64 dims (128-byte swizzle) leave through the warp's two 4 KB pieces of the slot; each
+      // is in registers before it waits until the one before last has been read out
 #pragma unroll 1
-      for (int cc = 0; cc < 8; ++cc) {
-        tmem_wait_ld();
-        uint32_t wv[16];
+      for (int x = 0; x < 4; ++x) {
+        uint32_t wv[32];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          __nv_bfloat162 v2 = __floats2bfloat162_rn(o[2 * j] * oscale, o[2 * j + 1] * oscale);
-          wv[j] = *reinterpret_cast<uint32_t*>(&v2) & emask;    // rows without a valid key: zeros
+        for (int cc = 0; cc < 2; ++cc) {      // 64 columns, scaled and rounded
+          float o[32];
+          tmem_ld32(e_ocol + 64 * x + 32 * cc, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float2 v = unpack2(mul2(pack2(o[2 * j], o[2 * j + 1]), os2));
+            const __nv_bfloat162 v2 = __floats2bfloat162_rn(v.x, v.y);
+            wv[16 * cc + j] = *reinterpret_cast<const uint32_t*>(&v2);
+          }
         }
-        if (cc < 7) {
-          tmem_ld32(e_ocol + (cc + 1) * 32, o);
-        } else {
-          // O has been read: the next item's first PV may overwrite it
+        if (some_no_key) {      // rows without a valid key: zeros, whatever O holds
+#pragma unroll
+          for (int j = 0; j < 32; ++j) wv[j] = no_key ? 0u : wv[j];
+        }
+        if (x == 3) {           // O has been read: the next item's first PV may overwrite it
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ms.o_free);
         }
-        // Two rounds make one box of 32 rows x 128 bytes (128-byte swizzle) in one of the warp's two 4 KB pieces of
-        // the slot; before the third and the fourth box the one before last must have been read out.  (With one
-        // piece, or from registers straight to memory, a row of 32 bytes per lane, it took 4500 cycles
-        // until the next item's first PV could start, and five blocks were waiting for that.)
-        if ((cc & 1) == 0 && cc >= 4) {
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          __syncwarp();
-        }
-        const uint32_t piece = stage + ((cc >> 1) & 1) * 4096;
+        if (x >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+        const uint32_t piece = stage + (x & 1) * 4096;
         uint8_t* st_row = sm + piece + lane * 128;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          *reinterpret_cast<uint4*>(st_row + (((4 * (cc & 1) + j) ^ (lane & 7)) << 4)) =
-              make_uint4(wv[4 * j], wv[4 * j + 1], wv[4 * j + 2], wv[4 * j + 3]);
-        if (cc & 1) {
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            // dims 256 (cc / 4) + 128 e_h + 64 (cc / 2 % 2)
-            tma_store_3d_hint(&map_out, sbase + piece, 256 * (cc >> 2) + 128 * e_h + 64 * ((cc >> 1) & 1), out_head, out_tok, pol_stream);
-            bulk_commit_group();
-          }
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<uint4*>(st_row + ((j ^ (lane & 7)) << 4)) = make_uint4(wv[4 * j], wv[4 * j + 1], wv[4 * j + 2], wv[4 * j + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          // dims 256 (x / 2) + 128 e_h + 64 (x % 2)
+          tma_store_3d_hint(&map_out, sbase + piece, 256 * (x >> 1) + 128 * e_h + 64 * (x & 1), out_head, out_tok, pol_stream);
+          bulk_commit_group();
         }
       }
       release(n);
@@ -752,25 +758,32 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
 }  // namespace r64
 
 // One launch over the 64-row tiles of dense q [T, h, 576] (ng = T h / 64).  a.nsplit, sinks, strides of q / out and
-// further destinations are not supported here.  With one token per tile every list entry is every row's.
-int run_fp8_rows64(const Fp8Args& a, void* out, void* stream) {
-  const int rc = check_fp8_args(a);
+// further destinations are not supported here.  With one token per tile every list entry is every row's.  q_codes:
+// rows64_scratch() bytes, used with bf16 queries.
+int64_t rows64_scratch(int ng) { return (int64_t)2 * min(ng, sm_count()) * r64::kSlot; }
+int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
+  Fp8Args c = a;
+  if (a.h_per_q == r64::kRows) c.memb_qm = reinterpret_cast<const uint32_t*>(a.indices);      // none there, and none read
+  const int rc = check_fp8_args(c);
   if (rc != LITEDSA_OK) return rc;
   // (row offsets are held in 32 bits of 16-byte units)
   if (a.h_per_q > r64::kRows || a.topk < 256 || ((uintptr_t)out & 15) || (int64_t)a.s_kv * (a.kv_row_stride >> 4) >= 0xffffffffll)
     return LITEDSA_ERR_UNSUPPORTED;
-  CUtensorMap map_q = {}, map_q_rope = {}, map_out;      // the first two are not used by the kernel with bf16 q
+  CUtensorMap map_q, map_q_rope, map_out;
   const int h = a.h_per_q, G = r64::kRows / h;
   const uint64_t tokens = (uint64_t)a.ng * G;
   const uint32_t ob_h = (uint32_t)min(h, 32);
+  const int ncta = min(a.ng, sm_count());
   if (!make_map_3d(&map_out, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, kDV, (uint64_t)h, tokens, kDV * 2, (uint64_t)h * kDV * 2,
                    64, ob_h, 32 / ob_h, CU_TENSOR_MAP_SWIZZLE_128B))
     return LITEDSA_ERR_CUDA;
-  if (!a.q_is_bf16 &&
-      (!make_map_3d(&map_q, a.q8, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, (uint64_t)h, tokens, kDQK, (uint64_t)h * kDQK, 128,
-                    (uint32_t)h, (uint32_t)G) ||
-       !make_map_3d(&map_q_rope, a.q8, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, (uint64_t)h, tokens, kDQK, (uint64_t)h * kDQK, 64,
-                    (uint32_t)h, (uint32_t)G, CU_TENSOR_MAP_SWIZZLE_64B)))
+  // Q: boxes of 64 rows x 128 bytes (128-byte swizzle) and the rope box of 64 rows x 64 bytes (64-byte swizzle)
+  const void* q = a.q_is_bf16 ? q_codes : a.q8;
+  const uint32_t qh = a.q_is_bf16 ? (uint32_t)r64::kRows : (uint32_t)h;
+  const uint64_t qz = a.q_is_bf16 ? (uint64_t)2 * ncta : tokens;
+  if (!make_map_3d(&map_q, q, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, qh, qz, kDQK, (uint64_t)qh * kDQK, 128, qh, r64::kRows / qh) ||
+      !make_map_3d(&map_q_rope, q, CU_TENSOR_MAP_DATA_TYPE_UINT8, kDQK, qh, qz, kDQK, (uint64_t)qh * kDQK, 64, qh, r64::kRows / qh,
+                   CU_TENSOR_MAP_SWIZZLE_64B))
     return LITEDSA_ERR_CUDA;
   r64::Params p;
   p.memb = G > 1 ? a.memb_qm : nullptr; p.indices = a.indices; p.counts = a.topk_length;
@@ -780,8 +793,9 @@ int run_fp8_rows64(const Fp8Args& a, void* out, void* stream) {
   p.scale_log2 = a.sm_scale * kLog2e; p.out_scale = a.out_scale;
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
   p.q_bf16 = a.q_is_bf16 ? reinterpret_cast<const uint4*>(a.q8) : nullptr; p.q_inv = a.q_inv;
+  p.q_codes = reinterpret_cast<uint8_t*>(q_codes);
   if (!ensure_smem<r64::masked_mla_fp8_r64_kernel>(current_device(), r64::Plan::kSmem)) return LITEDSA_ERR_CUDA;
-  return launch_pdl(r64::masked_mla_fp8_r64_kernel, dim3((unsigned)min(p.ng, sm_count())), r64::kThreads, r64::Plan::kSmem,
+  return launch_pdl(r64::masked_mla_fp8_r64_kernel, dim3((unsigned)ncta), r64::kThreads, r64::Plan::kSmem,
                     reinterpret_cast<cudaStream_t>(stream), map_q, map_q_rope, map_out, p);
 }
 

@@ -96,8 +96,8 @@ static int pick_slices(int tiles, int G, int k, bool bf16) {
 }
 
 // workspace layout: all offsets are multiples of 256 bytes
-struct Layout { int64_t counts, u, memb, part_o, part_ml, total; };
-static Layout layout_of(int ng, int G, int cap, int nsplit) {
+struct Layout { int64_t counts, u, memb, part_o, part_ml, q_codes, total; };
+static Layout layout_of(int ng, int G, int cap, int nsplit, bool rows64) {
   auto up = [](int64_t b) { return (b + 255) & ~(int64_t)255; };
   Layout l;
   l.counts = 0;
@@ -105,7 +105,8 @@ static Layout layout_of(int ng, int G, int cap, int nsplit) {
   l.memb = l.u + up(4 * (int64_t)ng * cap);
   l.part_o = l.memb + up(4 * (int64_t)ng * G * (cap / 32));
   l.part_ml = l.part_o + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 512 * 4) : 0);
-  l.total = l.part_ml + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 8) : 0);
+  l.q_codes = l.part_ml + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 8) : 0);
+  l.total = l.q_codes + (rows64 ? rows64_scratch(ng) : 0);
   return l;
 }
 
@@ -158,7 +159,7 @@ static Route route_of(int T, int h, int k, bool kv_bf16, int policy_tokens, bool
 static int64_t workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens, bool by_job) {
   if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
   const Route r = route_of(T, h, k, kv_is_bf16 != 0, policy_tokens, by_job);
-  return layout_of(r.ng, r.G, r.cap, r.ns).total;
+  return layout_of(r.ng, r.G, r.cap, r.ns, r.rows64).total;
 }
 
 static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, const int32_t* topk_idx, double sm_scale,
@@ -174,12 +175,12 @@ static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, con
     return LITEDSA_ERR_UNSUPPORTED;
   const Route r = route_of(T, h, k, kv_is_bf16 != 0, policy_tokens, by_job);
   const int G = r.G, ng = r.ng, cap = r.cap, ns = r.ns;
-  const Layout l = layout_of(ng, G, cap, ns);
+  const Layout l = layout_of(ng, G, cap, ns, r.rows64);
   if (workspace_bytes < l.total) return LITEDSA_ERR_SHAPE;
   char* ws = reinterpret_cast<char*>(workspace);
   int32_t* counts = reinterpret_cast<int32_t*>(ws + l.counts);
   int32_t* u = reinterpret_cast<int32_t*>(ws + l.u);
-  uint32_t* memb = reinterpret_cast<uint32_t*>(ws + l.memb);
+  uint32_t* memb = r.rows64 && G == 1 ? nullptr : reinterpret_cast<uint32_t*>(ws + l.memb);
   // fill 2: lists padded to whole 128-key blocks, nothing written beyond
   rc = run_union(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
   if (rc != LITEDSA_OK) return rc;
@@ -199,7 +200,7 @@ static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, con
             ng, s_kv, cap, 576, kv_row_stride, cap, nullptr, nullptr, 1};
   a.q_is_bf16 = q_is_bf16 != 0;
   a.q_inv = 1.0f / (float)q_scale;
-  if (r.rows64) return run_fp8_rows64(a, out, stream);
+  if (r.rows64) return run_fp8_rows64(a, out, ws + l.q_codes, stream);
   a.nsplit = ns;
   a.part_o = reinterpret_cast<float*>(ws + l.part_o);
   a.part_ml = ws + l.part_ml;

@@ -27,7 +27,7 @@ struct UnionParams {
   const int32_t* idx;       // [T, k]
   int32_t* u_phys;          // [ng, cap]
   int32_t* counts;          // [ng]
-  uint32_t* memb;           // [ng, G, cap/32]
+  uint32_t* memb;           // [ng, G, cap/32], or null: no membership words (one list per tile needs none)
   const int32_t* req_pg;    // [ng] or null (identity table)
   const int32_t* btab;      // [nreq, bt_stride] or null
   int bt_stride, bt_blocks, bsz;
@@ -76,7 +76,7 @@ union_qm_kernel(const UnionParams p) {
     uint4* b4 = reinterpret_cast<uint4*>(bm);
     for (int i = tid; i < (s_words >> 2); i += NT) b4[i] = make_uint4(0, 0, 0, 0);
     uint4* q4 = reinterpret_cast<uint4*>(qm_s);
-    for (int i = tid; i < (p.G * capw >> 2); i += NT) q4[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; p.memb && i < (p.G * capw >> 2); i += NT) q4[i] = make_uint4(0, 0, 0, 0);
   }
   pdl_trigger();
   pdl_wait();
@@ -160,7 +160,7 @@ union_qm_kernel(const UnionParams p) {
       if (RS)
         for (int x = (w >> RS) << RS; x < w; ++x) r += __popc(bm[x]);
       r += __popc(bm[w] & ((1u << (pos & 31)) - 1u));
-      atomicOr(row + (r >> 5), 1u << (r & 31));
+      if (p.memb) atomicOr(row + (r >> 5), 1u << (r & 31));
       int phys = pos;
       if (BT) {
         const int blk = fast_div(pos, p.bsz, p.bsz_mul);
@@ -216,7 +216,7 @@ union_qm_kernel(const UnionParams p) {
     const int runs = (per_row + 31) >> 5;                       // warp-wide pieces of a row
     uint4* dst = reinterpret_cast<uint4*>(p.memb + (size_t)g * p.G * capw);
     const uint4* s4 = reinterpret_cast<const uint4*>(qm_s);
-    for (int c = wid; c < p.G * runs; c += NW) {
+    for (int c = wid; p.memb && c < p.G * runs; c += NW) {
       const int q = c / runs, j = 32 * (c - q * runs) + lane;
       if (j < per_row) dst[q * c4 + j] = s4[q * c4 + j];
     }
@@ -241,7 +241,7 @@ int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uin
               const int32_t* block_table, int T, int k, int ng, int cap, int G, int bt_rows, int bt_blocks,
               int block_size, int64_t seq_space, int fill, void* stream) {
   // same argument checks as the reference launcher (litedsa.cu:43-59)
-  if (!topk_indices || !u_phys || !counts || !memb_qm) return LITEDSA_ERR_ARG;
+  if (!topk_indices || !u_phys || !counts || (!memb_qm && G != 1)) return LITEDSA_ERR_ARG;
   if (ng <= 0 || G <= 0 || k <= 0 || T != ng * G) return LITEDSA_ERR_SHAPE;
   if (cap < G * k || cap % 128 != 0) return LITEDSA_ERR_SHAPE;
   if (G > 16 || (int64_t)G * (cap / 32) > 16 * 1024) return LITEDSA_ERR_SHAPE;
@@ -307,7 +307,8 @@ extern "C" int litedsa_union_qm(const int32_t* topk_indices, int32_t* u_phys, in
                                 const int32_t* block_table, int T, int k, int ng, int cap, int G,
                                 int bt_rows, int bt_blocks, int block_size, int64_t seq_space,
                                 int fill_tail, void* stream) {
-  if (topk_indices && u_phys && counts && memb_qm && cap != G * k) return LITEDSA_ERR_SHAPE;
+  if (!topk_indices || !u_phys || !counts || !memb_qm) return LITEDSA_ERR_ARG;
+  if (cap != G * k) return LITEDSA_ERR_SHAPE;
   return lt::run_union(topk_indices, u_phys, counts, memb_qm, req_pg, block_table, T, k, ng, cap, G, bt_rows, bt_blocks,
                        block_size, seq_space, fill_tail != 0 ? 1 : 0, stream);
 }

@@ -49,6 +49,8 @@ def _agents(blocks, bf16_q, rescale):
                 g, land = f"g{s}{w}", f"land{s}{w}"
                 if it > 0:
                     wait(g, "q_taken", it - 1)
+                if bf16_q and nb:
+                    wait(g, "q_codes", it)
                 if e % 2 == s:
                     if e >= slots:
                         wait(g, f"slot_free{e % slots}", e // slots - 1)
@@ -122,10 +124,11 @@ def _agents(blocks, bf16_q, rescale):
     for it in range(-1, len(blocks)):
         staged = f"slot_free{q_entry[it + 1] % slots}"
         if it + 1 < len(blocks):
-            order = [("q_land", it + 1), ("q_free", it)]
-            for bar, phase in order if bf16_q else order[::-1]:
-                if phase >= 0:
-                    wait("epi", bar, phase)
+            if bf16_q:
+                ar("epi", "q_codes", it + 1)
+            if it >= 0:
+                wait("epi", "q_free", it)
+            wait("epi", "q_land", it + 1)
             ar("epi", "qt_ready", it + 1)
             ar("epi", "q_taken", it + 1)
         else:
