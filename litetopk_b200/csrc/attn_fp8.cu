@@ -49,9 +49,6 @@
 
 
 namespace lt {
-constexpr unsigned kIdleCheckEvery = 64;   // idle polls between two time-limit checks (power of two)
-constexpr unsigned kIdleSleepNs = 8;       // back-off of an idle poll
-
 
 constexpr int kSoftmaxWarps = 16, kProducerWarps = 8;
 constexpr int kWarpGather0 = 16, kWarpMma = 24, kWarpRelayK = 25, kWarpRelayV = 26, kWarpValid = 27, kWarpEpi0 = 28;
@@ -239,7 +236,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   };
 
   if (threadIdx.x == 0) {
-    mbar_init(&ms.q_land, 1);
+    mbar_init(&ms.q_land, kProducerWarps / 2);              // the K warps
     mbar_init(&ms.q_taken, 1);
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
@@ -247,8 +244,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     for (int i = 0; i < 8; ++i) {
       mbar_init(&ms.k_peer[i], 1);
       mbar_init(&ms.v_peer[i], 1);
-      mbar_init(&ms.k_land[i], kProducerWarps * 32);        // one async arrival per gather thread
-      mbar_init(&ms.v_land[i], kProducerWarps * 32);
+      mbar_init(&ms.k_land[i], kProducerWarps / 2 * 32);    // one async arrival per gather thread
+      mbar_init(&ms.v_land[i], kProducerWarps / 2 * 32);
       mbar_init(&ms.qk_done[i], 1);
     }
     for (int i = 0; i < 4; ++i) mbar_init(&ms.pv_done[i], 1);
@@ -487,154 +484,130 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     // directly in the 128-byte-swizzled tile layout, completion reported to an mbarrier by an
     // asynchronous arrival.  (TMA gather4 was measured at one instruction per ~8.5 ns per SM,
     // i.e. the same ~60 GB/s per SM that the L2 -> SM path gives these copies.)
-    // Two cursors: K rows of block ck (this CTA's 64 keys, all 576 bytes: warp pw rows
-    // [8pw, 8pw + 8), nine copies per lane) as soon as the stage's previous block has been through
-    // its PV; V rows of block cv (the PEER's 64 keys, this CTA's 256 value bytes, four copies per
-    // lane) into the dead half of the same stage as soon as the block's QK^T is complete.
-    const int pw = warp - kWarpGather0;
-    struct Cursor { int w, k, nb, kb, slot, ring, k0, lead; const int32_t* idx; };   // slot, ring: entry = 5 ring + slot
-    // The Q entry in front of an item's K entries belongs to warp 0: once the slot is free it
-    // requests the tile (TMA) or, for bf16 q, hands the slot to the epilogue warps.  (Only here: a
-    // slot's barrier may be waited on once every older entry has been through it, which this
-    // warp's own K copies prove.)
-    // The previous item's Q must have been moved on: with short items its bytes could still be in flight.
-    int q_w = cid, q_slot = 0, q_ring = 0, q_n = 0;      // q_n: items whose Q has been requested
-    bool q_pending = pw == 0 && cid < n_items;
-    const uint64_t pol_stream = l2_policy_evict_first();
-    auto cur_load = [&](Cursor& c) {
-      c.nb = 0;
-      if (c.w < n_items) {
-        const Item t = item_of(c.w);
-        c.nb = t.nb; c.k = 0; c.k0 = t.k0; c.lead = t.lead;
-        c.idx = p.indices + (size_t)t.tile * p.idx_stride;
-      }
-    };
-    auto advance = [&](Cursor& c) { if (++c.slot == kSlots) { c.slot = 0; ++c.ring; } };
-    auto cur_next = [&](Cursor& c) {
-      ++c.kb;
-      advance(c);
-      if (++c.k == c.nb) { c.w += ncl; cur_load(c); return true; }     // the next item's Q entry is next
-      return false;
-    };
-    Cursor ck, cv;
-    ck.w = cv.w = cid;
-    ck.kb = cv.kb = 0;
-    ck.slot = cv.slot = 1;                         // entry 0 is the first item's Q
-    ck.ring = cv.ring = 0;
-    cur_load(ck);
-    cur_load(cv);
-    // lane l holds the index of key 8 pw + l % 8 of the CTA's own (K) / the peer's (V) 64 keys
-    const int own_key = 64 * (int)cta + 8 * pw + (lane & 7);
-    auto load_idx = [&](const Cursor& c, int key) -> int {
-      return __ldcs(c.idx + (size_t)(!kSliced ? c.k : (c.k < c.lead ? 0 : c.k0 + c.k - c.lead)) * kBlockKeys + key);
-    };
-    auto in_range = [&](int v) -> int { return ((unsigned)v < (unsigned)p.s_kv) ? v : 0; };   // masked later
-    // The indices of a block are loaded right after the previous block's gather has been issued
-    // (one block ahead) and first looked at when the next gather goes out, so that nothing waits
-    // for a cold index line from HBM.
-    int kidx = 0, vidx = 0;
-    if (ck.w < n_items) { kidx = load_idx(ck, own_key); vidx = load_idx(cv, own_key ^ 64); }
+    // Four warps fetch K rows (this CTA's 64 keys, all 576 bytes: warp pw rows [16 pw, 16 pw + 16), 18 copies
+    // per lane) as soon as the slot's previous entry is dead, the other four V rows (the PEER's 64 keys,
+    // this CTA's 256 value bytes, eight copies per lane) into the dead half of the slot as soon as the block's QK^T
+    // is complete.  (Eight warps that polled for both in turn noticed a free slot 1500 cycles and a finished QK^T
+    // 1200 cycles late, out of the 11400 that a slot was held for; five slots make that the kernel's
+    // pace.)  Entries without a valid index become zeros without a read: all of them read from row 0, the padded
+    // blocks of all SMs met at one L2 slice (1.2 instead of 18 TB/s).
+    const int pw = (warp - kWarpGather0) & 3;
     const uint8_t* kvb = p.kv;
     const long long pitch = p.kv_pitch;
-    const int cj = lane >> 3, cc = lane & 7;       // latent piece `lane`: chunk cj, 16-byte slot cc
-    unsigned long long idle_since = 0;
-    unsigned idle_iters = 0;
-    bool aborted = false;
-    while (cv.w < n_items && !aborted) {           // the V cursor never runs ahead of the K cursor
-      bool did = false;
-      // V first: its block is further along, and P waits for it next
-      {
-        // the block's K tile must have been read by its QK^T
-        const bool ok = cv.kb < ck.kb && mbar_test(&ms.qk_done[cv.kb & 7], (cv.kb >> 3) & 1);
-        if (__all_sync(0xffffffffu, ok)) {
-          const int vcur = in_range(vidx);
-          // the dead half of the K tile: chunks 2-3 in CTA 0, chunks 0-1 in CTA 1
-          const uint32_t vst = sbase + kOffKV + cv.slot * kStageKV + (cta == 0 ? 2 * kChunkBytes : 0);
-          // lane: row 8 pw + 2i + lane / 16 of the peer's keys, 16-byte piece lane % 16 of this
-          // CTA's 256 value bytes
-          const int pc = lane & 15, nbk = pc >> 3, c8 = pc & 7;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int rloc = 2 * i + (lane >> 4);
-            const int ri = __shfl_sync(0xffffffffu, vcur, rloc);
-            const int row = 8 * pw + rloc;
-            cp_async16(vst + nbk * kChunkBytes + row * 128 + ((c8 ^ (row & 7)) << 4),
-                       kvb + (size_t)ri * pitch + 256 * cta + 16 * pc);
+    // lane l holds the index of key 16 pw + l % 16 of the CTA's own (K) / the peer's (V) 64 keys, -1 if it is out of
+    // range; a block's are loaded a block ahead, so that nothing waits for a cold line
+    const bool is_k = warp < kWarpGather0 + kProducerWarps / 2;
+    const int key = (64 * (int)cta + 16 * pw + (lane & 15)) ^ (is_k ? 0 : 64);
+    auto load_idx = [&](const Item& t, int k) -> int {
+      return __ldcs(p.indices + (size_t)t.tile * p.idx_stride + (size_t)t.block(k) * kBlockKeys + key);
+    };
+    Item nx = item_of(min(cid, n_items - 1));
+    int idx = load_idx(nx, 0);
+    int slot = 0, ring = 0, kb = 0, it = 0;        // entry = 5 ring + slot
+    auto advance = [&]() { if (++slot == kSlots) { slot = 0; ++ring; } };
+    // the block's index, with the next block's (of the next item behind the last) on its way
+    auto take_idx = [&](const Item& t, int k, int w) -> int {
+      const int cur = (unsigned)idx < (unsigned)p.s_kv ? idx : -1;
+      if (k + 1 < t.nb) idx = load_idx(t, k + 1);
+      else if (w + ncl < n_items) idx = load_idx(nx, 0);
+      return cur;
+    };
+    if (is_k) {
+      const uint64_t pol_stream = l2_policy_evict_first();
+      const int cj = lane >> 3, cc = lane & 7;     // latent piece `lane`: chunk cj, 16-byte slot cc
+      for (int w = cid; w < n_items; w += ncl, ++it) {
+        const Item t = nx;
+        if (w + ncl < n_items) nx = item_of(w + ncl);
+        // The item's Q entry, in front of its K entries.  Every warp goes through its slot's barrier and that of
+        // the previous Q (whose bytes could, with short items, still be in flight), and it counts as landed
+        // only when all of them have: no warp is overtaken and tests a phase that is two ahead.
+        if (it > 0) mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
+        if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
+        __syncwarp();
+        if (lane == 0) {
+          if (pw != 0 || p.q_bf16 != nullptr) {
+            mbar_arrive(&ms.q_land);               // bf16 q: the epilogue warps fill the slot
+          } else {
+            mbar_arrive_expect_tx(&ms.q_land, kStageKV);
+            // this CTA's 64 rows of the tile = (token, head) pairs starting at row 64 cta
+            const int qh = (64 * (int)cta) % p.h_per_q;
+            const int qt = t.tile / p.q_group_div * p.G + (64 * (int)cta) / p.h_per_q;
+            const uint32_t dst = sbase + kOffKV + slot * kStageKV;
+            for (int c = 0; c < 4; ++c)
+              tma_load_3d_hint(dst + c * kChunkBytes, &map_q, 128 * c, qh, qt, &ms.q_land, pol_stream);
+            tma_load_3d_hint(dst + kQLatent, &map_q_rope, 512, qh, qt, &ms.q_land, pol_stream);
           }
-          cp_async_mbar_arrive_noinc(&ms.v_land[cv.kb & 7]);
-          if (cur_next(cv)) advance(cv);
-          if (cv.w < n_items) vidx = load_idx(cv, own_key ^ 64);
-          did = true;
         }
-      }
-      if (q_pending) {                             // warp-uniform; warp 0 only
-        const bool ok = (q_ring == 0 || mbar_test(&ms.slot_free[q_slot], (q_ring - 1) & 1)) &&
-                        (q_n == 0 || mbar_test(&ms.q_taken, (q_n - 1) & 1));
-        if (__all_sync(0xffffffffu, ok)) {
-          if (lane == 0) {
-            if (p.q_bf16 != nullptr) {
-              mbar_arrive(&ms.q_land);
-            } else {
-              mbar_arrive_expect_tx(&ms.q_land, kStageKV);
-              // this CTA's 64 rows of the tile = (token, head) pairs starting at row 64 cta
-              const int qh = (64 * (int)cta) % p.h_per_q;
-              const int qt = item_of(q_w).tile / p.q_group_div * p.G + (64 * (int)cta) / p.h_per_q;
-              const uint32_t dst = sbase + kOffKV + q_slot * kStageKV;
-              for (int c = 0; c < 4; ++c)
-                tma_load_3d_hint(dst + c * kChunkBytes, &map_q, 128 * c, qh, qt, &ms.q_land, pol_stream);
-              tma_load_3d_hint(dst + kQLatent, &map_q_rope, 512, qh, qt, &ms.q_land, pol_stream);
+        __syncwarp();
+        advance();
+        for (int k = 0; k < t.nb; ++k, ++kb) {
+          const int cur = take_idx(t, k, w);
+          const bool full = __all_sync(0xffffffffu, cur >= 0);
+          if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
+          __syncwarp();
+          const uint32_t kst = sbase + kOffKV + slot * kStageKV;
+          const uint32_t kdst = kst + cj * kChunkBytes + 16 * pw * 128;
+          // rope bytes: compact 64-byte rows, 64-byte swizzle (16-byte unit ^ ((row / 2) % 4))
+          const uint32_t rdst = kst + kQLatent + (16 * pw + (lane >> 2)) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4);
+          if (full) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, i);
+              cp_async16(kdst + i * 128 + ((cc ^ (i & 7)) << 4), kvb + (size_t)ri * pitch + 16 * lane);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, 8 * i + (lane >> 2));
+              cp_async16(rdst + i * 512, kvb + (size_t)ri * pitch + 512 + 16 * (lane & 3));
+            }
+          } else {
+#pragma unroll 1
+            for (int i = 0; i < 16; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, i);
+              cp_async16_or_zero(kdst + i * 128 + ((cc ^ (i & 7)) << 4), kvb + (size_t)max(ri, 0) * pitch + 16 * lane, ri >= 0);
+            }
+#pragma unroll 1
+            for (int i = 0; i < 2; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, 8 * i + (lane >> 2));
+              cp_async16_or_zero(rdst + i * 512, kvb + (size_t)max(ri, 0) * pitch + 512 + 16 * (lane & 3), ri >= 0);
             }
           }
+          cp_async_mbar_arrive_noinc(&ms.k_land[kb & 7]);
+          advance();
+        }
+      }
+    } else {
+      // lane: rows 16 pw + 2 i + lane / 16 of the peer's keys, 16-byte piece lane % 16 of this CTA's 256 value bytes
+      const int pc = lane & 15, r2 = lane >> 4;
+      const uint8_t* src = kvb + 256 * cta + 16 * pc;
+      for (int w = cid; w < n_items; w += ncl) {
+        const Item t = nx;
+        if (w + ncl < n_items) nx = item_of(w + ncl);
+        advance();                                 // the item's Q
+        for (int k = 0; k < t.nb; ++k, ++kb) {
+          const int cur = take_idx(t, k, w);
+          const bool full = __all_sync(0xffffffffu, cur >= 0);
+          mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, k);
           __syncwarp();
-          q_pending = false;
-          ++q_n;
-          did = true;
-        }
-      }
-      if (ck.w < n_items && !q_pending) {
-        // the slot's previous entry must be dead
-        const bool ok = ck.ring == 0 || mbar_test(&ms.slot_free[ck.slot], (ck.ring - 1) & 1);
-        if (__all_sync(0xffffffffu, ok)) {
-          const int kcur = in_range(kidx);
-          const uint32_t kst = sbase + kOffKV + ck.slot * kStageKV;
+          // the dead half of the K tile: chunks 2-3 in CTA 0, chunks 0-1 in CTA 1
+          const uint32_t vst = sbase + kOffKV + slot * kStageKV + (cta == 0 ? 2 * kChunkBytes : 0) + (pc >> 3) * kChunkBytes +
+                               (16 * pw + r2) * 128;
+          if (full) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int ri = __shfl_sync(0xffffffffu, kcur, i);
-            const int row = 8 * pw + i;
-            cp_async16(kst + cj * kChunkBytes + row * 128 + ((cc ^ (row & 7)) << 4),
-                       kvb + (size_t)ri * pitch + 16 * lane);
+            for (int i = 0; i < 8; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, 2 * i + r2);
+              cp_async16(vst + i * 256 + (((pc & 7) ^ ((2 * i + r2) & 7)) << 4), src + (size_t)ri * pitch);
+            }
+          } else {
+#pragma unroll 1
+            for (int i = 0; i < 8; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, 2 * i + r2);
+              cp_async16_or_zero(vst + i * 256 + (((pc & 7) ^ ((2 * i + r2) & 7)) << 4), src + (size_t)max(ri, 0) * pitch, ri >= 0);
+            }
           }
-          {
-            const int ri = __shfl_sync(0xffffffffu, kcur, lane >> 2);
-            const int row = 8 * pw + (lane >> 2);
-            // rope bytes: compact 64-byte rows, 64-byte swizzle (16-byte unit ^ ((row / 2) % 4))
-            cp_async16(kst + kQLatent + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4),
-                       kvb + (size_t)ri * pitch + 512 + 16 * (lane & 3));
-          }
-          cp_async_mbar_arrive_noinc(&ms.k_land[ck.kb & 7]);
-          if (cur_next(ck)) {
-            if (pw == 0 && ck.w < n_items) { q_w = ck.w; q_slot = ck.slot; q_ring = ck.ring; q_pending = true; }
-            advance(ck);
-          }
-          if (ck.w < n_items) kidx = load_idx(ck, own_key);
-          did = true;
+          cp_async_mbar_arrive_noinc(&ms.v_land[kb & 7]);
+          advance();
         }
-      }
-      if (did) {
-        idle_since = 0;
-        idle_iters = 0;
-      } else if ((++idle_iters & (kIdleCheckEvery - 1)) != 0) {
-        __nanosleep(kIdleSleepNs);
-      } else {
-        // the (slow) time-limit and abort check runs once per kIdleCheckEvery idle polls
-        const unsigned long long now = globaltimer_ns();
-        if (idle_since == 0) idle_since = now;
-        bool stop = wt.aborting();
-        if (now - idle_since > wt.limit_ns) {
-          if (lane == 0) wt.fail(kSiteKFree, ck.k);
-          stop = true;
-        }
-        aborted = __any_sync(0xffffffffu, stop);
       }
     }
   } else if (warp < kWarpEpi0) {

@@ -133,37 +133,6 @@ __device__ __forceinline__ void commit_elect(uint64_t* bar) {
       "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
       ::"r"(smem_u32(bar)) : "memory");
 }
-// 16 bytes from global memory, or 16 zero bytes without a read
-__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst_smem, const void* src, bool read) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(read ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-  return v;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t v;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-  return v;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t v;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-  return v;
-}
-
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t v;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-  return v;
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
 masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_rope,
                           const __grid_constant__ CUtensorMap map_out, const Params p) {
