@@ -302,6 +302,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int capw = p.cap >> 5;
     const float c = p.scale_log2;
+    const uint64_t c2 = pack2(c, c);
     const uint32_t a_s_free = mapa(smem_u32(&ms.s_free[g]), 0);
     const uint32_t a_p_ready = mapa(smem_u32(&ms.p_ready[g]), 0);
     const uint32_t scol = tmem + lane_base + (g ? kTmemS1 : kTmemS0) + 32 * cs;
@@ -347,15 +348,19 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) mbar_arrive(&ms.valid_free[g]);
         mk = mk_next;
 
-        float c0 = -INFINITY, c1 = -INFINITY;
+        if (vm != ~0u) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          sv[j] = ((vm >> j) & 1u) ? sv[j] : -INFINITY;
-          sv[j + 1] = ((vm >> (j + 1)) & 1u) ? sv[j + 1] : -INFINITY;
-          c0 = fmaxf(c0, sv[j]);
-          c1 = fmaxf(c1, sv[j + 1]);
+          for (int j = 0; j < 32; ++j) sv[j] = ((vm >> j) & 1u) ? sv[j] : -INFINITY;
         }
-        float cur = fmaxf(c0, c1) * c;
+        float mx[4] = {sv[0], sv[1], sv[2], sv[3]};
+#pragma unroll
+        for (int j = 4; j < 32; j += 4) {
+          mx[0] = fmaxf(mx[0], sv[j]);
+          mx[1] = fmaxf(mx[1], sv[j + 1]);
+          mx[2] = fmaxf(mx[2], sv[j + 2]);
+          mx[3] = fmaxf(mx[3], sv[j + 3]);
+        }
+        float cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
         float (*xb)[128] = ms.xbuf[g][ph];
         xb[cs][tl] = cur;
         if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -381,22 +386,25 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
           for (int j = 0; j < 32; ++j) sv[j] = -INFINITY;      // only the maxima of this block count
         }
         const float nm = -new_m + kPScaleLog2;
+        const uint64_t nm2 = pack2(nm, nm);
         uint32_t pk[8];
-        float l1 = 0.f;
+        uint64_t l0 = 0, l1 = 0;      // two pairs of partial sums
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
-          float2 d0, d1;
-          d0.x = fast_exp2(fmaf(sv[j], c, nm));
-          d0.y = fast_exp2(fmaf(sv[j + 1], c, nm));
-          d1.x = fast_exp2(fmaf(sv[j + 2], c, nm));
-          d1.y = fast_exp2(fmaf(sv[j + 3], c, nm));
-          li += d0.x + d0.y;
-          l1 += d1.x + d1.y;
+          float2 d0 = unpack2(fma2(pack2(sv[j], sv[j + 1]), c2, nm2));
+          float2 d1 = unpack2(fma2(pack2(sv[j + 2], sv[j + 3]), c2, nm2));
+          d0.x = fast_exp2(d0.x);
+          d0.y = fast_exp2(d0.y);
+          d1.x = fast_exp2(d1.x);
+          d1.y = fast_exp2(d1.y);
+          l0 = add2(l0, pack2(d0.x, d0.y));
+          l1 = add2(l1, pack2(d1.x, d1.y));
           const uint32_t lo = __nv_cvt_float2_to_fp8x2(d0, __NV_SATFINITE, __NV_E4M3);
           const uint32_t hi = __nv_cvt_float2_to_fp8x2(d1, __NV_SATFINITE, __NV_E4M3);
           pk[j >> 2] = lo | (hi << 16);
         }
-        li += l1;
+        const float2 ls = unpack2(add2(l0, l1));
+        li += ls.x + ls.y;
         // the P buffer was last read by the PV of block kb-2
         if (kb >= 2) mbar_wait(&ms.pv_done[(kb - 2) & 3], ((kb - 2) >> 2) & 1, wt, kSitePFree, k);
         uint8_t* pdst = sm + kOffP + g * kPBytes + (4 * h + 2 * cs) * 1024 + r * 16;
