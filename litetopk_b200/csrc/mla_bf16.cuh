@@ -302,13 +302,13 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_res, 1);
-    mbar_init(&ms.q_land, kQEntries);
+    mbar_init(&ms.q_land, kQEntries + (kTma ? 0 : kGatherWarps / 2 - 1));      // gather: and the other K warps
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
     for (int i = 0; i < 8; ++i) {
-      mbar_init(&ms.k_full[i], kTma ? 1 : kGatherWarps * 32);     // gather: one async arrival per thread
-      mbar_init(&ms.v_full[i], kTma ? 1 : kGatherWarps * 32);
+      mbar_init(&ms.k_full[i], kTma ? 1 : kGatherWarps / 2 * 32);     // gather: one async arrival per thread
+      mbar_init(&ms.v_full[i], kTma ? 1 : kGatherWarps / 2 * 32);
       mbar_init(&ms.k_peer[i], 1);
       mbar_init(&ms.v_peer[i], 1);
       mbar_init(&ms.qk_done[i], 1);
@@ -369,6 +369,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int capw = p.cap >> 5;
     const float c = p.scale_log2;
+    const uint64_t c2 = pack2(c, c);
     const uint32_t a_s_free = mapa(smem_u32(&ms.s_free[g]), 0);
     const uint32_t a_p_ready = mapa(smem_u32(&ms.p_ready[g]), 0);
     const uint32_t scol = tmem + lane_base + (g ? kTmemS1 : kTmemS0);
@@ -437,15 +438,19 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           mk = mk_next;
         }
 
-        float c0 = -INFINITY, c1 = -INFINITY;
+        if (vm != ~0u) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          sv[j] = ((vm >> j) & 1u) ? sv[j] : -INFINITY;
-          sv[j + 1] = ((vm >> (j + 1)) & 1u) ? sv[j + 1] : -INFINITY;
-          c0 = fmaxf(c0, sv[j]);
-          c1 = fmaxf(c1, sv[j + 1]);
+          for (int j = 0; j < 32; ++j) sv[j] = ((vm >> j) & 1u) ? sv[j] : -INFINITY;
         }
-        float cur = fmaxf(c0, c1) * c;
+        float mx[4] = {sv[0], sv[1], sv[2], sv[3]};
+#pragma unroll
+        for (int j = 4; j < 32; j += 4) {
+          mx[0] = fmaxf(mx[0], sv[j]);
+          mx[1] = fmaxf(mx[1], sv[j + 1]);
+          mx[2] = fmaxf(mx[2], sv[j + 2]);
+          mx[3] = fmaxf(mx[3], sv[j + 3]);
+        }
+        float cur = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;
         float* xb = ms.xbuf[g][ph];
         xb[tl] = cur;
         if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -466,18 +471,20 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         li *= fast_exp2(m_mine - new_m);
         m_mine = new_m;
 
+        const uint64_t nm2 = pack2(-new_m, -new_m);
         uint32_t pk[16];
-        float l1 = 0.f;
+        uint64_t l2 = 0;              // a pair of partial sums
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
-          const float p0 = fast_exp2(fmaf(sv[j], c, -new_m));
-          const float p1 = fast_exp2(fmaf(sv[j + 1], c, -new_m));
-          li += p0;
-          l1 += p1;
-          const __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
+          float2 d = unpack2(fma2(pack2(sv[j], sv[j + 1]), c2, nm2));
+          d.x = fast_exp2(d.x);
+          d.y = fast_exp2(d.y);
+          l2 = add2(l2, pack2(d.x, d.y));
+          const __nv_bfloat162 b2 = __floats2bfloat162_rn(d.x, d.y);
           pk[j >> 1] = *reinterpret_cast<const uint32_t*>(&b2);
         }
-        li += l1;
+        const float2 ls = unpack2(l2);
+        li += ls.x + ls.y;
         // P: [64 rows][32 keys] per half, K-major core matrices (8-key group at 1024 * group + 16 * row).
         // Keys 0-31 go into the block's own rope chunk (576 dims); the other buffer was last read by
         // the PV of block kb - 2.
@@ -891,142 +898,103 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     tc_fence_before();
   } else if (!kTma) {
     // ------------------------------------------------------------ KV row gather (cp.async)
-    // 16-byte copies written straight into the 128-byte-swizzled layout, completion reported to an
-    // mbarrier by an asynchronous arrival.  Two cursors, whichever is ready goes first: V rows of
-    // block cv (the PEER's 32 keys, this CTA's 256 value dims; warp pw rows [4 pw, 4 pw + 4), one row
-    // per instruction) into the dead half of its slot once its QK^T is complete; K rows of block ck
-    // (this CTA's 32 keys, all dims) once its slot is free.
-    const int pw = warp - kWarpGather0;
-    struct Cursor { int w, k, nb, kb, slot, ring, k0, len; const int32_t* idx; };   // ring entry = kSlots ring + slot
-    // The Q entries in front of an item's K entries are requested by warp 0, once the previous item's Q
-    // has been moved on.  A parity test of slot_free answers for the slot's latest entry only if the
-    // warp knows that the one before it is dead, which it does when it filled the latest entry itself.
-    // The other warps have not: for them a slot that last held Q is free once that item's q_taken says
-    // so.  (Stepping over the Q entries and testing slot_free behind them let items of one or two blocks
-    // copy K over a block whose PV was pending.)  Two q_taken barriers are enough: the item after the
-    // next cannot have its Q moved before this warp has copied the next one's K.
-    // q_held: four bits per slot -- 1: Q was its last entry, 2: that item's ordinal % 2, 4: its phase.
-    int q_w = cid, q_slot = 0, q_ring = 0, q_left = pw == 0 && cid < n_items ? kQEntries : 0;
-    int q_n = 0;                                   // items whose Q has been requested
-    uint32_t q_held = 0x11u;                       // the first item's Q entries: slots 0 and 1
-    int k_it = 0;                                  // item ordinal of the K cursor
-    static_assert(kQEntries == 2 && kSlots <= 8, "q_held layout");
-    auto cur_load = [&](Cursor& c) {
-      c.nb = 0;
-      if (c.w < n_items) {
-        const Item t = item_of(c.w);
-        c.nb = t.nb; c.k = 0; c.k0 = t.k0; c.len = t.len0;
-        c.idx = p.indices + (size_t)t.tile * p.idx_stride;
-      }
-    };
-    auto advance = [&](Cursor& c) { if (++c.slot == kSlots) { c.slot = 0; ++c.ring; } };
-    auto cur_next = [&](Cursor& c) {
-      ++c.kb;
-      advance(c);
-      if (++c.k == c.nb) { c.w += ncl; cur_load(c); return true; }     // the next item's Q entries are next
-      return false;
-    };
-    Cursor ck, cv;
-    ck.w = cv.w = cid;
-    ck.kb = cv.kb = 0;
-    ck.slot = cv.slot = kQEntries;                 // behind the first item's Q
-    ck.ring = cv.ring = 0;
-    cur_load(ck);
-    cur_load(cv);
-    // lane l holds the index of key 4 pw + l % 4 of the CTA's own (K) / the peer's (V) 32 keys; loaded
-    // one block ahead, first looked at when that block's copies go out
-    const int key_l = 4 * pw + (lane & 3);
-    auto load_idx = [&](const Cursor& c, int half) -> int {
-      const int pos = (c.k0 + c.k) * kBlockKeys + kOwnKeys * half + key_l;
-      return pos < c.len ? __ldcs(c.idx + pos) : 0;
-    };
-    auto in_range = [&](int v) -> int { return ((unsigned)v < (unsigned)p.s_kv) ? v : 0; };   // masked later
-    int kidx = 0, vidx = 0;
-    if (ck.w < n_items) { kidx = load_idx(ck, (int)cta); vidx = load_idx(cv, (int)cta ^ 1); }
+    // 16-byte copies written straight into the 128-byte-swizzled layout, completion reported to an mbarrier by an
+    // asynchronous arrival.  Four warps fetch K rows (this CTA's 32 keys, all dims: warp pw rows [8 pw, 8 pw + 8)) as
+    // soon as the slot's previous entry is dead, the other four V rows (the PEER's 32 keys, this CTA's 256
+    // value dims) into the dead half of the slot as soon as the block's QK^T is complete.  (Eight warps that polled
+    // for both in turn were late for either: see attn_fp8.cu.  They kept in q_held which slots had last held
+    // a Q.)  Entries without a valid index become zeros without a read.
+    const int pw = (warp - kWarpGather0) & 3;
+    const bool is_k = warp < kWarpGather0 + kGatherWarps / 2;
     const uint8_t* kvb = p.kv;
     const long long pitch = p.kv_pitch;
     const int cj = lane >> 3, cc = lane & 7;       // piece `lane` of 32: chunk cj, 16-byte unit cc
-    unsigned long long idle_since = 0;
-    unsigned idle_iters = 0;
-    bool aborted = false;
-    while (cv.w < n_items && !aborted) {           // the V cursor never runs ahead of the K cursor
-      bool did = false;
-      {
-        const bool ok = cv.kb < ck.kb && mbar_test(&ms.qk_done[cv.kb & 7], (cv.kb >> 3) & 1);
-        if (__all_sync(0xffffffffu, ok)) {
-          const int vcur = in_range(vidx);
-          const uint32_t vst = sbase + PL::kOffKV + cv.slot * PL::kSlot + ((cta == 0 ? 4 : 0) + cj) * kChunkBytes;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int ri = __shfl_sync(0xffffffffu, vcur, i);
-            const int row = 4 * pw + i;
-            cp_async16(vst + row * 128 + ((cc ^ (row & 7)) << 4), kvb + (size_t)ri * pitch + 512 * (int)cta + 16 * lane);
-          }
-          cp_async_mbar_arrive_noinc(&ms.v_full[cv.kb & 7]);
-          if (cur_next(cv)) { advance(cv); advance(cv); }
-          if (cv.w < n_items) vidx = load_idx(cv, (int)cta ^ 1);
-          did = true;
-        }
-      }
-      if (q_left > 0) {                            // warp-uniform; warp 0 only
-        const bool ok = (q_ring == 0 || mbar_test(&ms.slot_free[q_slot], (q_ring - 1) & 1)) &&
-                        (q_n == 0 || mbar_test(&ms.q_taken[(q_n - 1) & 1], ((q_n - 1) >> 1) & 1));
-        if (__all_sync(0xffffffffu, ok)) {
-          if (lane == 0) request_q(q_w, kQEntries - q_left, q_slot);
+    // lane l holds the index of key 8 pw + l % 8 of the CTA's own (K) / the peer's (V) 32 keys, -1 if it has none;
+    // loaded one block ahead
+    const int key = kOwnKeys * ((int)cta ^ (is_k ? 0 : 1)) + 8 * pw + (lane & 7);
+    auto load_idx = [&](const Item& t, int k) -> int {
+      const int pos = (t.k0 + k) * kBlockKeys + key;
+      return pos < t.len0 ? __ldcs(p.indices + (size_t)t.tile * p.idx_stride + pos) : -1;
+    };
+    Item nx = item_of(min(cid, n_items - 1));
+    int idx = load_idx(nx, 0);
+    int slot = 0, ring = 0, kb = 0, it = 0;        // ring entry = kSlots ring + slot
+    auto advance = [&]() { if (++slot == kSlots) { slot = 0; ++ring; } };
+    // the block's index, with the next block's (of the next item behind the last) on its way
+    auto take_idx = [&](const Item& t, int k, int w) -> int {
+      const int cur = (unsigned)idx < (unsigned)p.s_kv ? idx : -1;
+      if (k + 1 < t.nb) idx = load_idx(t, k + 1);
+      else if (w + ncl < n_items) idx = load_idx(nx, 0);
+      return cur;
+    };
+    if (is_k) {
+      for (int w = cid; w < n_items; w += ncl, ++it) {
+        const Item t = nx;
+        if (w + ncl < n_items) nx = item_of(w + ncl);
+        // The item's Q entries, requested by warp 0.  Every warp goes through their slots' barriers and that of the
+        // previous Q (whose bytes could, with short items, still be in flight), and Q counts as landed only when
+        // all of them have: no warp is overtaken and tests a phase that is two ahead.
+        if (it > 0) mbar_wait(&ms.q_taken[(it - 1) & 1], ((it - 1) >> 1) & 1, wt, kSiteQ, it);
+        for (int e = 0; e < kQEntries; ++e) {
+          if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
           __syncwarp();
-          if (++q_slot == kSlots) { q_slot = 0; ++q_ring; }
-          if (--q_left == 0) ++q_n;
-          did = true;
+          if (pw == 0 && lane == 0) request_q(w, e, slot);
+          __syncwarp();
+          advance();
         }
-      }
-      if (ck.w < n_items && q_left == 0) {
-        const uint32_t held = q_held >> (4 * ck.slot);
-        const bool ok = (held & 1u) ? mbar_test(&ms.q_taken[(held >> 1) & 1u], (held >> 2) & 1u)
-                                    : (ck.ring == 0 || mbar_test(&ms.slot_free[ck.slot], (ck.ring - 1) & 1));
-        if (__all_sync(0xffffffffu, ok)) {
-          q_held &= ~(15u << (4 * ck.slot));
-          const int kcur = in_range(kidx);
-          const uint32_t kst = sbase + PL::kOffKV + ck.slot * PL::kSlot;
+        if (pw != 0 && lane == 0) mbar_arrive(&ms.q_land);
+        for (int k = 0; k < t.nb; ++k, ++kb) {
+          const int cur = take_idx(t, k, w);
+          const bool full = __all_sync(0xffffffffu, cur >= 0);
+          if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
+          __syncwarp();
+          const uint32_t kst = sbase + PL::kOffKV + slot * PL::kSlot + 8 * pw * 128;
+          if (full) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {            // 1024 latent bytes per row: two instructions
-            const int ri = __shfl_sync(0xffffffffu, kcur, i >> 1);
-            const int row = 4 * pw + (i >> 1);
-            cp_async16(kst + (4 * (i & 1) + cj) * kChunkBytes + row * 128 + ((cc ^ (row & 7)) << 4),
-                       kvb + (size_t)ri * pitch + 512 * (i & 1) + 16 * lane);
-          }
-          if (kD == 576) {                         // 128 rope bytes: four rows in one instruction
-            const int ri = __shfl_sync(0xffffffffu, kcur, cj);
-            const int row = 4 * pw + cj;
-            cp_async16(kst + 8 * kChunkBytes + row * 128 + ((cc ^ (row & 7)) << 4),
-                       kvb + (size_t)ri * pitch + 1024 + 16 * cc);
-          }
-          cp_async_mbar_arrive_noinc(&ms.k_full[ck.kb & 7]);
-          if (cur_next(ck)) {
-            if (pw == 0 && ck.w < n_items) { q_w = ck.w; q_slot = ck.slot; q_ring = ck.ring; q_left = kQEntries; }
-            ++k_it;
-            for (int e = 0; e < kQEntries; ++e) {
-              q_held = (q_held & ~(15u << (4 * ck.slot))) | ((1u | (uint32_t)(k_it & 3) << 1) << (4 * ck.slot));
-              advance(ck);
+            for (int i = 0; i < 16; ++i) {         // 1024 latent bytes per row: two instructions
+              const int ri = __shfl_sync(0xffffffffu, cur, i >> 1);
+              cp_async16(kst + (4 * (i & 1) + cj) * kChunkBytes + (i >> 1) * 128 + ((cc ^ (i >> 1)) << 4),
+                         kvb + (size_t)ri * pitch + 512 * (i & 1) + 16 * lane);
+            }
+          } else {
+#pragma unroll 1
+            for (int i = 0; i < 16; ++i) {
+              const int ri = __shfl_sync(0xffffffffu, cur, i >> 1);
+              cp_async16_or_zero(kst + (4 * (i & 1) + cj) * kChunkBytes + (i >> 1) * 128 + ((cc ^ (i >> 1)) << 4),
+                                 kvb + (size_t)max(ri, 0) * pitch + 512 * (i & 1) + 16 * lane, ri >= 0);
             }
           }
-          if (ck.w < n_items) kidx = load_idx(ck, (int)cta);
-          did = true;
+          if (kD == 576) {                         // 128 rope bytes: four rows in one instruction
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int rw = 4 * i + cj, ri = __shfl_sync(0xffffffffu, cur, rw);
+              cp_async16_or_zero(kst + 8 * kChunkBytes + rw * 128 + ((cc ^ rw) << 4),
+                                 kvb + (size_t)max(ri, 0) * pitch + 1024 + 16 * cc, ri >= 0);
+            }
+          }
+          cp_async_mbar_arrive_noinc(&ms.k_full[kb & 7]);
+          advance();
         }
       }
-      if (did) {
-        idle_since = 0;
-        idle_iters = 0;
-      } else if ((++idle_iters & 63u) != 0) {
-        __nanosleep(8);
-      } else {
-        const unsigned long long now = globaltimer_ns();
-        if (idle_since == 0) idle_since = now;
-        bool stop = wt.aborting();
-        if (now - idle_since > wt.limit_ns) {
-          if (lane == 0) wt.fail(kSiteKFree, ck.k);
-          stop = true;
+    } else {
+      const uint8_t* src = kvb + 512 * (int)cta + 16 * lane;
+      for (int w = cid; w < n_items; w += ncl) {
+        const Item t = nx;
+        if (w + ncl < n_items) nx = item_of(w + ncl);
+        for (int e = 0; e < kQEntries; ++e) advance();
+        for (int k = 0; k < t.nb; ++k, ++kb) {
+          const int cur = take_idx(t, k, w);
+          mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, k);
+          __syncwarp();
+          const uint32_t vst = sbase + PL::kOffKV + slot * PL::kSlot + ((cta == 0 ? 4 : 0) + cj) * kChunkBytes + 8 * pw * 128;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int ri = __shfl_sync(0xffffffffu, cur, i);
+            cp_async16_or_zero(vst + i * 128 + ((cc ^ i) << 4), src + (size_t)max(ri, 0) * pitch, ri >= 0);
+          }
+          cp_async_mbar_arrive_noinc(&ms.v_full[kb & 7]);
+          advance();
         }
-        aborted = __any_sync(0xffffffffu, stop);
       }
     }
   }

@@ -1,7 +1,8 @@
-"""The barrier protocol of the 64-row FP8 attention kernel (attn_fp8_r64.cuh), run on the CPU in random orders.
+"""The barrier protocols of the gathering attention kernels (attn_fp8_r64.cuh, attn_fp8.cu, mla_bf16.cuh), run on the CPU
+in random orders.
 
-Its warps wait on mbarriers by parity, which answers for the right phase only while a waiter is at most
-one phase behind and every arrival falls into the phase it is meant for.  One CTA is a set of agents --
+Their warps wait on mbarriers by parity, which answers for the right phase only while a waiter is at most
+one phase behind and every arrival falls into the phase it is meant for.  A CTA, or a pair, is a set of agents --
 gather sets, copies in flight, QK^T and PV issue, MMAs in flight, softmax groups, validity bits, epilogue --
 whose steps are taken in orders with random and changing priorities (an agent can be held up for
 as long as any other can go on); every wait and every arrival is checked against the phase it means."""
@@ -11,11 +12,12 @@ from pathlib import Path
 
 import pytest
 
-SRC = (Path(__file__).resolve().parents[1] / "litetopk_b200" / "csrc" / "attn_fp8_r64.cuh").read_text()
+CSRC = Path(__file__).resolve().parents[1] / "litetopk_b200" / "csrc"
+SRC, SRC_PAIR, SRC_BF16 = ((CSRC / f).read_text() for f in ("attn_fp8_r64.cuh", "attn_fp8.cu", "mla_bf16.cuh"))
 
 
-def _const(name):
-    return int(re.search(r"\b%s = (\d+)" % name, SRC).group(1))
+def _const(name, src=SRC):
+    return int(re.search(r"\b%s = (\d+)" % name, src).group(1))
 
 
 def _agents(blocks, bf16_q, rescale):
@@ -143,6 +145,129 @@ def _agents(blocks, bf16_q, rescale):
     return a, need
 
 
+def _pair_agents(blocks, bf16_q, rescale, src=SRC_PAIR, q_entries=1, q_depth=1):
+    """The same for the two CTAs that share a 128-row tile; names and barriers end in their CTA ("L": the leader's)."""
+    slots = _const("kSlots", src)
+    for name, n in (("k_peer", 8), ("v_peer", 8), ("qk_done", 8), ("pv_done", 4), ("s_free", 2), ("p_ready", 2), ("epi_ready", 2)):
+        assert re.search(r"uint64_t [^;]*\b%s\[%d\]" % (name, n), src), name
+    a, need = {}, {}
+
+    def do(agent, kind, what, phase=0):
+        a.setdefault(agent, []).append((kind, what, phase))
+
+    def ar(agent, bar, phase, n=1):
+        need[bar] = n
+        do(agent, "arrive", bar, phase)
+
+    def async_ar(agent, other, bar, phase, n=1):       # started by `agent`, arrives some time later, in order
+        do(agent, "issue", other)
+        do(other, "after", other)
+        ar(other, bar, phase, n)
+
+    def wait(agent, bar, phase):
+        do(agent, "wait", bar, phase)
+
+    e = kb0 = 0
+    q_entry = []
+    for it, nb in enumerate(blocks):
+        q_entry.append(e)
+        for c in (0, 1):
+            for w in (0, 1):
+                g = f"k{w}{c}"
+                if it > 0:
+                    wait(g, f"q_taken{(it - 1) % q_depth}{c}", (it - 1) // q_depth)
+                for x in range(e, e + q_entries):
+                    if x >= slots:
+                        wait(g, f"slot_free{x % slots}{c}", x // slots - 1)
+                    if w == 0:
+                        async_ar(g, f"qland{w}{c}", f"q_land{c}", it, q_entries + 1)
+                if w == 1:
+                    async_ar(g, f"qland{w}{c}", f"q_land{c}", it, q_entries + 1)
+                for k in range(nb):
+                    x, kb = e + q_entries + k, kb0 + k
+                    if x >= slots:
+                        wait(g, f"slot_free{x % slots}{c}", x // slots - 1)
+                    async_ar(g, f"kland{w}{c}", f"k_land{kb & 7}{c}", kb >> 3, 2)
+                    wait(f"v{w}{c}", f"qk_done{kb & 7}{c}", kb >> 3)
+                    async_ar(f"v{w}{c}", f"vland{w}{c}", f"v_land{kb & 7}{c}", kb >> 3, 2)
+        for k in range(nb):
+            kb, x = kb0 + k, e + q_entries + k
+            for what in "kv":                         # the peer's relays
+                wait(f"r{what}", f"{what}_land{kb & 7}1", kb >> 3)
+                ar(f"r{what}", f"{what}_peer{kb & 7}L", kb >> 3)
+            if k == 0:
+                wait("qk", "qt_readyL", it)
+            wait("qk", f"k_land{kb & 7}0", kb >> 3)
+            wait("qk", f"k_peer{kb & 7}L", kb >> 3)
+            if kb >= 2:
+                wait("qk", f"s_free{kb & 1}L", (kb >> 1) - 1)
+            for c in (0, 1):
+                async_ar("qk", "qkp", f"qk_done{kb & 7}{c}", kb >> 3)
+            if k == nb - 1:
+                for c in (0, 1):
+                    async_ar("qk", "qkp", f"q_free{c}", it)
+            wait("pv", f"v_land{kb & 7}0", kb >> 3)
+            wait("pv", f"v_peer{kb & 7}L", kb >> 3)
+            if k == 0 and it > 0:
+                wait("pv", "o_freeL", it - 1)
+            wait("pv", f"p_ready{kb & 1}L", kb >> 1)
+            for c in (0, 1):
+                async_ar("pv", "pvp", f"slot_free{x % slots}{c}", x // slots)
+                async_ar("pv", "pvp", f"pv_done{kb & 3}{c}", kb >> 2)
+            g = kb & 1
+            for c in (0, 1):
+                if kb >= 2:
+                    wait(f"valid{c}", f"valid_free{g}{c}", (kb >> 1) - 1)
+                ar(f"valid{c}", f"valid_ready{g}{c}", kb >> 1)
+                for w in (0, 1):
+                    s = f"s{g}{w}{c}"
+                    wait(s, f"qk_done{kb & 7}{c}", kb >> 3)
+                    ar(s, f"s_free{g}L", kb >> 1, 4)
+                    wait(s, f"valid_ready{g}{c}", kb >> 1)
+                    ar(s, f"valid_free{g}{c}", kb >> 1, 2)
+                    ar(s, f"group{g}{c}", kb >> 1, 2)
+                    wait(s, f"group{g}{c}", kb >> 1)
+                    if k > 0:
+                        wait(s, f"m_pub{g ^ 1}{c}", (kb - 1) >> 1)
+                    ar(s, f"m_pub{g}{c}", kb >> 1, 2)
+                    if kb >= 2:
+                        wait(s, f"pv_done{(kb - 2) & 3}{c}", (kb - 2) >> 2)
+                    if rescale and k > 0:
+                        wait(s, f"pv_done{(kb - 1) & 3}{c}", (kb - 1) >> 2)
+                    ar(s, f"p_ready{g}L", kb >> 1, 4)
+        for c in (0, 1):
+            for s in (f"s{g}{w}{c}" for g in (0, 1) for w in (0, 1)):
+                if it > 0:
+                    wait(s, f"epi_ready{(it - 1) & 1}{c}", (it - 1) >> 1)
+                ar(s, f"end{c}", it, 4)
+                wait(s, f"end{c}", it)
+                ar(s, f"epi_ready{it & 1}{c}", it >> 1, 4)
+        e += nb + q_entries
+        kb0 += nb
+    for c in (0, 1):
+        last, epi = -1, f"epi{c}"
+        for it in range(-1, len(blocks)):
+            if it + 1 < len(blocks):
+                order = [(f"q_land{c}", it + 1), (f"q_free{c}", it)]
+                for bar, phase in order if bf16_q else order[::-1]:
+                    if phase >= 0:
+                        wait(epi, bar, phase)
+                ar(epi, "qt_readyL", it + 1, 2)
+                for x in range(q_entry[it + 1], q_entry[it + 1] + q_entries):
+                    ar(epi, f"slot_free{x % slots}{c}", x // slots)
+                ar(epi, f"q_taken{(it + 1) % q_depth}{c}", (it + 1) // q_depth)
+            if it >= 0:
+                last += blocks[it]
+                wait(epi, f"epi_ready{it & 1}{c}", it >> 1)
+                wait(epi, f"pv_done{last & 3}{c}", last >> 2)
+                ar(epi, "o_freeL", it, 2)
+    return a, need
+
+
+def _bf16_agents(blocks, bf16_q, rescale):
+    return _pair_agents(blocks, bf16_q, rescale, SRC_BF16, _const("kQEntries", SRC_BF16), 2)
+
+
 def _run(agents, need, rng):
     """One random order; returns what went wrong, or None."""
     pos, issued, done = dict.fromkeys(agents, 0), dict.fromkeys(agents, 0), dict.fromkeys(agents, 0)
@@ -184,10 +309,11 @@ def _run(agents, need, rng):
 
 @pytest.mark.parametrize("bf16_q", [False, True])
 @pytest.mark.parametrize("rescale", [False, True])
-def test_no_order_of_the_warps_breaks_a_phase(bf16_q, rescale):
+@pytest.mark.parametrize("agents", [_agents, _pair_agents, _bf16_agents])
+def test_no_order_of_the_warps_breaks_a_phase(agents, bf16_q, rescale):
     rng = random.Random(64 + 2 * bf16_q + rescale)
-    for n in range(150):
+    for n in range(100):
         most = rng.choice([1, 2, 3, 9])
         blocks = [rng.randint(1, most) for _ in range(rng.randint(3, 9))]
-        fault = _run(*_agents(blocks, bf16_q, rescale), rng)
+        fault = _run(*agents(blocks, bf16_q, rescale), rng)
         assert fault is None, (blocks, fault)
