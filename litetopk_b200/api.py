@@ -13,6 +13,7 @@ There is no CPU path: tensors must live on a CUDA device.
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -42,6 +43,21 @@ def _on_device(dev: torch.device, fn, *args) -> int:
         return fn(*args, _raw_stream(index))
     with torch.cuda.device(index):
         return fn(*args, _raw_stream(index))
+
+
+def _empty(shape: tuple, dtype, dev: torch.device) -> torch.Tensor:
+    """torch.empty of a contiguous CUDA tensor, by way of empty_strided: 1.6 instead of 2.4 us of host time."""
+    strides = (1,)
+    for n in shape[:0:-1]:
+        strides = (strides[0] * max(n, 1),) + strides
+    return torch.empty_strided(shape, strides, dtype=dtype, device=dev)
+
+
+@functools.lru_cache(maxsize=1024)
+def _workspace_bytes(name: str, index: int, *shape: int) -> int:
+    """What the library's workspace function ``name`` says for these sizes on device ``index``."""
+    with torch.cuda.device(index):
+        return getattr(_lib.lib(), name)(*shape)
 
 
 def _need(t: torch.Tensor, name: str, dtype, ndim: Optional[int] = None) -> None:
@@ -475,14 +491,12 @@ def index_logits_fp8(q_idx8: torch.Tensor, k_idx8: torch.Tensor, weights: torch.
         if k_scale.numel() != S or not k_scale.is_contiguous():
             raise ValueError("k_scale must be a contiguous [S] tensor")
     if out is None:
-        out = torch.empty((T, S), dtype=torch.float32, device=q_idx8.device)
+        out = _empty((T, S), torch.float32, q_idx8.device)
     _need(out, "out", torch.float32, 2)
     if out.shape[0] != T or out.shape[1] < S or out.stride(1) != 1:
         raise ValueError("out must be [T, >= S] fp32 with unit inner stride")
-    with torch.cuda.device(q_idx8.device):
-        check(_lib.lib().litedsa_index_logits_fp8(_ptr(q_idx8), _ptr(k_idx8), _ptr(weights), _ptr(k_scale),
-                                                  _ptr(out), T, Hi, S, int(q_pos0), k_idx8.stride(0),
-                                                  out.stride(0), _stream(q_idx8)), "index_logits_fp8")
+    check(_on_device(q_idx8.device, _lib.lib().litedsa_index_logits_fp8, _ptr(q_idx8), _ptr(k_idx8), _ptr(weights),
+                     _ptr(k_scale), _ptr(out), T, Hi, S, int(q_pos0), k_idx8.stride(0), out.stride(0)), "index_logits_fp8")
     return out
 
 
@@ -502,13 +516,12 @@ def topk_select(logits: torch.Tensor, k: int, *, q_pos0: int = 0, lengths: Optio
         if lengths.numel() != T or not lengths.is_contiguous():
             raise ValueError("lengths must be a contiguous [T] int32 tensor")
     if out is None:
-        out = torch.empty((T, int(k)), dtype=torch.int32, device=logits.device)
+        out = _empty((T, int(k)), torch.int32, logits.device)
     _need(out, "out", torch.int32, 2)
     if tuple(out.shape) != (T, int(k)) or not out.is_contiguous():
         raise ValueError("out must be a contiguous [T, k] int32 tensor")
-    with torch.cuda.device(logits.device):
-        check(_lib.lib().litedsa_topk_select(_ptr(logits), _ptr(lengths), _ptr(out), T, S, int(k),
-                                             int(q_pos0), logits.stride(0), _stream(logits)), "topk_select")
+    check(_on_device(logits.device, _lib.lib().litedsa_topk_select, _ptr(logits), _ptr(lengths), _ptr(out), T, S, int(k),
+                     int(q_pos0), logits.stride(0)), "topk_select")
     return out
 
 
@@ -520,8 +533,7 @@ def lite_topk(q_idx8: torch.Tensor, k_idx8: torch.Tensor, weights: torch.Tensor,
     S = k_idx8.shape[0]
     if logits_workspace is None:
         # rows start on 16-byte boundaries whatever S is: the streaming selection kernels need that
-        logits_workspace = torch.empty((q_idx8.shape[0], (S + 3) // 4 * 4), dtype=torch.float32,
-                                       device=q_idx8.device)
+        logits_workspace = _empty((q_idx8.shape[0], (S + 3) // 4 * 4), torch.float32, q_idx8.device)
     logits = index_logits_fp8(q_idx8, k_idx8, weights, k_scale, q_pos0, out=logits_workspace)
     # a workspace wider than S: select over the first S columns of every row
     view = logits if logits.shape[1] == S else logits.as_strided((logits.shape[0], S), (logits.stride(0), 1))
@@ -829,14 +841,14 @@ def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_spac
     if q_bf16 and not kv_bf16 and _quantise_first(T * h // 128, 128 // h, 128 // h * k):
         q, q_bf16 = quantize_e4m3(q, q_scale), False
     if out is None:
-        out = torch.empty((T, h, 512), dtype=torch.bfloat16, device=dev)
+        out = _empty((T, h, 512), torch.bfloat16, dev)
     else:
         _need(out, "out", torch.bfloat16)
         if out.numel() != T * h * 512 or not out.is_contiguous():
             raise ValueError("out must be a contiguous [T,h,512] bf16 tensor")
         out = out.view(T, h, 512)
     if lse is None:
-        lse = torch.empty((T, h), dtype=torch.float32, device=dev)
+        lse = _empty((T, h), torch.float32, dev)
     else:
         _need(lse, "lse", torch.float32)
         if lse.numel() != T * h or not lse.is_contiguous():
@@ -844,9 +856,9 @@ def _sparse_prefill(q, kv_cache, topk_idx, sm_scale, kv_scale, q_scale, seq_spac
         lse = lse.view(T, h)
     lib = _lib.lib()
     space = kv_cache.shape[0] if seq_space is None else int(seq_space)
-    fn, size = (lib.litedsa_sparse_prefill_job, lib.litedsa_sparse_prefill_job_workspace) if by_job else \
-        (lib.litedsa_sparse_prefill, lib.litedsa_sparse_prefill_workspace)
-    ws = torch.empty((max(size(T, h, k, kv_bf16, job_tokens), 1),), dtype=torch.uint8, device=dev)
+    fn, size = (lib.litedsa_sparse_prefill_job, "litedsa_sparse_prefill_job_workspace") if by_job else \
+        (lib.litedsa_sparse_prefill, "litedsa_sparse_prefill_workspace")
+    ws = _empty((max(_workspace_bytes(size, dev.index, T, h, k, kv_bf16, job_tokens), 1),), torch.uint8, dev)
     check(_on_device(dev, fn, q.data_ptr(), q_bf16, kv.data_ptr(), kv_bf16, topk_idx.data_ptr(), float(sm_scale),
                      float(q_scale), float(kv_scale), out.data_ptr(), lse.data_ptr(), T, h, k, kv.shape[0], kv.stride(0),
                      (space + 1023) // 1024 * 1024, job_tokens, ws.data_ptr(), ws.numel()), "sparse_prefill")
@@ -1031,11 +1043,11 @@ def dsv4_c128a_bf16(q: torch.Tensor, kv_compressed: Optional[torch.Tensor], kv_r
         if out.shape[0] != T or out.shape[1] < h or out.shape[2] != 512 or out.stride(2) != 1:
             raise ValueError("out must be [T, H_padded >= heads, 512] with unit inner stride")
     else:
-        out = torch.empty((T, h, 512), dtype=torch.bfloat16, device=q.device)
-    lse = torch.empty((ng, 128), dtype=torch.float32, device=q.device)
+        out = _empty((T, h, 512), torch.bfloat16, q.device)
+    lse = _empty((ng, 128), torch.float32, q.device)
     lib = _lib.lib()
     ws_bytes = lib.litedsa_dsv4_workspace(ng, h, n_comp, int(q_pos0), int(window), int(ratio))
-    ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=q.device) if ws_bytes > 0 else None
+    ws = _empty((ws_bytes,), torch.uint8, q.device) if ws_bytes > 0 else None
     check(_on_device(q.device, lib.litedsa_dsv4_c128a_bf16_ws, q.data_ptr(),
                      kv_compressed.data_ptr() if n_comp else None, kv_raw.data_ptr(), ng, h, n_comp,
                      kv_raw.shape[0], int(q_pos0), int(window), int(ratio), sm_scale, _ptr(sink), h,
