@@ -133,6 +133,9 @@ __device__ __forceinline__ void commit_elect(uint64_t* bar) {
       "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
       ::"r"(smem_u32(bar)) : "memory");
 }
+// kWide: the cache is too large for row offsets in 32 bits of 16-byte units (64 GB); their products in 64 bits take 1 %
+// of the time (8192 tokens x 64 heads 1271 -> 1295 us)
+template <bool kWide>
 __global__ void __launch_bounds__(kThreads, 1)
 masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_rope,
                           const __grid_constant__ CUtensorMap map_out, const Params p) {
@@ -354,6 +357,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     static_assert(kSlots % 2 == 0, "two sets of gather warps");
     const int set = (warp - kWarpGather0) >> 2, pw = (warp - kWarpGather0) & 3;
     const uint64_t pol_stream = l2_policy_evict_first();
+    const size_t unit = kWide ? (size_t)p.kv_pitch : 16;
     const uint32_t pitch16 = (uint32_t)(p.kv_pitch >> 4);
     const int cj = lane >> 3, cc = lane & 7;       // latent piece `lane`: chunk cj, 16-byte slot cc
     const uint8_t* kv_lat = p.kv + 16 * lane;
@@ -395,10 +399,10 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       int k = first_k(e);
       if (k >= nb) kidx = next_tile_idx();
       for (; k < nb; k += 2) {
-        // this lane's row as an offset in 16-byte units; entries without a key become zeros.  (Indices are
-        // loaded a block ahead: nothing waits for a cold line.)
+        // this lane's row as an offset in 16-byte units (kWide: in rows); entries without a key become zeros.
+        // (Indices are loaded a block ahead: nothing waits for a cold line.)
         const bool has = (unsigned)kidx < (unsigned)p.s_kv;
-        const uint32_t off = has ? (uint32_t)kidx * pitch16 : 0xffffffffu;
+        const uint32_t row = has ? (kWide ? (uint32_t)kidx : (uint32_t)kidx * pitch16) : 0xffffffffu;
         const bool full = __all_sync(0xffffffffu, has);
         kidx = k + 2 < nb ? __ldcs(idx + (k + 2) * kBlockKeys) : next_tile_idx();
         if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
@@ -410,26 +414,26 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         if (full) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const uint32_t o = __shfl_sync(0xffffffffu, off, i);
-            cp_async16(kdst + i * 128 + ((cc ^ (i & 7)) << 4), kv_lat + (size_t)o * 16);
+            const uint32_t o = __shfl_sync(0xffffffffu, row, i);
+            cp_async16(kdst + i * 128 + ((cc ^ (i & 7)) << 4), kv_lat + (size_t)o * unit);
           }
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            const uint32_t o = __shfl_sync(0xffffffffu, off, 8 * i + (lane >> 2));
-            cp_async16(rdst + i * 512, kv_rope + (size_t)o * 16);
+            const uint32_t o = __shfl_sync(0xffffffffu, row, 8 * i + (lane >> 2));
+            cp_async16(rdst + i * 512, kv_rope + (size_t)o * unit);
           }
         } else {
 #pragma unroll 1
           for (int i = 0; i < 16; ++i) {
-            const uint32_t o = __shfl_sync(0xffffffffu, off, i);
+            const uint32_t o = __shfl_sync(0xffffffffu, row, i);
             const bool rd = o != 0xffffffffu;
-            cp_async16_or_zero(kdst + i * 128 + ((cc ^ (i & 7)) << 4), rd ? kv_lat + (size_t)o * 16 : p.kv, rd);
+            cp_async16_or_zero(kdst + i * 128 + ((cc ^ (i & 7)) << 4), rd ? kv_lat + (size_t)o * unit : p.kv, rd);
           }
 #pragma unroll 1
           for (int i = 0; i < 2; ++i) {
-            const uint32_t o = __shfl_sync(0xffffffffu, off, 8 * i + (lane >> 2));
+            const uint32_t o = __shfl_sync(0xffffffffu, row, 8 * i + (lane >> 2));
             const bool rd = o != 0xffffffffu;
-            cp_async16_or_zero(rdst + i * 512, rd ? kv_rope + (size_t)o * 16 : p.kv, rd);
+            cp_async16_or_zero(rdst + i * 512, rd ? kv_rope + (size_t)o * unit : p.kv, rd);
           }
         }
         cp_async_mbar_arrive_noinc(&ms.k_land[(e - it + k) & 7]);      // e - it: running number of the item's first block
@@ -735,9 +739,7 @@ int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
   if (a.h_per_q == r64::kRows) c.memb_qm = reinterpret_cast<const uint32_t*>(a.indices);      // none there, and none read
   const int rc = check_fp8_args(c);
   if (rc != LITEDSA_OK) return rc;
-  // (row offsets are held in 32 bits of 16-byte units)
-  if (a.h_per_q > r64::kRows || a.topk < 256 || ((uintptr_t)out & 15) || (int64_t)a.s_kv * (a.kv_row_stride >> 4) >= 0xffffffffll)
-    return LITEDSA_ERR_UNSUPPORTED;
+  if (a.h_per_q > r64::kRows || a.topk < 256 || ((uintptr_t)out & 15)) return LITEDSA_ERR_UNSUPPORTED;
   CUtensorMap map_q, map_q_rope, map_out;
   const int h = a.h_per_q, G = r64::kRows / h;
   const uint64_t tokens = (uint64_t)a.ng * G;
@@ -763,9 +765,13 @@ int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
   p.q_bf16 = a.q_is_bf16 ? reinterpret_cast<const uint4*>(a.q8) : nullptr; p.q_inv = a.q_inv;
   p.q_codes = reinterpret_cast<uint8_t*>(q_codes);
-  if (!ensure_smem<r64::masked_mla_fp8_r64_kernel>(current_device(), r64::Plan::kSmem)) return LITEDSA_ERR_CUDA;
-  return launch_pdl(r64::masked_mla_fp8_r64_kernel, dim3((unsigned)ncta), r64::kThreads, r64::Plan::kSmem,
-                    reinterpret_cast<cudaStream_t>(stream), map_q, map_q_rope, map_out, p);
+  const bool wide = (int64_t)a.s_kv * (a.kv_row_stride >> 4) >= 0xffffffffll;
+  const int dev = current_device();
+  if (!(wide ? ensure_smem<r64::masked_mla_fp8_r64_kernel<true>>(dev, r64::Plan::kSmem)
+             : ensure_smem<r64::masked_mla_fp8_r64_kernel<false>>(dev, r64::Plan::kSmem)))
+    return LITEDSA_ERR_CUDA;
+  return launch_pdl(wide ? r64::masked_mla_fp8_r64_kernel<true> : r64::masked_mla_fp8_r64_kernel<false>, dim3((unsigned)ncta),
+                    r64::kThreads, r64::Plan::kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_q_rope, map_out, p);
 }
 
 }  // namespace lt
