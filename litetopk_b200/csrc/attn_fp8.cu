@@ -28,7 +28,7 @@
 //                   32 S columns per thread: short chains, and eight warps per scheduler to hide
 //                   them);
 //       warps 16-23 KV row gather with 16-byte cp.async copies written straight into the
-//                   128-byte-swizzled tile layout;
+//                   128-byte-swizzled tile layout: K rows (16-19), the peer's value halves (20-23);
 //       warp 24     QK^T issue (leader CTA; whole warp polls, one elected lane issues);
 //       warps 25-26 in the peer CTA: relay "K / V landed" to the leader's barriers; in the leader
 //                   warp 25 issues PV;
@@ -490,8 +490,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
     // The union rows are fetched with 16-byte cp.async copies issued by all 256 threads of
     // these eight warps: fire-and-forget, any number of blocks in flight, destination written
     // directly in the 128-byte-swizzled tile layout, completion reported to an mbarrier by an
-    // asynchronous arrival.  (TMA gather4 was measured at one instruction per ~8.5 ns per SM,
-    // i.e. the same ~60 GB/s per SM that the L2 -> SM path gives these copies.)
+    // asynchronous arrival.  (These copies alone reach 17-20 TB/s from L2; TMA gather4 takes one request
+    // of 512 bytes per ~8.5 ns and SM, half of that.)
     // Four warps fetch K rows (this CTA's 64 keys, all 576 bytes: warp pw rows [16 pw, 16 pw + 16), 18 copies
     // per lane) as soon as the slot's previous entry is dead, the other four V rows (the PEER's 64 keys,
     // this CTA's 256 value bytes, eight copies per lane) into the dead half of the slot as soon as the block's QK^T

@@ -22,6 +22,10 @@
 //     warps 24, 27 QK^T issue, even and odd blocks;   warp 25  PV issue;   warp 26  index-validity bits;
 //     warps 28-31  Q tiles in, tile epilogue.
 //   * every wait is bounded (common.cuh).
+// What bounds it is shared memory: per block 640 wavefronts of 128 bytes for the MMAs' operands, 290 of the threads
+// and barriers, 288 of the copies, in 1030 cycles inside a tile and 1190 over tiles.  8192 tokens x 64
+// heads, top-2048, with the union: 1504 us on 128-row tiles, 1271 here; 16384 x 32, top-1024 1240 / 952; 16384 x 16,
+// top-2048 of 131072 1869 / 1308 (e4m3 queries, short runs; long ones meet the power limit: 1880 / 1570 for the first).
 #pragma once
 
 namespace lt {

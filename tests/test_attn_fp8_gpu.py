@@ -595,3 +595,21 @@ def test_calls_of_many_tokens_on_64_row_tiles(tokens, heads, topk, s_kv):
     out_e, lse_e = ao.mla_exact(q8[some].view(torch.float8_e4m3fn).float() * qs, kvf, uniq, synth.SM_SCALE)
     mad, cos = ao.compare(out[some].cpu(), out_e)
     assert cos >= 0.9995 and float((lse[some].cpu() - lse_e.float()).abs().max()) <= TOL_LSE, (mad, cos)
+
+
+def test_64_row_tiles_on_a_cache_beyond_32_bit_row_offsets():
+    # rows 16 MB apart: the last one starts beyond 64 GB, where offsets in 16-byte units leave 32 bits
+    tokens, s_kv, pitch = 380, 4160, 1 << 24
+    if torch.cuda.mem_get_info()[0] < s_kv * pitch + (8 << 30):
+        pytest.skip("needs 73 GB of free device memory")
+    w, idx, kv, q = _case(tokens, 64, 256, s_kv, (0.8, 0.8), seed=23)
+    q8, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    qd, kvd, idd = q8.view(tokens, 64, 576).to(DEV), kv8.to(DEV), idx.to(DEV)
+    assert bool((idd >= 4096).any())
+    want = api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    far = torch.empty((s_kv, pitch), dtype=torch.uint8, device=DEV)[:, :576]
+    far.copy_(kvd.view(torch.uint8))
+    got = api.sparse_prefill(qd, far, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and api.attn_status()[0] == 0
+    del far
+    torch.cuda.empty_cache()
