@@ -1,8 +1,8 @@
 // The FP8 attention kernel for tiles of 64 query rows: one CTA per tile (part of attn_fp8.cu).
 //
 // What it computes is masked_mla_fp8's operation on 64-row tiles (64 / h tokens x h heads) with the same
-// quantisation points; only blocks are 64 keys instead of 128, so a row's running max, and with it the
-// rounding of P to e4m3, takes another course.  sparse_prefill uses it for calls of many tokens (the
+// quantisation points; only blocks are 64 keys instead of 128 and the rule that moves a row's running max is
+// another one, so that it, and with it the rounding of P to e4m3, takes another course.  sparse_prefill uses it for calls of many tokens (the
 // rule and its reasons: use_rows64 in prefill.cu): a union of half as many lists is shorter -- 8 tokens
 // that share 70 % of their lists attend 3.1 k keys together, 4 of them 1.9 k -- and with 64 heads a tile
 // is a single token that needs no membership mask at all.
@@ -36,6 +36,8 @@ constexpr int kSlots = 6;
 constexpr int kWarpGather0 = 16, kWarpQk = 24, kWarpPv = 25, kWarpValid = 26, kWarpQkOdd = 27, kWarpEpi0 = 28;
 constexpr int kThreads = 1024, kRows = 64, kBlockKeys = 64;
 constexpr uint32_t kSlot = kStageKV;                  // 64 rows x 576 B, laid out as in attn_fp8.cu
+// By how much (log2) a row's maximum passes the running max before that moves: see the softmax warps.
+constexpr float kRescale = 5.5f;
 
 // Six slots, Q's rope chunk and the rest: P (64 rows x 64 keys e4m3) lies in the rope chunk of its own block's
 // slot, which is dead once QK^T has read it and of the same 4 KB; an item's output is staged in the slot of the
@@ -59,7 +61,6 @@ struct Misc {
   uint64_t slot_free[kSlots];       // the slot's entry is dead: block through its PV, or Q moved on and output staged
   uint64_t s_free[kGroups], valid_ready[kGroups], valid_free[kGroups];
   uint64_t m_pub[kGroups];          // running max after the group's latest block published
-  uint64_t pair_max;                // row maxima of an item's second block published
   uint64_t q_codes;                 // bf16 q: the item's codes are in q_codes
   uint64_t q_land;                  // the item's Q tile has landed in its slot
   uint64_t q_taken;                 // the item's Q has been moved out of its slot
@@ -71,7 +72,6 @@ struct Misc {
   uint32_t tmem_base, pad;
   float xbuf[kGroups][128];         // [group][lane]: row-max exchange between the key halves
   float mshare[kGroups][64];        // [group][row]: running max after the group's latest block
-  float second[64];                 // [row]: maxima of the item's second block
   float fin_l[kGroups][128], fin_m[kGroups][64];     // end of item: row sums per thread, relative to the group's last running max
 };
 static_assert(sizeof(Misc) <= Plan::kMiscBytes, "Misc too large");
@@ -170,7 +170,6 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       mbar_init(&ms.valid_free[i], kGroupWarps);
       mbar_init(&ms.m_pub[i], kGroupWarps);
     }
-    mbar_init(&ms.pair_max, kGroupWarps);
     mbar_init(&ms.q_codes, 1);
     mbar_init(&ms.q_land, kGatherWarps);
     mbar_init(&ms.q_taken, 1);
@@ -203,9 +202,13 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     // [32 h, +32) of the block with h = tl / 64.  (Two groups of eight warps with 16 columns per thread take as
     // long for a block, 1900 cycles: waits and exchanges, not arithmetic, are most of it.)  Block kb always
     // waits for block kb - 1's running max, also over the end of an item: that keeps every barrier's phases in step.
-    // An item's first running max is that of its first two blocks, as of one block of the 128-row kernel: the
-    // largest weight is exact in e4m3 if the running max is its own, and with 64 keys it less often was
-    // (top-256: 5 % more error against 64 bits).
+    // The largest weight of a row is exact in e4m3 if the running max is its own.  With the 128-row kernel's rule (it moves
+    // when a row of the warp's 32 passes it by more than 6) and 64 keys at a time it less often was: error against 64
+    // bits over the 128-row form's, 13 shapes, N(0, s) queries: s = 1 0.96-1.01, s = 2.5 1.00-1.10, s = 4 0.99-1.13.  So
+    // when it moves it also covers the maxima of the block behind (0.96-1.01, 0.92-1.01, 0.88-1.01: fewer
+    // moves, so it costs nothing), and it moves at 5.5: 0.95-1.00, 0.84-0.97, 0.83-0.97, for about 1 % of the time
+    // (4096 tokens x 64 heads, top-512: 212 -> 215 us; at 5.25 217).  The maxima of the block behind stay in their
+    // group's xbuf until they have been read: the group's next block comes behind this block's running max.
     const int g = warp >> 2;
     const int tl = ((warp & 3) << 5) | lane;
     const int r = tl & 63, h = tl >> 6;
@@ -214,7 +217,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     const float c = p.scale_log2;
     const uint64_t c2 = pack2(c, c);
     const uint32_t scol = tmem + lane_base + kTmemS + 32 * g;
-    int kb0 = 0, it = 0, pairs = 0, nb_next = blocks_of(cid);      // pairs: items of two blocks and more so far
+    int kb0 = 0, it = 0, nb_next = blocks_of(cid);
     // this thread's membership words: two per block of its token
     const uint32_t* mrow = p.memb ? p.memb + ((size_t)cid * p.G + r / p.h_per_q) * capw + h : nullptr;
     uint32_t mk_next = ~0u;
@@ -256,30 +259,25 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         ms.xbuf[g][tl] = cur;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
         cur = fmaxf(cur, ms.xbuf[g][tl ^ 64]);
-        // S, the validity bits and the exchanged maxima have been read: the group's next block may come
+        // S and the validity bits have been read, the maxima published: the group's next block may come
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&ms.s_free[g]);
           mbar_arrive(&ms.valid_free[g]);
         }
-        if (k == 1) {
-          // (behind block kb - 2's, so that every earlier item's maxima have been read)
-          if (kb > 1) mbar_wait(&ms.m_pub[(g + 2) & 3], ((kb - 2) >> 2) & 1, wt, kSiteMPub, k);
-          if (h == 0) ms.second[r] = cur;
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&ms.pair_max);
-        }
         float m_prev = kMInit;
         if (kb > 0) {
           mbar_wait(&ms.m_pub[(g + 3) & 3], ((kb - 1) >> 2) & 1, wt, kSiteMPub, k);
           if (k > 0) m_prev = ms.mshare[(g + 3) & 3][r];
         }
-        if (k == 0 && nb > 1) {
-          mbar_wait(&ms.pair_max, pairs & 1, wt, kSiteMPub, k);
-          cur = fmaxf(cur, ms.second[r]);
+        const bool rescale = __any_sync(0xffffffffu, cur - m_prev > kRescale);
+        if (rescale && k + 1 < nb) {
+          const int g2 = (g + 1) & 3;
+          mbar_wait(&ms.s_free[g2], ((kb + 1) >> 2) & 1, wt, kSiteMPub, k);
+          cur = fmaxf(cur, fmaxf(ms.xbuf[g2][r], ms.xbuf[g2][r + 64]));
+          __syncwarp();
         }
-        const bool rescale = __any_sync(0xffffffffu, cur - m_prev > kRescaleThreshold);
         const float new_m = rescale ? fmaxf(cur, m_prev) : m_prev;
         if (h == 0) ms.mshare[g][r] = new_m;
         __syncwarp();
@@ -348,7 +346,6 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       __syncwarp();
       if (lane == 0) mbar_arrive(&ms.fin_ready);
       kb0 += nb;
-      pairs += nb > 1;
     }
   } else if (warp < kWarpGather0 + kGatherWarps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");

@@ -597,6 +597,25 @@ def test_calls_of_many_tokens_on_64_row_tiles(tokens, heads, topk, s_kv):
     assert cos >= 0.9995 and float((lse[some].cpu() - lse_e.float()).abs().max()) <= TOL_LSE, (mad, cos)
 
 
+@pytest.mark.parametrize("tokens,heads,topk,s_kv,overlap", [(256, 64, 512, 4096, 0.8), (512, 64, 1024, 8192, 0.9),
+                                                            (1024, 16, 512, 8192, 0.9), (1024, 8, 256, 8192, 0.7)])
+@pytest.mark.parametrize("spread", [2.5, 4.0])
+def test_64_row_tiles_are_no_further_from_the_exact_result(tokens, heads, topk, s_kv, overlap, spread):
+    # with peaked logits a row's result hangs on the rounding of its largest weights, hence on how often the running
+    # max is theirs.  The ratio of the errors is 0.86 to 0.96 here; it varies by 0.01 from seed to seed
+    w, idx, kv, q = _case(tokens, heads, topk, s_kv, (overlap, overlap), seed=25)
+    q8, kv8, qs, ks = synth.refcompat_operands(q.float() * spread, kv)
+    q8, kvd, idd = q8.view(tokens, heads, 576).to(DEV), kv8.to(DEV), idx.to(DEV)
+    some = torch.arange(0, tokens, 4 if heads == 64 else 8)
+    exact, _ = ao.mla_exact(q8[some].cpu().view(torch.float8_e4m3fn).float() * qs, kv8.view(torch.float8_e4m3fn).float() * ks,
+                            idx[some], synth.SM_SCALE)
+    err = []
+    for by_job in (False, True):                                        # 128-row tiles, 64-row tiles
+        out, _ = api._sparse_prefill(q8, kvd, idd, synth.SM_SCALE, ks, qs, None, None, None, tokens, by_job)
+        err.append(float((out[some].cpu().double() - exact).norm()))
+    assert err[1] <= 1.01 * err[0], err
+
+
 def test_64_row_tiles_on_a_cache_beyond_32_bit_row_offsets():
     # rows 16 MB apart: the last one starts beyond 64 GB, where offsets in 16-byte units leave 32 bits
     tokens, s_kv, pitch = 380, 4160, 1 << 24

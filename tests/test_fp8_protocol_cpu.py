@@ -42,7 +42,7 @@ def _agents(blocks, bf16_q, rescale):
     def wait(agent, bar, phase):
         a[agent].append(("wait", bar, phase))
 
-    e = kb0 = pairs = 0
+    e = kb0 = 0
     q_entry = []
     for it, nb in enumerate([*blocks, 0]):          # behind the last item: an entry to stage its output in
         q_entry.append(e)
@@ -102,14 +102,10 @@ def _agents(blocks, bf16_q, rescale):
                 wait(s, f"group{g}", kb // groups)
                 ar(s, f"s_free{g}", kb // groups, 2)
                 ar(s, f"valid_free{g}", kb // groups, 2)
-                if k == 1:
-                    if kb > 1:
-                        wait(s, f"m_pub{(kb - 2) % groups}", (kb - 2) // groups)
-                    ar(s, "pair_max", pairs, 2)
                 if kb > 0:
                     wait(s, f"m_pub{before}", (kb - 1) // groups)
-                if k == 0 and nb > 1:
-                    wait(s, "pair_max", pairs)
+                if (rescale or k == 0) and k + 1 < nb:      # the next block's maxima
+                    wait(s, f"s_free{(g + 1) % groups}", (kb + 1) // groups)
                 ar(s, f"m_pub{g}", kb // groups, 2)
                 if rescale and k > 0:
                     wait(s, f"pv_done{(kb - 1) & 7}", (kb - 1) >> 3)
@@ -121,7 +117,6 @@ def _agents(blocks, bf16_q, rescale):
                 ar(f"s{g}{w}", "fin_ready", it, 2 * groups)
         e += nb + 1
         kb0 += nb
-        pairs += nb > 1
     last = -1
     for it in range(-1, len(blocks)):
         staged = f"slot_free{q_entry[it + 1] % slots}"
