@@ -181,6 +181,12 @@ static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, con
   int32_t* counts = reinterpret_cast<int32_t*>(ws + l.counts);
   int32_t* u = reinterpret_cast<int32_t*>(ws + l.u);
   uint32_t* memb = r.rows64 && G == 1 ? nullptr : reinterpret_cast<uint32_t*>(ws + l.memb);
+  // what the 128-row form of the call refuses (8 heads: lists of more than 2048 entries) is refused in either form
+  if (r.rows64) {
+    const int G2 = 128 / h;
+    rc = check_union(T, k, T / G2, G2 * k, G2, seq_space);
+    if (rc != LITEDSA_OK) return rc;
+  }
   // fill 2: lists padded to whole 128-key blocks, nothing written beyond
   rc = run_union(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
   if (rc != LITEDSA_OK) return rc;

@@ -236,22 +236,45 @@ static int launch_union(const UnionParams& p, int rank_shift, int ng, size_t sme
   return rank_shift ? launch_union_rs<NT, VPT, 2>(p, ng, smem, stream) : launch_union_rs<NT, VPT, 0>(p, ng, smem, stream);
 }
 
+// Shared memory (227 KB per CTA on sm_100): the whole list is staged if two CTAs fit on an SM then,
+// else its first 8192 entries (a union is usually well below G * k); one rank per bitmap word if
+// that fits, else one per quad.
+constexpr size_t kUnionSmemLimit = 220 * 1024;
+struct UnionSmem { int window, rank_shift; size_t bytes; };
+static UnionSmem union_smem(int s_words, int G, int cap) {
+  UnionSmem m{cap, 0, 0};
+  if (union_smem_bytes(s_words, 0, G, cap, cap) > 110 * 1024) m.window = cap < 8192 ? cap : 8192;
+  if (union_smem_bytes(s_words, 0, G, cap, m.window) > kUnionSmemLimit) m.window = cap < 1024 ? cap : 1024;
+  if (union_smem_bytes(s_words, 0, G, cap, m.window) > kUnionSmemLimit) m.rank_shift = 2;
+  m.bytes = union_smem_bytes(s_words, m.rank_shift, G, cap, m.window);
+  return m;
+}
+
+// The shapes that a union of G lists of k entries takes: no CUDA call.
+int check_union(int T, int k, int ng, int cap, int G, int64_t seq_space) {
+  if (ng <= 0 || G <= 0 || k <= 0 || T != ng * G) return LITEDSA_ERR_SHAPE;
+  if (cap < G * k || cap % 128 != 0) return LITEDSA_ERR_SHAPE;
+  if (G > 16 || (int64_t)G * (cap / 32) > 16 * 1024) return LITEDSA_ERR_SHAPE;
+  if (seq_space <= 0 || seq_space > (1 << 20)) return LITEDSA_ERR_SHAPE;
+  if ((seq_space + 31) / 32 % 32 != 0) return LITEDSA_ERR_SHAPE;   // 1024-position aligned
+  if (k % 4 != 0) return LITEDSA_ERR_UNSUPPORTED;    // 16-byte row loads
+  if (cap > 65536) return LITEDSA_ERR_UNSUPPORTED;   // 16-bit rank table
+  if (union_smem((int)((seq_space + 31) / 32), G, cap).bytes > kUnionSmemLimit) return LITEDSA_ERR_UNSUPPORTED;
+  return LITEDSA_OK;
+}
+
 // Checks and launch behind litedsa_union_qm and litedsa_sparse_prefill; fill as UnionParams::fill_tail.
 int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uint32_t* memb_qm, const int32_t* req_pg,
               const int32_t* block_table, int T, int k, int ng, int cap, int G, int bt_rows, int bt_blocks,
               int block_size, int64_t seq_space, int fill, void* stream) {
   // same argument checks as the reference launcher (litedsa.cu:43-59)
   if (!topk_indices || !u_phys || !counts || (!memb_qm && G != 1)) return LITEDSA_ERR_ARG;
-  if (ng <= 0 || G <= 0 || k <= 0 || T != ng * G) return LITEDSA_ERR_SHAPE;
-  if (cap < G * k || cap % 128 != 0) return LITEDSA_ERR_SHAPE;
-  if (G > 16 || (int64_t)G * (cap / 32) > 16 * 1024) return LITEDSA_ERR_SHAPE;
-  if (seq_space <= 0 || seq_space > (1 << 20)) return LITEDSA_ERR_SHAPE;
+  const int rc = check_union(T, k, ng, cap, G, seq_space);
+  if (rc == LITEDSA_ERR_SHAPE) return rc;
   const int s_words = (int)((seq_space + 31) / 32);
-  if (s_words % 32 != 0) return LITEDSA_ERR_SHAPE;   // 1024-position aligned
   if ((block_table != nullptr) != (req_pg != nullptr)) return LITEDSA_ERR_ARG;
   if (block_table && (block_size <= 0 || bt_blocks <= 0 || bt_rows <= 0)) return LITEDSA_ERR_SHAPE;
-  if (k % 4 != 0) return LITEDSA_ERR_UNSUPPORTED;    // 16-byte row loads
-  if (cap > 65536) return LITEDSA_ERR_UNSUPPORTED;   // 16-bit rank table
+  if (rc != LITEDSA_OK) return rc;
 
   UnionParams p;
   p.idx = topk_indices; p.u_phys = u_phys; p.counts = counts; p.memb = memb_qm;
@@ -260,17 +283,10 @@ int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uin
   p.bsz_mul = fast_div_mul(int64_t(s_words) * 32, p.bsz);
   p.kq = k / 4; p.kq_mul = fast_div_mul(int64_t(G) * (k / 4), k / 4);
   p.k = k; p.G = G; p.cap = cap; p.s_words = s_words; p.fill_tail = fill;
-  // Shared memory (227 KB per CTA on sm_100): the whole list is staged if two CTAs fit on an SM then,
-  // else its first 8192 entries (a union is usually well below G * k); one rank per bitmap word if
-  // that fits, else one per quad.
-  const size_t limit = 220 * 1024;
-  int rank_shift = 0;
-  p.window = cap;
-  if (union_smem_bytes(s_words, 0, G, cap, cap) > 110 * 1024) p.window = cap < 8192 ? cap : 8192;
-  if (union_smem_bytes(s_words, 0, G, cap, p.window) > limit) p.window = cap < 1024 ? cap : 1024;
-  if (union_smem_bytes(s_words, 0, G, cap, p.window) > limit) rank_shift = 2;
-  const size_t smem = union_smem_bytes(s_words, rank_shift, G, cap, p.window);
-  if (smem > limit) return LITEDSA_ERR_UNSUPPORTED;
+  const UnionSmem m = union_smem(s_words, G, cap);
+  p.window = m.window;
+  const int rank_shift = m.rank_shift;
+  const size_t smem = m.bytes;
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int quads = G * k / 4;

@@ -132,6 +132,13 @@ def test_entry_points_reject_bad_arguments_before_any_cuda_call(built_lib):
     outs2 = (ctypes.c_void_p * 2)(P, None)
     assert L.litedsa_masked_mla_fp8_multi(P, P, P, ok["sm"], ok["os"], None, P, 64, outs2, 2, None, P,
                                           2, 128, 128, 576, 576, 128, None) == ARG
+    # one call of many tokens: what it takes does not depend on the rows of a tile.  16 lists of 3072 entries are more
+    # than a union's membership words, also where the tiles of a large job unite 8
+    big, space = 16384, 65536
+    for fn in (L.litedsa_sparse_prefill, L.litedsa_sparse_prefill_job):
+        assert fn(P, 0, P, 0, P, 0.1, 1.0, 1.0, P, P, big, 8, 3072, space, 576, space, big, P, 1 << 40, None) == SHAPE
+        assert fn(P, 0, P, 0, P, 0.1, 1.0, 1.0, P, P, big, 8, 2048, space, 576, space + 512, big, P, 1 << 40, None) == SHAPE
+        assert fn(P, 0, P, 0, P, 0.1, 1.0, 1.0, P, P, big, 64, 2048, space, 576, 2 << 20, big, P, 1 << 40, None) == SHAPE
     # DSv4: queries outside the cache, heads not dividing 128
     assert L.litedsa_dsv4_c128a_bf16(P, None, P, 4, 64, 0, 4, 0, 128, 128, 0.1, None, P, P,
                                      576, 576, 576, 0, 0, 0, 0, None) == SHAPE
