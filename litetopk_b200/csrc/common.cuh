@@ -67,7 +67,9 @@ int run_fp8(const Fp8Args& a, void* const* outs, int n_outs, void* stream);
 // attn_fp8_r64.cuh: tiles of 64 rows; q_codes: rows64_scratch(ng) bytes
 int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream);
 int64_t rows64_scratch(int ng);
-// union_qm.cu; cap >= G * k, the row length of u_phys (a multiple of 128); memb_qm may be null with G = 1; fill 0: live prefixes only, 1: whole rows, 2: u_phys := -1 up to the next multiple of 128
+// union_qm.cu; cap >= G * k: the row length of u_phys, a multiple of 128.  memb_qm may be null with G = 1.  fill 0: live
+// prefixes only, 1: whole rows, 2: u_phys := -1 up to the next multiple of 128 (one block at least, which the
+// attention kernels run for an empty list)
 int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uint32_t* memb_qm, const int32_t* req_pg,
               const int32_t* block_table, int T, int k, int ng, int cap, int G, int bt_rows, int bt_blocks,
               int block_size, int64_t seq_space, int fill, void* stream);

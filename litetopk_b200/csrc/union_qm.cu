@@ -37,7 +37,7 @@ struct UnionParams {
   int k, G, cap, s_words;   // s_words = seq_space / 32
   int quads_per_thread;     // 16-byte bitmap quads a thread counts: 1 or odd (conflict-free reads)
   int window;               // list entries staged in shared memory; later ones are written directly
-  int fill_tail;            // 1: also write -1 / 0 beyond the live prefixes; 2: -1 up to the next multiple of 128
+  int fill_tail;            // 1: also write -1 / 0 beyond the live prefixes; 2: -1 up to the next multiple of 128, 128 entries at least
 };
 
 // Shared-memory carve-up (bytes): bitmap | rank table (u16) | qm accumulator | list window
@@ -132,7 +132,7 @@ union_qm_kernel(const UnionParams p) {
     const int t = __shfl_up_sync(0xffffffffu, wincl, off);
     if (lane >= off) wincl += t;
   }
-  const int live = __shfl_sync(0xffffffffu, wincl, NW - 1);     // <= G * k = cap
+  const int live = __shfl_sync(0xffffffffu, wincl, NW - 1);     // <= G * k <= cap
   int r0 = __shfl_sync(0xffffffffu, wincl - wt, wid) + incl - mine;
   if (tid == 0) p.counts[g] = live;
   for (int i = q0; i < q1; ++i) {
@@ -189,7 +189,7 @@ union_qm_kernel(const UnionParams p) {
 
   // ---- staged list -> global, 16-byte stores; the last quad is padded with -1
   {
-    const int end = p.fill_tail == 1 ? cap : (p.fill_tail == 2 ? ((live + 127) >> 7) << 7 : (live + 3) & ~3);
+    const int end = p.fill_tail == 1 ? cap : (p.fill_tail == 2 ? max(128, ((live + 127) >> 7) << 7) : (live + 3) & ~3);
     for (int i = tid; i < end >> 2; i += NT) {
       const int b = i << 2;
       if (b >= p.window && b + 3 < live) continue;              // written above (window % 4 == 0)

@@ -597,6 +597,40 @@ def test_calls_of_many_tokens_on_64_row_tiles(tokens, heads, topk, s_kv):
     assert cos >= 0.9995 and float((lse[some].cpu() - lse_e.float()).abs().max()) <= TOL_LSE, (mad, cos)
 
 
+@pytest.mark.parametrize("form", ["litedsa_sparse_prefill", "litedsa_sparse_prefill_job"])
+@pytest.mark.parametrize("tokens,heads,topk", [(600, 64, 256), (2400, 16, 256)])
+def test_an_empty_tile_has_a_list_of_padding(form, tokens, heads, topk):
+    # the attention kernels run one block for it: its entries are -1, not what the workspace held
+    from litetopk_b200 import _lib
+    def mutate(idx):
+        idx = idx.clone()
+        idx[32:64] = -1
+        idx[tokens - 16:] = -1
+        return idx
+    w, idx, kv, q = _case(tokens, heads, topk, 4096, (0.6, 0.8), seed=26, mutate=mutate)
+    q8, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    q8, kvd, idd = q8.to(DEV), kv8.to(DEV), idx.to(DEV)
+    rows = 64 if form.endswith("job") else 128
+    G, ng = rows // heads, tokens * heads // rows
+    cap = (G * topk + 127) // 128 * 128
+    out = torch.empty((tokens, heads, 512), dtype=torch.bfloat16, device=DEV)
+    lse = torch.empty((tokens, heads), dtype=torch.float32, device=DEV)
+    with torch.cuda.device(DEV):
+        ws = torch.full((getattr(_lib.lib(), form + "_workspace")(tokens, heads, topk, 0, tokens),), 7, dtype=torch.uint8, device=DEV)
+        _lib.check(getattr(_lib.lib(), form)(
+            q8.data_ptr(), 0, kvd.data_ptr(), 0, idd.data_ptr(), synth.SM_SCALE, qs, ks, out.data_ptr(), lse.data_ptr(),
+            tokens, heads, topk, 4096, 576, 4096, tokens, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), form)
+    torch.cuda.synchronize()
+    counts = ws[:4 * ng].view(torch.int32).cpu()
+    u = ws[(4 * ng + 255) // 256 * 256:][:4 * ng * cap].view(torch.int32).view(ng, cap).cpu()
+    assert int((counts == 0).sum()) == 48 // G
+    for g in range(ng):
+        n = int(counts[g])
+        end = max(128, (n + 127) // 128 * 128)
+        assert bool((u[g, n:end] == -1).all()) and bool((u[g, end:] == 0x07070707).all()), g
+    assert bool((out[32:64] == 0).all()) and bool(torch.isinf(lse[32:64]).all())
+
+
 @pytest.mark.parametrize("tokens,heads,topk,s_kv,overlap", [(256, 64, 512, 4096, 0.8), (512, 64, 1024, 8192, 0.9),
                                                             (1024, 16, 512, 8192, 0.9), (1024, 8, 256, 8192, 0.7)])
 @pytest.mark.parametrize("spread", [2.5, 4.0])
