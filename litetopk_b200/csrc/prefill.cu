@@ -103,7 +103,7 @@ static Layout layout_of(int ng, int G, int cap, int nsplit, bool rows64) {
   l.counts = 0;
   l.u = up(4 * (int64_t)ng);
   l.memb = l.u + up(4 * (int64_t)ng * cap);
-  l.part_o = l.memb + up(4 * (int64_t)ng * G * (cap / 32));
+  l.part_o = l.memb + (rows64 && G == 1 ? 0 : up(4 * (int64_t)ng * G * (cap / 32)));      // one token per tile: none
   l.part_ml = l.part_o + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 512 * 4) : 0);
   l.q_codes = l.part_ml + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 8) : 0);
   l.total = l.q_codes + (rows64 ? rows64_scratch(ng) : 0);
