@@ -181,10 +181,10 @@ struct ItemT {
   __device__ __forceinline__ bool leads(int k) const { return kSliced && k < lead; }
 };
 
-// wait sites reported in the status word
+// wait sites reported in the status word (kSiteAlign: the shared-memory base is not where the plan needs it)
 enum { kSiteQ = 1, kSiteKLand, kSiteQkDone, kSitePvDone,
        kSiteSFree, kSitePReady, kSiteValidReady, kSiteValidFree, kSiteKFree,
-       kSiteVFree, kSitePFree, kSiteEpi, kSiteRelayK, kSiteRelayV, kSiteMPub, kSiteQFree, kSiteOFree, kSiteSelfTest };
+       kSiteVFree, kSitePFree, kSiteEpi, kSiteRelayK, kSiteRelayV, kSiteMPub, kSiteQFree, kSiteOFree, kSiteSelfTest, kSiteAlign };
 
 // status block of the FP8 attention kernels (layout: see Waiter in common.cuh)
 __device__ int g_attn_status[8];

@@ -148,6 +148,13 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   const uint32_t sbase = smem_u32(sm);
   Misc& ms = *reinterpret_cast<Misc*>(sm + kOffMisc);
   const Waiter wt{g_attn_status, p.epoch, p.wait_limit_ns};
+  // The plan fills the shared memory, so the base cannot be rounded up: swizzled tiles on another one would be
+  // read wrongly without any error.
+  if ((sbase & 1023u) != 0) {
+    pdl_wait();
+    if (threadIdx.x == 0) wt.fail(kSiteAlign, (int)(sbase & 1023u));
+    return;
+  }
 
   const int cid = blockIdx.x, ncta = gridDim.x, ng = p.ng;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;

@@ -26,3 +26,13 @@ def test_a_kernels_shared_memory_limit_does_not_depend_on_the_call():
     assert calls
     for c in calls:
         assert not re.search(r"\b(bytes|dyn|smem)\b", c), c
+
+
+def test_a_kernel_with_swizzled_tiles_rounds_or_checks_its_shared_memory_base():
+    # the declared alignment of dynamic shared memory is no promise about its address at run time
+    found = 0
+    for f in sorted(CSRC.glob("*.cu*")):
+        for body in _code(f).split("extern __shared__ __align__(1024)")[1:]:
+            found += 1
+            assert re.search(r"\+ 1023u?\) & ~1023u?|& 1023u?\) != 0\)", body[:900]), f.name
+    assert found >= 5
