@@ -70,7 +70,7 @@ static int run(const Args& a, void* stream) {
   p.lse = a.lse; p.max_logits = a.max_logits; p.sink = a.sink; p.sink_mod = 128;
   p.ng = a.ng; p.G = 128 / a.h_per_q; p.h_per_q = a.h_per_q; p.nsplit = 1;
   p.scale_log2 = a.sm_scale * kLog2e;
-  p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
+  p.epoch = next_launch_epoch(); p.wait_limit = wait_limit_ticks();
   p.gate = a.gate; p.gate_value = 1;
   p.kv = reinterpret_cast<const uint8_t*>(a.kv); p.kv_pitch = a.kv_row_stride * 2;
   p.indices = a.indices; p.idx_stride = a.idx_row_stride;

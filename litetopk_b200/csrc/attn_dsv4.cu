@@ -82,7 +82,7 @@ static Params base_params(int ng, int h, float sm_scale, float* lse, const float
   p.ng = ng; p.G = 128 / h; p.h_per_q = h; p.nsplit = 1;
   p.window = p.ratio = 1;
   p.scale_log2 = sm_scale * kLog2e;
-  p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
+  p.epoch = next_launch_epoch(); p.wait_limit = wait_limit_ticks();
   return p;
 }
 

@@ -116,7 +116,9 @@ struct Misc {
                                     // be complete before the epilogue has looked at this one's
   uint32_t valid[2][4];             // 128 validity bits per stage
   uint32_t tmem_base;
-  uint32_t pad;
+  // for the tear-down of a launch that gives up: a wait of this block has; items whose Q has been requested from TMA
+  // and at whose q_land each K warp has arrived; leader: blocks whose QK^T and PV have been issued
+  uint32_t left, q_asked, q_passed[kProducerWarps / 2], qk_end, pv_end;
   float xbuf[2][2][2][128];         // [group][parity][column half][lane]: row-max exchange
   float mshare[2][128];             // [group][lane]: running max after the group's latest block
   float fin_l[512];                 // end of item: row sums per thread ...
@@ -146,7 +148,7 @@ struct AttnParams {
   long long idx_stride;
   float scale_log2, out_scale;
   int epoch;                          // this launch's epoch for the bounded waits
-  unsigned long long wait_limit_ns;
+  uint32_t wait_limit;       // of one wait, in ticks (BlockWaiter)
   // bf16 queries (dense packed layout), quantised to e4m3 on their way in: code = e4m3(q * q_inv);
   // null: q arrives as e4m3 through map_q / map_q_rope
   const uint4* q_bf16;
@@ -203,7 +205,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
   const uint32_t sbase = (raw + 1023u) & ~1023u;       // 128B-swizzle tiles need 1024-byte alignment
   uint8_t* sm = smem_raw + (sbase - raw);
   Misc& ms = *reinterpret_cast<Misc*>(sm + kOffMisc);
-  const Waiter wt{g_attn_status, p.epoch, p.wait_limit_ns};
+  const BlockWaiter wt{&ms.left, p.wait_limit};
 
   // Persistent: each cluster walks items cid, cid + #clusters, ...  Every role runs the same
   // item loop; stages, buffers and barrier phases are indexed by the cluster-wide running
@@ -237,6 +239,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
 
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_land, kProducerWarps / 2);              // the K warps
+    ms.left = ms.q_asked = ms.qk_end = ms.pv_end = 0;
+    for (int i = 0; i < kProducerWarps / 2; ++i) ms.q_passed[i] = 0;
     mbar_init(&ms.q_taken, 1);
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
@@ -520,22 +524,26 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       else if (w + ncl < n_items) idx = load_idx(nx, 0);
       return cur;
     };
+    bool ok = true, go = true;                     // none of this lane's / this warp's waits has given up: then it leaves
     if (is_k) {
       const uint64_t pol_stream = l2_policy_evict_first();
       const int cj = lane >> 3, cc = lane & 7;     // latent piece `lane`: chunk cj, 16-byte slot cc
-      for (int w = cid; w < n_items; w += ncl, ++it) {
+      for (int w = cid; go && w < n_items; w += ncl, ++it) {
         const Item t = nx;
         if (w + ncl < n_items) nx = item_of(w + ncl);
         // The item's Q entry, in front of its K entries.  Every warp goes through its slot's barrier and that of
         // the previous Q (whose bytes could, with short items, still be in flight), and it counts as landed
         // only when all of them have: no warp is overtaken and tests a phase that is two ahead.
-        if (it > 0) mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
-        if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
+        if (it > 0) ok &= mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
+        if (ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
         __syncwarp();
-        if (lane == 0) {
+        // (nothing behind a wait of any warp that gave up: the Q before could still be in flight)
+        if (lane == 0 && ok && !wt.aborting()) {
+          ms.q_passed[pw] = it + 1;
           if (pw != 0 || p.q_bf16 != nullptr) {
             mbar_arrive(&ms.q_land);               // bf16 q: the epilogue warps fill the slot
           } else {
+            ms.q_asked = it + 1;
             mbar_arrive_expect_tx(&ms.q_land, kStageKV);
             // this CTA's 64 rows of the tile = (token, head) pairs starting at row 64 cta
             const int qh = (64 * (int)cta) % p.h_per_q;
@@ -550,9 +558,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         advance();
         for (int k = 0; k < t.nb; ++k, ++kb) {
           const int cur = take_idx(t, k, w);
-          const bool full = __all_sync(0xffffffffu, cur >= 0);
-          if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
-          __syncwarp();
+          if (ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
+          const bool full = __all_sync(0xffffffffu, cur >= 0 && ok);
           const uint32_t kst = sbase + kOffKV + slot * kStageKV;
           const uint32_t kdst = kst + cj * kChunkBytes + 16 * pw * 128;
           // rope bytes: compact 64-byte rows, 64-byte swizzle (16-byte unit ^ ((row / 2) % 4))
@@ -569,6 +576,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
               cp_async16(rdst + i * 512, kvb + (size_t)ri * pitch + 512 + 16 * (lane & 3));
             }
           } else {
+            go = __all_sync(0xffffffffu, ok);
+            if (!go) break;
 #pragma unroll 1
             for (int i = 0; i < 16; ++i) {
               const int ri = __shfl_sync(0xffffffffu, cur, i);
@@ -588,15 +597,14 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       // lane: rows 16 pw + 2 i + lane / 16 of the peer's keys, 16-byte piece lane % 16 of this CTA's 256 value bytes
       const int pc = lane & 15, r2 = lane >> 4;
       const uint8_t* src = kvb + 256 * cta + 16 * pc;
-      for (int w = cid; w < n_items; w += ncl) {
+      for (int w = cid; go && w < n_items; w += ncl) {
         const Item t = nx;
         if (w + ncl < n_items) nx = item_of(w + ncl);
         advance();                                 // the item's Q
         for (int k = 0; k < t.nb; ++k, ++kb) {
           const int cur = take_idx(t, k, w);
-          const bool full = __all_sync(0xffffffffu, cur >= 0);
-          mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, k);
-          __syncwarp();
+          ok &= mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, k);
+          const bool full = __all_sync(0xffffffffu, cur >= 0 && ok);
           // the dead half of the K tile: chunks 2-3 in CTA 0, chunks 0-1 in CTA 1
           const uint32_t vst = sbase + kOffKV + slot * kStageKV + (cta == 0 ? 2 * kChunkBytes : 0) + (pc >> 3) * kChunkBytes +
                                (16 * pw + r2) * 128;
@@ -607,6 +615,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
               cp_async16(vst + i * 256 + (((pc & 7) ^ ((2 * i + r2) & 7)) << 4), src + (size_t)ri * pitch);
             }
           } else {
+            go = __all_sync(0xffffffffu, ok);
+            if (!go) break;
 #pragma unroll 1
             for (int i = 0; i < 8; ++i) {
               const int ri = __shfl_sync(0xffffffffu, cur, 2 * i + r2);
@@ -633,15 +643,8 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
      }
    };
    // the time-limit and abort check of a wait that has not been satisfied yet (warp-uniform answer)
-   auto mma_idle = [&](unsigned long long& since, int site, int kb) -> bool {
-     const unsigned long long now = globaltimer_ns();
-     if (since == 0) since = now;
-     bool stop = wt.aborting();
-     if (now - since > wt.limit_ns) {
-       if (lane == 0) wt.fail(site, kb);
-       stop = true;
-     }
-     return __any_sync(0xffffffffu, stop);
+   auto mma_idle = [&](uint32_t& since, int site, int kb) -> bool {
+     return __any_sync(0xffffffffu, wt.gives_up(since, site, kb));
    };
    if (warp == kWarpMma) {
     // ------------------------------------------------------------ MMA issue (leader CTA only)
@@ -672,7 +675,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       // breaks: 53 cycles to issue an MMA instead of 23).
       MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, 1};
       bool aborted = false;
-      unsigned long long since = 0;
+      uint32_t since = 0;
       while (c.w < n_items && !aborted) {
         // K rows landed on both CTAs, S buffer drained and, for an item's first block, Q in place
         const uint32_t ph = (c.kb >> 3) & 1;
@@ -691,6 +694,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
           aborted = mma_idle(since, kSiteKLand, c.kb);
         }
       }
+      if (lane == 0) ms.qk_end = c.kb;
     }
    } else if (warp == kWarpRelayK && cta == 0) {
       // ---------------------------------------------------------- PV issue (leader CTA)
@@ -711,7 +715,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       };
       MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, 1};
       bool aborted = false;
-      unsigned long long since = 0;
+      uint32_t since = 0;
       while (c.w < n_items && !aborted) {
         // V rows landed on both CTAs, P written; an item's first PV overwrites O: the previous item
         // must have read it out
@@ -727,6 +731,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
           aborted = mma_idle(since, kSitePReady, c.kb);
         }
       }
+      if (lane == 0) ms.pv_end = c.kb;
   } else if (warp == kWarpRelayK || warp == kWarpRelayV) {
     // ------------------------------------------------------------ "landed" relays to the leader CTA
     // The MMA thread lives in the leader CTA and can only wait on its own barriers: in the
@@ -953,10 +958,23 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
 
   // tear-down: nobody may still be reading TMEM of either CTA when it is released
   __syncthreads();
+  if (ms.left != 0) {
+    cp_async_wait_all();
+    if (threadIdx.x == 0) {
+      if (ms.q_asked != 0) {      // the last Q requested: with the arrivals of the warps that have left it counts as landed when it has
+        for (int i = 0; i < kProducerWarps / 2; ++i)
+          if (ms.q_passed[i] < ms.q_asked) mbar_arrive(&ms.q_land);
+        mbar_drain(&ms.q_land, (ms.q_asked - 1) & 1);
+      }
+      if (ms.qk_end != 0) mbar_drain(&ms.qk_done[(ms.qk_end - 1) & 7], ((ms.qk_end - 1) >> 3) & 1);
+      if (ms.pv_end != 0) mbar_drain(&ms.pv_done[(ms.pv_end - 1) & 3], ((ms.pv_end - 1) >> 2) & 1);
+    }
+  }
   __syncwarp();
   cluster_sync_all();
   if (warp == kWarpMma) tmem_dealloc_pair(tmem, kTmemCols);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_attn_status[3], 1);
+  if (threadIdx.x == 0) wt.report(g_attn_status, p.epoch);
 }
 
 // how many 2-CTA clusters of this kernel device `dev` (the current one) can hold at once
@@ -1028,7 +1046,7 @@ static int launch_fp8(const Fp8Args& a, void* const* outs, int n_out, cudaStream
   p.ng = a.ng; p.s_kv = a.s_kv; p.cap = a.topk; p.h_per_q = a.h_per_q; p.G = 128 / a.h_per_q;
   p.idx_stride = a.indices_row_stride;
   p.scale_log2 = a.sm_scale * kLog2e; p.out_scale = a.out_scale;
-  p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
+  p.epoch = next_launch_epoch(); p.wait_limit = wait_limit_ticks();
   p.q_bf16 = a.q_is_bf16 ? reinterpret_cast<const uint4*>(a.q8) : nullptr; p.q_inv = a.q_inv;
   p.nsplit = a.nsplit; p.part_o = a.part_o; p.part_ml = reinterpret_cast<float2*>(a.part_ml);
   return launch_fp8_t(map_q, map_q_rope, omaps, p, stream);

@@ -69,7 +69,10 @@ struct Misc {
   uint64_t o_free;                  // the item's O has been read out of TMEM
   uint64_t fin_ready, fin_free;     // the item's row sums are published / have been read
   uint32_t valid[kGroups][2];       // 64 validity bits
-  uint32_t tmem_base, pad;
+  uint32_t tmem_base;
+  // for the tear-down of a launch that gives up: a wait of this block has; items whose Q has been requested and at
+  // whose q_land each gather warp has arrived; blocks whose QK^T (per issuing warp) and PV have been issued
+  uint32_t left, q_asked, q_passed[kGatherWarps], qk_end[2], pv_end;
   float xbuf[kGroups][128];         // [group][lane]: row-max exchange between the key halves
   float mshare[kGroups][64];        // [group][row]: running max after the group's latest block
   float fin_l[kGroups][128], fin_m[kGroups][64];     // end of item: row sums per thread, relative to the group's last running max
@@ -86,7 +89,7 @@ struct Params {
   int ng, s_kv, cap, h_per_q, G;
   float scale_log2, out_scale;
   int epoch;
-  unsigned long long wait_limit_ns;
+  uint32_t wait_limit;       // of one wait, in ticks (BlockWaiter)
   // bf16 queries, quantised by the epilogue warps an item ahead into q_codes [2][CTAs][64, 576] (map_q and
   // map_q_rope are of that then); null: e4m3
   const uint4* q_bf16;
@@ -147,12 +150,12 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   extern __shared__ __align__(1024) uint8_t sm[];
   const uint32_t sbase = smem_u32(sm);
   Misc& ms = *reinterpret_cast<Misc*>(sm + kOffMisc);
-  const Waiter wt{g_attn_status, p.epoch, p.wait_limit_ns};
+  const BlockWaiter wt{&ms.left, p.wait_limit};
   // The plan fills the shared memory, so the base cannot be rounded up: swizzled tiles on another one would be
   // read wrongly without any error.
   if ((sbase & 1023u) != 0) {
     pdl_wait();
-    if (threadIdx.x == 0) wt.fail(kSiteAlign, (int)(sbase & 1023u));
+    if (threadIdx.x == 0) Waiter{g_attn_status, p.epoch, 0}.fail(kSiteAlign, (int)(sbase & 1023u));
     return;
   }
 
@@ -185,6 +188,8 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     mbar_init(&ms.o_free, kEpiWarps);
     mbar_init(&ms.fin_ready, kGroups * kGroupWarps);
     mbar_init(&ms.fin_free, kEpiWarps);
+    ms.left = ms.q_asked = 0;
+    for (int i = 0; i < kGatherWarps; ++i) ms.q_passed[i] = 0;
     fence_mbar_init();
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_q_rope);
@@ -375,7 +380,8 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     auto first_k = [&](int e0) -> int { return (set - e0 - 1) & 1; };      // first own block of an item whose Q is entry e0
     int kidx = __ldcs(p.indices + (size_t)cid * p.cap + first_k(0) * kBlockKeys + own_key);
     auto advance = [&]() { slot += 2; if (slot >= kSlots) { slot -= kSlots; ++ring; } };
-    for (int tile = cid; tile < ng + ncta; tile += ncta, ++it) {      // behind the last item: an entry to stage its output in
+    bool ok = true, go = true;                     // none of this lane's / this warp's waits has given up: then it leaves
+    for (int tile = cid; go && tile < ng + ncta; tile += ncta, ++it) {      // behind the last item: an entry to stage its output in
       const int nb = nb_next;
       nb_next = blocks_of(tile + ncta);
       const int32_t* idx = p.indices + (size_t)tile * p.cap + own_key;
@@ -385,15 +391,18 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       // With short items the previous Q could still be on its way.  Every warp goes through every item's barrier
       // and a Q counts as landed only when all of them have -- those of its set also through its slot's
       // barrier --, so that none is overtaken and tests a phase that is two ahead.
-      if (it > 0) mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
-      if (p.q_bf16 != nullptr && tile < ng) mbar_wait(&ms.q_codes, it & 1, wt, kSiteQ, it);
+      if (it > 0) ok &= mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
+      if (p.q_bf16 != nullptr && tile < ng) ok &= mbar_wait(&ms.q_codes, it & 1, wt, kSiteQ, it);
       const bool q_mine = (e & 1) == set;
-      if (q_mine && ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
+      if (q_mine && ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
       __syncwarp();
-      if (lane == 0) {
+      // (nothing behind a wait of any warp that gave up: the Q before could still be in flight)
+      if (lane == 0 && ok && !wt.aborting()) {
+        ms.q_passed[warp - kWarpGather0] = it + 1;
         if (!q_mine || pw != 0 || tile >= ng) {
           mbar_arrive(&ms.q_land);
         } else {
+          ms.q_asked = it + 1;
           mbar_arrive_expect_tx(&ms.q_land, kSlot);
           const uint32_t dst = sbase + kOffKV + slot * kSlot;
           const int z = p.q_bf16 != nullptr ? (it & 1) * ncta + cid : tile * p.G;
@@ -411,10 +420,9 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         // (Indices are loaded a block ahead: nothing waits for a cold line.)
         const bool has = (unsigned)kidx < (unsigned)p.s_kv;
         const uint32_t row = has ? (kWide ? (uint32_t)kidx : (uint32_t)kidx * pitch16) : 0xffffffffu;
-        const bool full = __all_sync(0xffffffffu, has);
         kidx = k + 2 < nb ? __ldcs(idx + (k + 2) * kBlockKeys) : next_tile_idx();
-        if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
-        __syncwarp();
+        if (ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
+        const bool full = __all_sync(0xffffffffu, has && ok);
         const uint32_t kst = sbase + kOffKV + slot * kSlot;
         const uint32_t kdst = kst + cj * kChunkBytes + 16 * pw * 128;
         // rope bytes: compact 64-byte rows, 64-byte swizzle (16-byte unit ^ ((row / 2) % 4))
@@ -431,6 +439,8 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
             cp_async16(rdst + i * 512, kv_rope + (size_t)o * unit);
           }
         } else {
+          go = __all_sync(0xffffffffu, ok);
+          if (!go) break;
 #pragma unroll 1
           for (int i = 0; i < 16; ++i) {
             const uint32_t o = __shfl_sync(0xffffffffu, row, i);
@@ -464,16 +474,9 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       }
     };
     // the time-limit and abort check of a wait, once per 64 polls (warp-uniform answer)
-    auto idle = [&](unsigned& polls, unsigned long long& since, int site, int kb) -> bool {
+    auto idle = [&](unsigned& polls, uint32_t& since, int site, int kb) -> bool {
       if ((++polls & 63u) != 0) return false;
-      const unsigned long long now = globaltimer_ns();
-      if (since == 0) since = now;
-      bool stop = wt.aborting();
-      if (now - since > wt.limit_ns) {
-        if (lane == 0) wt.fail(site, kb);
-        stop = true;
-      }
-      return __any_sync(0xffffffffu, stop);
+      return __any_sync(0xffffffffu, wt.gives_up(since, site, kb));
     };
     if (warp == kWarpQk || warp == kWarpQkOdd) {
       // ---------------------------------------------------------- QK^T issue (every decision a vote: see attn_fp8.cu)
@@ -491,7 +494,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       };
       const int mine = warp == kWarpQkOdd ? 1 : 0;
       bool aborted = false;
-      unsigned long long since = 0;
+      uint32_t since = 0;
       unsigned polls = 0;
       while (c.tile < ng && !aborted) {
         // One barrier per lane, tested by one instruction: K rows landed, S buffer drained and, at an item's
@@ -517,12 +520,13 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
           aborted = idle(polls, since, kSiteKLand, c.kb);
         }
       }
+      if (lane == 0) ms.qk_end[mine] = (c.kb + 1 - mine) / 2;      // of its own
     } else if (warp == kWarpPv) {
       // ---------------------------------------------------------- PV issue
       constexpr uint32_t idesc_pv = umma_idesc(0, 0, false, true, 64, 256);
       Cursor c{cid, 0, blocks_of(cid), 0, 0, 1, blocks_of(cid + ncta)};
       bool aborted = false;
-      unsigned long long since = 0;
+      uint32_t since = 0;
       unsigned polls = 0;
       while (c.tile < ng && !aborted) {
         // P written (its QK^T has read the K rows that are V here, so they have landed); an item's first PV
@@ -544,6 +548,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
           aborted = idle(polls, since, kSitePReady, c.kb);
         }
       }
+      if (lane == 0) ms.pv_end = c.kb;
     } else if (warp == kWarpValid) {
       // ---------------------------------------------------------- index-validity bits
       int kb = 0, lim_next = live_of(cid);
@@ -728,9 +733,25 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   }
 
   __syncthreads();
+  if (ms.left != 0) {
+    cp_async_wait_all();
+    if (threadIdx.x == 0) {
+      if (ms.q_asked != 0) {      // the last Q requested: with the arrivals of the warps that have left it counts as landed when it has
+        for (int i = 0; i < kGatherWarps; ++i)
+          if (ms.q_passed[i] < ms.q_asked) mbar_arrive(&ms.q_land);
+        mbar_drain(&ms.q_land, (ms.q_asked - 1) & 1);
+      }
+      for (int i = 0; i < 2; ++i) {      // block 2 (n - 1) + i was the warp's last
+        const uint32_t kb = 2 * (ms.qk_end[i] - 1) + i;
+        if (ms.qk_end[i] != 0) mbar_drain(&ms.qk_done[kb & 7], (kb >> 3) & 1);
+      }
+      if (ms.pv_end != 0) mbar_drain(&ms.pv_done[(ms.pv_end - 1) & 7], ((ms.pv_end - 1) >> 3) & 1);
+    }
+  }
   __syncwarp();
   if (warp == kWarpQk) tmem_dealloc_cta(tmem, kTmemCols);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_attn_status[3], 1);
+  if (threadIdx.x == 0) wt.report(g_attn_status, p.epoch);
 }
 #undef LT_WS_TS
 #undef LT_WS_SS
@@ -770,7 +791,7 @@ int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
   p.lse = a.lse;
   p.ng = a.ng; p.s_kv = a.s_kv; p.cap = a.topk; p.h_per_q = h; p.G = G;
   p.scale_log2 = a.sm_scale * kLog2e; p.out_scale = a.out_scale;
-  p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
+  p.epoch = next_launch_epoch(); p.wait_limit = wait_limit_ticks();
   p.q_bf16 = a.q_is_bf16 ? reinterpret_cast<const uint4*>(a.q8) : nullptr; p.q_inv = a.q_inv;
   p.q_codes = reinterpret_cast<uint8_t*>(q_codes);
   const bool wide = (int64_t)a.s_kv * (a.kv_row_stride >> 4) >= 0xffffffffll;

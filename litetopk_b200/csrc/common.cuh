@@ -22,6 +22,10 @@ namespace lt {
 // of a single device-side wait (default kWaitLimitNs; litedsa_set_wait_limit_ns changes it).
 int next_launch_epoch();
 unsigned long long wait_limit_ns();
+inline uint32_t wait_limit_ticks() {      // rounded up
+  const unsigned long long t = wait_limit_ns() >> 20;
+  return (uint32_t)(t < 0x7fffffffull ? t : 0x7fffffffull) + 1u;
+}
 
 // Arguments of the FP8 attention operator as every entry point of the library passes them
 // to the shared checker / launcher (attn_fp8.cu).
@@ -280,6 +284,46 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   return true;
 }
 
+// The same for kernels of many roles, whose some forty waits would each carry that report (as the kernels' code grew
+// by it, tiles of four blocks took 4 % longer): a wait that gives up leaves its site and iteration in a word of the
+// block's shared memory, which makes all others of the block give up, and the block reports it when it ends.
+struct BlockWaiter {
+  volatile uint32_t* left;      // 0: no wait of this block has given up; else site | iteration << 8
+  uint32_t limit;               // how long one wait may take, in ticks of 2^20 ns (wait_limit_ticks())
+  __device__ __forceinline__ static uint32_t ticks() {      // never 0
+    return (uint32_t)(globaltimer_ns() >> 20) | 1u;
+  }
+  __device__ __forceinline__ bool aborting() const { return *left != 0; }
+  // whether a wait that has not been satisfied gives up; `since` is 0 at its first look
+  __device__ __forceinline__ bool gives_up(uint32_t& since, int site, int iter) const {
+    const uint32_t now = ticks();
+    if (since == 0) since = now;
+    const bool gone = aborting(), late = now - since > limit;
+    if (late && !gone) *left = (uint32_t)site | (uint32_t)iter << 8;
+    return gone || late;
+  }
+  // at the end of the block, one thread
+  __device__ __forceinline__ void report(int* status, int epoch) const {
+    const uint32_t v = *left;
+    if (v != 0) Waiter{status, epoch, 0}.fail((int)(v & 255u), (int)(v >> 8));
+  }
+};
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const BlockWaiter& w, int site, int iter = 0) {
+  uint32_t since = 0;
+  while (!mbar_try_wait(bar, parity))
+    if (w.gives_up(since, site, iter)) return false;
+  return true;
+}
+
+// A launch that gives up still waits for what it has in flight before its blocks retire: a bulk load that lands later
+// would write shared memory that already belongs to another block, and tensor memory would be freed under running
+// MMAs.  What is in flight ends by itself within some microseconds; the limit is for arrivals that never come.
+constexpr unsigned long long kDrainLimitNs = 1000000ull;
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const unsigned long long t0 = globaltimer_ns();
+  while (!mbar_test(bar, parity) && globaltimer_ns() - t0 < kDrainLimitNs) {}
+}
+
 // release at cluster scope: orders this thread's earlier (distributed) shared-memory stores
 __device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
@@ -400,6 +444,8 @@ __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src) {
 __device__ __forceinline__ void cp_async16_or_zero(uint32_t dst_smem, const void* src, bool read) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(read ? 16 : 0) : "memory");
 }
+// all cp.async of this thread have landed
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

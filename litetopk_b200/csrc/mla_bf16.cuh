@@ -104,7 +104,10 @@ struct Misc {
                                     // items of one or two blocks the next item's can be complete before the
                                     // epilogue has looked at this one's
   uint32_t valid[2][2];             // 64 validity bits per stage (gather)
-  uint32_t tmem_base, pad;
+  uint32_t tmem_base;
+  // for the tear-down of a launch that gives up: a wait of this block has; ring entries of Q that have been requested, items
+  // whose resident chunks have, and at whose q_land each K warp has arrived; leader: blocks whose QK^T and PV have been issued
+  uint32_t left, q_asked, q_res_asked, q_passed[kGatherWarps / 2], qk_end, pv_end;
   float xbuf[2][2][128];            // [group][parity][lane]: row-max exchange between key halves
   float mshare[2][64];              // [group][row]: running max after the group's latest block
   float fin_l[256];                 // end of item: row sums per thread,
@@ -121,7 +124,7 @@ struct Params {
   int ng, G, h_per_q;
   float scale_log2;
   int epoch;                          // this launch's epoch for the bounded waits
-  unsigned long long wait_limit_ns;
+  uint32_t wait_limit;       // of one wait, in ticks (BlockWaiter)
   // slices: every tile's blocks are cut into nsplit > 1 work items, each leaving its unnormalised
   // O (fp32 [ng * nsplit, 128, 512]) and (running max, row sum) for merge_slices
   int nsplit;
@@ -256,7 +259,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const uint32_t sbase = (raw + 1023u) & ~1023u;       // 128B-swizzle tiles need 1024-byte alignment
   uint8_t* sm = smem_raw + (sbase - raw);
   Misc& ms = *reinterpret_cast<Misc*>(sm + PL::kOffMisc);
-  const Waiter wt{g_status, p.epoch, p.wait_limit_ns};
+  const BlockWaiter wt{&ms.left, p.wait_limit};
   pdl_trigger();
   pdl_wait();
   if (p.gate != nullptr && *reinterpret_cast<const volatile int*>(p.gate) != p.gate_value) return;   // grid-uniform
@@ -303,6 +306,8 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_res, 1);
     mbar_init(&ms.q_land, kQEntries + (kTma ? 0 : kGatherWarps / 2 - 1));      // gather: and the other K warps
+    ms.left = ms.q_asked = ms.q_res_asked = ms.qk_end = ms.pv_end = 0;
+    for (int i = 0; i < kGatherWarps / 2; ++i) ms.q_passed[i] = 0;
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
     mbar_init(&ms.q_free, 1);
     mbar_init(&ms.o_free, 2 * kEpiWarps);
@@ -341,11 +346,14 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   const uint32_t tmem = __shfl_sync(0xffffffffu, ms.tmem_base, 0);
 
   // Requests half `e` of an item's Q chunks for tensor memory into ring slot `slot` (one thread); the
-  // other chunks go into L2, for the fetch that follows the previous item's last QK^T.
+  // other chunks go into L2, for the fetch that follows the previous item's last QK^T.  (Nothing behind a wait that gave
+  // up: the Q before could still be in flight.)
   const uint64_t pol_stream = l2_policy_evict_first();
   const int q_head = (64 * (int)cta) % p.h_per_q, q_tok0 = (64 * (int)cta) / p.h_per_q;
-  auto request_q = [&](int w, int e, int slot) {
+  auto request_q = [&](int w, int it, int e, int slot) {
     constexpr int kPer = kQChunksTmem / kQEntries;
+    if (wt.aborting()) return;
+    ms.q_asked = kQEntries * it + e + 1;
     const int qt = (kSliced ? w / p.nsplit : w) * p.G + q_tok0;
     mbar_arrive_expect_tx(&ms.q_land, kPer * kQChunkBytes);
     for (int j = 0; j < kPer; ++j)
@@ -585,15 +593,8 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
      }
    };
    // the time-limit and abort check of a wait that has not been satisfied yet (warp-uniform answer)
-   auto mma_idle = [&](unsigned long long& since, int site, int kb) -> bool {
-     const unsigned long long now = globaltimer_ns();
-     if (since == 0) since = now;
-     bool stop = wt.aborting();
-     if (now - since > wt.limit_ns) {
-       if (lane == 0) wt.fail(site, kb);
-       stop = true;
-     }
-     return __any_sync(0xffffffffu, stop);
+   auto mma_idle = [&](uint32_t& since, int site, int kb) -> bool {
+     return __any_sync(0xffffffffu, wt.gives_up(since, site, kb));
    };
    if (warp == kWarpMma) {
     // ------------------------------------------------------------ QK^T issue (leader CTA)
@@ -622,7 +623,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       };
       MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, kQEntries};
       bool aborted = false;
-      unsigned long long since = 0;
+      uint32_t since = 0;
       while (c.w < n_items && !aborted) {
         // K rows landed on both CTAs, S buffer drained and, for an item's first block, Q in place
         const uint32_t ph = (c.kb >> 3) & 1;
@@ -637,6 +638,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           aborted = mma_idle(since, kSiteKFull, c.kb);
         }
       }
+      if (lane == 0) ms.qk_end = c.kb;
     }
    } else if (warp == (kTma ? kWarpValid : kWarpK) && cta == 0) {
     // ------------------------------------------------------------ PV issue (leader CTA)
@@ -663,7 +665,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       };
       MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, kQEntries};
       bool aborted = false;
-      unsigned long long since = 0;
+      uint32_t since = 0;
       while (c.w < n_items && !aborted) {
         // V rows landed on both CTAs, P written; an item's first PV overwrites O: the previous item
         // must have read it out
@@ -679,6 +681,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           aborted = mma_idle(since, kSitePReady, c.kb);
         }
       }
+      if (lane == 0) ms.pv_end = c.kb;
    } else if (kTma && (warp == kWarpK || warp == kWarpV)) {
     // ------------------------------------------------------------ TMA producers (tiled loads, one lane)
     if (lane == 0) {
@@ -694,7 +697,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         for (int e = 0; e < kQEntries && ok; ++e) {
           if (!is_v) {
             if (ring > 0) ok = mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteQFree, kb);
-            if (ok) request_q(w, e, slot);
+            if (ok) request_q(w, it, e, slot);
           }
           advance();
         }
@@ -795,7 +798,8 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // (chunk -> 32 columns; lane = row, duplicated in lanes 64-127)
     auto bring_q = [&](int w, int j, int n) {
       if (j > 0) mbar_wait(&ms.q_free, (j - 1) & 1, wt, kSiteQFree, j);
-      if (e_tid == 0) {
+      if (e_tid == 0 && !wt.aborting()) {
+        ms.q_res_asked = j + 1;
         const int qt = (kSliced ? w / p.nsplit : w) * p.G + q_tok0;
         if (cta == 0) mbar_arrive_expect_tx(&ms.q_res, 2 * kQRes * kQChunkBytes);
         for (int i = 0; i < kQRes; ++i)
@@ -927,27 +931,30 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       else if (w + ncl < n_items) idx = load_idx(nx, 0);
       return cur;
     };
+    bool ok = true, go = true;                     // none of this lane's / this warp's waits has given up: then it leaves
     if (is_k) {
-      for (int w = cid; w < n_items; w += ncl, ++it) {
+      for (int w = cid; go && w < n_items; w += ncl, ++it) {
         const Item t = nx;
         if (w + ncl < n_items) nx = item_of(w + ncl);
         // The item's Q entries, requested by warp 0.  Every warp goes through their slots' barriers and that of the
         // previous Q (whose bytes could, with short items, still be in flight), and Q counts as landed only when
         // all of them have: no warp is overtaken and tests a phase that is two ahead.
-        if (it > 0) mbar_wait(&ms.q_taken[(it - 1) & 1], ((it - 1) >> 1) & 1, wt, kSiteQ, it);
+        if (it > 0) ok &= mbar_wait(&ms.q_taken[(it - 1) & 1], ((it - 1) >> 1) & 1, wt, kSiteQ, it);
         for (int e = 0; e < kQEntries; ++e) {
-          if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
+          if (ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
           __syncwarp();
-          if (pw == 0 && lane == 0) request_q(w, e, slot);
+          if (pw == 0 && lane == 0 && ok) request_q(w, it, e, slot);
           __syncwarp();
           advance();
         }
-        if (pw != 0 && lane == 0) mbar_arrive(&ms.q_land);
+        if (pw != 0 && lane == 0 && ok && !wt.aborting()) {
+          ms.q_passed[pw] = it + 1;
+          mbar_arrive(&ms.q_land);
+        }
         for (int k = 0; k < t.nb; ++k, ++kb) {
           const int cur = take_idx(t, k, w);
-          const bool full = __all_sync(0xffffffffu, cur >= 0);
-          if (ring > 0) mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
-          __syncwarp();
+          if (ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, k);
+          const bool full = __all_sync(0xffffffffu, cur >= 0 && ok);
           const uint32_t kst = sbase + PL::kOffKV + slot * PL::kSlot + 8 * pw * 128;
           if (full) {
 #pragma unroll
@@ -957,6 +964,8 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                          kvb + (size_t)ri * pitch + 512 * (i & 1) + 16 * lane);
             }
           } else {
+            go = __all_sync(0xffffffffu, ok);
+            if (!go) break;
 #pragma unroll 1
             for (int i = 0; i < 16; ++i) {
               const int ri = __shfl_sync(0xffffffffu, cur, i >> 1);
@@ -978,14 +987,15 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       }
     } else {
       const uint8_t* src = kvb + 512 * (int)cta + 16 * lane;
-      for (int w = cid; w < n_items; w += ncl) {
+      for (int w = cid; go && w < n_items; w += ncl) {
         const Item t = nx;
         if (w + ncl < n_items) nx = item_of(w + ncl);
         for (int e = 0; e < kQEntries; ++e) advance();
         for (int k = 0; k < t.nb; ++k, ++kb) {
           const int cur = take_idx(t, k, w);
-          mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, k);
-          __syncwarp();
+          ok &= mbar_wait(&ms.qk_done[kb & 7], (kb >> 3) & 1, wt, kSiteVFree, k);
+          go = __all_sync(0xffffffffu, ok);
+          if (!go) break;
           const uint32_t vst = sbase + PL::kOffKV + slot * PL::kSlot + ((cta == 0 ? 4 : 0) + cj) * kChunkBytes + 8 * pw * 128;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -1001,10 +1011,30 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   // tear-down: nobody may still be reading TMEM of either CTA when it is released
   __syncthreads();
+  if (ms.left != 0) {
+    cp_async_wait_all();
+    if (threadIdx.x == 0) {
+      const unsigned long long t0 = globaltimer_ns();
+      const uint32_t n = ms.q_asked, items = (n + kQEntries - 1) / kQEntries;
+      if (n != 0) {               // the last Q requested: with the arrivals that are missing it counts as landed when it has
+        for (uint32_t i = n; i < kQEntries * items; ++i) mbar_arrive(&ms.q_land);
+        for (int i = 1; !kTma && i < kGatherWarps / 2; ++i)
+          if (ms.q_passed[i] < items) mbar_arrive(&ms.q_land);
+        mbar_drain(&ms.q_land, (items - 1) & 1);
+      }
+      if (cta == 0 && ms.q_res_asked != 0) mbar_drain(&ms.q_res, (ms.q_res_asked - 1) & 1);      // both CTAs' bytes
+      if (ms.qk_end != 0) mbar_drain(&ms.qk_done[(ms.qk_end - 1) & 7], ((ms.qk_end - 1) >> 3) & 1);
+      if (ms.pv_end != 0) mbar_drain(&ms.pv_done[(ms.pv_end - 1) & 3], ((ms.pv_end - 1) >> 2) & 1);
+      // K and V by TMA: the leader's barriers count the bytes of both CTAs, of which one may have asked for none.  No load
+      // takes a tenth of this.
+      while (kTma && globaltimer_ns() - t0 < 100000ull) {}
+    }
+  }
   __syncwarp();
   cluster_sync_all();
   if (warp == kWarpMma) tmem_dealloc_pair(tmem, kTmemCols);
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&g_status[3], 1);
+  if (threadIdx.x == 0) wt.report(g_status, p.epoch);
 }
 
 // how many 2-CTA clusters of this kernel device `dev` (the current one) can hold at once
