@@ -134,7 +134,7 @@ def masked_mla_refnum(q8f: torch.Tensor, kv8f: torch.Tensor, union_idx: torch.Te
                       p_quant: str = "e4m3", block: int = BLOCK, p_scale_log2: float = P_SCALE_LOG2,
                       attn_sink: Optional[torch.Tensor] = None,
                       topk_length_per_q: Optional[torch.Tensor] = None, q_group_div: int = 1,
-                      ranges=None):
+                      ranges=None, threshold: float = RESCALE_THRESHOLD, ahead: bool = False):
     """Reference-numerics oracle of the masked MLA kernels.
 
     Defaults restate the FP8 kernel (kernels/b200/dsa/litedsa_attention_sm100.cuh:1961-2189):
@@ -145,6 +145,9 @@ def masked_mla_refnum(q8f: torch.Tensor, kv8f: torch.Tensor, union_idx: torch.Te
     keys, P = e4m3(7 * 2^(s*c - m)).
     With ``block=64, p_quant="bf16", p_scale_log2=0`` and bf16-representable q / kv it restates
     the bf16 kernel (litedsa_attention_sm100_dsv4.cuh:2015-2157).
+
+    With ``q8f`` [ng,64,d], ``block=64, threshold=5.5, ahead=True`` it restates the FP8 kernel on tiles of 64 rows, where a
+    running max that moves also covers the maxima of the block behind.
 
     Optional modes of the kernels' parameter block: ``attn_sink`` [128] per packed row joins
     the output normaliser only (litedsa_attention_sm100.cuh:2127-2133); ``topk_length_per_q``
@@ -160,7 +163,7 @@ def masked_mla_refnum(q8f: torch.Tensor, kv8f: torch.Tensor, union_idx: torch.Te
     """
     ng, cap = union_idx.shape
     rows, d = q8f.shape[1], q8f.shape[2]
-    assert rows == 128 and q8f.shape[0] * q_group_div == ng
+    assert rows in (64, 128) and q8f.shape[0] * q_group_div == ng
     s_kv = kv8f.shape[0]
     G = rows // h_per_q
     c = torch.tensor(sm_scale, dtype=torch.float32) * torch.tensor(LOG2E, dtype=torch.float32)
@@ -194,20 +197,27 @@ def masked_mla_refnum(q8f: torch.Tensor, kv8f: torch.Tensor, union_idx: torch.Te
         li = torch.zeros((n, rows), dtype=torch.float32)
         real_m = torch.full((n, rows), float("-inf"), dtype=torch.float32)
         O = torch.zeros((n, rows, d_v), dtype=torch.float32)
-        for b in range(nblk):
+        def logits(b):                                                  # of block b, its rows' maxima, its keys
             idx = union_idx[g0:g1, b * block:(b + 1) * block].long()    # [n,block]
             rank = b * block + torch.arange(block)[None, :]
             ok = (idx >= 0) & (idx < s_kv)
             kvb = kv_pad[torch.where(ok, idx, torch.full_like(idx, s_kv))]  # [n,block,d]
             col_valid = ok & (rank < cnt[:, None])
-            bits = tok[:, :, b * block:(b + 1) * block].repeat_interleave(h_per_q, dim=1)  # [n,128,block]
+            bits = tok[:, :, b * block:(b + 1) * block].repeat_interleave(h_per_q, dim=1)  # [n,rows,block]
             valid = bits & col_valid[:, None, :]
             s = torch.einsum("grd,gkd->grk", qf, kvb)                   # fp32 accumulate
             s = s.masked_fill(~valid, float("-inf"))
-            cur = s.amax(dim=2) * c                                     # [n,128]
+            return s, s.amax(dim=2) * c, kvb
+
+        behind = logits(0)
+        for b in range(nblk):
+            s, cur, kvb = behind
+            behind = logits(b + 1) if b + 1 < nblk else (None, torch.full_like(cur, float("-inf")), None)
             real_m = torch.maximum(real_m, cur)
-            over = (cur - m) > RESCALE_THRESHOLD
-            vote = over.view(n, 4, 32).any(dim=2, keepdim=True).expand(n, 4, 32).reshape(n, rows)
+            over = (cur - m) > threshold
+            vote = over.view(n, rows // 32, 32).any(dim=2, keepdim=True).expand(n, rows // 32, 32).reshape(n, rows)
+            if ahead:
+                cur = torch.maximum(cur, behind[1])
             new_m = torch.where(vote, torch.maximum(cur, m), m)
             scale_old = torch.where(vote, torch.exp2(m - new_m), torch.ones_like(m))
             m = new_m

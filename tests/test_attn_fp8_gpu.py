@@ -471,7 +471,8 @@ def test_sparse_prefill_in_one_call_equals_its_operators(tokens, heads, topk, s_
     api.attn_status(reset=True)
     want_o, want_l = api.masked_mla_fp8(q8.view(tokens, heads, 576).to(DEV), kvd, u, m, synth.SM_SCALE, counts=c,
                                         kv_scale=ks, q_scale=qs)
-    # a chunk of a large job: no slices, the same kernels on the same operands
+    # the 128-row form without slices (that of litedsa_sparse_prefill for a chunk of a large job): the same kernels on the
+    # same operands.  (sparse_prefill runs such a job on 64-row tiles, whose P are rounded to other maxima: below.)
     o1, l1 = api._sparse_prefill(qd, kvd, idd, synth.SM_SCALE, ks, qs, None, None, None, 100000)
     assert torch.equal(o1, want_o) and torch.equal(l1, want_l)
     # on its own: slices.  Their running maxima differ from the unsliced tile's, hence the e4m3
@@ -595,6 +596,52 @@ def test_calls_of_many_tokens_on_64_row_tiles(tokens, heads, topk, s_kv):
     out_e, lse_e = ao.mla_exact(q8[some].view(torch.float8_e4m3fn).float() * qs, kvf, uniq, synth.SM_SCALE)
     mad, cos = ao.compare(out[some].cpu(), out_e)
     assert cos >= 0.9995 and float((lse[some].cpu() - lse_e.float()).abs().max()) <= TOL_LSE, (mad, cos)
+
+
+@pytest.mark.parametrize("tokens,heads,topk,s_kv", [
+    (380, 64, 256, 4096),        # four blocks of one token's list
+    (602, 64, 960, 7777),        # fifteen: the last one has none behind it
+    (1300, 32, 512, 5001),
+    (2376, 16, 256, 3000),
+    (4752, 8, 272, 2500),        # a union row that is no multiple of 128
+])
+@pytest.mark.parametrize("spread", [1.0, 4.0])           # no move of the running max behind the first block / many
+def test_64_row_tiles_match_their_numerics_tile_by_tile(tokens, heads, topk, s_kv, spread):
+    # the restatement on some tiles, each held to the 128-row kernels' tolerances by itself: one wrong value row shows
+    G = 64 // heads
+
+    def mutate(idx):
+        idx = idx.clone()
+        for i, n in enumerate((0, 1, 63, 64, 65, 127, 128, 129)):
+            idx[8 * i:8 * i + 8, n:] = -1
+        return idx
+    w, idx, kv, q = _case(tokens, heads, topk, s_kv, (0.5, 0.9), seed=27, mutate=mutate)
+    q8, kv8, qs, ks = synth.refcompat_operands(q.float() * spread, kv)
+    q8 = q8.view(tokens, heads, 576)
+    api.attn_status(reset=True)
+    out, lse = api.sparse_prefill(q8.to(DEV), kv8.to(DEV), idx.to(DEV), synth.SM_SCALE, kv_scale=ks, q_scale=qs)
+    torch.cuda.synchronize()
+    assert api.attn_status()[0] == 0
+    ng = tokens // G
+    tiles = torch.tensor(sorted({*range(0, min(64 // G, ng), max(1, 8 // G)), *range(64 // G, ng, ng // 16)}))
+    t = (tiles[:, None] * G + torch.arange(G)).flatten()
+    lists = idx[t]
+    if G * topk % 128:                                   # the oracle's rows are G * k entries; the kernel's are padded
+        lists = torch.cat([lists, torch.full((len(t), 128 // G - topk % (128 // G)), -1, dtype=lists.dtype)], dim=1)
+    u, c, m = uo.union_qm_oracle(lists.numpy(), G, (s_kv + 1023) // 1024 * 1024)
+    want_o, want_l, _ = ao.masked_mla_refnum(
+        q8[t].view(torch.float8_e4m3fn).float().view(len(tiles), 64, 576), kv8.view(torch.float8_e4m3fn).float(), torch.from_numpy(u),
+        torch.from_numpy(c), torch.from_numpy(m.astype(np.int64)), synth.SM_SCALE * qs * ks, ks, heads, block=64, threshold=5.5, ahead=True)
+    out, lse = out.cpu().view(ng, 64, 512)[tiles], lse.cpu().view(ng, 64)[tiles]
+    fin = torch.isfinite(want_l)
+    assert torch.equal(torch.isfinite(lse), fin) and float((lse[fin] - want_l[fin]).abs().max()) <= TOL_LSE
+    for i in range(len(tiles)):
+        if not bool(fin[i].any()):
+            assert not bool(out[i].any())
+            continue
+        # (few keys per row: |out| reaches several units, where one bf16 ulp exceeds 1e-2 absolute)
+        mad, cos = ao.compare(out[i], want_o[i])
+        assert mad <= TOL_ABS * max(1.0, float(want_o[i].float().abs().max())) and cos >= TOL_COS, (int(tiles[i]), mad, cos)
 
 
 @pytest.mark.parametrize("form", ["litedsa_sparse_prefill", "litedsa_sparse_prefill_job"])
