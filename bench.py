@@ -696,7 +696,7 @@ def stock_sparse_mla(w, dev, steps):
            "out_cosine": float(torch.nn.functional.cosine_similarity(a, b, dim=0)),
            "out_max_abs_diff": float((a - b).abs().max()),
            "lse_max_abs_diff": float((lse - lse_ref[:, :w.heads]).abs().max()),
-           "note": "ours = union_qm + masked_mla_fp8 (e4m3 P): cosine ~0.9998 against a bf16 kernel is its quantisation"}
+           "note": "ours = sparse_prefill (union and FP8 attention, e4m3 P): cosine ~0.9998 against a bf16 kernel is its quantisation"}
     del idx, q8, kv8, kv_bf16, q_bf16, ind, o_ref, lse_ref, out, lse
     torch.cuda.empty_cache()
     return rec

@@ -12,8 +12,8 @@
 //   * tcgen05.mma.ws with M = 64: the form that spreads 64 rows over all 128 TMEM lanes (lanes 0-63 the
 //     first half of an instruction's columns, lanes 64-127 the second), which plain M = 64 does not (half
 //     the rate).  A block's 64 K rows are also its V rows: nothing is fetched twice and nothing crosses CTAs.
-//     Measured cycles per K step of 32 bytes: QK^T (N = 64, A in TMEM) 28, PV (N = 256) 80 -- operand
-//     bytes / 128, the shared-memory rate -- so 830 per block of 64 x 64.
+//     Measured cycles per K step of 32 bytes: QK^T (N = 64, A in TMEM) 28, although its K rows are 16 shared-memory
+//      wavefronts of 128 bytes; PV (N = 256) 80, the wavefronts of both operands.  So 830 per block of 64 x 64.
 //   * six 36 KB slots in a ring hold the blocks in flight (and each item's Q on its way to TMEM).
 //   * warps 0-15   softmax, four groups of four warps on every fourth block each (TMEM lane x 32 columns per
 //                  thread); the running max is handed from group to group, row sums are merged by the
@@ -22,10 +22,11 @@
 //     warps 24, 27 QK^T issue, even and odd blocks;   warp 25  PV issue;   warp 26  index-validity bits;
 //     warps 28-31  Q tiles in, tile epilogue.
 //   * every wait is bounded (common.cuh).
-// What bounds it is shared memory: per block 640 wavefronts of 128 bytes for the MMAs' operands, 290 of the threads
-// and barriers, 288 of the copies, in 1030 cycles inside a tile and 1190 over tiles.  8192 tokens x 64
-// heads, top-2048, with the union: 1504 us on 128-row tiles, 1271 here; 16384 x 32, top-1024 1240 / 952; 16384 x 16,
-// top-2048 of 131072 1869 / 1308 (e4m3 queries, short runs; long ones meet the power limit: 1880 / 1570 for the first).
+// What bounds it is not settled: 1170 cycles per block over tiles, about 1030 inside one, against 830 of the MMAs.  Of the
+// shared-memory pipe's wavefronts the MMAs' operands take 640 per block and threads, barriers and copies 338,
+// 83 % of the cycles together; the tensor pipe is busy 48 % of them, issue slots 59 %.  With the union, e4m3 queries, us on
+// 128-row tiles and here: 8192 tokens x 64 heads, top-2048 1420 / 1265; 16384 x 32, top-1024 1201 / 961; 16384 x 16,
+// top-2048 of 131072 1780 / 1330-1490 (long runs meet the power limit); 4096 x 64, top-256 181 / 137.
 #pragma once
 
 namespace lt {

@@ -905,9 +905,8 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // 16-byte copies written straight into the 128-byte-swizzled layout, completion reported to an mbarrier by an
     // asynchronous arrival.  Four warps fetch K rows (this CTA's 32 keys, all dims: warp pw rows [8 pw, 8 pw + 8)) as
     // soon as the slot's previous entry is dead, the other four V rows (the PEER's 32 keys, this CTA's 256
-    // value dims) into the dead half of the slot as soon as the block's QK^T is complete.  (Eight warps that polled
-    // for both in turn were late for either: see attn_fp8.cu.  They kept in q_held which slots had last held
-    // a Q.)  Entries without a valid index become zeros without a read.
+    // value dims) into the dead half of the slot as soon as the block's QK^T is complete.  (Eight warps that polled for both
+    // in turn were late for either: see attn_fp8.cu.)  Entries without a valid index become zeros without a read.
     const int pw = (warp - kWarpGather0) & 3;
     const bool is_k = warp < kWarpGather0 + kGatherWarps / 2;
     const uint8_t* kvb = p.kv;

@@ -120,10 +120,16 @@ static int check_shape(int T, int h, int k, int policy_tokens) {
 // Whether a job of `tokens` tokens runs on 64-row tiles (attn_fp8_r64.cuh) instead of 128-row ones: with an FP8
 // cache, up to 64 heads, lists of a tile of 256 entries and more, a tile for every other SM and at least ten key
 // blocks per SM.  (Fewer tiles run faster as slices of 128-row ones: 40 tiles of 16 heads, top-2048, 60 us
-// against 65; with less work both forms take the 23 us of a call's launches.)  128-row / 64-row tiles, e4m3 queries, half and nine tenths of the lists shared, us: 74 tiles x 64 heads, top-2048 39 / 30 and
-// 35 / 29; 16 heads, top-2048 71 / 59 and 45 / 39; 222 x 32 heads, top-2048 104 / 76
-// and 63 / 65; 1184 tiles x 64 heads, top-256 59 / 51 and 84 / 51, top-2048 276 / 199 and 233 / 202; 32 heads
-// 430 / 295 and 263 / 246; 16 heads 770 / 456 and 376 / 296; 8 heads 1403 / 806 and 572 / 429.
+// against 65 when the line was drawn; with less work both forms take the 23 us of a call's launches.)
+// 128-row / 64-row tiles, half and nine tenths of the lists shared, e4m3 queries, us (bf16 queries: much the same, but
+// 67 / 70 at 222 tiles and nine tenths, 87 / 82 with top-256):
+//   74 tiles of 64 rows: 64 heads, top-2048    35 / 28 and 32 / 28;    16 heads 64 / 57 and 41 / 37
+//   222: 32 heads, top-2048                    98 / 75 and 72 / 71
+//   1184: 64 heads, top-256 58 / 45 and 57 / 45, top-2048 249 / 189 and 196 / 188;    32 heads, top-2048 394 / 274 and
+//         228 / 220;    16 heads 687 / 442 and 300 / 262;    8 heads 1298 / 779 and 448 / 352
+// The more of the lists is shared, the less there is to gain: over 7700 calls (sharing 30 to 97 %, both query types) 6 % were
+// slower, by up to 13 %, nearly all with nine tenths shared and more and two or three rounds of tiles.  How
+// much is shared is not known on the host.
 static bool use_rows64(int tokens, int h, int k, bool kv_bf16) {
   if (kv_bf16 || h > 64 || (int64_t)(128 / h) * k % 128 != 0) return false;
   const int64_t tiles = (int64_t)tokens * h / 64, list = (int64_t)(64 / h) * k;
