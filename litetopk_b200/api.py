@@ -687,7 +687,8 @@ def _quantise_first(ng: int, G: int, cap: int) -> bool:
     the kernel / with the pass: top-256 579 / 445 us, top-512 614 / 543, top-1024 823 / 843).  The union
     of several tokens is not known here: only tiles of a single block (4096 x 64 heads, top-64 278 / 221
     and 288 / 268 us at half and nine tenths sharing; top-256 302 / 252 but 327 / 344).  Few tiles
-    have nothing to hide."""
+    have nothing to hide.  (``ng`` and ``cap`` are of 128-row tiles.  Jobs on 64-row tiles have lists of 512 entries a pair of
+    tiles and more, so there this is never true: their queries are quantised a tile ahead.)"""
     return ng > 296 and cap <= (512 if G == 1 else 128)
 
 

@@ -234,7 +234,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  Every wait in the library goes through here: it gives up after the
+// Bounded wait.  Every wait in the library goes through this or the form for many roles below: it gives up after the
 // launch's time limit, or as soon as any other wait of the SAME launch gave up (the abort
 // word carries that launch's epoch), records where, and returns false.  Callers then fall
 // through to their normal tear-down, so a lost arrival costs a wrong result and an error
