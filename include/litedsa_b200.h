@@ -196,7 +196,8 @@ int litedsa_attn_status(int* out4_host, int reset);
 
 /*
  * Limit of one device-side wait for all later launches of this process, in nanoseconds
- * (0 restores the default, 2 s).  *previous_ns (may be NULL) receives the old value.
+ * (0 restores the default, 2 s).  *previous_ns (may be NULL) receives the old value.  The attention kernels
+ * count in units of 2^20 ns (1.05 ms), rounded up.
  */
 int litedsa_set_wait_limit_ns(uint64_t limit_ns, uint64_t* previous_ns);
 

@@ -803,7 +803,7 @@ def sparse_prefill(q: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_idx: torch.
     fp32; one of many tokens with an FP8 cache and up to 64 heads unites the lists of 64 query rows
     instead of 128.  Either way softmax weights are rounded relative to another running maximum, so the
     result of some tokens alone and inside a larger call can differ by that rounding (e4m3 or bf16; none
-    is closer to the exact result).  What a tile is and how it is cut depends on ``job_tokens`` alone, by
+    is further from the exact result than that of the operators).  What a tile is and how it is cut depends on ``job_tokens`` alone, by
     default the call's own number of tokens: state the tokens of the whole job when this call is a part of
     it, and its tokens get the bits that they have in one call of the job.
     """
