@@ -26,14 +26,14 @@
 //     other chunks stay in shared memory and are fetched as soon as the previous item's last QK^T is
 //     complete (prefetched into L2 before).
 //   * half of P lies in the block's own rope chunk, dead after QK^T, too (576 dims).
-// Roles (16 warps, 24 with the gather):
+// Roles (17 warps, 24 with the gather):
 //   warps 0-7   softmax, two groups of four on alternate blocks (TMEM lane x 32 columns per thread);
-//   warp 8      QK^T issue (leader CTA);
+//   warp 8      QK^T issue of even blocks (leader CTA);
 //   warps 9-10  TMA producers of Q / K and of V -- or, with the gather, relays of "K / V landed" from
-//               the peer CTA to the leader, and in the leader PV issue (warp 9);
+//               the peer CTA to the leader, and in the leader PV issue (warp 9) and QK^T issue of odd blocks (warp 10);
 //   warp 11     PV issue (leader CTA) -- or, with the gather, index-validity bits;
 //   warps 12-15 Q into tensor memory; tile epilogue: O out of TMEM, x 1 / normaliser, bf16, TMA stores;
-//   warps 16-23 KV row gather (gather only).
+//   warp 16     QK^T issue of odd blocks (leader CTA) -- or, warps 16-23, KV row gather.
 // No TMA multicast of any kind.  Every wait is bounded (common.cuh).
 #pragma once
 #include "common.cuh"
@@ -56,7 +56,7 @@ constexpr uint32_t kPHalf = 64 * kOwnKeys * 2;        // 64 rows x 32 keys of P
 constexpr uint32_t kStageBytes = 4 * 2048;            // output staging, one slice per epilogue warp
 constexpr uint32_t kMiscBytes = 6144;
 
-constexpr int threads_of(Source src) { return src == kGather ? 768 : 512; }
+constexpr int threads_of(Source src) { return src == kGather ? 768 : 544; }
 
 template <int kD>
 struct Plan {
@@ -106,8 +106,8 @@ struct Misc {
   uint32_t valid[2][2];             // 64 validity bits per stage (gather)
   uint32_t tmem_base;
   // for the tear-down of a launch that gives up: a wait of this block has; ring entries of Q that have been requested, items
-  // whose resident chunks have, and at whose q_land each K warp has arrived; leader: blocks whose QK^T and PV have been issued
-  uint32_t left, q_asked, q_res_asked, q_passed[kGatherWarps / 2], qk_end, pv_end;
+  // whose resident chunks have, and at whose q_land each K warp has arrived; leader: blocks whose QK^T (per issuing warp) and PV have been issued
+  uint32_t left, q_asked, q_res_asked, q_passed[kGatherWarps / 2], qk_end[2], pv_end;
   float xbuf[2][2][128];            // [group][parity][lane]: row-max exchange between key halves
   float mshare[2][64];              // [group][row]: running max after the group's latest block
   float fin_l[256];                 // end of item: row sums per thread,
@@ -254,6 +254,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   using PL = Plan<kD>;
   constexpr int kChunks = PL::kChunks, kQRes = PL::kQRes;
   constexpr bool kTma = kSrc != kGather;
+  constexpr int kWarpQkOdd = kTma ? kWarpGather0 : kWarpV;      // second QK^T warp: where the gather's peer has its V relay
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;       // 128B-swizzle tiles need 1024-byte alignment
@@ -306,10 +307,10 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (threadIdx.x == 0) {
     mbar_init(&ms.q_res, 1);
     mbar_init(&ms.q_land, kQEntries + (kTma ? 0 : kGatherWarps / 2 - 1));      // gather: and the other K warps
-    ms.left = ms.q_asked = ms.q_res_asked = ms.qk_end = ms.pv_end = 0;
+    ms.left = ms.q_asked = ms.q_res_asked = ms.qk_end[0] = ms.qk_end[1] = ms.pv_end = 0;
     for (int i = 0; i < kGatherWarps / 2; ++i) ms.q_passed[i] = 0;
     mbar_init(&ms.qt_ready, 2 * kEpiWarps);
-    mbar_init(&ms.q_free, 1);
+    mbar_init(&ms.q_free, 2);              // both QK^T warps
     mbar_init(&ms.o_free, 2 * kEpiWarps);
     for (int i = 0; i < 8; ++i) {
       mbar_init(&ms.k_full[i], kTma ? 1 : kGatherWarps / 2 * 32);     // gather: one async arrival per thread
@@ -578,7 +579,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       kb0 += nb;
       ++it;
     }
-  } else if (warp < kWarpEpi0) {
+  } else if (warp < kWarpEpi0 || (kTma && warp == kWarpQkOdd)) {
    // running position of an MMA-issuing warp: work item, block of the item, blocks of the item, item
    // ordinal, running block number, ring slot
    struct MmaCursor { int w, k, nb, it, kb, slot; };
@@ -596,11 +597,14 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
    auto mma_idle = [&](uint32_t& since, int site, int kb) -> bool {
      return __any_sync(0xffffffffu, wt.gives_up(since, site, kb));
    };
-   if (warp == kWarpMma) {
+   if (warp == kWarpMma || (warp == kWarpQkOdd && (kTma || cta == 0))) {
     // ------------------------------------------------------------ QK^T issue (leader CTA)
-    // Two warps issue the MMAs, one QK^T and one PV: each waits for its own operands and the tensor
-    // pipe takes what comes first.  (One warp polling for both needed 150-300 cycles per look and
-    // could not look at all while its MMAs filled the queue.)
+    // Three warps issue the MMAs, two QK^T, of even and odd blocks, and one PV: each waits for its own operands and the
+    // tensor pipe takes what comes first.  (One warp polling for all needed 150-300 cycles per look and
+    // could not look at all while its MMAs filled the queue.  With one for QK^T there were 600 cycles, 420 without the gather,
+    // from its last MMA of a block to its first of the next, cursor, polls and commits, with the pipe idle as soon as it had
+    // caught up: per 64-key block 1880 and 1450 cycles; native cache, 1184 tokens x 64 heads, top-2048 375 -> 354 us,
+    // ranges, 1184 x 64 at 131072 159 -> 156.)
     if (cta == 0) {
       constexpr uint32_t idesc_qk = umma_idesc(1, 1, false, false, 128, kBlockKeys);
       const uint32_t a_qk_done = smem_u32(&ms.qk_done[0]), a_qk_done_peer = mapa(a_qk_done, 1);
@@ -608,7 +612,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const uint64_t q_desc = umma_desc(sbase + PL::kOffQ, 16, 1024, kSwz128);
       static_assert(kChunkBytes >> 4 == 256 && kQChunkBytes >> 4 == 512, "strides of the MMA loops");
       // S of block kb goes into S buffer kb % 2
-      auto issue_qk = [&](int kb, int slot, bool last) {
+      auto issue_qk = [&](int kb, int slot) {
         if (!kTma) fence_proxy_async_smem();     // rows written by cp.async, read through the async proxy
         tc_fence_after();
         const uint64_t kd = umma_desc(sbase + PL::kOffKV + slot * PL::kSlot, 16, 1024, kSwz128);
@@ -617,28 +621,41 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                    (uint32_t)(kd >> 32), idesc_qk);
         commit_one(a_qk_done + 8u * (uint32_t)(kb & 7));
         commit_one(a_qk_done_peer + 8u * (uint32_t)(kb & 7));
-        if (last) { commit_one(a_q_free); commit_one(a_q_free_peer); }
         }
         __syncwarp();
       };
+      const int mine = warp == kWarpMma ? 0 : 1;
       MmaCursor c{cid, 0, cid < n_items ? item_of(cid).nb : 0, 0, 0, kQEntries};
+      auto step = [&]() {
+        const int it = c.it;
+        mma_next(c);
+        if (c.it != it && elect_one()) {      // this warp's QK^T of the item, if it had any
+          commit_one(a_q_free);
+          commit_one(a_q_free_peer);
+        }
+        __syncwarp();
+      };
       bool aborted = false;
       uint32_t since = 0;
       while (c.w < n_items && !aborted) {
-        // K rows landed on both CTAs, S buffer drained and, for an item's first block, Q in place
+        // K rows landed on both CTAs, S buffer drained and, for an item's first block, Q in place.  Both warps stop at
+        // every item's first block, whoever's it is: one that had none in an item could otherwise report two items
+        // as read before the other has read one.
         const uint32_t ph = (c.kb >> 3) & 1;
+        const bool own = (c.kb & 1) == mine;
         const bool ok = (c.k > 0 || (mbar_try_wait(&ms.qt_ready, c.it & 1) && mbar_try_wait(&ms.q_res, c.it & 1))) &&
-                        mbar_try_wait(&ms.k_full[c.kb & 7], ph) && (kTma || mbar_try_wait(&ms.k_peer[c.kb & 7], ph)) &&
-                        (c.kb < 2 || mbar_try_wait(&ms.s_free[c.kb & 1], ((c.kb >> 1) & 1) ^ 1));
+                        (!own || (mbar_try_wait(&ms.k_full[c.kb & 7], ph) && (kTma || mbar_try_wait(&ms.k_peer[c.kb & 7], ph)) &&
+                                  (c.kb < 2 || mbar_try_wait(&ms.s_free[c.kb & 1], ((c.kb >> 1) & 1) ^ 1))));
         if (__all_sync(0xffffffffu, ok)) {
-          issue_qk(c.kb, c.slot, c.k == c.nb - 1);
-          mma_next(c);
+          if (own) issue_qk(c.kb, c.slot);
+          step();
+          if (own && c.k != 0) step();      // the other warp's block
           since = 0;
         } else {
           aborted = mma_idle(since, kSiteKFull, c.kb);
         }
       }
-      if (lane == 0) ms.qk_end = c.kb;
+      if (lane == 0) ms.qk_end[mine] = (c.kb + 1 - mine) / 2;      // of its own
     }
    } else if (warp == (kTma ? kWarpValid : kWarpK) && cta == 0) {
     // ------------------------------------------------------------ PV issue (leader CTA)
@@ -1022,7 +1039,10 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         mbar_drain(&ms.q_land, (items - 1) & 1);
       }
       if (cta == 0 && ms.q_res_asked != 0) mbar_drain(&ms.q_res, (ms.q_res_asked - 1) & 1);      // both CTAs' bytes
-      if (ms.qk_end != 0) mbar_drain(&ms.qk_done[(ms.qk_end - 1) & 7], ((ms.qk_end - 1) >> 3) & 1);
+      for (int i = 0; i < 2; ++i) {      // block 2 (n - 1) + i was the warp's last
+        const uint32_t kb = 2 * (ms.qk_end[i] - 1) + i;
+        if (ms.qk_end[i] != 0) mbar_drain(&ms.qk_done[kb & 7], (kb >> 3) & 1);
+      }
       if (ms.pv_end != 0) mbar_drain(&ms.pv_done[(ms.pv_end - 1) & 3], ((ms.pv_end - 1) >> 2) & 1);
       // K and V by TMA: the leader's barriers count the bytes of both CTAs, of which one may have asked for none.  No load
       // takes a tenth of this.

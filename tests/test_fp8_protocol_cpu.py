@@ -204,6 +204,7 @@ def pair(blocks, bf16_q=False, moves=lambda kb, w: False, warps=(0, 1), inline=F
         assert re.search(r"uint64_t [^;]*\b%s\[%d\]" % (name, n), SRC[f]), name
     full = {"k": "k_land", "v": "v_land"} if f == "attn_fp8.cu" else {"k": "k_full", "v": "v_full"}
     p_in_slot = f == "mla_bf16.cuh"                      # half of P in the block's rope chunk
+    qks = ("even", "odd") if re.search(r"int mine = warp == kWarpMma \? 0 : 1;", SRC[f]) else ("all",)       # QK^T warps
     m = Model(inline)
     e = kb0 = 0
     o_gen = dict.fromkeys(ctas, 0)
@@ -239,21 +240,25 @@ def pair(blocks, bf16_q=False, moves=lambda kb, w: False, warps=(0, 1), inline=F
                 for what in "kv":                        # the peer's relays
                     m.wait(f"relay.{what}", f"{full[what]}.{kb & 7}1", kb >> 3)
                     m.ar(f"relay.{what}", f"{what}_peer.{kb & 7}L", kb >> 3)
+            qk, qk_mma = (f"qk.{qks[kb % len(qks)]}", f"qk_mma.{qks[kb % len(qks)]}")
             if k == 0:
-                m.wait("qk", "qt_ready.L", it)
-                if p_in_slot:
-                    m.wait("qk", "q_res.L", it)
-            m.wait("qk", f"{full['k']}.{kb & 7}0", kb >> 3)
+                for i in qks:                            # both warps, whoever's the block is
+                    m.wait(f"qk.{i}", "qt_ready.L", it)
+                    if p_in_slot:
+                        m.wait(f"qk.{i}", "q_res.L", it)
+            m.wait(qk, f"{full['k']}.{kb & 7}0", kb >> 3)
             if 1 in ctas:
-                m.wait("qk", f"k_peer.{kb & 7}L", kb >> 3)
+                m.wait(qk, f"k_peer.{kb & 7}L", kb >> 3)
             if kb >= 2:
-                m.wait("qk", f"s_free.{g}L", (kb >> 1) - 1)
+                m.wait(qk, f"s_free.{g}L", (kb >> 1) - 1)
             uses = []
             for c in ctas:
                 uses += [("r", f"{part}.{x % slots}{c}", 2 * x) for part in "abr"] + [("r", f"q.{c}", it), ("w", f"s.{g}{c}", kb)] + \
                     ([("r", f"q_res.{c}", it)] if p_in_slot else [])
-            m.later("qk", "qk_mma", uses, [(f"qk_done.{kb & 7}{c}", kb >> 3) for c in ctas] +
-                    [(f"q_free.{c}", it) for c in ctas if k == nb - 1])
+            m.later(qk, qk_mma, uses, [(f"qk_done.{kb & 7}{c}", kb >> 3) for c in ctas])
+            if k == nb - 1:
+                for i in qks:
+                    m.later(f"qk.{i}", f"qk_mma.{i}", [], [(f"q_free.{c}", it) for c in ctas])
             for c in ctas:
                 if kb >= 2:
                     m.wait(f"valid.{c}", f"valid_free.{g}{c}", (kb >> 1) - 1)
