@@ -885,18 +885,29 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       mbar_wait(&ms.pv_done[kbl & 3], (kbl >> 2) & 1, wt, kSiteEpi, item.nb);
       __syncwarp();      // lanes leave the wait loop one by one: re-converge before .aligned ops
       tc_fence_after();
+      // Behind the cluster's last item nothing is loaded any more, and with its PVs complete the ring is free for all of O.
+      const bool last = w + ncl >= n_items;
       if (kSliced) {
-        // a slice: unnormalised fp32 O straight to its slot (few slices exist, all of them in L2)
+        // a slice: unnormalised fp32 O to its slot (few slices exist, all of them in L2), a row's half per thread: in one
+        // bulk copy through the ring, or directly
         float4* dst = reinterpret_cast<float4*>(p.part_o + ((size_t)w * 128 + 64 * cta + e_r) * kDV + 256 * e_h);
+        const uint32_t row_off = kOffKV + (64 * e_h + e_r) * 1024;
+        float4* to = last ? reinterpret_cast<float4*>(sm + row_off) : dst;
+        static_assert(128 * 1024 <= kSlots * kStageKV, "O of a slice fits into the ring");
         float o[32];
 #pragma unroll 1
         for (int cc = 0; cc < 8; ++cc) {
           tmem_ld32(e_ocol + cc * 32, o);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) dst[cc * 8 + j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          for (int j = 0; j < 8; ++j) to[part_unit(cc * 8 + j, e_r)] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         }
         tc_fence_before();
+        if (last) {
+          fence_proxy_async_smem();
+          bulk_store_1d(dst, sbase + row_off, 1024);
+          bulk_commit_group();
+        }
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(a_o_free);
         kb0 += item.nb;
@@ -929,22 +940,23 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
         {
           // two rounds make one box of 32 rows x 128 bytes (128-byte swizzle) in the warp's 4 KB
           // slice; before the first of them the previous box must have been read out
-          if ((cc & 1) == 0) {
+          if ((cc & 1) == 0 && !last) {
             if (lane == 0) bulk_wait_read_all();
             __syncwarp();
           }
-          const uint32_t slice = kOffStage + (uint32_t)ew * 4096;
+          const uint32_t slice = last ? kOffKV + (uint32_t)ew * 16384 + (cc >> 1) * 4096 : kOffStage + (uint32_t)ew * 4096;
           uint8_t* st_row = sm + slice + (e_r & 31) * 128;
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             *reinterpret_cast<uint4*>(st_row + (((4 * (cc & 1) + j) ^ (e_r & 7)) << 4)) =
                 make_uint4(wv[4 * j], wv[4 * j + 1], wv[4 * j + 2], wv[4 * j + 3]);
-          if (cc & 1) {
+          if (last ? cc == 7 : (cc & 1) != 0) {
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              for (int d = 0; d < p.n_out; ++d)
-                tma_store_3d_hint(&omaps.m[d], sbase + slice, 256 * e_h + 64 * (cc >> 1), out_head, out_tok, pol_stream);
+              for (int x = last ? 0 : cc >> 1; x <= cc >> 1; ++x)
+                for (int d = 0; d < p.n_out; ++d)
+                  tma_store_3d_hint(&omaps.m[d], sbase + slice - 4096 * ((cc >> 1) - x), 256 * e_h + 64 * x, out_head, out_tok, pol_stream);
               bulk_commit_group();
             }
           }
@@ -952,7 +964,7 @@ masked_mla_fp8_kernel(const __grid_constant__ CUtensorMap map_q,
       }
       kb0 += item.nb;
     }
-    if (lane == 0) bulk_wait_all();   // output boxes written before the CTA retires
+    if (kSliced || lane == 0) bulk_wait_all();   // output boxes and rows written before the CTA retires
     tc_fence_before();
   }
 

@@ -83,6 +83,9 @@ int run_bf16_slices(const void* q, const void* kv, const int32_t* indices, float
                     int nsplit, float* part_o, float2* part_ml, void* stream);      // attn_bf16.cu
 // prefill.cu: merge of the slices of ng tiles (see there); out strides in ELEMENTS
 constexpr int kMaxSlices = 16;
+// A slice's O [128, 512] fp32 has its rows' 16-byte units swapped in eights, unit u of row r at u ^ (r % 8): that is how
+// they lie in shared memory without bank conflicts when every thread has a row.
+__device__ __forceinline__ int part_unit(int u, int row) { return u ^ (row & 7); }
 int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
                  const float* sink, int sink_mod, void* out, int64_t out_token_stride, int64_t out_head_stride,
                  float* lse, cudaStream_t stream);
@@ -406,6 +409,11 @@ __device__ __forceinline__ void tma_store_3d_hint(const void* map, uint32_t src_
                :: "l"(map), "r"(src_smem), "r"(x), "r"(y), "r"(z), "l"(pol) : "memory");
 }
 
+// untiled bulk copy this CTA's shared memory -> global (both addresses 16-byte aligned, size a multiple of 16; bulk
+// async-group completion)
+__device__ __forceinline__ void bulk_store_1d(void* dst, uint32_t src_smem, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_smem), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void bulk_commit_group() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -586,6 +594,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {      // 16 columns
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
   asm volatile(
@@ -604,6 +622,12 @@ __device__ __forceinline__ void tmem_wait_ld() {
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// 32 bytes (one sector; 32-byte aligned) to global memory in one instruction
+__device__ __forceinline__ void st_global_32(void* dst, const uint32_t* w) {
+  asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
 }
 
 // ---------------------------------------------------------------- UMMA descriptors

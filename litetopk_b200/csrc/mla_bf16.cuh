@@ -580,6 +580,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       ++it;
     }
   } else if (warp < kWarpEpi0 || (kTma && warp == kWarpQkOdd)) {
+   if (!kTma) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
    // running position of an MMA-issuing warp: work item, block of the item, blocks of the item, item
    // ordinal, running block number, ring slot
    struct MmaCursor { int w, k, nb, it, kb, slot; };
@@ -798,6 +799,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
    }
   } else if (warp < kWarpGather0) {
+    if (!kTma) asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");      // 80 x 2 + 48 + 48 x 2 + 176 = 480 = 80 x 6, as launched
     // ------------------------------------------------------------ epilogue warps
     // Bring the Q tiles in, then write out O: a warp reads the TMEM lanes of its quarter (warp % 4),
     // i.e. rows e_r of key half e_h, dims [256 e_h, +256) in 8 rounds of 32.  A round (32 rows x 64
@@ -861,63 +863,131 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       tc_fence_after();
       const uint32_t ocol = tmem + e_lane + kTmemO;
       float o[32];
+      // Behind the cluster's last item nothing is loaded any more, and with its PVs complete the ring is free for all of O:
+      // one fence and one group of stores instead of eight rounds at the end of every launch.  (2 tokens x 64 heads, top-2048, in
+      // slices 24.2 -> 21.9 us on a native cache, FP8 22.2 -> 20.1; ranges, 34 x 64 11.3 -> 10.5.)
+      const bool last = w + ncl >= n_items;
       if (kSliced) {
-        // a slice: unnormalised fp32 O straight to its slot (few slices exist, all of them in L2)
+        // a slice: unnormalised fp32 O to its slot (few slices exist, all of them in L2), a row's half per thread: in one
+        // bulk copy through the ring, or directly
         float4* dst = reinterpret_cast<float4*>(p.part_o + ((size_t)w * 128 + 64 * cta + e_r) * kDV + 256 * e_h);
+        const uint32_t row_off = PL::kOffKV + (64 * e_h + e_r) * 1024;
+        float4* to = last ? reinterpret_cast<float4*>(sm + row_off) : dst;
+        static_assert(128 * 1024 <= kSlots * PL::kSlot, "O of a slice fits into the ring");
 #pragma unroll 1
         for (int cc = 0; cc < 8; ++cc) {
           tmem_ld32(ocol + cc * 32, o);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) dst[cc * 8 + j] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          for (int j = 0; j < 8; ++j) to[part_unit(cc * 8 + j, e_r)] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
         }
         tc_fence_before();
+        if (last) {
+          fence_proxy_async_smem();
+          bulk_store_1d(dst, sbase + row_off, 1024);
+          bulk_commit_group();
+        }
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(a_o_free);
+      } else if (last) {
+        const float oscale = ms.oscale[it & 1][e_r];
+        const uint32_t emask = oscale != 0.f ? 0xffffffffu : 0u;
+        const int r0 = (int)cta * 64 + 32 * (warp & 1);
+        const int out_head = r0 % p.h_per_q, out_tok = item.tile * p.G + r0 / p.h_per_q;
+        const uint32_t all = PL::kOffKV + (warp - kWarpEpi0) * 16384;
+        uint8_t* row_off = sm + all + (e_r & 31) * 64;
+#pragma unroll 1
+        for (int cc = 0; cc < 8; ++cc) {
+          tmem_ld32(ocol + cc * 32, o);
+          tmem_wait_ld();
+          uint32_t w16[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const __nv_bfloat162 v2 = __floats2bfloat162_rn(o[2 * j] * oscale, o[2 * j + 1] * oscale);
+            w16[j] = *reinterpret_cast<const uint32_t*>(&v2) & emask;      // rows without a key: zeros
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<uint4*>(row_off + cc * 2048 + ((j ^ sw) << 4)) =
+                make_uint4(w16[4 * j], w16[4 * j + 1], w16[4 * j + 2], w16[4 * j + 3]);
+        }
+        tc_fence_before();
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          for (int cc = 0; cc < 8; ++cc)
+            tma_store_3d_hint(&map_out, sbase + all + cc * 2048, 256 * e_h + 32 * cc, out_head, out_tok, pol_stream);
+          bulk_commit_group();
+          mbar_arrive_cluster(a_o_free);
+        }
       } else {
         const float oscale = ms.oscale[it & 1][e_r];
         const uint32_t emask = oscale != 0.f ? 0xffffffffu : 0u;
         // this warp's 32 rows of the tile = (token, head) pairs starting at row r0
         const int r0 = (int)cta * 64 + 32 * (warp & 1);
         const int out_head = r0 % p.h_per_q, out_tok = item.tile * p.G + r0 / p.h_per_q;
-        tmem_ld32(ocol, o);
-#pragma unroll 1
-        for (int cc = 0; cc < 8; ++cc) {
-          tmem_wait_ld();
-          uint32_t wv[16];
+        // The last kHeld boxes are scaled, rounded and kept in registers, so that the next item's first PV may overwrite O
+        // before they are handed over: a box's way through the warp's slice takes some 500 cycles, all eight 4000, by
+        // which that PV was late.  With the gather the block's registers are redistributed for it (7 boxes; native cache,
+        // 1184 tokens x 64 heads, top-2048 354 -> 343 us); the tiled forms lose more by that than they gain (items of
+        // four blocks 52.5 -> 54 us) and hold what fits without (3 boxes: 1184 x 64 at 65536 100.0 -> 97.9; 4 spill).  Straight to
+        // memory from registers, a row per lane, O is free after 4000 cycles, too.
+        constexpr int kHeld = kTma ? 3 : 7;
+        uint32_t wv[kHeld][16];
+        auto pack = [&](int cc, uint32_t (&w)[16]) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const __nv_bfloat162 v2 = __floats2bfloat162_rn(o[2 * j] * oscale, o[2 * j + 1] * oscale);
-            wv[j] = *reinterpret_cast<const uint32_t*>(&v2) & emask;      // rows without a key: zeros
+          for (int i = 0; i < 2; ++i) {
+            float x[16];
+            tmem_ld16(ocol + 32 * cc + 16 * i, x);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const __nv_bfloat162 v2 = __floats2bfloat162_rn(x[2 * j] * oscale, x[2 * j + 1] * oscale);
+              w[8 * i + j] = *reinterpret_cast<const uint32_t*>(&v2) & emask;      // rows without a key: zeros
+            }
           }
-          if (cc < 7) {
-            tmem_ld32(ocol + (cc + 1) * 32, o);
-          } else {
-            // O has been read: the next item's first PV may overwrite it
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(a_o_free);
-          }
-          // the previous round's box must have been read out of the slice
+        };
+        auto put = [&](const uint32_t (&w)[16]) {      // once the slice's previous box has been read out of it
           if (lane == 0) bulk_wait_read_all();
           __syncwarp();
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<uint4*>(st_row + ((j ^ sw) << 4)) =
-                make_uint4(wv[4 * j], wv[4 * j + 1], wv[4 * j + 2], wv[4 * j + 3]);
+            *reinterpret_cast<uint4*>(st_row + ((j ^ sw) << 4)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+        };
+        auto send = [&](int cc) {
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
             tma_store_3d_hint(&map_out, sbase + stage_off, 256 * e_h + 32 * cc, out_head, out_tok, pol_stream);
             bulk_commit_group();
           }
+        };
+#pragma unroll 1
+        for (int cc = 0; cc < 7 - kHeld; ++cc) {
+          pack(cc, wv[0]);
+          put(wv[0]);
+          send(cc);
+        }
+        pack(7 - kHeld, wv[0]);
+        put(wv[0]);
+#pragma unroll
+        for (int cc = 0; cc < kHeld; ++cc) pack(8 - kHeld + cc, wv[cc]);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(a_o_free);
+        send(7 - kHeld);
+#pragma unroll
+        for (int cc = 0; cc < kHeld; ++cc) {
+          put(wv[cc]);
+          send(8 - kHeld + cc);
         }
       }
       kb0 += item.nb;
     }
-    if (lane == 0) bulk_wait_all();   // boxes written before the CTA retires
+    if (kSliced || lane == 0) bulk_wait_all();   // boxes and rows written before the CTA retires
     tc_fence_before();
   } else if (!kTma) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     // ------------------------------------------------------------ KV row gather (cp.async)
     // 16-byte copies written straight into the 128-byte-swizzled layout, completion reported to an mbarrier by an
     // asynchronous arrival.  Four warps fetch K rows (this CTA's 32 keys, all dims: warp pw rows [8 pw, 8 pw + 8)) as

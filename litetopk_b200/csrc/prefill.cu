@@ -22,7 +22,7 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 // out = out_scale * sum_j O_j 2^(m_j - M) / (sum_j l_j 2^(m_j - M) + sink), lse = ln(sum) + M ln 2 - lse_off
 // (the sink joins the output's normaliser only; row r of a tile = token r / h, head r % h).
-// One warp per row: lane i holds dims 128 c + 4 i .. + 3 of the four 128-dim pieces.  HBM / L2
+// One warp per row: lane i holds unit i (4 dims) of the four 128-dim pieces, as part_unit() has swapped them.  HBM / L2
 // bound in principle (2 KB per slice and row), latency-bound at the sizes it runs at: all slices'
 // loads of a piece are independent.
 __global__ void __launch_bounds__(128)
@@ -62,7 +62,7 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
   float denom = l;
   if (sink != nullptr && l > 0.f) denom += fast_exp2(__ldcg(sink + r % sink_mod) * kLog2e - m);
   const float os = l > 0.f ? __fdividef(out_scale, denom) : 0.f;
-  uint2* dst = reinterpret_cast<uint2*>(out + (row / h) * out_ts + (row % h) * out_hs) + lane;
+  uint2* dst = reinterpret_cast<uint2*>(out + (row / h) * out_ts + (row % h) * out_hs) + part_unit(lane, r);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const __nv_bfloat162 a = __floats2bfloat162_rn(acc[c].x * os, acc[c].y * os);

@@ -345,6 +345,8 @@ def pair(blocks, bf16_q=False, moves=lambda kb, w: False, warps=(0, 1), inline=F
                 m.wait(epi, f"pv_done.{last & 3}{c}", last >> 2)
                 m.use(epi, ("r", f"oscale.{it & 1}{c}", it), ("r", f"o.{c}", o_last[it][c]))
                 m.ar(epi, "o_free.L", it)
+                if it + 1 == len(blocks):                # the last item's output, staged in the ring
+                    m.use(epi, *(("w", f"{part}.{x}{c}", 1 << 20) for x in range(slots) for part in "abr"))
     return m
 
 
@@ -577,6 +579,7 @@ def _give_up(model, rng, q_entries, leaves, asks_if_all_well):
     lost = rng.choice(arrivals + [None])
     late = rng.choice([0, 1, 2, 1 << 30]) * q_entries    # this and later Qs land when all warps are done
     giving_up, left, gone, gave = False, set(), set(), set()          # (giving up: the limit has run out)
+    withheld = set()                                     # arrivals for Q that were passed by
 
     def step(a):
         kind, i, n = run.steps[a][run.pos[a]]
@@ -591,6 +594,8 @@ def _give_up(model, rng, q_entries, leaves, asks_if_all_well):
                 return True
         elif kind == "arrive":
             held = bar == "q_land" and not role[a].endswith("copy") and asks_if_all_well and (cta[a] in left or a in gave)
+            if held:
+                withheld.add((a, run.pos[a]))
             if (a, run.pos[a]) != lost and not held:
                 run.pending[i] += 1
                 if bar == "q_land" and run.pending[i] > run.need[i]:
@@ -640,7 +645,7 @@ def _give_up(model, rng, q_entries, leaves, asks_if_all_well):
         for a, r in enumerate(role):
             if r in ("gather", "k") and cta[a] == cta[i]:
                 made = [j for j, x in enumerate(run.steps[a]) if x[:2] == ("arrive", land) and x[2] == items - 1]
-                run.pending[land] += sum(j >= run.pos[a] or (a, j) == lost for j in made)
+                run.pending[land] += sum(j >= run.pos[a] or (a, j) == lost or (a, j) in withheld for j in made)
         run.pending[land] += items * q_entries - run.issued[i]
         if run.passes(land, items - 1):
             return "the tear-down does not wait for Q"
