@@ -262,8 +262,10 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   Misc& ms = *reinterpret_cast<Misc*>(sm + PL::kOffMisc);
   const BlockWaiter wt{&ms.left, p.wait_limit};
   pdl_trigger();
-  pdl_wait();
-  if (p.gate != nullptr && *reinterpret_cast<const volatile int*>(p.gate) != p.gate_value) return;   // grid-uniform
+  if (p.gate != nullptr) {      // grid-uniform
+    pdl_wait();
+    if (*reinterpret_cast<const volatile int*>(p.gate) != p.gate_value) return;
+  }
 
   // Persistent: each cluster walks items cid, cid + #clusters, ...  Every role runs the same item
   // loop; slots, buffers and barrier phases are indexed by the cluster-wide running block number kb,
@@ -345,6 +347,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, ms.tmem_base, 0);
+  if (p.gate == nullptr) pdl_wait();      // (the set-up overlaps the kernel before)
 
   // Requests half `e` of an item's Q chunks for tensor memory into ring slot `slot` (one thread); the
   // other chunks go into L2, for the fetch that follows the previous item's last QK^T.  (Nothing behind a wait that gave
