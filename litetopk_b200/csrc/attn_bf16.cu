@@ -31,7 +31,7 @@ struct Args {
   float sm_scale;
   // in-place addressing of q / out inside [T, H_padded, d] tensors (ELEMENTS, 0 = dense packed)
   int64_t q_token_stride, q_head_stride, out_token_stride, out_head_stride;
-  const int* gate = nullptr;      // run only if *gate == 1 (see Params)
+  const int4* runs = nullptr;     // run only if a tile's list is not two runs (see Params)
   // nsplit > 1 (d = 576): every tile's blocks are cut into slices whose fp32 results go to part_o / part_ml
   int nsplit = 1;
   float* part_o = nullptr;
@@ -71,7 +71,7 @@ static int run(const Args& a, void* stream) {
   p.ng = a.ng; p.G = 128 / a.h_per_q; p.h_per_q = a.h_per_q; p.nsplit = 1;
   p.scale_log2 = a.sm_scale * kLog2e;
   p.epoch = next_launch_epoch(); p.wait_limit = wait_limit_ticks();
-  p.gate = a.gate; p.gate_value = 1;
+  p.runs = a.runs;
   p.kv = reinterpret_cast<const uint8_t*>(a.kv); p.kv_pitch = a.kv_row_stride * 2;
   p.indices = a.indices; p.idx_stride = a.idx_row_stride;
   p.memb = a.memb; p.s_kv = a.s_kv; p.cap = a.topk;
@@ -174,7 +174,7 @@ extern "C" int litedsa_dsv4_masked_mla_bf16(const void* q, const void* kv, const
                                           out_token_stride, out_head_stride, workspace,
                                           reinterpret_cast<cudaStream_t>(stream));
     if (rc2 != LITEDSA_OK) return rc2;
-    a.gate = reinterpret_cast<const int*>(workspace);
+    a.runs = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(workspace) + 16);
   }
   return run(a, stream);
 }

@@ -16,39 +16,54 @@ namespace dsv4 {
 
 using namespace mla16;
 
-// One warp per tile: is the tile's gathered index list (its first counts[tile] entries) two
-// contiguous ascending runs of valid rows?  runs[tile] = (first row of run 0, its length, first
-// row of run 1, its length); a tile that is not sets *gate (cleared by the host beforehand) to 1.
-__global__ void __launch_bounds__(128)
+// One warp per tile: is the tile's gathered index list (its first counts[tile] entries) two contiguous ascending runs of
+// valid rows?  runs[tile] = (first row of run 0, its length, first row of run 1, its length), and a mark if one of a
+// block's tiles is not (kRunGroup): nothing has to be cleared beforehand.  Latency-bound, so sixteen loads of a lane are in
+// flight (2048 lists of 641 entries: 10 us with one after the other, and a launch to clear a word, 1.5, before it).
+__global__ void __launch_bounds__(32 * kRunGroup)
 classify_runs_kernel(const int32_t* __restrict__ indices, long long idx_stride, int topk,
-                     const int32_t* __restrict__ counts, int ng, int s_kv, int4* __restrict__ runs,
-                     int* __restrict__ gate) {
-  const int tile = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (tile >= ng) return;
-  const int32_t* row = indices + (size_t)tile * idx_stride;
-  const int cnt = min(max(counts ? __ldg(counts + tile) : topk, 0), topk);
-  int breaks = 0, first_break = 0x7fffffff, bad = 0;
-  for (int j = lane; j < cnt; j += 32) {
-    const int v = __ldg(row + j);
-    bad |= (v < 0 || v >= s_kv);
-    if (j + 1 < cnt && __ldg(row + j + 1) != v + 1) {
-      ++breaks;
-      first_break = min(first_break, j);
-    }
-  }
+                     const int32_t* __restrict__ counts, int ng, int s_kv, int4* __restrict__ runs) {
+  const int tile = (int)(blockIdx.x * kRunGroup + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  pdl_trigger();
+  pdl_wait();
+  int scattered = 0;
+  int4 r = make_int4(0, 0, 0, 0);
+  if (tile < ng) {
+    const int32_t* row = indices + (size_t)tile * idx_stride;
+    const int cnt = min(max(counts ? __ldcg(counts + tile) : topk, 0), topk);
+    int breaks = 0, first_break = 0x7fffffff, bad = 0;
+    for (int j0 = lane; j0 < cnt; j0 += 32 * 8) {
+      int v[8], next[8];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    breaks += __shfl_xor_sync(0xffffffffu, breaks, off);
-    first_break = min(first_break, __shfl_xor_sync(0xffffffffu, first_break, off));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, off);
+      for (int u = 0; u < 8; ++u) {
+        const int j = j0 + 32 * u;
+        v[u] = j < cnt ? __ldcg(row + j) : 0;
+        next[u] = j + 1 < cnt ? __ldcg(row + j + 1) : v[u] + 1;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        bad |= v[u] < 0 || v[u] >= s_kv;
+        if (next[u] != v[u] + 1) {
+          ++breaks;
+          first_break = min(first_break, j0 + 32 * u);
+        }
+      }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      breaks += __shfl_xor_sync(0xffffffffu, breaks, off);
+      first_break = min(first_break, __shfl_xor_sync(0xffffffffu, first_break, off));
+      bad |= __shfl_xor_sync(0xffffffffu, bad, off);
+    }
+    r.y = breaks ? first_break + 1 : cnt;
+    r.w = cnt - r.y;
+    if (cnt > 0) r.x = __ldcg(row);
+    if (r.w > 0) r.z = __ldcg(row + r.y);
+    scattered = bad || breaks > 1;
   }
-  if (lane == 0) {
-    const int l0 = breaks ? first_break + 1 : cnt;
-    const int a0 = cnt > 0 ? __ldg(row) : 0;
-    const int b0 = l0 < cnt ? __ldg(row + l0) : 0;
-    runs[tile] = make_int4(a0, l0, b0, cnt - l0);
-    if (bad || breaks > 1) atomicOr(gate, 1);
-  }
+  scattered = __syncthreads_or(scattered);
+  if (threadIdx.x == 0 && scattered) r.x |= (int)0x80000000;
+  if (lane == 0 && tile < ng) runs[tile] = r;
 }
 
 
@@ -91,7 +106,7 @@ static Params base_params(int ng, int h, float sm_scale, float* lse, const float
 // Rank mode of the range kernel for the reference operator's argument list (see
 // litedsa_dsv4_masked_mla_bf16): classifies every tile's index list on the device, then enqueues
 // the range kernel gated on "every tile is two contiguous runs".  workspace: 16 + 16 * ng bytes
-// (gate word, then runs[ng]); the caller enqueues the gather kernel behind it, gated on the
+// (runs[ng] from byte 16); the caller enqueues the gather kernel behind it, gated on the
 // opposite value, so exactly one of the two does the work -- no host synchronisation.
 int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, const int32_t* pref,
                       const int32_t* win_lo, const int32_t* win_hi, const int32_t* counts,
@@ -101,17 +116,15 @@ int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, con
                       int64_t out_token_stride, int64_t out_head_stride, void* workspace,
                       cudaStream_t stream) {
   using namespace dsv4;
-  int* gate = reinterpret_cast<int*>(workspace);
   int4* runs = reinterpret_cast<int4*>(reinterpret_cast<char*>(workspace) + 16);
-  if (cudaMemsetAsync(gate, 0, 16, stream) != cudaSuccess) return LITEDSA_ERR_CUDA;
-  classify_runs_kernel<<<(ng + 3) / 4, 128, 0, stream>>>(indices, indices_row_stride, topk, counts, ng, s_kv,
-                                                         runs, gate);
+  const int rc = launch_pdl(classify_runs_kernel, dim3((unsigned)(ng + kRunGroup - 1) / kRunGroup), 32 * kRunGroup, 0, stream, indices,
+                            (long long)indices_row_stride, topk, counts, ng, s_kv, runs);
+  if (rc != LITEDSA_OK) return rc;
   CUtensorMap mq, mkv, mout;
   const QOutArgs a{q, out, d, ng, h_per_q, q_row_stride, q_token_stride, q_head_stride, out_token_stride, out_head_stride};
   if (!make_q_out_maps(a, &mq, &mout) || !make_kv_map(&mkv, kv, d, s_kv, kv_row_stride)) return LITEDSA_ERR_CUDA;
   Params p = base_params(ng, h_per_q, sm_scale, lse, attn_sink, 128);
   p.runs = runs; p.pref = pref; p.win_lo = win_lo; p.win_hi = win_hi; p.counts = counts;
-  p.gate = gate; p.gate_value = 0;
   return d == 576 ? launch<576, kRank, false>(mq, mkv, mkv, mout, p, stream)
                   : launch<512, kRank, false>(mq, mkv, mkv, mout, p, stream);
 }

@@ -59,7 +59,7 @@ struct Fp8Args {
 constexpr float kFp8LseOffset = 1.9459101090932196f;   // ln 7: the FP8 kernel's P carry a factor 7
 int check_fp8_args(const Fp8Args& a);                                   // no CUDA call
 // attn_dsv4.cu: classify the tiles' index lists and enqueue the range kernel in rank mode, gated on
-// "every list is two contiguous runs" (workspace: 16 + 16 * ng bytes; word 0 is the gate)
+// "every list is two contiguous runs" (workspace: 16 + 16 * ng bytes)
 int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, const int32_t* pref,
                       const int32_t* win_lo, const int32_t* win_hi, const int32_t* counts,
                       float sm_scale, int h_per_q, void* out, float* lse, const float* attn_sink,

@@ -43,6 +43,8 @@ namespace lt {
 namespace mla16 {
 
 enum Source { kRange, kRank, kGather };
+// The first of each kRunGroup tiles has the sign bit of its first row set if the list of one of them is not two runs.
+constexpr int kRunGroup = 16;
 
 constexpr int kSoftmaxWarps = 8, kGatherWarps = 8, kEpiWarps = 4;
 constexpr int kWarpMma = 8, kWarpK = 9, kWarpV = 10, kWarpValid = 11, kWarpEpi0 = 12, kWarpGather0 = 16;
@@ -130,14 +132,11 @@ struct Params {
   int nsplit;
   float* part_o;
   float2* part_ml;
-  // the launch runs only if *gate == gate_value (null: always): the device-side choice between the
-  // rank and the gather form of one call
-  const int* gate;
-  int gate_value;
+  // The device-side choice between the rank and the gather form of one call: the rank form runs if no group of tiles is
+  // marked in `runs` (kGather: null: it always runs), the gather form if one is.
+  const int4* runs;          // [ng]: (first row of run 0, its length, first row of run 1, its length); groups: see kRunGroup
   // kRange: token t of the call sits at pos0 + t
   int n_comp, pos0, window, ratio;
-  // kRank: runs[tile] = (first row of run 0, its length, first row of run 1, its length)
-  const int4* runs;
   // kGather: rows of kv (kv_pitch bytes apart) by index
   const uint8_t* kv;
   long long kv_pitch, idx_stride;
@@ -262,9 +261,15 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   Misc& ms = *reinterpret_cast<Misc*>(sm + PL::kOffMisc);
   const BlockWaiter wt{&ms.left, p.wait_limit};
   pdl_trigger();
-  if (p.gate != nullptr) {      // grid-uniform
+  // whether a list of the call is not two runs (grid-uniform)
+  auto scattered = [&]() -> bool {
+    int marked = 0;
+    for (int i = threadIdx.x * kRunGroup; i < p.ng; i += blockDim.x * kRunGroup) marked |= __ldcg(&p.runs[i].x) < 0;
+    return __syncthreads_or(marked) != 0;
+  };
+  if (kSrc == kGather && p.runs != nullptr) {
     pdl_wait();
-    if (*reinterpret_cast<const volatile int*>(p.gate) != p.gate_value) return;
+    if (!scattered()) return;
   }
 
   // Persistent: each cluster walks items cid, cid + #clusters, ...  Every role runs the same item
@@ -347,7 +352,12 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, ms.tmem_base, 0);
-  if (p.gate == nullptr) pdl_wait();      // (the set-up overlaps the kernel before)
+  if (kSrc != kGather || p.runs == nullptr) pdl_wait();      // (the set-up overlaps the kernel before)
+  if (kSrc == kRank && scattered()) {
+    cluster_sync_all();
+    if (warp == kWarpMma) tmem_dealloc_pair(tmem, kTmemCols);
+    return;
+  }
 
   // Requests half `e` of an item's Q chunks for tensor memory into ring slot `slot` (one thread); the
   // other chunks go into L2, for the fetch that follows the previous item's last QK^T.  (Nothing behind a wait that gave
@@ -933,9 +943,9 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         // before they are handed over: a box's way through the warp's slice takes some 500 cycles, all eight 4000, by
         // which that PV was late.  With the gather the block's registers are redistributed for it (7 boxes; native cache,
         // 1184 tokens x 64 heads, top-2048 354 -> 343 us); the tiled forms lose more by that than they gain (items of
-        // four blocks 52.5 -> 54 us) and hold what fits without (3 boxes: 1184 x 64 at 65536 100.0 -> 97.9; 4 spill).  Straight to
+        // four blocks 52.5 -> 54 us) and hold what fits without (ranges 3 boxes: 1184 x 64 at 65536 100.0 -> 97.9; 4 spill, with runs 3).  Straight to
         // memory from registers, a row per lane, O is free after 4000 cycles, too.
-        constexpr int kHeld = kTma ? 3 : 7;
+        constexpr int kHeld = kSrc == kRange ? 3 : kSrc == kRank ? 2 : 7;
         uint32_t wv[kHeld][16];
         auto pack = [&](int cc, uint32_t (&w)[16]) {
 #pragma unroll

@@ -340,6 +340,37 @@ def test_dsv4_one_scattered_list_sends_the_whole_call_to_the_gather_kernel():
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
 
 
+@pytest.mark.parametrize("tile", [None, 0, 15, 16, 31, 32])
+def test_dsv4_a_scattered_list_of_any_group_of_tiles_is_found(tile):
+    # the classification marks groups of 16 tiles; lists that end around its steps of 256 entries stay two runs
+    ng, heads, topk, s_kv, d = 33, 64, 576, 4096, 512
+    q, kv, idx, pref, wlo, whi, counts, _ = _two_run_case(ng, heads, topk, s_kv, d, seed=30)
+    for t, n in enumerate((0, 1, 2, 255, 256, 257, 511, 512, 513)):
+        idx[3 * t] = -1
+        idx[3 * t, :n] = torch.cat([torch.arange(7, 7 + n // 2), torch.arange(900, 900 + n - n // 2)]).to(torch.int32)
+        counts[3 * t] = n
+    if tile is not None:
+        idx[tile] = -1
+        idx[tile, :30] = torch.cat([torch.arange(100, 110), torch.arange(200, 210), torch.arange(300, 310)]).to(torch.int32)
+        counts[tile] = 30
+    dev = [t.to(DEV) for t in (q, kv, idx, pref, wlo, whi, counts)]
+    res = []
+    for detect in (True, False):
+        out = torch.empty((ng, 128, 512), dtype=torch.bfloat16, device=DEV)
+        lse = torch.empty((ng, 128), dtype=torch.float32, device=DEV)
+        api.dsv4_status(reset=True)
+        api.dsv4_masked_mla_bf16_out(*dev, synth.SM_SCALE, heads, out, lse, None, detect_runs=detect)
+        torch.cuda.synchronize()
+        assert api.dsv4_status()[3] == (1 if detect and tile is None else 0)
+        res.append((out, lse))
+    if tile is not None:      # the same kernel
+        assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    else:
+        mad, cos = ao.compare(res[0][0].cpu(), res[1][0].cpu().float())
+        scale = max(1.0, float(res[1][0].abs().max()))
+        assert mad <= TOL_ABS * scale and cos >= TOL_COS, (mad, cos)
+
+
 def test_dsv4_two_run_lists_in_place_padded_heads():
     # rank mode of the range kernel with q / out addressed inside [T, 64, d] / [T, 64, 512]
     ng, heads, hpad, topk, s_kv, d = 6, 16, 64, 320, 4096, 512
