@@ -22,20 +22,35 @@ constexpr float kLn2 = 0.6931471805599453f;
 
 // out = out_scale * sum_j O_j 2^(m_j - M) / (sum_j l_j 2^(m_j - M) + sink), lse = ln(sum) + M ln 2 - lse_off
 // (the sink joins the output's normaliser only; row r of a tile = token r / h, head r % h).
-// One warp per row: lane i holds unit i (4 dims) of the four 128-dim pieces, as part_unit() has swapped them.  HBM / L2
-// bound in principle (2 KB per slice and row), latency-bound at the sizes it runs at: all slices'
-// loads of a piece are independent.
-__global__ void __launch_bounds__(128)
+// A warp has kPieces of a row's four 128-dim pieces, lane i unit i (4 dims) of each, as part_unit() has swapped them.  Latency-
+// bound at the sizes it runs at (2 KB per slice and row): the loads of eight (two) slices are under way with that of the
+// maxima, before a weight is known.  One piece per warp as long as all blocks are on the chip at once, else four.  (A warp per
+// row that went from slice to slice: 2 tokens x 64 heads in five slices 20.3 -> 18.6 us, in eight of a native cache 20.6 -> 18.3;
+// 68 x 64 in two 30.8, with one piece per warp 33.0, four of them 31.1.)
+template <int kPieces>
+__global__ void __launch_bounds__(256)
 merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml, int nsplit, int n_rows, int h,
                     float out_scale, float lse_off, const float* __restrict__ sink, int sink_mod,
                     __nv_bfloat16* __restrict__ out, long long out_ts, long long out_hs, float* __restrict__ lse) {
-  const int row = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  constexpr int kPer = 4 / kPieces, kBatch = 8 / kPieces;
+  const int w = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  const int row = w / kPer, c0 = w % kPer * kPieces;
   if (row >= n_rows) return;
   pdl_wait();
   const int tile = row >> 7, r = row & 127;
   const size_t p0 = (size_t)tile * nsplit * 128 + r;            // slice j of the row: p0 + 128 j
   float2 ml = make_float2(-INFINITY, 0.f);
   if (lane < nsplit) ml = __ldcg(part_ml + p0 + (size_t)lane * 128);
+  const float4* src = reinterpret_cast<const float4*>(part_o + p0 * 512) + 32 * c0 + lane;
+  float4 v[kBatch][kPieces];
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+      for (int c = 0; c < kPieces; ++c)
+        if (j0 + u < nsplit) v[u][c] = __ldcg(src + (size_t)(j0 + u) * (128 * 128) + 32 * c);
+  };
+  fetch(0);
   float m = ml.y > 0.f ? ml.x : -INFINITY;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -43,33 +58,34 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
   float l = ml.y * f;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-  float4 acc[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int j = 0; j < nsplit; ++j) {
-    const float fj = __shfl_sync(0xffffffffu, f, j);
-    if (fj == 0.f) continue;                                    // warp-uniform
-    const float4* src = reinterpret_cast<const float4*>(part_o + (p0 + (size_t)j * 128) * 512) + lane;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float4 v = __ldcg(src + 32 * c);
-      acc[c].x = fmaf(v.x, fj, acc[c].x);
-      acc[c].y = fmaf(v.y, fj, acc[c].y);
-      acc[c].z = fmaf(v.z, fj, acc[c].z);
-      acc[c].w = fmaf(v.w, fj, acc[c].w);
-    }
-  }
   float denom = l;
   if (sink != nullptr && l > 0.f) denom += fast_exp2(__ldcg(sink + r % sink_mod) * kLog2e - m);
-  const float os = l > 0.f ? __fdividef(out_scale, denom) : 0.f;
-  uint2* dst = reinterpret_cast<uint2*>(out + (row / h) * out_ts + (row % h) * out_hs) + part_unit(lane, r);
+  float4 acc[kPieces];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(acc[c].x * os, acc[c].y * os);
-    const __nv_bfloat162 b = __floats2bfloat162_rn(acc[c].z * os, acc[c].w * os);
+  for (int c = 0; c < kPieces; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j0 = 0; j0 < nsplit; j0 += kBatch) {
+    if (j0 > 0) fetch(j0);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const float fj = j0 + u < nsplit ? __shfl_sync(0xffffffffu, f, j0 + u) : 0.f;
+      if (fj == 0.f) continue;                                  // warp-uniform; whatever the slice holds
+#pragma unroll
+      for (int c = 0; c < kPieces; ++c) {
+        acc[c].x = fmaf(v[u][c].x, fj, acc[c].x);
+        acc[c].y = fmaf(v[u][c].y, fj, acc[c].y);
+        acc[c].z = fmaf(v[u][c].z, fj, acc[c].z);
+        acc[c].w = fmaf(v[u][c].w, fj, acc[c].w);
+      }
+    }
+  }
+  const float os = l > 0.f ? __fdividef(out_scale, denom) : 0.f;
+  uint2* dst = reinterpret_cast<uint2*>(out + (row / h) * out_ts + (row % h) * out_hs) + 32 * c0 + part_unit(lane, r);
+#pragma unroll
+  for (int c = 0; c < kPieces; ++c) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(acc[c].x * os, acc[c].y * os), b = __floats2bfloat162_rn(acc[c].z * os, acc[c].w * os);
     dst[32 * c] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
   }
-  if (lane == 0) lse[row] = l > 0.f ? __logf(l) + m * kLn2 - lse_off : INFINITY;
+  if (lane == 0 && c0 == 0) lse[row] = l > 0.f ? __logf(l) + m * kLn2 - lse_off : INFINITY;
 }
 
 // How many slices a tile is cut into when a launch has `tiles` tiles of G lists of k entries: as many as
@@ -141,8 +157,9 @@ static bool use_rows64(int tokens, int h, int k, bool kv_bf16) {
 int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
                  const float* sink, int sink_mod, void* out, int64_t out_token_stride, int64_t out_head_stride,
                  float* lse, cudaStream_t stream) {
-  return launch_pdl(prefill::merge_slices_kernel, dim3((ng * 128 + 3) / 4), 128, 0, stream, part_o, part_ml, nsplit,
-                    ng * 128, h, out_scale, lse_off, sink, sink_mod, reinterpret_cast<__nv_bfloat16*>(out),
+  const bool few = ng * 64 <= 8 * sm_count();      // blocks of 256 threads, eight on an SM
+  return launch_pdl(few ? prefill::merge_slices_kernel<1> : prefill::merge_slices_kernel<4>, dim3(ng * (few ? 64 : 16)), 256, 0, stream,
+                    part_o, part_ml, nsplit, ng * 128, h, out_scale, lse_off, sink, sink_mod, reinterpret_cast<__nv_bfloat16*>(out),
                     (long long)out_token_stride, (long long)out_head_stride, lse);
 }
 }  // namespace lt
