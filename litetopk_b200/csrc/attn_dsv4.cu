@@ -67,19 +67,6 @@ classify_runs_kernel(const int32_t* __restrict__ indices, long long idx_stride, 
 }
 
 
-// Slices of a tile when a call has `tiles` tiles of up to `blocks` key blocks: as many as there are
-// idle clusters for, at least five blocks each, none below 20 blocks.  They cost a launch for the merge and
-// fp32 partial results, which grow with their number, so they have to shorten a tile by at least 4 +
-// 0.1 tiles n of its blocks of 0.75 us.  (24 tokens against 77777 positions in slices from six blocks on
-// 25.5 us, unsliced 20; 37 tiles of 20 blocks in two slices 26.6, unsliced 24.7, of 26 blocks 28.8 and 29.3;
-// one tile of 26 blocks in five 18.4 and 28.4.)
-static int pick_slices(int tiles, int blocks) {
-  if (blocks < 20) return 1;
-  int n = sm_count() / 2 / tiles;
-  if (n > blocks / 5) n = blocks / 5;
-  if (n > kMaxSlices) n = kMaxSlices;
-  return n >= 2 && blocks - (double)blocks / n >= 4.0 + 0.1 * tiles * n ? n : 1;
-}
 // most blocks a tile of the call can have: its last tile has the longest prefix
 static int most_blocks(int ng, int G, int n_comp, int pos0, int window, int ratio) {
   const int64_t last = (int64_t)pos0 + (int64_t)ng * G - 1;
@@ -135,7 +122,7 @@ int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, con
 extern "C" int64_t litedsa_dsv4_workspace(int ng, int h_per_q, int n_comp, int pos0, int window, int ratio) {
   using namespace lt::dsv4;
   if (ng <= 0 || h_per_q <= 0 || 128 % h_per_q || n_comp < 0 || pos0 < 0 || window <= 0 || ratio <= 0) return 0;
-  return slice_bytes(ng, pick_slices(ng, most_blocks(ng, 128 / h_per_q, n_comp, pos0, window, ratio)));
+  return slice_bytes(ng, lt::bf16_slices(ng, most_blocks(ng, 128 / h_per_q, n_comp, pos0, window, ratio)));
 }
 
 // DSv4 packed BF16 attention over (compressed prefix, sliding window).  Replaces the
@@ -198,7 +185,7 @@ extern "C" int litedsa_dsv4_c128a_bf16_ws(const void* q, const void* kv_comp, co
   p.n_comp = n_comp; p.pos0 = pos0; p.window = window; p.ratio = ratio;
   if (workspace) {
     if ((uintptr_t)workspace & 255) return LITEDSA_ERR_UNSUPPORTED;
-    const int ns = pick_slices(ng, most_blocks(ng, G, n_comp, pos0, window, ratio));
+    const int ns = bf16_slices(ng, most_blocks(ng, G, n_comp, pos0, window, ratio));
     if (ns > 1 && workspace_bytes >= slice_bytes(ng, ns)) {
       p.nsplit = ns;
       p.part_o = reinterpret_cast<float*>(workspace);

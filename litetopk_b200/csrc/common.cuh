@@ -83,6 +83,8 @@ int run_bf16_slices(const void* q, const void* kv, const int32_t* indices, float
                     int nsplit, float* part_o, float2* part_ml, void* stream);      // attn_bf16.cu
 // prefill.cu: merge of the slices of ng tiles (see there); out strides in ELEMENTS
 constexpr int kMaxSlices = 16;
+// prefill.cu: slices of `tiles` tiles of up to `blocks` 64-key blocks in the bf16 kernel
+int bf16_slices(int tiles, int blocks);
 // A slice's O [128, 512] fp32 has its rows' 16-byte units swapped in eights, unit u of row r at u ^ (r % 8): that is how
 // they lie in shared memory without bank conflicts when every thread has a row.
 __device__ __forceinline__ int part_unit(int u, int row) { return u ^ (row & 7); }

@@ -88,27 +88,32 @@ merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__
   if (lane == 0 && c0 == 0) lse[row] = l > 0.f ? __logf(l) + m * kLn2 - lse_off : INFINITY;
 }
 
-// How many slices a tile is cut into when a launch has `tiles` tiles of G lists of k entries: as many as
-// there are idle clusters for, of at least four 128-key blocks (bf16 kernel: five of 64), if a tile has
-// 12 (20).  A union is not known on the host; neighbouring tokens share about three quarters of their
-// lists, so it is taken as k (3 + G) / 4 entries.  Slices cost a launch for the merge, a block each for the
-// running max, and fp32 partial results, which grow with their number; a block of an unsliced tile takes
-// 1.1 us (0.8).  FP8 slices that shorten a tile by less than 4 + 0.08 tiles n blocks even when only half of
-// the lists is shared are not made (128 heads, 37 tiles of 12 blocks: 30.5 us in two slices, 25.6 whole).
-// Graph replays of 1440 calls (8 to 128 heads, 1 to 37 tiles, 256 to 3072 entries, 50 to 90 % sharing): FP8
-// 0.80 of the unsliced time in the mean, 59 of 660 calls more than 2 % slower, all of them with unions
-// much shorter than taken here (8 heads, 24 tiles, top-384: nine tenths shared 28.8 and 23.1 us, half
-// shared 36.0 and 41.8); bf16 0.61 and 6 of 780.  Two tokens x 64 heads, top-2048:
-// FP8 32.2 -> 24.1 us.
+// Slices of a tile of `blocks` key blocks that are worth what they cost when nothing else runs: what each costs grows with
+// their number, the time that they save does less and less.
+static int most_slices(int blocks) {
+  int n = 1;
+  while (n < kMaxSlices && (n + 1) * (n + 1) <= 4 * blocks) ++n;
+  return n;
+}
+
+// How many slices a tile is cut into when a launch has `tiles` tiles of G lists of k entries: no more than there are clusters
+// for.  A union is not known on the host; neighbouring tokens share about three quarters of their lists, so it is taken as
+// k (3 + G) / 4 entries.  Slices cost a launch for the merge, fp32 partial results, which grow with their number, and, FP8, a
+// block each for the running max; a block of an unsliced tile takes 1.1 us (bf16: bf16_slices).  FP8: tiles of ten blocks and more; with
+// a few tiles in slices of two to three blocks, with many of four.  Slices that shorten a tile by less than 4 + 0.08 tiles n blocks even
+// when only half of the lists is shared are not made (128 heads, 37 tiles of 12 blocks: 30.5 us in two slices, 25.6 whole).  us, whole / in n:
+// 2 tokens x 64 heads, top-2048 30.4, five 18.7, eight 18.0; 8 x 64 30.6, five 19.6, eight 19.2; 18 x 64 31.5, five 21.0, eight 22.3;
+// top-1024 20.8, three 19.5, five 18.3; 36 x 64, top-2048 31.7, two 27.7, four 25.3; 68 x 64 33.3, two 30.4, top-1024 22.0 and 24.5;
+// 16 x 8, top-1024, half shared 81.5, eight 28.7, twelve 26.5, nine tenths shared 35.1, 22.1, 21.8.
 static int pick_slices(int tiles, int G, int k, bool bf16) {
   const int blocks = (int)((int64_t)k * (3 + G) / 4 / (bf16 ? 64 : 128));
-  if (blocks < (bf16 ? 20 : 12)) return 1;
-  int n = sm_count() / 2 / tiles;
-  if (n > blocks / (bf16 ? 5 : 4)) n = blocks / (bf16 ? 5 : 4);
-  if (n > kMaxSlices) n = kMaxSlices;
+  if (bf16) return bf16_slices(tiles, blocks);
+  if (blocks < 10) return 1;
+  const int few = min(most_slices(blocks), 48 / tiles);
+  const int n = min(min(sm_count() / 2 / tiles, max(blocks / 4, few)), kMaxSlices);
   if (n < 2) return 1;
   const double half = (double)k * (1 + G) / 2 / 128;
-  return bf16 || half - (half / n + 1.0) >= 4.0 + 0.08 * tiles * n ? n : 1;
+  return half - (half / n + 1.0) >= 4.0 + 0.08 * tiles * n ? n : 1;
 }
 
 // workspace layout: all offsets are multiples of 256 bytes
@@ -153,6 +158,16 @@ static bool use_rows64(int tokens, int h, int k, bool kv_bf16) {
 }
 
 }  // namespace prefill
+
+// What the slices save (0.75 us a block) has to be more than the merge and the items cost.  us, whole / in n slices: 2 tokens x 64
+// heads at 131072 (18.5 blocks) 21.3, two 18.5, four 14.5, eight 13.1; at 65536 (10.5) 14.9, two 15.2, six 12.5; 8 x 16 at 40000 (7.5)
+// 13.1, five 12.3, at 32768 (6.5) 12.4 and 12.4; 16 x 64 at 131072 22.0, four 16.3, eight 15.5; 40 x 64 22.8, three 19.5; 70 x 64 23.4,
+// two 24.0.  Unions on a native cache: 2 x 64, top-2048 43.7, five 21.2, twelve 18.4; 18 x 64 44.6, four 25.1, eight 22.8, top-1024 28.1, four
+// 19.9, eight 20.1; 68 x 64, top-2048 50.4, two 38.6, top-1024 30.4 and 27.8; 40 x 64, top-512 19.7, three 19.8.
+int bf16_slices(int tiles, int blocks) {
+  const int n = min(prefill::most_slices(blocks), sm_count() / 2 / tiles);
+  return n >= 2 && 0.75 * blocks * (n - 1) / n >= 4.0 + 0.045 * tiles * n ? n : 1;
+}
 
 int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
                  const float* sink, int sink_mod, void* out, int64_t out_token_stride, int64_t out_head_stride,
