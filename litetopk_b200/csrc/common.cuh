@@ -403,6 +403,10 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src,
       ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(smem_u32(mbar))
       : "memory");
 }
+// `bytes` (a multiple of 16) from a 16-byte aligned address into L2
+__device__ __forceinline__ void l2_prefetch_1d(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // TMA 3-D tile store shared -> global (bulk async-group completion)
 __device__ __forceinline__ void tma_store_3d_hint(const void* map, uint32_t src_smem, int x, int y,
                                                   int z, uint64_t pol) {
