@@ -84,6 +84,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = False                          # not looked for yet
 
 
 class LiteDSAError(RuntimeError):
@@ -108,6 +109,30 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+def host():
+    """The module of host_binding.cpp, or None where it was not built, or for another torch: the short way into the same
+    library for plain calls; everything else, and everything without it, goes by ctypes."""
+    global _host
+    if _host is False:
+        lib()
+        _host = None
+        path = LIB_PATH.with_name("litedsa_host.so")
+        if path.exists():
+            import importlib.machinery
+            import importlib.util
+
+            import torch
+            try:
+                loader = importlib.machinery.ExtensionFileLoader("litedsa_host", str(path))
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("litedsa_host", loader))
+                if module.built_for == torch.__version__:
+                    _host = module
+            except ImportError as e:
+                import warnings
+                warnings.warn(f"{path.name} cannot be loaded, calls go by ctypes: {e}")
+    return _host
 
 
 def check(code: int, where: str) -> None:

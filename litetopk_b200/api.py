@@ -360,8 +360,14 @@ def dsv4_masked_mla_bf16_out(q: torch.Tensor, kv: torch.Tensor, indices: torch.T
     ``detect_runs`` (default): the index lists are classified on the device and, when every
     tile's list is two contiguous runs of rows (the packed prefix + window pattern), the
     attention runs in the kernel that reads K / V with tiled TMA loads instead of gathering
-    rows; otherwise in the gather kernel.  No host synchronisation either way; a small cached
-    device workspace (16 + 16 * ng bytes per device) carries the decision."""
+    rows; otherwise in the gather kernel.  No host synchronisation either way; a small
+    device workspace (16 + 16 * ng bytes) carries the decision."""
+    if detect_runs and not in_place_heads and (host := _lib.host()) is not None:
+        r = host.dsv4_masked_mla_bf16_out(q, kv, indices, pref, win_lo, win_hi, counts, sm_scale, h_per_q, out, lse, attn_sink)
+        if r is not None:
+            if r is not True:
+                check(r, "dsv4_masked_mla_bf16")
+            return
     G = 128 // int(h_per_q)
     strides = (0, 0, 0, 0)
     if in_place_heads:
@@ -530,6 +536,12 @@ def lite_topk(q_idx8: torch.Tensor, k_idx8: torch.Tensor, weights: torch.Tensor,
               logits_workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Indexer + selection in one call: ``topk_idx`` [T, k] int32 (-1 padded) for the T query
     tokens at positions ``q_pos0 ...`` -- the input of ``union_qm`` / ``sparse_prefill``."""
+    if logits_workspace is None and (host := _lib.host()) is not None:
+        r = host.lite_topk(q_idx8, k_idx8, weights, k_scale, k, q_pos0)
+        if r is not None:
+            if type(r) is tuple:
+                check(*r)
+            return r
     S = k_idx8.shape[0]
     if logits_workspace is None:
         # rows start on 16-byte boundaries whatever S is: the streaming selection kernels need that
@@ -807,6 +819,12 @@ def sparse_prefill(q: torch.Tensor, kv_cache_fp8: torch.Tensor, topk_idx: torch.
     default the call's own number of tokens: state the tokens of the whole job when this call is a part of
     it, and its tokens get the bits that they have in one call of the job.
     """
+    if out is None and lse is None and (host := _lib.host()) is not None:
+        r = host.sparse_prefill(q, kv_cache_fp8, topk_idx, sm_scale, kv_scale, q_scale, seq_space, job_tokens)
+        if r is not None:
+            if type(r) is int:
+                check(r, "sparse_prefill")
+            return r
     if job_tokens is not None and int(job_tokens) < q.shape[0]:
         raise ValueError("job_tokens must be at least the call's number of tokens")
     return _sparse_prefill(q, kv_cache_fp8, topk_idx, sm_scale, kv_scale, q_scale, seq_space, out, lse,
@@ -1010,6 +1028,12 @@ def dsv4_c128a_bf16(q: torch.Tensor, kv_compressed: Optional[torch.Tensor], kv_r
     fp32; a slice rounds its softmax weights to bf16 relative to its own running maximum, so the result of a
     few tokens alone and inside a larger call can differ by that rounding.
     """
+    if heads is None and out is None and (host := _lib.host()) is not None:
+        r = host.dsv4_c128a_bf16(q, kv_compressed, kv_raw, q_pos0, sm_scale, window, ratio, attn_sink)
+        if r is not None:
+            if type(r) is int:
+                check(r, "dsv4_c128a_bf16")
+            return r
     _need(q, "q", torch.bfloat16, 3)
     _need(kv_raw, "kv_raw", torch.bfloat16, 2)
     T, hq, d = q.shape

@@ -1,0 +1,142 @@
+"""The short way into the library (host_binding.cpp) against the general one (ctypes): the same results bit for bit over the forms
+that it accepts, and whatever else it is handed goes the general way, with that way's results and errors."""
+import pytest
+import torch
+
+from litetopk_b200 import _lib, api, synth
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+SC = synth.REFCOMPAT_SCALE
+
+
+@pytest.fixture
+def both(monkeypatch):
+    """f -> (result of f by the short way, by the general one), and whether the short way took it."""
+    host = _lib.host()
+    assert host is not None, "litedsa_host.so is missing"
+
+    def run(f):
+        took = []
+
+        class Spy:
+            def __getattr__(self, name):
+                def call(*args):
+                    took.append(getattr(host, name)(*args))
+                    return took[-1]
+                return call
+        monkeypatch.setattr(_lib, "_host", Spy())
+        short = f()
+        monkeypatch.setattr(_lib, "_host", None)
+        general = f()
+        torch.cuda.synchronize()
+        return short, general, [r is not None for r in took]
+    return run
+
+
+def _same(a, b):
+    a, b = (x if isinstance(x, (tuple, list)) else (x,) for x in (a, b))
+    assert len(a) == len(b)
+    for x, y in zip(a, b):
+        assert x.shape == y.shape and x.dtype == y.dtype and x.stride() == y.stride() and torch.equal(x, y)
+
+
+def _prefill(T, h, k, S, q_type, cache):
+    w = synth.Workload("t", tokens=T, heads=h, topk=k, s_kv=S, overlap=(0.7, 0.7))
+    idx = synth.make_topk(w, seed=5).to(DEV)
+    rows = synth.make_kv_cache(S, seed=5, device=DEV, mode="native" if cache == "native" else "refcompat")
+    kv = api.prepare_kv(rows) if cache == "native" else api.prepare_kv(rows, SC)
+    x = torch.randn((T, h, 576), generator=torch.Generator().manual_seed(5)).to(DEV)
+    q = x.to(torch.bfloat16) if q_type == "bf16" else synth.e4m3_codes(x / SC)
+    return q, kv, idx, ({} if cache == "native" else dict(kv_scale=SC, q_scale=SC))
+
+
+@pytest.mark.parametrize("T,h,k,S,q_type,cache", [
+    (2, 64, 256, 2048, "bf16", "fp8"), (2, 64, 1024, 4096, "e4m3", "fp8"), (16, 8, 128, 999, "e4m3", "fp8"), (1, 128, 256, 777, "bf16", "fp8"),
+    (6, 64, 512, 3001, "bf16", "native"), (200, 64, 256, 2048, "bf16", "fp8"), (8, 32, 32, 640, "e4m3", "fp8")])
+def test_sparse_prefill(both, T, h, k, S, q_type, cache):
+    q, kv, idx, scales = _prefill(T, h, k, S, q_type, cache)
+    for q_, kv_, extra in ((q, kv, {}), (q if q_type == "bf16" else q.view(torch.float8_e4m3fn), kv, dict(seq_space=S + 1, job_tokens=T + 4 * 128 // h)),
+                           (q, torch.cat([kv, kv], dim=1)[:, :576], {})):                    # rows of a wider pitch
+        short, general, took = both(lambda: api.sparse_prefill(q_, kv_, idx, synth.SM_SCALE, **scales, **extra))
+        assert took == [True]
+        _same(short, general)
+
+
+def test_what_is_not_plain_goes_the_general_way(both):
+    q, kv, idx, scales = _prefill(4, 64, 256, 2048, "bf16", "fp8")
+    call = lambda q=q, kv=kv, idx=idx, **kw: api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **{**scales, **kw})      # noqa: E731
+    plain = call()
+    wide = torch.cat([q, q], dim=2)[:, :, :576]
+    for f in (lambda: call(q=wide), lambda: call(idx=torch.cat([idx, idx], dim=1)[:, :256]), lambda: call(kv=kv[:, None]),
+              lambda: call(kv_scale=torch.tensor(SC))):
+        short, general, took = both(f)
+        assert took == [False]
+        _same(short, general)
+        _same(short, plain)
+    short, general, took = both(lambda: call(out=torch.empty_like(plain[0])))
+    assert took == []
+    _same(short, plain)
+    short, general, took = both(lambda: call(q_scale=None))                                  # derived with a synchronisation
+    assert took == [False]
+    _same(short, general)
+    for kw, exc in ((dict(q=q[:, :48]), ValueError), (dict(q=q.float()), TypeError), (dict(idx=idx.long()), TypeError),
+                    (dict(idx=idx[:2]), ValueError), (dict(kv=kv[:, :512]), ValueError), (dict(q=q.cpu()), ValueError),
+                    (dict(job_tokens=2), ValueError), (dict(q=None), TypeError)):
+        for way in (_lib.host(), None):
+            with pytest.MonkeyPatch.context() as m:
+                m.setattr(_lib, "_host", way)
+                with pytest.raises((exc, AttributeError) if kw.get("q", 0) is None else exc):
+                    call(**kw)
+    for way in (_lib.host(), None):                                                          # refused by the library
+        with pytest.MonkeyPatch.context() as m:
+            m.setattr(_lib, "_host", way)
+            with pytest.raises(_lib.LiteDSAError) as e:
+                call(idx=idx[:, :254].contiguous())
+            assert e.value.code == _lib.ERR_SHAPE
+            with pytest.raises(_lib.LiteDSAError) as e:
+                call(q_scale=0.0)
+            assert e.value.code == _lib.ERR_SHAPE
+
+
+@pytest.mark.parametrize("T,h,S,n_comp,sink", [(2, 64, 300, 0, False), (24, 16, 77777, 607, True), (4, 32, 5000, 39, True)])
+def test_dsv4_ranges(both, T, h, S, n_comp, sink):
+    g = torch.Generator(device=DEV).manual_seed(6)
+    q, kr = (torch.empty(s, dtype=torch.bfloat16, device=DEV).normal_(generator=g) for s in ((T, h, 576), (S, 576)))
+    kc = torch.empty((n_comp, 576), dtype=torch.bfloat16, device=DEV).normal_(generator=g) if n_comp else None
+    sk = torch.randn((h,), generator=g, device=DEV) if sink else None
+    short, general, took = both(lambda: api.dsv4_c128a_bf16(q, kc, kr, S - T, synth.SM_SCALE, attn_sink=sk))
+    assert took == [True]
+    _same(short, general)
+    short, general, took = both(lambda: api.dsv4_c128a_bf16(q, q.new_empty((0, 576)), kr, S - T, synth.SM_SCALE, heads=h))
+    assert took == []
+    _same(short, general)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+def test_dsv4_lists(both, dims):
+    T, h, S = 8, 32, 3000
+    g = torch.Generator(device=DEV).manual_seed(7)
+    q, kc, kr = (torch.empty(s, dtype=torch.bfloat16, device=DEV).normal_(generator=g) for s in ((T, h, 512), (S // 128, 512), (S, 512)))
+    q, kv, idx, pref, lo, hi, counts = synth.dsv4_rank_space_operands(q, kc, kr, S - T, h, 128, 128)
+    kv, idx = (x.reshape(x.shape[0], -1) if dims == 2 else x.reshape(x.shape[0], 1, -1) for x in (kv, idx))
+    sink = torch.randn((128,), generator=g, device=DEV)
+
+    def call(in_place=False):
+        out, lse = torch.empty((T * h // 128, 128, 512), dtype=torch.bfloat16, device=DEV), torch.empty((T * h // 128, 128), device=DEV)
+        api.dsv4_masked_mla_bf16_out(q, kv, idx, pref, lo, hi, counts, synth.SM_SCALE, h, out, lse, sink)
+        return out, lse
+    short, general, took = both(call)
+    assert took == [True]
+    _same(short, general)
+
+
+@pytest.mark.parametrize("T,Hi,S,k,scale", [(3, 32, 1001, 64, True), (36, 64, 5000, 1024, True), (2, 128, 4096, 512, False)])
+def test_lite_topk(both, T, Hi, S, k, scale):
+    q, kk, w, ks = (x.to(DEV) for x in synth.make_indexer_operands(T, S, Hi, seed=8))
+    short, general, took = both(lambda: api.lite_topk(q, kk, w, ks if scale else None, k, S - T))
+    assert took == [True]
+    _same(short, general)
+    short, general, took = both(lambda: api.lite_topk(q, kk, w, ks, k, S - T, logits_workspace=torch.empty((T, S + 5), device=DEV)))
+    assert took == []
+    assert torch.equal(short.sort(dim=1).values, general.sort(dim=1).values)
