@@ -90,7 +90,8 @@ __device__ __forceinline__ bool elect_one() {
   return e != 0;
 }
 
-template <int HI>
+// accs: accumulators in use, a CTA's tokens are accs * 128 / HI (a run-time number costs spills)
+template <int HI, int accs>
 __global__ void __launch_bounds__(kThreads, 1)
 index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const LogitParams p) {
@@ -104,8 +105,8 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   constexpr int tpa = kCols / HI;               // tokens per accumulator
-  const int tok0 = blockIdx.x * kAccs * tpa;    // first token of this CTA
-  const int tok_end = min(p.T, tok0 + kAccs * tpa);
+  const int tok0 = blockIdx.x * accs * tpa;     // first token of this CTA
+  const int tok_end = min(p.T, tok0 + accs * tpa);
   // key tiles up to the causal bound of the CTA's last token, and this CTA's share [j0, j0 + n)
   const int pos_max = p.q_pos0 + tok_end - 1;
   const int all_tiles = (p.S + kKeyTile - 1) / kKeyTile;
@@ -143,8 +144,8 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0 && n_tiles > 0) {
       const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
-      mbar_arrive_expect_tx(&bar.q_full, kAccs * kQTile);
-      for (int a = 0; a < kAccs; ++a)
+      mbar_arrive_expect_tx(&bar.q_full, accs * kQTile);
+      for (int a = 0; a < accs; ++a)
         tma_load_2d_hint(sbase + kOffQ + a * kQTile, &map_q, 0, tok0 * HI + a * kCols, &bar.q_full, pol_stream);
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % kStages;
@@ -163,7 +164,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         ok = mbar_wait(&bar.k_full[s], (j / kStages) & 1, wt, kSiteKFull, j);
         if (!ok) break;
         const uint64_t ad = umma_desc(sbase + kOffK + s * kKTile, 16, 1024, kSwz128);
-        for (int a = 0; a < kAccs && ok; ++a) {
+        for (int a = 0; a < accs && ok; ++a) {
           // accumulator a still holds tile j-1 until its four warps have read it
           if (j > 0) ok = mbar_wait(&bar.acc_free[a], (j - 1) & 1, wt, kSiteAccFree, j);
           if (!ok) break;
@@ -178,7 +179,7 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
     __syncwarp();
-  } else {
+  } else if (warp < kDrainWarp0 + 4 * accs) {
     // ---------------------------------------------------------------- accumulator drain
     // Sixteen warps: accumulator a, TMEM lane quarter q4.  The four warps of one scheduler (one lane
     // quarter) serve four accumulators, which are filled in turn, so that they are in different phases:
@@ -291,23 +292,25 @@ index_logits_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(&g_status[3], 1);
 }
 
+template <int N> struct Int { static constexpr int value = N; };
+
 // How many key ranges the grid splits every token group's keys into.  A CTA occupies an SM by
-// itself (all of TMEM) and works about one unit of time per key tile after a start-up worth about
-// four (TMEM and barrier set-up, the 64 KB of Q, the first K tile), so the launch takes
+// itself (all of TMEM) and works about one unit of time per key tile -- less with fewer accumulators in use -- after a start-up
+// worth about four (TMEM and barrier set-up, the 64 KB of Q, the first K tile), so the launch takes
 // waves(ctas_x * splits) * (4 + tiles per split): few tokens need many splits to fill the SMs (36
 // tokens of 32 heads are 3 CTAs: 867 -> 22 us against 100K keys), many tokens a few so that the
 // last wave is full.  The tiles beyond every token's position are only filled with -inf, at about a 90th of
 // a unit per tile and token of the CTA, and shared out among the same CTAs.  (A CTA per range of the
 // whole cache paid the start-up for each of them: 150 tokens of 128 heads at position 0 of 131072
 // 507 us; with ranges of the live tiles alone 20.)
-static int pick_splits(int ctas_x, int live, int dead, int tok_per_cta, int sms) {
+static int pick_splits(int ctas_x, int live, int dead, int tok_per_cta, int accs, int sms) {
   int best = 1;
   long long best_cost = -1;
   for (int n = 1; n <= 64 && n <= live + dead; ++n) {
     const int per = (live + n - 1) / n;
     const long long ranges = dead > 0 ? n : (live + per - 1) / per;      // CTAs with something to do
     const long long waves = (ctas_x * ranges + sms - 1) / sms;
-    const long long cost = waves * (90LL * (4 + per) + (long long)((dead + n - 1) / n) * tok_per_cta);
+    const long long cost = waves * (90LL * 4 + 18LL * (accs + 1) * per + (long long)((dead + n - 1) / n) * tok_per_cta);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = n; }
   }
   return best;
@@ -1144,21 +1147,28 @@ extern "C" int litedsa_index_logits_fp8(const void* q_idx8, const void* k_idx8, 
   p.T = T; p.Hi = Hi; p.S = S; p.q_pos0 = q_pos0; p.ld = logits_row_stride;
   p.epoch = next_launch_epoch(); p.wait_limit_ns = wait_limit_ns();
   const int dev = current_device();
-  if (!(Hi == 32 ? ensure_smem<index_logits_kernel<32>>(dev, kSmem)
-                 : (Hi == 64 ? ensure_smem<index_logits_kernel<64>>(dev, kSmem) : ensure_smem<index_logits_kernel<128>>(dev, kSmem))))
-    return LITEDSA_ERR_CUDA;
-  const int tok_per_cta = kAccs * (kCols / Hi);
-  const int ctas_x = (T + tok_per_cta - 1) / tok_per_cta;
+  // The tokens are dealt to as few CTAs as hold them, evenly: the drain of a key tile, which paces a CTA, takes as long as its
+  // accumulators are many (36 tokens of 32 heads: three CTAs of three accumulators each, not of four, four and one:
+  // 100003 keys 24.4 -> 20.8 us; two tokens of 64 heads, one accumulator, 65536 keys 12.0 -> 8.1).
+  const int groups = (T + kCols / Hi - 1) / (kCols / Hi), ctas_x = (groups + kAccs - 1) / kAccs;
+  const int accs = (groups + ctas_x - 1) / ctas_x, tok_per_cta = accs * (kCols / Hi);
   // the tiles that do work: up to the last token's causal bound
   const int all_tiles = (S + kKeyTile - 1) / kKeyTile;
   const int live_tiles = (int)min((long long)all_tiles, ((long long)q_pos0 + T - 1) / kKeyTile + 1);
   const int dead_tiles = all_tiles - live_tiles;
-  const int splits = pick_splits(ctas_x, live_tiles, dead_tiles, tok_per_cta, sm_count());
+  const int splits = pick_splits(ctas_x, live_tiles, dead_tiles, tok_per_cta, accs, sm_count());
   p.live_tiles = live_tiles;
   p.tiles_per_split = (live_tiles + splits - 1) / splits;
   const int grid_y = dead_tiles > 0 ? splits : (live_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
-  return launch_pdl(Hi == 32 ? index_logits_kernel<32> : (Hi == 64 ? index_logits_kernel<64> : index_logits_kernel<128>),
-                    dim3(ctas_x, grid_y), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_k, p);
+  auto go = [&](auto hi, auto use) -> int {
+    constexpr auto* kern = index_logits_kernel<decltype(hi)::value, decltype(use)::value>;
+    if (!ensure_smem<index_logits_kernel<decltype(hi)::value, decltype(use)::value>>(dev, kSmem)) return LITEDSA_ERR_CUDA;
+    return launch_pdl(kern, dim3(ctas_x, grid_y), kThreads, kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_k, p);
+  };
+  auto with_accs = [&](auto hi) -> int {
+    return accs == 1 ? go(hi, Int<1>()) : accs == 2 ? go(hi, Int<2>()) : accs == 3 ? go(hi, Int<3>()) : go(hi, Int<4>());
+  };
+  return Hi == 32 ? with_accs(Int<32>()) : Hi == 64 ? with_accs(Int<64>()) : with_accs(Int<128>());
 }
 
 // Exact top-k per row of `logits`: topk_idx[t, :] = the k positions i < len(t) with the largest

@@ -55,6 +55,21 @@ def test_index_logits_match_the_formula(T, S, Hi, pos0):
     assert bool(torch.isinf(got[~valid]).all()) and bool((got[~valid] < 0).all())
 
 
+@pytest.mark.parametrize("Hi,tokens", [(32, (1, 4, 5, 8, 9, 13, 17, 20, 33)), (64, (1, 3, 5, 7, 9, 11)), (128, (1, 2, 3, 4, 5, 6, 9))])
+def test_index_logits_of_few_tokens_on_one_to_four_accumulators(Hi, tokens):
+    # a CTA has as many accumulators in use as its share of the tokens needs; the last CTA's share is cut
+    for T in tokens:
+        for S, pos0 in ((1001, 1001 - T), (2500, 700)):                 # the second: key tiles beyond every token
+            q8, k8, w, ks = _ops(T, S, Hi, seed=T + S)
+            ref = io.index_logits(q8, k8, w, ks, pos0)
+            got = api.index_logits_fp8(q8.to(DEV), k8.to(DEV), w.to(DEV), ks.to(DEV), pos0).cpu().double()
+            assert api.index_status(reset=True)[0] == 0
+            valid = torch.arange(S)[None, :] <= (pos0 + torch.arange(T))[:, None]
+            scale = ref[valid].abs().max().item()
+            assert (got[valid] - ref[valid]).abs().max().item() <= 2e-6 * scale * Hi ** 0.5, T      # as above
+            assert bool(torch.isinf(got[~valid]).all()) and bool((got[~valid] < 0).all()), T
+
+
 def test_index_logits_agree_with_the_deepgemm_kernel():
     # an independent production kernel of the same operator: DeepGEMM's fp8 MQA logits as shipped
     # inside the vLLM package of this image (JIT-compiled on first use); skipped where it is absent
