@@ -1091,17 +1091,17 @@ topk_select_cluster_kernel(const SelParams p, int nc) {
 
 constexpr size_t kChunkDyn = (size_t)2 * kChunk * 4 + (size_t)kSurvCap * 8;
 
-// how many clusters of nc (2, 4 or 8) CTAs of topk_select_cluster_kernel device `dev` holds at once
+// how many clusters of nc (2 .. 8) CTAs of topk_select_cluster_kernel device `dev` holds at once
 static int row_clusters(int dev, int nc, int sms) {
-  static thread_local int cached_dev = -1, cached[3];
+  static thread_local int cached_dev = -1, cached[9];
   if (dev != cached_dev) {
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 2; i <= 8; ++i) {
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)((sms >> (i + 1)) << (i + 1))); cfg.blockDim = dim3(kStreamThreads);
+      cfg.gridDim = dim3((unsigned)(sms / i * i)); cfg.blockDim = dim3(kStreamThreads);
       cfg.dynamicSmemBytes = kChunkDyn;
       cudaLaunchAttribute at;
       at.id = cudaLaunchAttributeClusterDimension;
-      at.val.clusterDim.x = 2u << i; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+      at.val.clusterDim.x = (unsigned)i; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
       cfg.attrs = &at; cfg.numAttrs = 1;
       int n = 0;
       if (!ensure_smem<topk_select_cluster_kernel>(dev, kChunkDyn) ||
@@ -1112,7 +1112,7 @@ static int row_clusters(int dev, int nc, int sms) {
     }
     cached_dev = dev;
   }
-  return cached[nc == 8 ? 2 : nc >> 2];
+  return cached[nc];
 }
 
 }  // namespace idx
@@ -1199,9 +1199,10 @@ extern "C" int litedsa_topk_select(const float* logits, const int32_t* lengths, 
   // filter saves (20000 entries, k = 2048: 11.9 us, one CTA per row 10.3; 32768: 12.2 and 12.3; 131072:
   // 14.1 and 28.8).  What counts is how many clusters fit, not how many SMs there are: 18 clusters of eight are
   // 144 CTAs but more than the chip's GPCs hold, and the second wave made 18 rows of 32768 entries take
-  // 20.3 us.
+  // 20.3 us.  Sizes that are no powers of two fit where the next power does not: 36 rows of 100003 entries in clusters of three
+  // 16.2 us, of two 18.2.
   int nc = aligned ? 8 : 1;
-  while (nc > 1 && (S <= 24576 || S < 8192 * nc || T > row_clusters(dev, nc, sms))) nc >>= 1;
+  while (nc > 1 && (S <= 24576 || S < 8192 * nc || T > row_clusters(dev, nc, sms))) --nc;
   if (nc > 1) {
     if (!lt::ensure_smem<topk_select_cluster_kernel>(dev, kChunkDyn)) return LITEDSA_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};

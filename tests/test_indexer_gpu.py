@@ -314,6 +314,17 @@ def test_topk_select_few_rows_shared_by_clusters(T, S, k):
     assert np.array_equal(_canon(got), ref)
 
 
+@pytest.mark.parametrize("T", [16, 20, 24, 28, 36, 48, 60, 80])
+def test_topk_select_rows_shared_by_clusters_of_any_size(T):
+    # as many CTAs per row as fit on the chip for all rows at once: two to eight, three, five and six among them
+    S, k = 70003, 777
+    logits = torch.empty((T, 70004), device=DEV).normal_(generator=torch.Generator(device=DEV).manual_seed(T))[:, :S]
+    sel = api.topk_select(logits, k, q_pos0=S - T)
+    torch.cuda.synchronize()
+    assert api.index_status(reset=True)[0] == 0
+    assert np.array_equal(_canon(sel), io.topk_exact(logits.cpu(), k, q_pos0=S - T))
+
+
 def test_index_logits_of_a_long_cache_before_its_tokens_arrive():
     # tokens at the start of a cache of more than 65535 key tiles, all but the first beyond their positions
     T, S, Hi, pos0 = 3, 65536 * 128 + 5, 64, 70
