@@ -65,6 +65,11 @@ PyObject* pair(const Tensor& a, const Tensor& b) {
   Py_XDECREF(pb);
   return r;
 }
+// allocations and launches can block: other Python threads run meanwhile, as with ctypes
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 // C++ exceptions (out of memory, say) leave as the Python exceptions that torch makes of them
 template <class F>
 PyObject* guarded(F&& f) {
@@ -107,13 +112,18 @@ PyObject* sparse_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     else if (!integer(a[6], &space)) Py_RETURN_NONE;
     if (a[7] == Py_None) job = T;
     else if (!integer(a[7], &job) || job < T) Py_RETURN_NONE;
-    Tensor out = empty({T, h, 512}, at::kBFloat16, *q), lse = empty({T, h}, at::kFloat, *q);
-    const int64_t bytes = litedsa_sparse_prefill_job_workspace((int)T, (int)h, (int)k, kv_bf16, (int)job);
-    Tensor ws = empty({bytes > 0 ? bytes : 1}, at::kByte, *q);
-    const int rc = litedsa_sparse_prefill_job(q->data_ptr(), q_bf16, kv->data_ptr(), kv_bf16, static_cast<const int32_t*>(idx->data_ptr()), sm,
-                                              q_scale, kv_scale, out.data_ptr(), static_cast<float*>(lse.data_ptr()), (int)T, (int)h, (int)k,
-                                              (int)s_kv, kv->stride(0), (space + 1023) / 1024 * 1024, (int)job, ws.data_ptr(), ws.numel(),
-                                              stream_of(dev));
+    Tensor out, lse;
+    int rc;
+    {
+      NoGil unlocked;
+      out = empty({T, h, 512}, at::kBFloat16, *q);
+      lse = empty({T, h}, at::kFloat, *q);
+      const int64_t bytes = litedsa_sparse_prefill_job_workspace((int)T, (int)h, (int)k, kv_bf16, (int)job);
+      Tensor ws = empty({bytes > 0 ? bytes : 1}, at::kByte, *q);
+      rc = litedsa_sparse_prefill_job(q->data_ptr(), q_bf16, kv->data_ptr(), kv_bf16, static_cast<const int32_t*>(idx->data_ptr()), sm, q_scale,
+                                      kv_scale, out.data_ptr(), static_cast<float*>(lse.data_ptr()), (int)T, (int)h, (int)k, (int)s_kv,
+                                      kv->stride(0), (space + 1023) / 1024 * 1024, (int)job, ws.data_ptr(), ws.numel(), stream_of(dev));
+    }
     return rc == LITEDSA_OK ? pair(out, lse) : PyLong_FromLong(rc);
   });
 }
@@ -139,14 +149,20 @@ PyObject* dsv4_c128a_bf16(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (T <= 0 || !small(T) || !heads_ok(h) || T % (128 / h) != 0) Py_RETURN_NONE;
     if (sink && (sink->scalar_type() != at::kFloat || sink->dim() != 1 || sink->size(0) != h || !sink->is_contiguous())) Py_RETURN_NONE;
     const int ng = (int)(T * h / 128), n_comp = kc ? (int)kc->size(0) : 0;
-    Tensor out = empty({T, h, 512}, at::kBFloat16, *q), lse = empty({T, h}, at::kFloat, *q), ws;
-    const int64_t bytes = litedsa_dsv4_workspace(ng, (int)h, n_comp, (int)pos0, (int)window, (int)ratio);
-    if (bytes > 0) ws = empty({bytes}, at::kByte, *q);
-    const int rc = litedsa_dsv4_c128a_bf16_ws(q->data_ptr(), kc ? kc->data_ptr() : nullptr, kr->data_ptr(), ng, (int)h, n_comp,
-                                              (int)kr->size(0), (int)pos0, (int)window, (int)ratio, (float)sm,
-                                              sink ? static_cast<const float*>(sink->data_ptr()) : nullptr, (int)h, out.data_ptr(),
-                                              static_cast<float*>(lse.data_ptr()), 576, kc ? kc->stride(0) : 576, kr->stride(0), h * 576,
-                                              576, h * 512, 512, bytes > 0 ? ws.data_ptr() : nullptr, bytes, stream_of(dev));
+    Tensor out, lse;
+    int rc;
+    {
+      NoGil unlocked;
+      Tensor ws;
+      out = empty({T, h, 512}, at::kBFloat16, *q);
+      lse = empty({T, h}, at::kFloat, *q);
+      const int64_t bytes = litedsa_dsv4_workspace(ng, (int)h, n_comp, (int)pos0, (int)window, (int)ratio);
+      if (bytes > 0) ws = empty({bytes}, at::kByte, *q);
+      rc = litedsa_dsv4_c128a_bf16_ws(q->data_ptr(), kc ? kc->data_ptr() : nullptr, kr->data_ptr(), ng, (int)h, n_comp, (int)kr->size(0),
+                                      (int)pos0, (int)window, (int)ratio, (float)sm, sink ? static_cast<const float*>(sink->data_ptr()) : nullptr,
+                                      (int)h, out.data_ptr(), static_cast<float*>(lse.data_ptr()), 576, kc ? kc->stride(0) : 576,
+                                      kr->stride(0), h * 576, 576, h * 512, 512, bytes > 0 ? ws.data_ptr() : nullptr, bytes, stream_of(dev));
+    }
     return rc == LITEDSA_OK ? pair(out, lse) : PyLong_FromLong(rc);
   });
 }
@@ -180,13 +196,17 @@ PyObject* dsv4_masked_mla_bf16_out(PyObject*, PyObject* const* a, Py_ssize_t n) 
         !out->is_contiguous() || lse->scalar_type() != at::kFloat || lse->numel() != ng * 128 || !lse->is_contiguous())
       Py_RETURN_NONE;
     if (sink && (sink->scalar_type() != at::kFloat || sink->dim() != 1 || sink->size(0) != 128 || !sink->is_contiguous())) Py_RETURN_NONE;
-    Tensor ws = empty({16 + 16 * ng}, at::kByte, *q);
     auto ints = [](const Tensor* t) { return static_cast<const int32_t*>(t->data_ptr()); };
-    const int rc = litedsa_dsv4_masked_mla_bf16(q->data_ptr(), kv->data_ptr(), ints(idx), ints(range[0]), ints(range[1]), ints(range[2]),
-                                                ints(counts), (float)sm, (int)h, out->data_ptr(), static_cast<float*>(lse->data_ptr()),
-                                                sink ? static_cast<const float*>(sink->data_ptr()) : nullptr, (int)ng, (int)kv->size(0),
-                                                (int)idx->size(-1), (int)d, q->stride(1), kv->stride(0), idx->stride(0), 0, 0, 0, 0,
-                                                ws.data_ptr(), ws.numel(), stream_of(dev));
+    int rc;
+    {
+      NoGil unlocked;
+      Tensor ws = empty({16 + 16 * ng}, at::kByte, *q);
+      rc = litedsa_dsv4_masked_mla_bf16(q->data_ptr(), kv->data_ptr(), ints(idx), ints(range[0]), ints(range[1]), ints(range[2]), ints(counts),
+                                        (float)sm, (int)h, out->data_ptr(), static_cast<float*>(lse->data_ptr()),
+                                        sink ? static_cast<const float*>(sink->data_ptr()) : nullptr, (int)ng, (int)kv->size(0),
+                                        (int)idx->size(-1), (int)d, q->stride(1), kv->stride(0), idx->stride(0), 0, 0, 0, 0, ws.data_ptr(),
+                                        ws.numel(), stream_of(dev));
+    }
     if (rc != LITEDSA_OK) return PyLong_FromLong(rc);
     Py_RETURN_TRUE;
   });
@@ -207,16 +227,24 @@ PyObject* lite_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
       Py_RETURN_NONE;
     if (ks && (ks->scalar_type() != at::kFloat || ks->dim() != 1 || ks->size(0) != S || !ks->is_contiguous())) Py_RETURN_NONE;
     // rows start on 16-byte boundaries whatever S is: the streaming selection kernels need that
-    Tensor logits = empty({T, ld}, at::kFloat, *q), out = empty({T, k}, at::kInt, *q);
-    void* stream = stream_of(dev);
-    int rc = litedsa_index_logits_fp8(q->data_ptr(), k8->data_ptr(), static_cast<const float*>(w->data_ptr()),
-                                      ks ? static_cast<const float*>(ks->data_ptr()) : nullptr, static_cast<float*>(logits.data_ptr()), (int)T,
-                                      (int)Hi, (int)S, (int)pos0, k8->stride(0), ld, stream);
-    if (rc != LITEDSA_OK) return Py_BuildValue("(is)", rc, "index_logits_fp8");
-    rc = litedsa_topk_select(static_cast<const float*>(logits.data_ptr()), nullptr, static_cast<int32_t*>(out.data_ptr()), (int)T, (int)S, (int)k,
-                             (int)pos0, ld, stream);
-    if (rc != LITEDSA_OK) return Py_BuildValue("(is)", rc, "topk_select");
-    return THPVariable_Wrap(out);
+    Tensor out;
+    int rc;
+    const char* where = "index_logits_fp8";
+    {
+      NoGil unlocked;
+      Tensor logits = empty({T, ld}, at::kFloat, *q);
+      void* stream = stream_of(dev);
+      rc = litedsa_index_logits_fp8(q->data_ptr(), k8->data_ptr(), static_cast<const float*>(w->data_ptr()),
+                                    ks ? static_cast<const float*>(ks->data_ptr()) : nullptr, static_cast<float*>(logits.data_ptr()), (int)T,
+                                    (int)Hi, (int)S, (int)pos0, k8->stride(0), ld, stream);
+      if (rc == LITEDSA_OK) {
+        where = "topk_select";
+        out = empty({T, k}, at::kInt, *q);
+        rc = litedsa_topk_select(static_cast<const float*>(logits.data_ptr()), nullptr, static_cast<int32_t*>(out.data_ptr()), (int)T, (int)S,
+                                 (int)k, (int)pos0, ld, stream);
+      }
+    }
+    return rc == LITEDSA_OK ? THPVariable_Wrap(out) : Py_BuildValue("(is)", rc, where);
   });
 }
 

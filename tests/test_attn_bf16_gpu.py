@@ -448,8 +448,10 @@ def test_native_many_short_tiles(tokens, heads, topk):
 
 
 @pytest.mark.parametrize("tokens,heads,topk", [
-    (2, 64, 2048),         # one tile, eight slices
-    (24, 32, 1536),        # six tiles, eight slices
+    (2, 64, 2048),         # one tile, twelve slices
+    (2, 64, 512),          # a short one, six slices
+    (8, 16, 256),          # ... of eight tokens
+    (24, 32, 1536),        # six tiles, twelve slices
     (8, 16, 2048),         # one tile of eight tokens, sixteen slices
     (30, 64, 1984),        # 15 tiles, four slices; a list that is not a multiple of the block
 ])

@@ -447,12 +447,14 @@ def test_path_agrees_with_the_stock_per_token_sparse_mla_kernel():
 
 
 @pytest.mark.parametrize("tokens,heads,topk,s_kv", [
-    (2, 64, 2048, 32768),       # one tile, five slices of four blocks
+    (2, 64, 2048, 32768),       # one tile, eight slices of two or three blocks
+    (2, 64, 1024, 8192),        # the shortest tile that is cut, six slices
+    (18, 64, 1024, 9000),       # nine of them, five slices each
     (2, 64, 512, 4096),         # too short to slice
     (34, 64, 1024, 8192),       # 17 tiles, too short to slice
     (34, 64, 1536, 16384),      # 17 tiles, three slices
     (34, 64, 2048, 16384),      # 17 tiles, four slices
-    (8, 16, 2048, 20000),       # one tile of eight tokens, eleven slices
+    (8, 16, 2048, 20000),       # one tile of eight tokens, thirteen slices
     (8, 16, 4096, 20000),       # ... sixteen slices
     (300, 32, 256, 5000),       # 75 tiles: one more than clusters
 ])

@@ -96,11 +96,12 @@ def test_dsv4_in_place_padded_heads(h, hpad):
 
 
 @pytest.mark.parametrize("T,h,S,Nc,pos0,sink", [
-    (24, 16, 77777, 607, 77777 - 24, True),     # three tiles of 12 blocks: too short to slice; sink per head
-    (24, 16, 140000, 1093, 140000 - 24, True),  # three tiles, four slices each, sink per head
-    (8, 16, 300000, 2343, 300000 - 8, False),   # one tile of 39 blocks, seven slices
+    (24, 16, 77777, 607, 77777 - 24, True),     # three tiles of 12 blocks, six slices each; sink per head
+    (24, 16, 140000, 1093, 140000 - 24, True),  # three tiles, eight slices each, sink per head
+    (8, 16, 300000, 2343, 300000 - 8, False),   # one tile of 40 blocks, twelve slices
+    (8, 16, 40000, 312, 40000 - 8, False),      # one of eight blocks, five slices: the shortest that is cut
     (16, 8, 300000, 2343, 160001, True),        # one tile of sixteen tokens in the middle of the cache
-    (2, 64, 9000, 70, 300, False),              # five blocks: one slice
+    (2, 64, 9000, 70, 300, False),              # three blocks: one slice
 ])
 def test_dsv4_few_tiles_run_in_slices(T, h, S, Nc, pos0, sink):
     _run(T, h, S, Nc, pos0, sink=sink, seed=T + h)
