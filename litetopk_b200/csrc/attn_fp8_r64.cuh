@@ -85,6 +85,7 @@ struct Params {
   const uint32_t* memb;      // [ng, G, cap / 32], or null: every list entry is every row's
   const int32_t* indices;    // [ng, cap], -1 up to the next multiple of 64
   const int32_t* counts;     // [ng]
+  const int2* order;         // [ng] (tile, keys) in the order in which they are dealt out, or null: as they come
   const uint8_t* kv;         // [s_kv, kv_pitch] e4m3 rows (576 bytes used)
   long long kv_pitch;
   float* lse;                // [ng, 64]
@@ -144,7 +145,7 @@ __device__ __forceinline__ void commit_elect(uint64_t* bar) {
 }
 // kWide: the cache is too large for row offsets in 32 bits of 16-byte units (64 GB); their products in 64 bits take 1 %
 // of the time (8192 tokens x 64 heads 1271 -> 1295 us)
-template <bool kWide>
+template <bool kWide, bool kOrdered>
 __global__ void __launch_bounds__(kThreads, 1)
 masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_rope,
                           const __grid_constant__ CUtensorMap map_out, const Params p) {
@@ -163,10 +164,19 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
 
   const int cid = blockIdx.x, ncta = gridDim.x, ng = p.ng;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  auto live_of = [&](int tile) -> int { return min(max(p.counts[tile], 0), p.cap); };
-  // key blocks of a tile, 0 past the last one.  Every role loads the next tile's number a tile ahead: a
-  // dependent load at the change of tiles would hold up all of them.
-  auto blocks_of = [&](int tile) -> int { return tile < ng ? max((live_of(tile) + kBlockKeys - 1) / kBlockKeys, 1) : 0; };
+  // item i: its tile (x) and that one's keys (y), and the key blocks of these, 0 past the last one.  Every role loads the next
+  // item's a tile ahead: a dependent load at the change of tiles would hold up all of them.
+  auto item_at = [&](int i) -> int2 {
+    if (i >= ng) return make_int2(0, -1);
+    return kOrdered ? __ldcg(p.order + i) : make_int2(i, min(max(p.counts[i], 0), p.cap));
+  };
+  struct Next { int tile, nb; };
+  auto next_at = [&](int i) -> Next {
+    const int2 v = item_at(i);
+    return {v.x, v.y >= 0 ? max((v.y + kBlockKeys - 1) / kBlockKeys, 1) : 0};
+  };
+  // the tile of item i, `known` where that has to be loaded
+  auto tile_at = [&](int i, int known) -> int { return kOrdered ? known : i; };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 8; ++i) {
@@ -231,15 +241,17 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     const float c = p.scale_log2;
     const uint64_t c2 = pack2(c, c);
     const uint32_t scol = tmem + lane_base + kTmemS + 32 * g;
-    int kb0 = 0, it = 0, nb_next = blocks_of(cid);
+    int kb0 = 0, it = 0;
+    Next next = next_at(cid);
     // this thread's membership words: two per block of its token
-    const uint32_t* mrow = p.memb ? p.memb + ((size_t)cid * p.G + r / p.h_per_q) * capw + h : nullptr;
+    const uint32_t* mrow = p.memb ? p.memb + ((size_t)tile_at(cid, next.tile) * p.G + r / p.h_per_q) * capw + h : nullptr;
     uint32_t mk_next = ~0u;
     if (mrow) mk_next = __ldcs(mrow + 2 * g);      // (cap >= 256: a group's first word exists even if its block does not)
 
-    for (int tile = cid; tile < ng; tile += ncta, ++it) {
-      const int nb = nb_next;
-      nb_next = blocks_of(tile + ncta);
+    for (int i = cid; i < ng; i += ncta, ++it) {
+      const Next cur = next;
+      const int nb = cur.nb;
+      next = next_at(i + ncta);
       float m_mine = kMInit;      // the running max my row sum is relative to
       float li = 0.f;
 
@@ -349,8 +361,8 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         if (lane == 0) mbar_arrive(&ms.p_ready[kb & 7]);
       }
 
-      if (mrow && tile + ncta < ng) {
-        mrow += (size_t)ncta * p.G * capw;
+      if (mrow && i + ncta < ng) {
+        mrow += (kOrdered ? (ptrdiff_t)(next.tile - cur.tile) : (ptrdiff_t)ncta) * p.G * capw;
         mk_next = __ldcs(mrow + 2 * ((g - kb0 - nb) & (kGroups - 1)));
       }
       // end of item: row sums, each relative to its own group's latest running max, for the epilogue
@@ -378,30 +390,32 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     const uint8_t* kv_lat = p.kv + 16 * lane;
     const uint8_t* kv_rope = p.kv + 512 + 16 * (lane & 3);
     const int own_key = 16 * pw + (lane & 15);
-    int slot = set, ring = 0, e = 0, it = 0, nb_next = blocks_of(cid);
+    int slot = set, ring = 0, e = 0, it = 0;
+    Next next = next_at(cid);
     auto first_k = [&](int e0) -> int { return (set - e0 - 1) & 1; };      // first own block of an item whose Q is entry e0
-    int kidx = __ldcs(p.indices + (size_t)cid * p.cap + first_k(0) * kBlockKeys + own_key);
+    int kidx = __ldcs(p.indices + (size_t)tile_at(cid, next.tile) * p.cap + first_k(0) * kBlockKeys + own_key);
     auto advance = [&]() { slot += 2; if (slot >= kSlots) { slot -= kSlots; ++ring; } };
     bool ok = true, go = true;                     // none of this lane's / this warp's waits has given up: then it leaves
-    for (int tile = cid; go && tile < ng + ncta; tile += ncta, ++it) {      // behind the last item: an entry to stage its output in
-      const int nb = nb_next;
-      nb_next = blocks_of(tile + ncta);
+    for (int i = cid; go && i < ng + ncta; i += ncta, ++it) {      // behind the last item: an entry to stage its output in
+      const int tile = tile_at(i, next.tile), nb = next.nb;
+      next = next_at(i + ncta);
       const int32_t* idx = p.indices + (size_t)tile * p.cap + own_key;
       auto next_tile_idx = [&]() -> int {
-        return tile + ncta < ng ? __ldcs(idx + (size_t)ncta * p.cap + first_k(e + nb + 1) * kBlockKeys) : 0;
+        return i + ncta < ng ? __ldcs((kOrdered ? p.indices + (size_t)next.tile * p.cap + own_key : idx + (size_t)ncta * p.cap) +
+                                     first_k(e + nb + 1) * kBlockKeys) : 0;
       };
       // With short items the previous Q could still be on its way.  Every warp goes through every item's barrier
       // and a Q counts as landed only when all of them have -- those of its set also through its slot's
       // barrier --, so that none is overtaken and tests a phase that is two ahead.
       if (it > 0) ok &= mbar_wait(&ms.q_taken, (it - 1) & 1, wt, kSiteQ, it);
-      if (p.q_bf16 != nullptr && tile < ng) ok &= mbar_wait(&ms.q_codes, it & 1, wt, kSiteQ, it);
+      if (p.q_bf16 != nullptr && i < ng) ok &= mbar_wait(&ms.q_codes, it & 1, wt, kSiteQ, it);
       const bool q_mine = (e & 1) == set;
       if (q_mine && ring > 0) ok &= mbar_wait(&ms.slot_free[slot], (ring - 1) & 1, wt, kSiteKFree, it);
       __syncwarp();
       // (nothing behind a wait of any warp that gave up: the Q before could still be in flight)
       if (lane == 0 && ok && !wt.aborting()) {
         ms.q_passed[warp - kWarpGather0] = it + 1;
-        if (!q_mine || pw != 0 || tile >= ng) {
+        if (!q_mine || pw != 0 || i >= ng) {
           mbar_arrive(&ms.q_land);
         } else {
           ms.q_asked = it + 1;
@@ -463,16 +477,16 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     }
   } else if (warp < kWarpEpi0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
-    // running position of an MMA-issuing warp: tile, block of the tile, its blocks, item ordinal, running block, slot
-    struct Cursor { int tile, k, nb, it, kb, slot, nb_next; };
+    // running position of an MMA-issuing warp: item, block of its tile, its blocks, item ordinal, running block, slot
+    struct Cursor { int i, k, nb, it, kb, slot, nb_next; };
     auto next = [&](Cursor& c) {
       ++c.kb;
       if (++c.slot == kSlots) c.slot = 0;
       if (++c.k == c.nb) {
-        c.tile += ncta; c.k = 0; ++c.it;
+        c.i += ncta; c.k = 0; ++c.it;
         if (++c.slot == kSlots) c.slot = 0;       // the next item's Q entry
         c.nb = c.nb_next;
-        c.nb_next = blocks_of(c.tile + ncta);
+        c.nb_next = next_at(c.i + ncta).nb;
       }
     };
     // the time-limit and abort check of a wait that has not been satisfied yet (warp-uniform answer)
@@ -487,7 +501,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       const uint32_t hi128 = (uint32_t)(umma_desc(0, 16, 1024, kSwz128) >> 32);
       const uint32_t hi64 = (uint32_t)(umma_desc(0, 16, 512, kSwz64) >> 32);
       const uint32_t a_rope_lo = (uint32_t)umma_desc(sbase + kOffRope, 16, 512, kSwz64);
-      Cursor c{cid, 0, blocks_of(cid), 0, 0, 1, blocks_of(cid + ncta)};
+      Cursor c{cid, 0, next_at(cid).nb, 0, 0, 1, next_at(cid + ncta).nb};
       auto step = [&]() {
         const int it = c.it;
         next(c);
@@ -496,7 +510,7 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       const int mine = warp == kWarpQkOdd ? 1 : 0;
       bool aborted = false;
       uint32_t since = 0;
-      while (c.tile < ng && !aborted) {
+      while (c.i < ng && !aborted) {
         // K rows landed, S buffer drained and, at an item's first block, Q in place, waited for one after the other and
         // suspended.  (One barrier per lane, all tested by one instruction in a loop, took issue slots and power from the
         // warps beside: 1184 tokens x 64 heads, top-2048 189.3 -> 181.1 us, top-512 71.8 -> 68.3; long runs at the power
@@ -525,10 +539,10 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     } else if (warp == kWarpPv) {
       // ---------------------------------------------------------- PV issue
       constexpr uint32_t idesc_pv = umma_idesc(0, 0, false, true, 64, 256);
-      Cursor c{cid, 0, blocks_of(cid), 0, 0, 1, blocks_of(cid + ncta)};
+      Cursor c{cid, 0, next_at(cid).nb, 0, 0, 1, next_at(cid + ncta).nb};
       bool aborted = false;
       uint32_t since = 0;
-      while (c.tile < ng && !aborted) {
+      while (c.i < ng && !aborted) {
         // P written (its QK^T has read the K rows that are V here, so they have landed); an item's first PV
         // overwrites O: the previous item must have been read out
         const bool ok = (c.k > 0 || c.it == 0 || mbar_try_wait(&ms.o_free, (c.it - 1) & 1)) &&
@@ -550,19 +564,20 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       if (lane == 0) ms.pv_end = c.kb;
     } else if (warp == kWarpValid) {
       // ---------------------------------------------------------- index-validity bits
-      int kb = 0, lim_next = live_of(cid);
-      const int32_t* idx = p.indices + (size_t)cid * p.cap + lane;
+      int kb = 0;
+      int2 next = item_at(cid);
+      const int32_t* idx = p.indices + (size_t)tile_at(cid, next.x) * p.cap + lane;
       int i0 = __ldcs(idx), i1 = __ldcs(idx + 32);
-      for (int tile = cid; tile < ng; tile += ncta) {
-        const int lim = lim_next, nb = max((lim + kBlockKeys - 1) / kBlockKeys, 1);
-        if (tile + ncta < ng) lim_next = live_of(tile + ncta);
+      for (int i = cid; i < ng; i += ncta) {
+        const int lim = next.y, nb = max((lim + kBlockKeys - 1) / kBlockKeys, 1);
+        next = item_at(i + ncta);
         for (int k = 0; k < nb; ++k, ++kb) {
           const int s = kb & (kGroups - 1), rank = k * kBlockKeys + lane;
           const uint32_t w0 = __ballot_sync(0xffffffffu, (unsigned)i0 < (unsigned)p.s_kv && rank < lim);
           const uint32_t w1 = __ballot_sync(0xffffffffu, (unsigned)i1 < (unsigned)p.s_kv && rank + 32 < lim);
           idx += kBlockKeys;
-          if (k + 1 == nb) idx = p.indices + (size_t)(tile + ncta) * p.cap + lane;
-          if (k + 1 < nb || tile + ncta < ng) {
+          if (k + 1 == nb) idx = p.indices + (size_t)tile_at(i + ncta, next.x) * p.cap + lane;
+          if (k + 1 < nb || i + ncta < ng) {
             i0 = __ldcs(idx);
             i1 = __ldcs(idx + 32);
           }
@@ -587,12 +602,14 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     const uint32_t e_ocol = tmem + lane_base + kTmemO;
     // bf16 q: item j's codes into q_codes, an item ahead.  (Straight into the Q's ring slot, which is free only when
     // the item before it ends, the loads' latency held up each item by some 6000 cycles.)
-    auto quantise_q = [&](int tile, int j, bool ahead) {
+    // (behind: the item behind that)
+    auto quantise_q = [&](int tile, int j, bool ahead, int behind) {
       const uint4* src = p.q_bf16 + (size_t)tile * kRows * (kDQK / 8);
       uint4* dst = reinterpret_cast<uint4*>(p.q_codes + (size_t)((j & 1) * ncta + cid) * kSlot);
       // The Q of the item behind that into L2 -- with short items only, whose pace these loads' latency bounds (1184 tokens x 64
       // heads, top-256 82.3 -> 78.0 us; top-2048 199.5 -> 202.6).
-      if (ahead && e_tid == 0 && tile + ncta < ng) l2_prefetch_1d(src + (size_t)ncta * kRows * (kDQK / 8), kRows * kDQK * 2);
+      if (ahead && e_tid == 0 && behind < ng)
+        l2_prefetch_1d(p.q_bf16 + (size_t)tile_at(behind, item_at(behind).x) * kRows * (kDQK / 8), kRows * kDQK * 2);
       // 64 rows x 36 units of 16 codes = 18 units per thread, six under way: a unit's registers take the next one's loads as
       // soon as its codes are on their way
       uint4 a[kFillBatch], b[kFillBatch];
@@ -652,16 +669,17 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       asm volatile("bar.sync 5, 128;" ::: "memory");
       if (e_tid == 0) mbar_arrive(&ms.slot_free[n % kSlots]);
     };
-    int kb0 = 0, it = 0, nb_next = blocks_of(cid);
-    if (p.q_bf16 != nullptr) quantise_q(cid, 0, false);
+    int kb0 = 0, it = 0;
+    Next next = next_at(cid);
+    if (p.q_bf16 != nullptr) quantise_q(tile_at(cid, next.tile), 0, false, 0);
     transfer_q(0, 0);
     release(0);
-    for (int tile = cid; tile < ng; tile += ncta, ++it) {
-      const int nb = nb_next, kbl = kb0 + nb - 1;           // last block of the item
-      nb_next = blocks_of(tile + ncta);
+    for (int i = cid; i < ng; i += ncta, ++it) {
+      const int tile = tile_at(i, next.tile), nb = next.nb, kbl = kb0 + nb - 1;           // last block of the item
+      next = next_at(i + ncta);
       const int n = kb0 + nb + it + 1;             // entry number of the next item's Q
-      if (tile + ncta < ng) {
-        if (p.q_bf16 != nullptr) quantise_q(tile + ncta, it + 1, nb <= 12);
+      if (i + ncta < ng) {
+        if (p.q_bf16 != nullptr) quantise_q(tile_at(i + ncta, next.tile), it + 1, nb <= 12, i + 2 * ncta);
         transfer_q(it + 1, n);
       } else {
         mbar_wait(&ms.q_land, (it + 1) & 1, wt, kSiteQ, it + 1);      // an empty entry
@@ -767,9 +785,9 @@ masked_mla_fp8_r64_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
 
 // One launch over the 64-row tiles of dense q [T, h, 576] (ng = T h / 64).  a.nsplit, sinks, strides of q / out and
 // further destinations are not supported here.  With one token per tile every list entry is every row's.  q_codes:
-// rows64_scratch() bytes, used with bf16 queries.
+// rows64_scratch() bytes, used with bf16 queries.  order: see Params.
 int64_t rows64_scratch(int ng) { return (int64_t)2 * min(ng, sm_count()) * r64::kSlot; }
-int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
+int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, const int2* order, void* stream) {
   Fp8Args c = a;
   if (a.h_per_q == r64::kRows) c.memb_qm = reinterpret_cast<const uint32_t*>(a.indices);      // none there, and none read
   const int rc = check_fp8_args(c);
@@ -792,7 +810,7 @@ int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
                    CU_TENSOR_MAP_SWIZZLE_64B))
     return LITEDSA_ERR_CUDA;
   r64::Params p;
-  p.memb = G > 1 ? a.memb_qm : nullptr; p.indices = a.indices; p.counts = a.topk_length;
+  p.memb = G > 1 ? a.memb_qm : nullptr; p.indices = a.indices; p.counts = a.topk_length; p.order = order;
   p.kv = reinterpret_cast<const uint8_t*>(a.kv8); p.kv_pitch = a.kv_row_stride;
   p.lse = a.lse;
   p.ng = a.ng; p.s_kv = a.s_kv; p.cap = a.topk; p.h_per_q = h; p.G = G;
@@ -802,11 +820,15 @@ int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream) {
   p.q_codes = reinterpret_cast<uint8_t*>(q_codes);
   const bool wide = (int64_t)a.s_kv * (a.kv_row_stride >> 4) >= 0xffffffffll;
   const int dev = current_device();
-  if (!(wide ? ensure_smem<r64::masked_mla_fp8_r64_kernel<true>>(dev, r64::Plan::kSmem)
-             : ensure_smem<r64::masked_mla_fp8_r64_kernel<false>>(dev, r64::Plan::kSmem)))
-    return LITEDSA_ERR_CUDA;
-  return launch_pdl(wide ? r64::masked_mla_fp8_r64_kernel<true> : r64::masked_mla_fp8_r64_kernel<false>, dim3((unsigned)ncta),
-                    r64::kThreads, r64::Plan::kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_q_rope, map_out, p);
+  auto launch = [&](auto is_wide, auto is_ordered) -> int {
+    constexpr auto kern = r64::masked_mla_fp8_r64_kernel<decltype(is_wide)::value, decltype(is_ordered)::value>;
+    if (!ensure_smem<kern>(dev, r64::Plan::kSmem)) return LITEDSA_ERR_CUDA;
+    return launch_pdl(kern, dim3((unsigned)ncta), r64::kThreads, r64::Plan::kSmem, reinterpret_cast<cudaStream_t>(stream), map_q, map_q_rope,
+                      map_out, p);
+  };
+  using Yes = std::true_type;
+  using No = std::false_type;
+  return order != nullptr ? (wide ? launch(Yes{}, Yes{}) : launch(No{}, Yes{})) : (wide ? launch(Yes{}, No{}) : launch(No{}, No{}));
 }
 
 }  // namespace lt

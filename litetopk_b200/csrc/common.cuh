@@ -69,7 +69,7 @@ int dsv4_rank_enqueue(const void* q, const void* kv, const int32_t* indices, con
                       cudaStream_t stream);
 int run_fp8(const Fp8Args& a, void* const* outs, int n_outs, void* stream);
 // attn_fp8_r64.cuh: tiles of 64 rows; q_codes: rows64_scratch(ng) bytes
-int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, void* stream);
+int run_fp8_rows64(const Fp8Args& a, void* out, void* q_codes, const int2* order, void* stream);
 int64_t rows64_scratch(int ng);
 // union_qm.cu; cap >= G * k: the row length of u_phys, a multiple of 128.  memb_qm may be null with G = 1.  fill 0: live
 // prefixes only, 1: whole rows, 2: u_phys := -1 up to the next multiple of 128 (one block at least, which the

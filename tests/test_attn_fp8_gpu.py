@@ -552,6 +552,31 @@ def test_a_part_of_a_job_gives_the_bits_of_the_job():
 
 
 @pytest.mark.parametrize("tokens,heads,topk,s_kv", [
+    (3760, 8, 1024, 9000),       # eight tokens per tile; four rounds of tiles, the last not full
+    (7400, 16, 512, 5001),       # four; a full window of eight rounds and half of one
+    (4740, 32, 2048, 7777),      # two; the last window has two tiles
+])
+def test_tiles_in_order_of_their_size_give_the_bits_of_tiles_as_they_come(tokens, heads, topk, s_kv):
+    # parts of fewer tiles than SMs are not ordered
+    g = torch.Generator().manual_seed(22)
+    idx = torch.randint(0, s_kv, (tokens, topk), generator=g, dtype=torch.int32)
+    n = torch.randint(0, topk + 1, (tokens, 1), generator=g)
+    n[torch.rand((tokens, 1), generator=g) < 0.3] = topk
+    n[:64] = 0                                           # empty tiles
+    idx[torch.arange(topk)[None] >= n] = -1
+    w, _, kv, q = _case(16, 64, 16, s_kv, (0.5, 0.5), seed=22)
+    _, kv8, qs, ks = synth.refcompat_operands(q, kv)
+    q8 = torch.randint(0, 120, (tokens, heads, 576), generator=g, dtype=torch.uint8).to(DEV)
+    kvd, idd = kv8.to(DEV), idx.to(DEV)
+    out, lse = api.sparse_prefill(q8, kvd, idd, synth.SM_SCALE / 8, kv_scale=ks, q_scale=qs)
+    part = 128 * 64 // heads
+    for t0 in range(0, tokens, part):
+        rows = slice(t0, t0 + part)
+        o, l = api.sparse_prefill(q8[rows], kvd, idd[rows], synth.SM_SCALE / 8, kv_scale=ks, q_scale=qs, job_tokens=tokens)
+        assert torch.equal(out[rows], o) and torch.equal(lse[rows], l)
+
+
+@pytest.mark.parametrize("tokens,heads,topk,s_kv", [
     (380, 64, 256, 4096),        # one token per tile, four blocks
     (602, 64, 960, 7777),        # a list that is no multiple of 128, ten more tiles in the last round
     (1300, 32, 512, 5001),       # two tokens per tile
