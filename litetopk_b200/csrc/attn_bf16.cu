@@ -36,6 +36,7 @@ struct Args {
   int nsplit = 1;
   float* part_o = nullptr;
   float2* part_ml = nullptr;
+  const int2* order = nullptr;    // d = 576, unsliced (see Params)
 };
 
 // argument rules shared by both entry points (no CUDA call)
@@ -80,6 +81,10 @@ static int run(const Args& a, void* stream) {
   if (a.nsplit > 1) {
     p.nsplit = a.nsplit; p.part_o = a.part_o; p.part_ml = a.part_ml;
     return launch<576, kGather, true>(mq, mq, mq, mout, p, st);
+  }
+  if (a.order != nullptr) {
+    p.order = a.order;
+    return launch<576, kGather, false, true>(mq, mq, mq, mout, p, st);
   }
   return a.d == 576 ? launch<576, kGather, false>(mq, mq, mq, mout, p, st)
                     : launch<512, kGather, false>(mq, mq, mq, mout, p, st);
@@ -127,13 +132,13 @@ __global__ void __launch_bounds__(256) dequant_kv656_kernel(const uint8_t* __res
 
 }  // namespace b16
 
-// the union form on dense packed operands of 576 dims, in nsplit slices (prefill.cu)
-int run_bf16_slices(const void* q, const void* kv, const int32_t* indices, float sm_scale, const int32_t* counts,
+// the union form on dense packed operands of 576 dims, in nsplit slices or in an order (prefill.cu)
+int run_bf16_union(const void* q, const void* kv, const int32_t* indices, float sm_scale, const int32_t* counts,
                     const uint32_t* memb, int h, void* out, float* lse, int ng, int s_kv, int cap, int64_t kv_row_stride,
-                    int nsplit, float* part_o, float2* part_ml, void* stream) {
+                    int nsplit, float* part_o, float2* part_ml, const int2* order, void* stream) {
   b16::Args a{q, kv, indices, counts, memb, nullptr, nullptr, nullptr, nullptr, out, nullptr, lse,
               ng, s_kv, cap, 576, h, 576, kv_row_stride, cap, sm_scale, 0, 0, 0, 0};
-  a.nsplit = nsplit; a.part_o = part_o; a.part_ml = part_ml;
+  a.nsplit = nsplit; a.part_o = part_o; a.part_ml = part_ml; a.order = order;
   return b16::run(a, stream);
 }
 }  // namespace lt

@@ -78,9 +78,9 @@ int run_union(const int32_t* topk_indices, int32_t* u_phys, int32_t* counts, uin
               const int32_t* block_table, int T, int k, int ng, int cap, int G, int bt_rows, int bt_blocks,
               int block_size, int64_t seq_space, int fill, void* stream);
 int check_union(int T, int k, int ng, int cap, int G, int64_t seq_space);      // its shape rules alone
-int run_bf16_slices(const void* q, const void* kv, const int32_t* indices, float sm_scale, const int32_t* counts,
+int run_bf16_union(const void* q, const void* kv, const int32_t* indices, float sm_scale, const int32_t* counts,
                     const uint32_t* memb, int h, void* out, float* lse, int ng, int s_kv, int cap, int64_t kv_row_stride,
-                    int nsplit, float* part_o, float2* part_ml, void* stream);      // attn_bf16.cu
+                    int nsplit, float* part_o, float2* part_ml, const int2* order, void* stream);      // attn_bf16.cu
 // prefill.cu: merge of the slices of ng tiles (see there); out strides in ELEMENTS
 constexpr int kMaxSlices = 16;
 // prefill.cu: slices of `tiles` tiles of up to `blocks` 64-key blocks in the bf16 kernel

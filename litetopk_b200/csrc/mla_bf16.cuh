@@ -148,6 +148,7 @@ struct Params {
   const int32_t* win_lo;
   const int32_t* win_hi;
   const int32_t* counts;     // [ng] or null
+  const int2* order;         // kOrdered: [ng] (tile, its counts clamped to cap) in the order in which they are dealt out
 };
 
 enum { kSiteQ = 101, kSiteKFull, kSiteQkDone, kSitePvDone, kSiteValidReady, kSiteValidFree,
@@ -245,7 +246,7 @@ __device__ __forceinline__ void mma_pv(uint32_t d, uint32_t v_lo, uint32_t p0_lo
   for (int i = 0; i < 2; ++i) mma4_pv(d + 128 * i, p0_lo, p1_lo, v_lo + 512 * i, p_hi, v_hi, idesc, accumulate);
 }
 
-template <int kD, Source kSrc, bool kSliced>
+template <int kD, Source kSrc, bool kSliced, bool kOrdered>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads_of(kSrc), 1)
 mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv0,
                 const __grid_constant__ CUtensorMap map_kv1, const __grid_constant__ CUtensorMap map_out,
@@ -283,11 +284,18 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // broadcast so the compiler knows the role index is warp-uniform
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   auto halves_of = [](int n) -> int { return (n + kOwnKeys - 1) / kOwnKeys; };
+  auto tile_of = [&](int w) -> int { return kSliced ? w / p.nsplit : kOrdered ? __ldcg(&p.order[w].x) : w; };
   auto item_of = [&](int w) -> Item {
     Item t;
-    t.tile = kSliced ? w / p.nsplit : w;
     t.row0 = t.row1 = t.len1 = 0;
-    if (kSrc == kRange) {
+    if (kOrdered) {
+      const int2 v = __ldcg(p.order + w);
+      t.tile = v.x; t.len0 = v.y;
+    } else {
+      t.tile = tile_of(w);
+    }
+    if (kOrdered) {
+    } else if (kSrc == kRange) {
       const int p0 = p.pos0 + t.tile * p.G, plast = p0 + p.G - 1;
       t.len0 = min(plast / p.ratio, p.n_comp);
       t.row1 = max(0, p0 - p.window + 1);
@@ -368,7 +376,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     constexpr int kPer = kQChunksTmem / kQEntries;
     if (wt.aborting()) return;
     ms.q_asked = kQEntries * it + e + 1;
-    const int qt = (kSliced ? w / p.nsplit : w) * p.G + q_tok0;
+    const int qt = tile_of(w) * p.G + q_tok0;
     mbar_arrive_expect_tx(&ms.q_land, kPer * kQChunkBytes);
     for (int j = 0; j < kPer; ++j)
       tma_load_3d_hint(sbase + PL::kOffKV + slot * PL::kSlot + j * kQChunkBytes, &map_q, 64 * (kPer * e + j), q_head,
@@ -832,7 +840,7 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (j > 0) mbar_wait(&ms.q_free, (j - 1) & 1, wt, kSiteQFree, j);
       if (e_tid == 0 && !wt.aborting()) {
         ms.q_res_asked = j + 1;
-        const int qt = (kSliced ? w / p.nsplit : w) * p.G + q_tok0;
+        const int qt = tile_of(w) * p.G + q_tok0;
         if (cta == 0) mbar_arrive_expect_tx(&ms.q_res, 2 * kQRes * kQChunkBytes);
         for (int i = 0; i < kQRes; ++i)
           tma_load_3d_pair_hint(sbase + PL::kOffQ + i * kQChunkBytes, &map_q, 64 * (kQChunksTmem + i), q_head, qt,
@@ -1154,8 +1162,8 @@ static int max_clusters(int dev) {
   at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
   int q = 0;
-  if (ensure_smem<mla_bf16_kernel<kD, kSrc, false>>(dev, Plan<kD>::kSmem) &&
-      cudaOccupancyMaxActiveClusters(&q, mla_bf16_kernel<kD, kSrc, false>, &cfg) == cudaSuccess && q > 0)
+  if (ensure_smem<mla_bf16_kernel<kD, kSrc, false, false>>(dev, Plan<kD>::kSmem) &&
+      cudaOccupancyMaxActiveClusters(&q, mla_bf16_kernel<kD, kSrc, false, false>, &cfg) == cudaSuccess && q > 0)
     n = q;
   cudaGetLastError();
   cached_dev = dev; cached = n;
@@ -1189,13 +1197,13 @@ inline bool make_kv_map(CUtensorMap* m, const void* kv, int d, int64_t rows, int
 }
 
 // Launch over p.ng tiles of p.nsplit slices (a merge has to follow when they are sliced).
-template <int kD, Source kSrc, bool kSliced>
+template <int kD, Source kSrc, bool kSliced, bool kOrdered = false>
 static int launch(const CUtensorMap& mq, const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& mout,
                   const Params& p, cudaStream_t stream) {
   const int dev = current_device();
-  if (!ensure_smem<mla_bf16_kernel<kD, kSrc, kSliced>>(dev, Plan<kD>::kSmem)) return LITEDSA_ERR_CUDA;
+  if (!ensure_smem<mla_bf16_kernel<kD, kSrc, kSliced, kOrdered>>(dev, Plan<kD>::kSmem)) return LITEDSA_ERR_CUDA;
   const int items = kSliced ? p.ng * p.nsplit : p.ng;
-  return launch_pdl(mla_bf16_kernel<kD, kSrc, kSliced>, dim3(2 * min(items, max_clusters<kD, kSrc>(dev))),
+  return launch_pdl(mla_bf16_kernel<kD, kSrc, kSliced, kOrdered>, dim3(2 * min(items, max_clusters<kD, kSrc>(dev))),
                     threads_of(kSrc), Plan<kD>::kSmem, stream, mq, m0, m1, mout, p);
 }
 

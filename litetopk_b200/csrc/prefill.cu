@@ -116,13 +116,14 @@ static int pick_slices(int tiles, int G, int k, bool bf16) {
   return half - (half / n + 1.0) >= 4.0 + 0.08 * tiles * n ? n : 1;
 }
 
-// In which order 64-row tiles are dealt out to the CTAs.  Unions of several lists differ in size, and a CTA that has every
-// 148th tile as they come can have more to do than the others: with half to nine tenths of the lists shared, 16384 tokens x 32 heads
-// 4 % more than the mean, 8192 x 16 10 %, 8192 x 8 22 %.  A block of this kernel takes eight rounds of tiles, sorts them by
-// their key blocks (a counting sort) and deals them out to and fro: 1 to 2 %.  Not all tiles at once, so that neighbours, whose
-// tokens attend much the same keys, still run at about the same time.  Order among equals is of no matter to a tile's result.
+// In which order the tiles are dealt out to the CTAs (64-row tiles) or clusters (a native cache).  Unions of several lists differ in
+// size, and a CTA that has every 148th tile as they come can have more to do than the others: with half to nine tenths of the lists
+// shared, 16384 tokens x 32 heads 4 % more than the mean, 8192 x 16 10 %, 8192 x 8 22 %.  A block of this kernel takes eight rounds
+// of tiles, sorts them by their key blocks (a counting sort) and deals them out to and fro: 1 to 2 %.  Not all tiles at once, so
+// that neighbours, whose tokens attend much the same keys, still run at about the same time.  A tile's result does not depend on
+// its place.
 constexpr int kMostBlocks = 1024;      // of 64 keys: 65536
-static int order_window() { return sm_count() * max(min(8, 2048 / sm_count()), 1); }      // at most 2048 tiles
+static int order_window(int ncta) { return ncta * max(min(8, 2048 / ncta), 1); }      // at most 2048 tiles
 __global__ void __launch_bounds__(1024)
 order_tiles_kernel(const int32_t* __restrict__ counts, int ng, int cap, int ncta, int window, int2* __restrict__ order) {
   __shared__ int place[kMostBlocks], warp_sum[32];
@@ -169,10 +170,14 @@ struct Layout { int64_t counts, u, memb, part_o, part_ml, q_codes, order, total;
 // less.  As they come / ordered, us: half to nine tenths of the lists shared 8192 x 8, top-1024 296 / 261; 8192 x 16 345 / 325; 4096 x
 // 16, bf16 queries 197 / 184; 16384 x 32 933 / 925; below the line, with it none: 4096 x 16, top-512 111 / 106, 2048 x 32, top-1024
 // 132 / 130.  Seven tenths shared by all: 8192 x 16, top-2048 637 / 641, top-512 226 / 227; below the line 1776 x 16, top-256 32 / 34.
-static bool ordered(int ng, int G, int cap) {
-  return G > 1 && ng > sm_count() && (int64_t)ng * cap >= (int64_t)(G > 2 ? 400 : 1000) * 64 * sm_count();
+// Native cache, half to nine tenths shared: 4096 x 8, top-512 241 / 196; 2048 x 16, top-1024 256 / 215; 2048 x 32 263 / 242; 2050 x 64,
+// top-1984 616 / 605; three quarters shared by all 174 / 175, 193 / 195, and 583 / 585.
+static bool ordered(int ng, int G, int cap, bool rows64, bool kv_bf16) {
+  const int ncta = rows64 ? sm_count() : sm_count() / 2;
+  if (G == 1 || ng <= ncta || !(rows64 || kv_bf16)) return false;
+  return (int64_t)ng * cap >= (int64_t)(rows64 ? (G > 2 ? 400 : 1000) : (G > 2 ? 280 : 700)) * 64 * ncta;
 }
-static Layout layout_of(int ng, int G, int cap, int nsplit, bool rows64) {
+static Layout layout_of(int ng, int G, int cap, int nsplit, bool rows64, bool kv_bf16) {
   auto up = [](int64_t b) { return (b + 255) & ~(int64_t)255; };
   Layout l;
   l.counts = 0;
@@ -182,7 +187,7 @@ static Layout layout_of(int ng, int G, int cap, int nsplit, bool rows64) {
   l.part_ml = l.part_o + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 512 * 4) : 0);
   l.q_codes = l.part_ml + (nsplit > 1 ? up((int64_t)ng * nsplit * 128 * 8) : 0);
   l.order = l.q_codes + (rows64 ? rows64_scratch(ng) : 0);
-  l.total = l.order + (rows64 && ordered(ng, G, cap) ? up(8 * (int64_t)ng) : 0);
+  l.total = l.order + (nsplit == 1 && ordered(ng, G, cap, rows64, kv_bf16) ? up(8 * (int64_t)ng) : 0);
   return l;
 }
 
@@ -252,7 +257,7 @@ static Route route_of(int T, int h, int k, bool kv_bf16, int policy_tokens, bool
 static int64_t workspace(int T, int h, int k, int kv_is_bf16, int policy_tokens, bool by_job) {
   if (check_shape(T, h, k, policy_tokens) != LITEDSA_OK) return 0;
   const Route r = route_of(T, h, k, kv_is_bf16 != 0, policy_tokens, by_job);
-  return layout_of(r.ng, r.G, r.cap, r.ns, r.rows64).total;
+  return layout_of(r.ng, r.G, r.cap, r.ns, r.rows64, kv_is_bf16 != 0).total;
 }
 
 static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, const int32_t* topk_idx, double sm_scale,
@@ -268,7 +273,7 @@ static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, con
     return LITEDSA_ERR_UNSUPPORTED;
   const Route r = route_of(T, h, k, kv_is_bf16 != 0, policy_tokens, by_job);
   const int G = r.G, ng = r.ng, cap = r.cap, ns = r.ns;
-  const Layout l = layout_of(ng, G, cap, ns, r.rows64);
+  const Layout l = layout_of(ng, G, cap, ns, r.rows64, kv_is_bf16 != 0);
   if (workspace_bytes < l.total) return LITEDSA_ERR_SHAPE;
   char* ws = reinterpret_cast<char*>(workspace);
   int32_t* counts = reinterpret_cast<int32_t*>(ws + l.counts);
@@ -283,11 +288,20 @@ static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, con
   // fill 2: lists padded to whole 128-key blocks, nothing written beyond
   rc = run_union(topk_idx, u, counts, memb, nullptr, nullptr, T, k, ng, cap, G, 0, 0, 1, seq_space, 2, stream);
   if (rc != LITEDSA_OK) return rc;
-  if (kv_is_bf16 && ns > 1) {
+  // tiles in order of their size
+  int2* order = nullptr;
+  if (ns == 1 && ordered(ng, G, cap, r.rows64, kv_is_bf16 != 0)) {
+    order = reinterpret_cast<int2*>(ws + l.order);
+    const int ncta = r.rows64 ? sm_count() : sm_count() / 2, window = order_window(ncta);
+    rc = launch_pdl(order_tiles_kernel, dim3((ng + window - 1) / window), 1024, 0, reinterpret_cast<cudaStream_t>(stream), counts, ng, cap,
+                    ncta, window, order);
+    if (rc != LITEDSA_OK) return rc;
+  }
+  if (kv_is_bf16 && (ns > 1 || order != nullptr)) {
     float* part_o = reinterpret_cast<float*>(ws + l.part_o);
     float2* part_ml = reinterpret_cast<float2*>(ws + l.part_ml);
-    rc = run_bf16_slices(q, kv, u, (float)sm_scale, counts, memb, h, out, lse, ng, s_kv, cap, kv_row_stride, ns, part_o, part_ml, stream);
-    if (rc != LITEDSA_OK) return rc;
+    rc = run_bf16_union(q, kv, u, (float)sm_scale, counts, memb, h, out, lse, ng, s_kv, cap, kv_row_stride, ns, part_o, part_ml, order, stream);
+    if (rc != LITEDSA_OK || ns == 1) return rc;
     return merge_slices(part_o, part_ml, ns, ng, h, 1.f, 0.f, nullptr, 1, out, (int64_t)h * 512, 512, lse,
                         reinterpret_cast<cudaStream_t>(stream));
   }
@@ -299,17 +313,7 @@ static int run(const void* q, int q_is_bf16, const void* kv, int kv_is_bf16, con
             ng, s_kv, cap, 576, kv_row_stride, cap, nullptr, nullptr, 1};
   a.q_is_bf16 = q_is_bf16 != 0;
   a.q_inv = 1.0f / (float)q_scale;
-  if (r.rows64) {
-    int2* order = nullptr;
-    if (ordered(ng, G, cap)) {
-      order = reinterpret_cast<int2*>(ws + l.order);
-      const int window = order_window();
-      rc = launch_pdl(order_tiles_kernel, dim3((ng + window - 1) / window), 1024, 0, reinterpret_cast<cudaStream_t>(stream), counts, ng,
-                      cap, sm_count(), window, order);
-      if (rc != LITEDSA_OK) return rc;
-    }
-    return run_fp8_rows64(a, out, ws + l.q_codes, order, stream);
-  }
+  if (r.rows64) return run_fp8_rows64(a, out, ws + l.q_codes, order, stream);
   a.nsplit = ns;
   a.part_o = reinterpret_cast<float*>(ws + l.part_o);
   a.part_ml = ws + l.part_ml;

@@ -551,28 +551,33 @@ def test_a_part_of_a_job_gives_the_bits_of_the_job():
         api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs, job_tokens=tokens - 2)
 
 
-@pytest.mark.parametrize("tokens,heads,topk,s_kv", [
-    (3760, 8, 1024, 9000),       # eight tokens per tile; four rounds of tiles, the last not full
-    (7400, 16, 512, 5001),       # four; a full window of eight rounds and half of one
-    (4740, 32, 2048, 7777),      # two; the last window has two tiles
+@pytest.mark.parametrize("tokens,heads,topk,s_kv,cache", [
+    (3760, 8, 1024, 9000, "fp8"),       # eight tokens per tile; four rounds of tiles, the last not full
+    (7400, 16, 512, 5001, "fp8"),       # four; a full window of eight rounds and half of one
+    (4740, 32, 2048, 7777, "fp8"),      # two; the last window has two tiles
+    (2640, 8, 512, 5001, "native"),     # sixteen; three rounds on the clusters, the last not full
+    (1680, 64, 1984, 7777, "native"),   # two; a window and a part of one
 ])
-def test_tiles_in_order_of_their_size_give_the_bits_of_tiles_as_they_come(tokens, heads, topk, s_kv):
-    # parts of fewer tiles than SMs are not ordered
+def test_tiles_in_order_of_their_size_give_the_bits_of_tiles_as_they_come(tokens, heads, topk, s_kv, cache):
+    # parts of no more tiles than CTAs or clusters are not ordered
     g = torch.Generator().manual_seed(22)
     idx = torch.randint(0, s_kv, (tokens, topk), generator=g, dtype=torch.int32)
     n = torch.randint(0, topk + 1, (tokens, 1), generator=g)
     n[torch.rand((tokens, 1), generator=g) < 0.3] = topk
     n[:64] = 0                                           # empty tiles
     idx[torch.arange(topk)[None] >= n] = -1
-    w, _, kv, q = _case(16, 64, 16, s_kv, (0.5, 0.5), seed=22)
-    _, kv8, qs, ks = synth.refcompat_operands(q, kv)
-    q8 = torch.randint(0, 120, (tokens, heads, 576), generator=g, dtype=torch.uint8).to(DEV)
-    kvd, idd = kv8.to(DEV), idx.to(DEV)
-    out, lse = api.sparse_prefill(q8, kvd, idd, synth.SM_SCALE / 8, kv_scale=ks, q_scale=qs)
-    part = 128 * 64 // heads
+    if cache == "native":
+        kv = api.prepare_kv(synth.make_kv_cache(s_kv, seed=22, device=DEV, mode="native"))
+        q, kw, part = torch.randn((tokens, heads, 576), generator=g).to(torch.bfloat16).to(DEV), {}, 64 * 128 // heads
+    else:
+        kv = api.prepare_kv(synth.make_kv_cache(s_kv, seed=22, device=DEV, mode="refcompat"), synth.REFCOMPAT_SCALE)
+        q = torch.randint(0, 120, (tokens, heads, 576), generator=g, dtype=torch.uint8).to(DEV)
+        kw, part = dict(kv_scale=synth.REFCOMPAT_SCALE, q_scale=synth.REFCOMPAT_SCALE), 128 * 64 // heads
+    idd = idx.to(DEV)
+    out, lse = api.sparse_prefill(q, kv, idd, synth.SM_SCALE / 8, **kw)
     for t0 in range(0, tokens, part):
         rows = slice(t0, t0 + part)
-        o, l = api.sparse_prefill(q8[rows], kvd, idd[rows], synth.SM_SCALE / 8, kv_scale=ks, q_scale=qs, job_tokens=tokens)
+        o, l = api.sparse_prefill(q[rows], kv, idd[rows], synth.SM_SCALE / 8, job_tokens=tokens, **kw)
         assert torch.equal(out[rows], o) and torch.equal(lse[rows], l)
 
 
