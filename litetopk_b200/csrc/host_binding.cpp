@@ -14,6 +14,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/litedsa_b200.h"
@@ -70,23 +71,13 @@ struct NoGil {
   PyThreadState* state = PyEval_SaveThread();
   ~NoGil() { PyEval_RestoreThread(state); }
 };
-// C++ exceptions (out of memory, say) leave as the Python exceptions that torch makes of them
+// Exceptions and warnings leave as they do from torch's own functions: a Python exception raised below a call as itself, a C++ one as
+// the Python class that torch has for it.
 template <class F>
 PyObject* guarded(F&& f) {
-  try {
-    return f();
-  } catch (const c10::OutOfMemoryError& e) {
-    PyObject* torch = PyImport_ImportModule("torch");
-    PyObject* type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
-    PyErr_SetString(type ? type : PyExc_RuntimeError, e.what_without_backtrace());
-    Py_XDECREF(type);
-    Py_XDECREF(torch);
-  } catch (const c10::Error& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-  }
-  return nullptr;
+  HANDLE_TH_ERRORS
+  return f();
+  END_HANDLE_TH_ERRORS
 }
 
 // (q, kv, topk_idx, sm_scale, kv_scale, q_scale, seq_space, job_tokens)

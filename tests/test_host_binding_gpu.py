@@ -140,3 +140,40 @@ def test_lite_topk(both, T, Hi, S, k, scale):
     short, general, took = both(lambda: api.lite_topk(q, kk, w, ks, k, S - T, logits_workspace=torch.empty((T, S + 5), device=DEV)))
     assert took == []
     assert torch.equal(short.sort(dim=1).values, general.sort(dim=1).values)
+
+
+@pytest.mark.filterwarnings("ignore:Warning only once for all operators")      # that kernels are overridden
+def test_exceptions_below_are_those_of_the_general_way(both):
+    q, kv, idx, scales = _prefill(256, 64, 256, 2048, "e4m3", "fp8")
+    xi = [x.to(DEV) for x in synth.make_indexer_operands(8, 1024, 32, seed=8)]
+    r = torch.randn((24, 16, 576), device=DEV).to(torch.bfloat16)
+    calls = (lambda: api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales), lambda: api.lite_topk(*xi, 64, 1016),
+             lambda: api.dsv4_c128a_bf16(r, None, r[:, 0], 0, synth.SM_SCALE))
+
+    class Own(Exception):
+        pass
+
+    def refuse(*args, **kwargs):
+        raise Own("from below")
+    for way in (_lib.host(), None):
+        with pytest.MonkeyPatch.context() as m:
+            m.setattr(_lib, "_host", way)
+            for f in calls:
+                f()
+                lib = torch.library.Library("aten", "IMPL")      # noqa: TOR901
+                try:
+                    for op in ("empty.memory_format", "empty_strided"):
+                        lib.impl(op, refuse, "CUDA")
+                    with pytest.raises(Own, match="from below"):
+                        f()
+                finally:
+                    lib._destroy()
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            torch.cuda.set_per_process_memory_fraction(1e-6)
+            try:
+                with pytest.raises(torch.OutOfMemoryError):      # the output has 16 MB
+                    calls[0]()
+            finally:
+                torch.cuda.set_per_process_memory_fraction(1.0)
+            calls[0]()
