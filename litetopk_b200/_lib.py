@@ -116,7 +116,10 @@ def host():
     library for plain calls; everything else, and everything without it, goes by ctypes."""
     global _host
     if _host is False:
-        lib()
+        try:
+            lib()
+        except (ImportError, OSError, AttributeError):      # said by the general way, behind its checks of the arguments
+            return None
         _host = None
         path = LIB_PATH.with_name("litedsa_host.so")
         if path.exists():
