@@ -111,9 +111,18 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def host_path() -> Path:
+    """Where the module of host_binding.cpp for this interpreter and this torch lies, whose binary interfaces it uses both: under
+    a name of theirs, so that no other pair's is ever loaded."""
+    import sysconfig
+
+    import torch
+    return LIB_PATH.with_name(f"litedsa_host-torch{torch.__version__}-cxx{int(torch._C._GLIBCXX_USE_CXX11_ABI)}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
 def host():
-    """The module of host_binding.cpp, or None where it was not built, or for another torch: the short way into the same
-    library for plain calls; everything else, and everything without it, goes by ctypes."""
+    """The module of host_binding.cpp, or None where it was not built: the short way into the same library for plain
+    calls; everything else, and everything without it, goes by ctypes."""
     global _host
     if _host is False:
         try:
@@ -121,20 +130,20 @@ def host():
         except (ImportError, OSError, AttributeError):      # said by the general way, behind its checks of the arguments
             return None
         _host = None
-        path = LIB_PATH.with_name("litedsa_host.so")
+        path, why = host_path(), None
         if path.exists():
             import importlib.machinery
             import importlib.util
-
-            import torch
             try:
                 loader = importlib.machinery.ExtensionFileLoader("litedsa_host", str(path))
-                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("litedsa_host", loader))
-                if module.built_for == torch.__version__:
-                    _host = module
+                _host = importlib.util.module_from_spec(importlib.util.spec_from_loader("litedsa_host", loader))
             except ImportError as e:
-                import warnings
-                warnings.warn(f"{path.name} cannot be loaded, calls go by ctypes: {e}")
+                why = f"{path.name} cannot be loaded: {e}"
+        elif any(path.parent.glob("litedsa_host*.so")):
+            why = f"{path.name} is missing, there are only those of another Python or torch"
+        if why:
+            import warnings
+            warnings.warn(f"{why}.  Calls take up to twice the host time, by ctypes, until `python -m litetopk_b200.build` has been run")
     return _host
 
 

@@ -4,8 +4,9 @@
 
 The library lands in litetopk_b200/_C/ (git-ignored, but shipped with the source tree to
 the GPU machine).  Only nvcc and the CUDA runtime are needed: no CUTLASS, no Python
-headers, no torch headers.  Beside it, litedsa_host.so, the short way from Python to the library's
-calls (csrc/host_binding.cpp), needs both; where it cannot be built the package goes by ctypes alone.
+headers, no torch headers.  Beside it, litedsa_host-*.so, the short way from Python to the library's
+calls (csrc/host_binding.cpp), needs both and is one interpreter's and one torch's; where it cannot be built
+the package goes by ctypes alone.
 """
 from __future__ import annotations
 
@@ -19,7 +20,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT_DIR = PKG / "_C"
 LIB = OUT_DIR / "liblitedsa_b200.so"
-HOST_SRC, HOST = CSRC / "host_binding.cpp", OUT_DIR / "litedsa_host.so"
+HOST_SRC = CSRC / "host_binding.cpp"
 SOURCES = ["abi.cu", "union_qm.cu", "attn_fp8.cu", "prep.cu", "noalloc.cu", "attn_dsv4.cu", "attn_bf16.cu", "peak_probe.cu", "index_topk.cu",
            "prefill.cu"]
 
@@ -43,14 +44,23 @@ def is_stale() -> bool:
 
 
 def build_host(verbose: bool = False) -> None:
-    """litedsa_host.so for the installed torch, linked against the library beside it."""
+    """The module of host_binding.cpp for this interpreter and torch, linked against the library beside it, unless it is there;
+    modules of an earlier library, whoever's they are, leave."""
+    newest = max(HOST_SRC.stat().st_mtime, LIB.stat().st_mtime)
+    for f in OUT_DIR.glob("litedsa_host*.so"):
+        if f.stat().st_mtime < newest:
+            f.unlink()
     try:
         import sysconfig
         import torch
         from torch.utils import cpp_extension as ext
+        from ._lib import host_path
+        path = OUT_DIR / host_path().name
+        if path.exists():
+            return
         includes = [sysconfig.get_paths()["include"], *ext.include_paths(), str(Path(_nvcc()).parents[1] / "include")]
-        tmp = HOST.with_suffix(".so.tmp")
-        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-DLITEDSA_BUILT_FOR=\"{torch.__version__}\"",
+        tmp = path.with_suffix(".so.tmp")
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in includes), str(HOST_SRC), "-o", str(tmp),
                *(f"-L{d}" for d in ext.library_paths()), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
                f"-L{OUT_DIR}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
@@ -59,16 +69,14 @@ def build_host(verbose: bool = False) -> None:
         p = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if p.returncode != 0:
             raise RuntimeError(p.stdout[-2000:])
-        os.replace(tmp, HOST)
+        os.replace(tmp, path)
     except Exception as e:      # no Python or torch headers, no g++: the package goes by ctypes
-        HOST.unlink(missing_ok=True)
-        sys.stderr.write(f"litedsa_host.so not built: {e}\n")
+        sys.stderr.write(f"the module of {HOST_SRC.name} was not built: {e}\n")
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and not is_stale():
-        if not HOST.exists() or HOST.stat().st_mtime < max(HOST_SRC.stat().st_mtime, LIB.stat().st_mtime):
-            build_host(verbose)
+        build_host(verbose)
         return LIB
     OUT_DIR.mkdir(exist_ok=True)
     objs = []

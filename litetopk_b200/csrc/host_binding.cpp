@@ -249,8 +249,4 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "litedsa_host", nullptr, -1, kMeth
 
 }  // namespace
 
-extern "C" __attribute__((visibility("default"))) PyObject* PyInit_litedsa_host() {
-  PyObject* m = PyModule_Create(&kModule);
-  if (m && PyModule_AddStringConstant(m, "built_for", LITEDSA_BUILT_FOR) != 0) Py_CLEAR(m);
-  return m;
-}
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit_litedsa_host() { return PyModule_Create(&kModule); }

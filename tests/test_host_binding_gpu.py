@@ -14,7 +14,7 @@ SC = synth.REFCOMPAT_SCALE
 def both(monkeypatch):
     """f -> (result of f by the short way, by the general one), and whether the short way took it."""
     host = _lib.host()
-    assert host is not None, "litedsa_host.so is missing"
+    assert host is not None, "the module of host_binding.cpp is missing"
 
     def run(f):
         took = []
