@@ -3,9 +3,9 @@
 // Python, its host side took as long or longer and was what such calls were bound by: sparse_prefill of 2 tokens 22 us (11 this
 // way), dsv4_c128a_bf16 of 24 tokens 19 (9), lite_topk and sparse_prefill of 36 tokens 48 (19).
 //
-// Each function takes the arguments of its operator in api.py and returns the result, the status code of a call
-// that the library refused, or None for whatever is not plain: then nothing has been done, and api.py goes its own way, checks and
-// errors included.  Plain are dense CUDA tensors of the expected types, shapes and strides on the current device that
+// Each function takes the arguments of its operator in api.py and returns the result (True from dsv4_masked_mla_bf16_out, whose caller
+// has it), the status code of a call that the library refused (lite_topk, which makes two: with the refused one's name), or None for
+// whatever is not plain: then nothing has been done, and api.py goes its own way, checks and errors included.  Plain are dense CUDA tensors of the expected types, shapes and strides on the current device that
 // no dispatch mode, function transform or subclass stands behind.
 #include <Python.h>
 

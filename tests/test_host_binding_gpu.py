@@ -1,7 +1,12 @@
 """The short way into the library (host_binding.cpp) against the general one (ctypes): the same results bit for bit over the forms
 that it accepts, and whatever else it is handed goes the general way, with that way's results and errors."""
+import sys
+import threading
+import time
+
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from litetopk_b200 import _lib, api, synth
 
@@ -143,8 +148,8 @@ def test_lite_topk(both, T, Hi, S, k, scale):
 
 
 @pytest.mark.filterwarnings("ignore:Warning only once for all operators")      # that kernels are overridden
-def test_exceptions_below_are_those_of_the_general_way(both):
-    q, kv, idx, scales = _prefill(256, 64, 256, 2048, "e4m3", "fp8")
+def test_exceptions_below_are_those_of_the_general_way():
+    q, kv, idx, scales = _prefill(2, 64, 256, 2048, "e4m3", "fp8")
     xi = [x.to(DEV) for x in synth.make_indexer_operands(8, 1024, 32, seed=8)]
     r = torch.randn((24, 16, 576), device=DEV).to(torch.bfloat16)
     calls = (lambda: api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales), lambda: api.lite_topk(*xi, 64, 1016),
@@ -169,11 +174,131 @@ def test_exceptions_below_are_those_of_the_general_way(both):
                 finally:
                     lib._destroy()
             torch.cuda.synchronize()
-            torch.cuda.empty_cache()
             torch.cuda.set_per_process_memory_fraction(1e-6)
             try:
-                with pytest.raises(torch.OutOfMemoryError):      # the output has 16 MB
-                    calls[0]()
+                with pytest.raises(torch.OutOfMemoryError):      # 64 GB of positions
+                    api.lite_topk(*xi, 2 ** 31 - 1, 1016)
             finally:
                 torch.cuda.set_per_process_memory_fraction(1.0)
             calls[0]()
+
+
+@pytest.mark.parametrize("T,h,k", [(592, 64, 64), (594, 64, 64), (594, 64, 128), (296, 128, 512), (297, 128, 512), (297, 128, 640)])
+def test_bf16_queries_with_a_pass_of_their_own_go_the_general_way(both, T, h, k):
+    """The line between both ways (296 tiles, lists of 512 entries or unions of 128) is drawn in both."""
+    q, kv, idx, scales = _prefill(T, h, k, 2048, "bf16", "fp8")
+    short, general, took = both(lambda: api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales))
+    assert took == [not api._quantise_first(T * h // 128, 128 // h, 128 // h * k)]
+    _same(short, general)
+
+
+class _Count(TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.n = getattr(self, "n", 0) + 1
+        return func(*args, **(kwargs or {}))
+
+
+def test_modes_and_transforms(both):
+    q, kv, idx, scales = _prefill(2, 64, 256, 2048, "bf16", "fp8")
+    call = lambda q=q: api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales)      # noqa: E731
+    plain = call()
+
+    def counted():
+        with _Count() as mode:
+            r = call()
+        assert mode.n == 3                                                            # out, lse, workspace
+        return r
+    short, general, took = both(counted)
+    assert took == [False]
+    _same(short, plain)
+    _same(general, plain)
+    ones = torch.ones(3, device=DEV)
+    short, general, took = both(lambda: torch.func.vmap(lambda x: (call(), x)[0], out_dims=(None, None))(ones))
+    _same(short, plain)
+    _same(general, plain)
+    for f in (lambda: torch.func.vmap(lambda x: call(x))(torch.stack([q, q])), lambda: torch.func.grad(lambda x: call(x)[0].float().sum())(q),
+              lambda: torch.func.jvp(call, (q,), (q,)), lambda: torch.func.grad(lambda x: call()[0].float().sum() + x.sum())(ones)):
+        for way in (_lib.host(), None):
+            with pytest.MonkeyPatch.context() as m:
+                m.setattr(_lib, "_host", way)
+                with pytest.raises(RuntimeError, match="data pointer"):
+                    f()
+
+
+def test_capture(both):
+    q, kv, idx, scales = _prefill(2, 64, 1024, 4096, "bf16", "fp8")
+    q2 = _prefill(2, 64, 1024, 4096, "e4m3", "fp8")[0].float().to(torch.bfloat16).mul_(2.0 ** -6)
+
+    def captured():
+        x = q.clone()
+        api.sparse_prefill(x, kv, idx, synth.SM_SCALE, **scales)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out, lse = api.sparse_prefill(x, kv, idx, synth.SM_SCALE, **scales)
+        x.copy_(q2)
+        g.replay()
+        torch.cuda.synchronize()
+        return out.clone(), lse.clone()
+    short, general, took = both(captured)
+    assert took == [True, True]
+    _same(short, general)
+    _same(short, api.sparse_prefill(q2, kv, idx, synth.SM_SCALE, **scales))
+
+
+def test_threads_on_streams_of_their_own():
+    q, kv, idx, scales = _prefill(8, 64, 1024, 4096, "bf16", "fp8")
+    xi = [x.to(DEV) for x in synth.make_indexer_operands(8, 3000, 32, seed=8)]
+    r = torch.randn((24, 16, 576), device=DEV).to(torch.bfloat16)
+    kr = torch.randn((20000, 576), device=DEV).to(torch.bfloat16)
+
+    def all_three():
+        return (*api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales), api.lite_topk(*xi, 64, 2992).sort(dim=1).values,
+                *api.dsv4_c128a_bf16(r, kr[:156], kr, 19976, synth.SM_SCALE))
+    want, got = all_three(), [None] * 4
+    torch.cuda.synchronize()
+
+    def work(i):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            results = [all_three() for _ in range(50)]
+        stream.synchronize()
+        got[i] = results
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    for results in got:
+        for x in results:
+            _same(x, want)
+
+
+def test_other_threads_run_during_calls():
+    q, kv, idx, scales = _prefill(2, 64, 256, 2048, "bf16", "fp8")
+    keep, n, done = [], [0], threading.Event()
+
+    def count():
+        while not done.is_set():
+            n[0] += 1
+            time.sleep(0)
+    interval, thread = sys.getswitchinterval(), threading.Thread(target=count)
+    api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales)
+    try:
+        sys.setswitchinterval(1000.0)      # nobody has to hand over: the calls do so of their own accord
+        thread.start()
+        before = n[0]
+        for _ in range(200):
+            keep.append(api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales))
+        assert n[0] > before
+    finally:
+        done.set()
+        sys.setswitchinterval(interval)
+        thread.join()
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="two GPUs")
+def test_another_current_device(both):
+    q, kv, idx, scales = _prefill(2, 64, 256, 2048, "bf16", "fp8")
+    with torch.cuda.device(1):
+        short, general, took = both(lambda: api.sparse_prefill(q, kv, idx, synth.SM_SCALE, **scales))
+    assert took == [False]
+    _same(short, general)
