@@ -3,6 +3,8 @@
 Tolerances are the benchmark's: out max-abs <= 1e-2 and cosine >= 0.9999, LSE <= 1e-3,
 measured against the reference's own numerics (oracle.attention_oracle.masked_mla_refnum,
 pinned to the reference module by tests/golden/)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -551,15 +553,27 @@ def test_a_part_of_a_job_gives_the_bits_of_the_job():
         api.sparse_prefill(qd, kvd, idd, synth.SM_SCALE, kv_scale=ks, q_scale=qs, job_tokens=tokens - 2)
 
 
-@pytest.mark.parametrize("tokens,heads,topk,s_kv,cache", [
-    (3760, 8, 1024, 9000, "fp8"),       # eight tokens per tile; four rounds of tiles, the last not full
-    (7400, 16, 512, 5001, "fp8"),       # four; a full window of eight rounds and half of one
-    (4740, 32, 2048, 7777, "fp8"),      # two; the last window has two tiles
-    (2640, 8, 512, 5001, "native"),     # sixteen; three rounds on the clusters, the last not full
-    (1680, 64, 1984, 7777, "native"),   # two; a window and a part of one
+def _launches(f):
+    """How many launches f() makes: the nodes of a graph that captures it."""
+    graph, n = torch.cuda.CUDAGraph(keep_graph=True), ctypes.c_size_t()
+    with torch.cuda.graph(graph):
+        f()
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(n)) == 0
+    return n.value
+
+
+@pytest.mark.parametrize("rounds,more,heads,topk,s_kv,cache", [      # whole rounds of tiles, and tiles more
+    (3, 60, 8, 1024, 9000, "fp8"),         # eight tokens per tile; four rounds, the last not full
+    (13, 30, 16, 512, 5001, "fp8"),        # four; a full window of eight rounds and most of one
+    (16, 2, 32, 2048, 7777, "fp8"),        # two; the last window has two tiles
+    (2, 40, 8, 512, 5001, "native"),       # sixteen; three rounds on the clusters, the last not full
+    (11, 60, 64, 1984, 7777, "native"),    # two; a window and a part of one
 ])
-def test_tiles_in_order_of_their_size_give_the_bits_of_tiles_as_they_come(tokens, heads, topk, s_kv, cache):
-    # parts of no more tiles than CTAs or clusters are not ordered
+def test_tiles_in_order_of_their_size_give_the_bits_of_tiles_as_they_come(rounds, more, heads, topk, s_kv, cache):
+    sms, rows = torch.cuda.get_device_properties(DEV).multi_processor_count, 128 if cache == "native" else 64
+    ncta = sms * 64 // rows                              # CTAs or clusters
+    tokens = (rounds * ncta + more) // 2 * 2 * rows // heads
+    part = ncta * 7 // 8 // 2 * 2 * rows // heads        # parts of no more tiles than CTAs or clusters are not ordered
     g = torch.Generator().manual_seed(22)
     idx = torch.randint(0, s_kv, (tokens, topk), generator=g, dtype=torch.int32)
     n = torch.randint(0, topk + 1, (tokens, 1), generator=g)
@@ -568,17 +582,20 @@ def test_tiles_in_order_of_their_size_give_the_bits_of_tiles_as_they_come(tokens
     idx[torch.arange(topk)[None] >= n] = -1
     if cache == "native":
         kv = api.prepare_kv(synth.make_kv_cache(s_kv, seed=22, device=DEV, mode="native"))
-        q, kw, part = torch.randn((tokens, heads, 576), generator=g).to(torch.bfloat16).to(DEV), {}, 64 * 128 // heads
+        q, kw = torch.randn((tokens, heads, 576), generator=g).to(torch.bfloat16).to(DEV), {}
     else:
         kv = api.prepare_kv(synth.make_kv_cache(s_kv, seed=22, device=DEV, mode="refcompat"), synth.REFCOMPAT_SCALE)
         q = torch.randint(0, 120, (tokens, heads, 576), generator=g, dtype=torch.uint8).to(DEV)
-        kw, part = dict(kv_scale=synth.REFCOMPAT_SCALE, q_scale=synth.REFCOMPAT_SCALE), 128 * 64 // heads
+        kw = dict(kv_scale=synth.REFCOMPAT_SCALE, q_scale=synth.REFCOMPAT_SCALE)
     idd = idx.to(DEV)
-    out, lse = api.sparse_prefill(q, kv, idd, synth.SM_SCALE / 8, **kw)
+    call = lambda s: api.sparse_prefill(q[s], kv, idd[s], synth.SM_SCALE / 8, job_tokens=tokens, **kw)      # noqa: E731
+    out, lse = call(slice(0, tokens))
     for t0 in range(0, tokens, part):
-        rows = slice(t0, t0 + part)
-        o, l = api.sparse_prefill(q[rows], kv, idd[rows], synth.SM_SCALE / 8, job_tokens=tokens, **kw)
-        assert torch.equal(out[rows], o) and torch.equal(lse[rows], l)
+        s = slice(t0, t0 + part)
+        o, l = call(s)
+        assert torch.equal(out[s], o) and torch.equal(lse[s], l)
+    assert _launches(lambda: call(slice(0, tokens))) == 3      # union, order, attention
+    assert _launches(lambda: call(slice(0, part))) == 2
 
 
 @pytest.mark.parametrize("tokens,heads,topk,s_kv", [
