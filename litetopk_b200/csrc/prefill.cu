@@ -24,9 +24,8 @@ constexpr float kLn2 = 0.6931471805599453f;
 // (the sink joins the output's normaliser only; row r of a tile = token r / h, head r % h).
 // A warp has kPieces of a row's four 128-dim pieces, lane i unit i (4 dims) of each, as part_unit() has swapped them.  Latency-
 // bound at the sizes it runs at (2 KB per slice and row): the loads of eight (two) slices are under way with that of the
-// maxima, before a weight is known.  One piece per warp as long as all blocks are on the chip at once, else four.  (A warp per
-// row that went from slice to slice: 2 tokens x 64 heads in five slices 20.3 -> 18.6 us, in eight of a native cache 20.6 -> 18.3;
-// 68 x 64 in two 30.8, with one piece per warp 33.0, four of them 31.1.)
+// maxima, before a weight is known.  One piece per warp for few tiles, else four (merge_slices).  (A warp per row that went from slice to
+// slice: 2 tokens x 64 heads in five slices 20.3 -> 18.6 us, in eight of a native cache 20.6 -> 18.3.)
 template <int kPieces>
 __global__ void __launch_bounds__(256)
 merge_slices_kernel(const float* __restrict__ part_o, const float2* __restrict__ part_ml, int nsplit, int n_rows, int h,
@@ -232,7 +231,11 @@ int bf16_slices(int tiles, int blocks) {
 int merge_slices(const float* part_o, const float2* part_ml, int nsplit, int ng, int h, float out_scale, float lse_off,
                  const float* sink, int sink_mod, void* out, int64_t out_token_stride, int64_t out_head_stride,
                  float* lse, cudaStream_t stream) {
-  const bool few = ng * 64 <= 8 * sm_count();      // blocks of 256 threads, eight on an SM
+  // One piece per warp makes blocks of 256 threads (57 registers), of which an SM holds four: nine tiles are all of them at once.  The line is
+  // where both forms take the same time, at 11 tiles.  Calls with their merge, four pieces / one, us, top-2048, native cache and ranges at 131072: 1 tile
+  // 18.4 / 17.0, 19.2 / 17.6, 13.8 / 12.3; 9 tiles 20.4 / 20.1, 24.1 / 22.0, 17.5 / 15.4; 10 tiles 21.3 / 20.7, 24.4 / 23.7, 17.0 / 16.6; 12 tiles 22.1 /
+  // 22.3, 25.3 / 25.3, 17.3 / 17.5; 18 tiles 24.3 / 24.9, 27.7 / 28.4, 17.9 / 18.7; 34 tiles 30.4 / 32.2, 38.5 / 40.2, 23.5 / 25.3.
+  const bool few = ng * 64 <= 5 * sm_count();
   return launch_pdl(few ? prefill::merge_slices_kernel<1> : prefill::merge_slices_kernel<4>, dim3(ng * (few ? 64 : 16)), 256, 0, stream,
                     part_o, part_ml, nsplit, ng * 128, h, out_scale, lse_off, sink, sink_mod, reinterpret_cast<__nv_bfloat16*>(out),
                     (long long)out_token_stride, (long long)out_head_stride, lse);
