@@ -23,11 +23,11 @@
 //     warps 28-31  Q tiles in, tile epilogue.
 //   * every wait is bounded (common.cuh).
 // What bounds it inside a tile is latency x slots: stamps per role show a slot held 6100 cycles (copies 1700, QK^T and its queue
-// 700, softmax 2500, wait for PV 700, PV 330), six of them 1015 per block, against 830 of the MMAs; the shared-memory pipe is 83 %
+// 700, softmax 2500, wait for PV 700, PV 330), six of them 1015 per block, against 830 of the MMAs; the shared-memory pipe is 87 %
 // busy beside.  Between tiles 2.3 to 3 us pass: Q's entry takes a turn of the ring, and its slot stays until the output
-// staged in it has left.  Long runs are at the power limit.  With the union, e4m3 queries, us on
-// 128-row tiles and here, before the issuing warps waited suspended: 8192 tokens x 64 heads, top-2048 1420 / 1265; 16384 x 32, top-1024 1201 / 961; 16384 x 16,
-// top-2048 of 131072 1780 / 1330-1490 (long runs meet the power limit); 4096 x 64, top-256 181 / 137.
+// staged in it has left.  Long runs are at the power limit.  With the union, e4m3 queries, three quarters
+// of the lists shared, us on 128-row tiles and here: 8192 tokens x 64 heads, top-2048 1430 / 1237; 16384 x 32, top-1024 of 65535 1065 / 875; 16384 x 16,
+// top-2048 of 131072 1597 / 1181; 4096 x 64, top-256 183 / 144.
 #pragma once
 
 namespace lt {

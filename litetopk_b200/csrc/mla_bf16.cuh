@@ -951,8 +951,8 @@ mla_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         // before they are handed over: a box's way through the warp's slice takes some 500 cycles, all eight 4000, by
         // which that PV was late.  With the gather the block's registers are redistributed for it (7 boxes; native cache,
         // 1184 tokens x 64 heads, top-2048 354 -> 343 us); the tiled forms lose more by that than they gain (items of
-        // four blocks 52.5 -> 54 us) and hold what fits without (ranges 3 boxes: 1184 x 64 at 65536 100.0 -> 97.9; 4 spill, with runs 3).  Straight to
-        // memory from registers, a row per lane, O is free after 4000 cycles, too.
+        // four blocks 52.5 -> 54 us) and hold the boxes for which their registers suffice: ranges 3 (1184 x 64 at 65536 100.0 -> 97.9; 4 would
+        // spill), runs 2 (3 would spill).  Straight to memory from registers, a row per lane, O is free after 4000 cycles, too.
         constexpr int kHeld = kSrc == kRange ? 3 : kSrc == kRank ? 2 : 7;
         uint32_t wv[kHeld][16];
         auto pack = [&](int cc, uint32_t (&w)[16]) {

@@ -199,16 +199,17 @@ static int check_shape(int T, int h, int k, int policy_tokens) {
 
 // Whether a job of `tokens` tokens runs on 64-row tiles (attn_fp8_r64.cuh) instead of 128-row ones: with an FP8
 // cache, up to 64 heads, lists of a tile of 256 entries and more, a tile for every other SM and at least ten key
-// blocks per SM.  (Fewer tiles run faster as slices of 128-row ones: 40 tiles of 16 heads, top-2048, 60 us
-// against 65 when the line was drawn; with less work both forms take the 23 us of a call's launches.)
+// blocks per SM.  Fewer tiles run faster as slices of 128-row ones: 40 tiles of 16 heads, top-2048, 48 us against 56.  (Of the line of
+// ten blocks that no longer holds: 148 tiles of 64 heads, top-512, 21.1 / 16.4 us, 296 of top-256 22.3 / 18.3, 60 of top-1024 23.2 / 18.3.  It was drawn when
+// both forms took the 23 us of a call's launches there; such calls keep the rounding that 128-row tiles give them.)
 // 128-row / 64-row tiles, half and nine tenths of the lists shared, e4m3 queries, us (bf16 queries: much the same, but
-// 67 / 70 at 222 tiles and nine tenths, 87 / 82 with top-256):
-//   74 tiles of 64 rows: 64 heads, top-2048    35 / 28 and 32 / 28;    16 heads 64 / 57 and 41 / 37
-//   222: 32 heads, top-2048                    98 / 75 and 72 / 71
-//   1184: 64 heads, top-256 58 / 45 and 57 / 45, top-2048 249 / 189 and 196 / 188;    32 heads, top-2048 394 / 274 and
-//         228 / 220;    16 heads 687 / 442 and 300 / 262;    8 heads 1298 / 779 and 448 / 352
-// The more of the lists is shared, the less there is to gain: over 7700 calls (sharing 30 to 97 %, both query types) 6 % were
-// slower, by up to 13 %, nearly all with nine tenths shared and more and two or three rounds of tiles.  How
+// 69 / 68 at 222 tiles and nine tenths, 90 / 79 with top-256):
+//   74 tiles of 64 rows: 64 heads, top-2048    34 / 28 and 31 / 28;    16 heads 65 / 58 and 41 / 37
+//   222: 32 heads, top-2048                    106 / 75 and 65 / 63
+//   1184: 64 heads, top-256 59 / 46 both, top-2048 249 / 183 and 199 / 184;    32 heads, top-2048 392 / 266 and
+//         231 / 217;    16 heads 690 / 430 and 306 / 261;    8 heads 1322 / 754 and 449 / 347
+// The more of the lists is shared, the less there is to gain: of 402 calls above the line (74 to 1200 tiles, sharing 30 to 97 %, both query
+// types) four were slower, by 1 to 3 %, all of 32 heads with 95 % shared and more; 0.75 of the time in the mean.  How
 // much is shared is not known on the host.
 static bool use_rows64(int tokens, int h, int k, bool kv_bf16) {
   if (kv_bf16 || h > 64 || (int64_t)(128 / h) * k % 128 != 0) return false;
